@@ -120,6 +120,13 @@ enum mb_body {
                                   after MB_CELLS_X_WAIT: every CTA makes its stores visible
                                   (a gpu-scope fence) before it reports the phase finished   */
 
+#define MB_FLAG_RELAY 8        /* decode: the phase's results (and its copy of the gathered rows)
+                                  go to later phases of the launch only, through memory of the
+                                  plan's own in which every word not yet written in this launch
+                                  is recognisable; readers poll the words they need.  Takes
+                                  precedence over MB_CELLS_* and MB_FLAG_FENCE for these tensors;
+                                  the slots they name are not written                         */
+
 /* bits of MB_GV_I_CELLS / MB_AT_I_CELLS: which tensors of the phase are flagged cells */
 #define MB_CELLS_X 1           /* activations in (GEMV x; attention q, k and v)            */
 #define MB_CELLS_OUT 2         /* every output segment                                     */

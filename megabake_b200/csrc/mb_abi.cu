@@ -47,6 +47,13 @@ struct DeviceGuard {
 };
 
 
+// Which operands of a decode phase live in the plan's relay arena, and where.
+struct Relay {
+    unsigned long long modes = 0;
+    unsigned long long offset[MB_PHASE_SLOTS] = {};
+    bool used[MB_PHASE_SLOTS] = {};
+};
+
 }  // namespace
 
 struct mb_plan {
@@ -62,10 +69,19 @@ struct mb_plan {
     int threads = 0;
     int smem_bytes = 0;
     int stages = 0;
-    int stage_bytes = 0;
+    int head_dim = 64;  // decode: of all attention phases, 0 if they differ
     int barriers = 0;
+    bool counters = false;
     unsigned int wait_limit_us = 2000000u;
+    std::vector<Relay> relays;            // per phase (decode)
+    unsigned long long relay_bytes = 0;   // one half of the arena
+    void* d_relay = nullptr;              // both halves
     mb::PhaseEntry* d_entries = nullptr;
+    mb::StreamDesc* d_streams = nullptr;
+    void* d_maps = nullptr;               // tensor maps of weights and caches, decode_map_bytes() per phase
+    std::vector<unsigned char> maps;      // the same on the host
+    std::vector<size_t> late_maps;        // phases with such an operand that comes with the launch
+    std::vector<mb::PhaseEntry> entries;  // as bound
     mb::Control* d_ctl = nullptr;
     unsigned long long trace = 0;
     mb::PrefillState* prefill = nullptr;  // MB_MODE_PREFILL plans only
@@ -179,6 +195,99 @@ int validate_attention(const mb_plan_desc* d, const mb_phase& P) {
     return MB_OK;
 }
 
+// Gives every tensor that a phase with MB_FLAG_RELAY produces a place of its own in the relay arena
+// and points the phases that read it there.  No place is used twice in a launch, so nothing ever
+// has to wait before it overwrites.  Sets `counters` if some hand-off still needs the
+// finished-phase counters: plain results behind MB_CELLS_X_WAIT, or cells, whose buffers are
+// written again.
+int lower_relays(mb_plan* plan) {
+    plan->relays.assign(plan->phases.size(), Relay());
+    bool any = false;
+    for (const mb_phase& P : plan->phases) any = any || (P.flags & MB_FLAG_RELAY) != 0;
+    plan->relay_bytes = any ? static_cast<unsigned long long>(plan->phases.size()) * mb::kHintBytes : 0;
+    plan->relay_bytes = (plan->relay_bytes + 255) / 256 * 256;
+    std::vector<long long> place(plan->slots.size(), -1);  // slot -> arena offset of its live contents
+    auto produce = [&](Relay& r, const mb_phase& P, int s, unsigned long long bytes) {
+        const int slot = P.slot[s];
+        if (slot < 0) return MB_OK;
+        if (!(P.flags & MB_FLAG_RELAY)) {
+            place[slot] = -1;
+            return MB_OK;
+        }
+        if (static_cast<unsigned int>(slot) < plan->n_dynamic) return MB_ERR_INVALID;
+        place[slot] = static_cast<long long>(plan->relay_bytes);
+        r.offset[s] = plan->relay_bytes;
+        r.used[s] = true;
+        plan->relay_bytes += (bytes + 255) / 256 * 256;
+        return MB_OK;
+    };
+    auto consume = [&](Relay& r, const mb_phase& P, int s) {
+        const int slot = P.slot[s];
+        if (slot < 0 || place[slot] < 0) return false;
+        r.offset[s] = static_cast<unsigned long long>(place[slot]);
+        r.used[s] = true;
+        return true;
+    };
+    for (size_t i = 0; i < plan->phases.size(); ++i) {
+        const mb_phase& P = plan->phases[i];
+        Relay& r = plan->relays[i];
+        if (P.body == MB_BODY_GEMV) {
+            const int cells = P.i[MB_GV_I_CELLS];
+            if (!P.i[MB_GV_I_GATHER]) {
+                if (consume(r, P, MB_GV_S_X))
+                    r.modes |= mb::kModeInRelay;
+                else if (cells & (MB_CELLS_X | MB_CELLS_X_WAIT))
+                    plan->counters = true;
+            }
+            if (P.i[MB_GV_I_EPILOGUE] == MB_EPI_RESIDUAL) {
+                if (consume(r, P, MB_GV_S_RESIDUAL))
+                    r.modes |= mb::kModeResidualRelay;
+                else if (cells & MB_CELLS_RESIDUAL)
+                    plan->counters = true;
+            }
+            if (P.i[MB_GV_I_GATHER] && P.i[MB_GV_I_STORE_X]) {
+                if (P.flags & MB_FLAG_RELAY) r.modes |= mb::kModeStoreRelay;
+                const int rc = produce(r, P, MB_GV_S_XSTORE, 2ull * P.i[MB_GV_I_ROWS] * P.i[MB_GV_I_K]);
+                if (rc != MB_OK) return rc;
+            }
+            if (P.flags & MB_FLAG_RELAY) r.modes |= mb::kModeOutRelay;
+            for (int s = 0; s < P.i[MB_GV_I_NSEG]; ++s) {
+                const int rc = produce(r, P, MB_GV_S_OUT0 + s, 2ull * P.i[MB_GV_I_ROWS] * P.i[MB_GV_I_N0 + s]);
+                if (rc != MB_OK) return rc;
+            }
+        } else if (P.body == MB_BODY_ATTN_DECODE) {
+            const bool q = consume(r, P, MB_AT_S_Q), k = consume(r, P, MB_AT_S_K), v = consume(r, P, MB_AT_S_V);
+            if (q != k || q != v) return MB_ERR_INVALID;
+            if (q)
+                r.modes |= mb::kModeInRelay;
+            else if (P.i[MB_AT_I_CELLS] & (MB_CELLS_X | MB_CELLS_X_WAIT))
+                plan->counters = true;
+            if (P.flags & MB_FLAG_RELAY) r.modes |= mb::kModeOutRelay;
+            const int rc = produce(r, P, MB_AT_S_OUT,
+                                   2ull * P.i[MB_AT_I_BATCH] * P.i[MB_AT_I_HEADS] * P.i[MB_AT_I_HEAD_DIM]);
+            if (rc != MB_OK) return rc;
+        }
+    }
+    return MB_OK;
+}
+
+// Phases that read weights or caches from addresses known at launch only.
+bool has_late_map(const mb::PhaseEntry& entry) {
+    const bool gemv = entry.rec.body == MB_BODY_GEMV;
+    static const int weights[] = {MB_GV_S_W0, MB_GV_S_W0 + 1, MB_GV_S_W0 + 2, MB_GV_S_W_PAIR};
+    static const int caches[] = {MB_AT_S_KCACHE, MB_AT_S_VCACHE};
+    if (!gemv && entry.rec.body != MB_BODY_ATTN_DECODE) return false;
+    for (int k = 0; k < (gemv ? 4 : 2); ++k)
+        if (entry.addr[gemv ? weights[k] : caches[k]] & mb::kDynamicTag) return true;
+    return false;
+}
+
+// Blank arena: every word says "not written in this launch".
+cudaError_t blank_relays(const mb_plan* plan) {
+    if (plan->d_relay == nullptr) return cudaSuccess;
+    return cudaMemset(plan->d_relay, 0xff, 2 * plan->relay_bytes);
+}
+
 // A prefill plan is a list of kernel launches; it shares the descriptor, the slot table, the
 // status word and the entry points with decode plans.
 int create_prefill_plan(const mb_plan_desc* desc, mb_plan** out) {
@@ -276,7 +385,7 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
         desc->stage_bytes > static_cast<unsigned int>(mb::decode_stage_bytes()))
         return MB_ERR_INVALID;
 
-    int barriers = 1;  // the closing barrier
+    int barriers = 1;  // the last arrival closes the launch
     for (unsigned int i = 0; i < desc->n_phases; ++i) {
         const mb_phase& P = desc->phases[i];
         int rc = MB_OK;
@@ -301,19 +410,18 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     }
     if (!prop.cooperativeLaunch) return MB_ERR_UNSUPPORTED;
 
-    const int fixed = mb::decode_fixed_smem();
-    const int stage = plan_stage_bytes(desc);
     const int limit = static_cast<int>(prop.sharedMemPerBlockOptin);
-    int stages = (limit - fixed - static_cast<int>(desc->activation_bytes)) / stage;
-    if (stages > mb::decode_max_stages()) stages = mb::decode_max_stages();
+    const int head_dim = mb::decode_head_dim(desc->phases, desc->n_phases);
+    const int rope_bytes = mb::decode_rope_bytes(desc->phases, desc->n_phases);
+    const int stages = mb::decode_ring_stages(rope_bytes, desc->n_phases, limit);
     if (stages < 2) return MB_ERR_RESOURCE;
-    const int smem = fixed + static_cast<int>(desc->activation_bytes) + stages * stage;
+    const int smem = mb::decode_smem_bytes(rope_bytes, desc->n_phases, stages);
 
     // The attribute belongs to the kernel, not to a plan: set it to the device's opt-in limit so
     // that plans of different sizes (two batch sizes, two models) can be launched in any order.
-    MB_CUDA(mb::decode_configure(limit));
+    MB_CUDA(mb::decode_configure(head_dim, limit));
     int per_sm = 0;
-    MB_CUDA(mb::decode_occupancy(smem, &per_sm));
+    MB_CUDA(mb::decode_occupancy(head_dim, smem, &per_sm));
     if (per_sm < 1) return MB_ERR_RESOURCE;
     int ctas = desc->ctas == 0 ? prop.multiProcessorCount : static_cast<int>(desc->ctas);
     if (ctas < 1 || ctas > prop.multiProcessorCount * per_sm) return MB_ERR_RESOURCE;
@@ -340,14 +448,25 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     plan->threads = mb::decode_threads();
     plan->smem_bytes = smem;
     plan->stages = stages;
-    plan->stage_bytes = stage;
+    plan->head_dim = head_dim;
     plan->barriers = barriers;
     if (desc->wait_limit_ms != 0)
         plan->wait_limit_us = desc->wait_limit_ms > 4000000u ? 4000000000u : desc->wait_limit_ms * 1000u;
 
+    const int lowered = lower_relays(plan);
+    if (lowered != MB_OK) {
+        mb_plan_destroy(plan);
+        return lowered;
+    }
+
     cudaError_t err = cudaMalloc(&plan->d_entries, sizeof(mb::PhaseEntry) * desc->n_phases);
+    if (err == cudaSuccess) err = cudaMalloc(&plan->d_streams, sizeof(mb::StreamDesc) * desc->n_phases);
+    if (err == cudaSuccess) err = cudaMalloc(&plan->d_maps, mb::decode_map_bytes() * desc->n_phases);
+    if (err == cudaSuccess && plan->relay_bytes > 0) err = cudaMalloc(&plan->d_relay, 2 * plan->relay_bytes);
+    if (err == cudaSuccess) err = blank_relays(plan);
     if (err == cudaSuccess) err = cudaMalloc(&plan->d_ctl, sizeof(mb::Control));
     if (err == cudaSuccess) err = cudaMemset(plan->d_ctl, 0, sizeof(mb::Control));
+    if (err == cudaSuccess) err = cudaStreamSynchronize(cudaStreamLegacy);  // launches may use any stream
     if (err != cudaSuccess) {
         cuda_fail(err, "plan table allocation");
         mb_plan_destroy(plan);
@@ -391,22 +510,40 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     // Resolve every slot a phase names into its entry, so the kernel reads one record per
     // phase and never a second table.
     std::vector<mb::PhaseEntry> entries(plan->phases.size());
+    std::vector<mb::StreamDesc> streams(plan->phases.size());
+    plan->maps.assign(plan->phases.size() * mb::decode_map_bytes(), 0);
+    plan->late_maps.clear();
     for (size_t ph = 0; ph < plan->phases.size(); ++ph) {
         entries[ph].rec = plan->phases[ph];
+        entries[ph].modes = plan->relays[ph].modes;
         for (int j = 0; j < MB_PHASE_SLOTS; ++j) {
             const int slot = plan->phases[ph].slot[j];
             if (slot < 0)
                 entries[ph].addr[j] = 0ull;
+            else if (plan->relays[ph].used[j])
+                entries[ph].addr[j] = mb::kRelayTag | plan->relays[ph].offset[j];
             else if (static_cast<unsigned int>(slot) < plan->n_dynamic)
                 entries[ph].addr[j] = mb::kDynamicTag | static_cast<unsigned long long>(slot);
             else
                 entries[ph].addr[j] = plan->slots[slot];
+        }
+        mb::decode_stream(plan->phases[ph], entries[ph].addr, plan->ctas, &streams[ph]);
+        if (has_late_map(entries[ph])) {
+            plan->late_maps.push_back(ph);
+        } else if (!mb::decode_encode_maps(plan->phases[ph], entries[ph].addr, plan->ctas,
+                                           plan->maps.data() + ph * mb::decode_map_bytes())) {
+            g_last_cuda_error = "tensor map encoding failed";
+            return MB_ERR_CUDA;
         }
     }
     DeviceGuard guard(plan->device);
     if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
     MB_CUDA(cudaMemcpy(plan->d_entries, entries.data(), sizeof(mb::PhaseEntry) * entries.size(),
                        cudaMemcpyHostToDevice));
+    MB_CUDA(cudaMemcpy(plan->d_maps, plan->maps.data(), plan->maps.size(), cudaMemcpyHostToDevice));
+    MB_CUDA(cudaMemcpy(plan->d_streams, streams.data(), sizeof(mb::StreamDesc) * streams.size(),
+                       cudaMemcpyHostToDevice));
+    plan->entries = std::move(entries);
     plan->bound = true;
     return MB_OK;
 }
@@ -429,6 +566,11 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     mb::KernelParams params;
     std::memset(&params, 0, sizeof(params));
     params.entries = plan->d_entries;
+    params.streams = plan->d_streams;
+    params.maps = plan->d_maps;
+    params.stages = plan->stages;
+    params.relay = reinterpret_cast<unsigned long long>(plan->d_relay);
+    params.relay_bytes = plan->relay_bytes;
     params.ctl = plan->d_ctl;
     params.trace = reinterpret_cast<unsigned long long*>(plan->trace);
     for (size_t i = 0; i < n; ++i) {
@@ -437,14 +579,24 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     }
     params.n_phases = static_cast<int>(plan->phases.size());
     params.n_dynamic = static_cast<int>(plan->n_dynamic);
-    params.barriers_per_launch = plan->barriers;
-    params.stages = plan->stages;
-    params.stage_bytes = plan->stage_bytes;
-    params.activation_bytes = static_cast<int>(plan->activation_bytes);
+    params.barriers_per_launch = plan->barriers - 1;
+    params.counters = plan->counters ? 1 : 0;
     params.wait_limit_us = plan->wait_limit_us;
     DeviceGuard guard(plan->device);
     if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
-    MB_CUDA(mb::decode_launch(params, plan->ctas, plan->smem_bytes,
+    for (size_t ph : plan->late_maps) {
+        mb::PhaseEntry entry = plan->entries[ph];
+        for (unsigned long long& a : entry.addr)
+            if (a & mb::kDynamicTag) a = dynamic_addresses[a & (MB_MAX_DYNAMIC - 1)];
+        unsigned char* maps = plan->maps.data() + ph * mb::decode_map_bytes();
+        if (!mb::decode_encode_maps(plan->phases[ph], entry.addr, plan->ctas, maps)) {
+            g_last_cuda_error = "tensor map encoding failed";
+            return MB_ERR_CUDA;
+        }
+        MB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(plan->d_maps) + ph * mb::decode_map_bytes(), maps,
+                                mb::decode_map_bytes(), cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)));
+    }
+    MB_CUDA(mb::decode_launch(params, plan->head_dim, plan->ctas, plan->smem_bytes,
                               static_cast<cudaStream_t>(stream)));
     return MB_OK;
 }
@@ -486,6 +638,8 @@ int mb_plan_reset(mb_plan* plan) {
     epoch += 1;
     MB_CUDA(cudaMemset(plan->d_ctl, 0, sizeof(mb::Control)));
     MB_CUDA(cudaMemcpy(&plan->d_ctl->epoch, &epoch, sizeof(epoch), cudaMemcpyHostToDevice));
+    MB_CUDA(blank_relays(plan));
+    MB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return MB_OK;
 }
 
@@ -494,6 +648,9 @@ void mb_plan_destroy(mb_plan* plan) {
     {
         DeviceGuard guard(plan->device);
         if (plan->d_entries) cudaFree(plan->d_entries);
+        if (plan->d_streams) cudaFree(plan->d_streams);
+        if (plan->d_maps) cudaFree(plan->d_maps);
+        if (plan->d_relay) cudaFree(plan->d_relay);
         if (plan->d_ctl) cudaFree(plan->d_ctl);
         mb::prefill_destroy(plan->prefill);
     }

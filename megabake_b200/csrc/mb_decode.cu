@@ -1,14 +1,25 @@
 // Decode megakernel: one cooperative persistent launch runs every phase of a one-token
-// decoder step.  Phases hand activations to one another through flagged cells (two bf16 values
-// and a sequence number per 8-byte store, polled by the consumers), so that a layer needs no
-// grid barrier; a record may still ask for one.  Thread layout per CTA (one CTA per SM):
-//   warps 0..7   consumers: activation prologues (RMSNorm, embedding gather), the skinny
-//                GEMM inner loop on mma.sync with fp32 accumulation, epilogues, decode
-//                attention, and the grid barriers between barrier intervals
-//   warp 8       weight producer: walks the same phase table and streams this CTA's weight
-//                rows into a shared-memory ring with bulk async copies (TMA, 1-D), running
-//                ahead of the consumers across phase and grid-barrier boundaries because
-//                weights never depend on earlier phases
+// decoder step.  One CTA per SM, nine warps:
+//
+//   warp 8       streams weight rows through a ring of 16 KB stages in shared memory, one
+//                tensor-map copy per stage, a ring length ahead of the others and across phase
+//                boundaries, because weights depend on nothing in the launch: HBM keeps streaming
+//                while a phase waits for its activations.  The box of a copy is 32 reduction
+//                elements x 8 or 16 rows x 16 or 32 such groups, which lands as the mma.sync fragments
+//                of the lanes that read it: 16 bytes per lane, no bank conflicts, no padding, no
+//                address arithmetic.  (Measured with nothing but the copies: 6.6 TB/s; 16-byte
+//                copies by one producer warp reach 3.4 TB/s and by all warps 6.9, but then every
+//                warp spends about as many instructions on copying as on everything else.)
+//   warps 0..7   consumers: activation prologues (RMSNorm, embedding gather), the skinny GEMM on
+//                mma.sync, epilogues, decode attention.
+//
+// Phases hand activations to one another through the plan's relay arena: every word of it that has
+// not been written in this launch holds a pattern no result can have, so a consumer simply loads
+// the activations it needs, in fragment layout, until they are there.  Data and "ready" are one L2
+// round trip; there is no fence and no grid barrier.  (Records may also ask for plain
+// tensors behind a counter, flagged cells, or a grid barrier.)  A warp multiplies a slice of the
+// reduction for all rows of the CTA, keeps its activations in registers, and the slices are added
+// in shared memory in a fixed order.
 //
 // Replaces, for decode, the reference's generated persistent kernel
 // (src/megabake/codegen.py:1634-1703), its sm100 swapAB GEMM bodies
@@ -17,6 +28,9 @@
 // map bodies used for RMSNorm, RoPE, residual and gated activations
 // (src/megabake/bodies/cuda/generic.py:175-613) and the counting grid barrier
 // (src/megabake/runtime.py:153-190).
+#include <cuda.h>
+
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -27,1852 +41,1983 @@
 namespace mb {
 namespace decode {
 
-constexpr int kConsumerWarps = 8;
-constexpr int kConsumerThreads = kConsumerWarps * 32;
-constexpr int kThreads = kConsumerThreads + 32;
-constexpr int kMaxStages = 16;
-constexpr int kRowTile = 8;          // weight rows of one n8 MMA tile; a stage holds one or two
-constexpr int kRowPad = 64;          // bytes added to each staged row: with row lengths that are
-                                     // multiples of 128 B this makes 16-byte fragment loads of
-                                     // two neighbouring rows hit disjoint banks
-constexpr int kStageBytes = 34816;   // largest ring stage: 8 rows x (2048 * 2 + 64) B plus slack,
-                                     // whole 4 KB rows; plans may ask for smaller stages
-constexpr int kCtlBytes = 2048;
-constexpr int kReduceBytes = 16384;  // partial sums of one reduction group of row blocks
-constexpr int kFixedBytes = kCtlBytes + kReduceBytes;
-constexpr int kBarConsumers = 1;     // named barrier id of the consumer warps
-constexpr int kFoldFloats = 8 * 64 + 16;  // attention: chunk weights + denominators
+constexpr int kWarps = 8;
+constexpr int kThreads = kWarps * 32;        // consumers
+constexpr int kAllThreads = kThreads + 32;   // and the producer warp
+constexpr int kRowTile = 8;          // ROW_TILE and K_CHUNK of a record describe the staging of
+constexpr int kRowPad = 64;          // weight rows in units of these; the kernel's own stages are
+constexpr int kStageBytes = 34816;   // 16 KB whatever they say
+constexpr int kRingStage = 16384;    // 16 groups of 16 rows, 32 groups of 8, or 2 x 16 groups of 8
+constexpr int kMaxStages = 8;
+constexpr int kMapsPerPhase = 6;     // tensor maps: three weights, or keys and values for three boxes
+// Partial sums: two halves of 256 results (two blocks of 16 rows x 8 tokens; four blocks of 8) from
+// eight slices each.
+constexpr int kScratchBytes = 2 * 4 * kWarps * 512;
+// Keys are cut over CTAs once a (row, kv head) has more than kWholeBlocks 16-key blocks: up to four
+// rounds of the eight warps cost less than meeting through global memory (about 1.5 us), and
+// a part is never shorter than kRunBlocks.
+constexpr int kWholeBlocks = 32, kRunBlocks = 16, kSeamBlocks = 16;
+constexpr int kBarAll = 1;           // named barrier of the consumer warps
+constexpr int kRopeRows = 8;         // batch rows the cos / sin table holds
 constexpr int kEntryVectors = sizeof(PhaseEntry) / 16;
 constexpr int kTraceEvents = 8;  // stamps per phase and CTA in the optional trace buffer
 
-// Trace stamp from inside a body (events 4..7 are body-specific); thread 0 only.
-__device__ __forceinline__ void trace_stamp(const KernelParams& p, int ph, int event, int tid) {
-    if (p.trace != nullptr && tid == 0)
-        p.trace[(static_cast<size_t>(blockIdx.x) * p.n_phases + ph) * kTraceEvents + event] =
+// How the key blocks of an attention phase are dealt over the CTAs, one piece of it: see
+// find_segment.
+struct Segment {
+    int b, h, pair;
+    int length;          // cached keys of the row
+    int blk0, blk1;      // this CTA's blocks of the (row, kv head) pair
+    int index, parts;    // which part of the pair this is, of how many
+};
+
+struct SharedCtl {
+    unsigned long long full[kMaxStages];   // a stage's copies have landed
+    unsigned long long empty[kMaxStages];  // all consumer warps have read it
+    unsigned long long entry_full;         // the next phase record has landed
+    volatile unsigned int issued;          // stages the producer armed
+    unsigned long long limit_ns;           // bound of every wait of this launch
+    unsigned long long relay_now, relay_next;  // this launch's half of the arena, the other half
+    volatile int abort_flag;
+    volatile int verdict;            // thread 0's decision at a grid barrier / at the end
+    unsigned int tag_base;           // cells of phase q carry tag_base + q + 1 in this launch
+    unsigned int calls;              // launches completed before this one
+    Control* ctl;
+    unsigned long long* trace;
+    const PhaseEntry* entries;
+    const CUtensorMap* maps;         // kMapsPerPhase per phase
+    unsigned long long dyn[MB_MAX_DYNAMIC];
+    int n_phases, stages;
+    unsigned long long rope_pos, rope_freq;  // what the cos / sin table was made from
+    int rope_shape;
+    float rope_scale;
+    Segment segment[kWarps + 1];     // the segment a warp works on, the one the producer streams
+    __align__(16) float norm_part[8][kWarps];      // sums of squares per activation row and slice
+    float stat[kWarps][8][2];        // attention: (maximum, sum) per warp and head
+    float exchange[2][kWarps][8];    // attention, exact mode: maxima and sums of the warps
+    __align__(16) unsigned short new_row[2][256];  // rotated new key and new value of an item
+    __align__(16) PhaseEntry entry[4];  // phase records ph - 1 .. ph + 2
+};
+constexpr int kCtlBytes = 5120;
+constexpr int kFixedBytes = kCtlBytes + kScratchBytes;
+static_assert(sizeof(SharedCtl) <= kCtlBytes, "control block too large");
+
+// Shared activations of GEMV phases, 8 KB per warp; attention dumps its states there.
+constexpr int kSlicesBytes = kWarps * 8 * 1024;
+// After the fixed part: the slices, the ring, the stream table, the cos / sin table.
+// The weight ring starts on a 1024-byte boundary.
+constexpr unsigned int kSliceOffset = kFixedBytes;
+constexpr unsigned int kRingOffset = kSliceOffset + kSlicesBytes;
+static_assert(kRingOffset % 1024 == 0, "stages are 1024-byte aligned");
+__host__ __device__ constexpr unsigned int table_offset(int stages) {
+    return kRingOffset + static_cast<unsigned int>(stages) * kRingStage;
+}
+__host__ __device__ constexpr unsigned int rope_offset(int stages, unsigned int n_phases) {
+    return table_offset(stages) + (n_phases * static_cast<unsigned int>(sizeof(StreamDesc)) + 127u) / 128u * 128u;
+}
+
+extern __shared__ __align__(1024) char g_smem[];
+__device__ __forceinline__ SharedCtl* ctl_of() { return reinterpret_cast<SharedCtl*>(g_smem); }
+__device__ __forceinline__ float* scratch_of() { return reinterpret_cast<float*>(g_smem + kCtlBytes); }
+__device__ __forceinline__ StreamDesc* table_of() {
+    return reinterpret_cast<StreamDesc*>(g_smem + table_offset(ctl_of()->stages));
+}
+__device__ __forceinline__ unsigned int* rope_of() {
+    return reinterpret_cast<unsigned int*>(g_smem + rope_offset(ctl_of()->stages, ctl_of()->n_phases));
+}
+
+__device__ __forceinline__ void trace_stamp(int ph, int event) {
+    SharedCtl* sc = ctl_of();
+    if (threadIdx.x == 0 && sc->trace != nullptr)
+        sc->trace[(static_cast<size_t>(blockIdx.x) * sc->n_phases + ph) * kTraceEvents + event] =
             global_timer_ns();
 }
 
-struct SharedCtl {
-    unsigned long long full[kMaxStages];
-    unsigned long long empty[kMaxStages];
-    unsigned long long act_full;     // bulk copies of the current GEMV phase's prologue have landed
-    unsigned long long limit_ns;     // bound of every wait of this launch
-    volatile int abort_flag;
-    volatile unsigned int issued;    // stages the producer armed
-    int bcast[4];                    // small broadcasts (attention chunking, arrival order)
-    volatile int verdict;            // thread 0's go / drain decision at a barrier
-    unsigned int tag_base;           // cells of phase q carry tag_base + q + 1 in this launch
-    unsigned int calls;              // launches completed before this one
-    __align__(16) unsigned int guard[4];  // a counter of Control::finished, fetched asynchronously
-    float red[kConsumerWarps][8];    // per-warp partials of the activation prologue
-    __align__(16) PhaseEntry entry[2];  // current / next phase record with resolved addresses
-    __align__(16) PhaseEntry producer_entry;  // the producer warp's own copy of its phase
-};
-static_assert(sizeof(SharedCtl) <= kCtlBytes, "control block too large");
-static_assert(sizeof(PhaseEntry) % 16 == 0, "phase entries are copied in 16-byte vectors");
-
-// Entries reach the bodies with per-launch (dynamic) slots already replaced by their addresses
-// (patch_dynamic below), so reading an address is one shared-memory load.
-__device__ __forceinline__ unsigned long long entry_address(const KernelParams&,
-                                                            const PhaseEntry* e, int j) {
-    return e->addr[j];
-}
-
-__device__ __forceinline__ unsigned long long resolve_dynamic(const KernelParams& p,
-                                                              unsigned long long v) {
-    if (v >> 63) {  // dynamic slot: the address comes with the launch
-        const int s = static_cast<int>(v & 0xffu);
-        unsigned long long a = p.dyn[0];
-#pragma unroll
-        for (int i = 1; i < MB_MAX_DYNAMIC; ++i)
-            if (s == i) a = p.dyn[i];
-        return a;
-    }
+__device__ __forceinline__ unsigned long long resolve_address(unsigned long long v) {
+    const SharedCtl* sc = ctl_of();
+    if (v & kDynamicTag) return sc->dyn[v & (MB_MAX_DYNAMIC - 1)];  // the address comes with the launch
+    if (v & kRelayTag) return sc->relay_now + (v & ~kRelayTag);
     return v;
 }
 
-// One thread per slot rewrites the tagged slots of an entry that sits in shared memory.
-__device__ __forceinline__ void patch_dynamic(const KernelParams& p, PhaseEntry* e, int lane) {
-    if (lane < MB_PHASE_SLOTS) e->addr[lane] = resolve_dynamic(p, e->addr[lane]);
-}
-
 // ---------------------------------------------------------------------------------------
-// Waiting for flagged cells.  The fast path (the cell already carries the expected sequence
-// number) is inline at the call sites; these are the retry loops.  A wait gives up when the
-// launch's limit has run out (status MB_ST_HANDOFF_TIMEOUT) or when this CTA or any other has
-// recorded a fault; the caller goes on with whatever it has and the CTA drains at the end of
-// the phase.
+// Bounded waits.  A wait gives up when the launch's limit has run out (status
+// MB_ST_HANDOFF_TIMEOUT) or when this CTA or any other has recorded a fault; the caller goes on
+// with whatever it has and the CTA drains at the next barrier all its threads meet at.
 // ---------------------------------------------------------------------------------------
-__device__ __noinline__ bool wait_gave_up(const KernelParams& p, SharedCtl* sc, int ph,
-                                          unsigned long long start) {
+__device__ __forceinline__ bool wait_gave_up(int ph, unsigned long long start) {
+    SharedCtl* sc = ctl_of();
     if (sc->abort_flag) return true;
-    if (peek_status(p.ctl) != 0) {
+    if (peek_status(sc->ctl) != 0) {
         sc->abort_flag = 1;
         return true;
     }
     if (global_timer_ns() - start > sc->limit_ns) {
-        record_status(p.ctl, MB_ST_HANDOFF_TIMEOUT, ph, static_cast<int>(blockIdx.x));
+        record_status(sc->ctl, MB_ST_HANDOFF_TIMEOUT, ph, static_cast<int>(blockIdx.x));
         sc->abort_flag = 1;
         return true;
     }
     return false;
 }
 
-__device__ __noinline__ void cell_pair_wait(const void* src, unsigned int tag,
-                                            unsigned long long& a, unsigned long long& b,
-                                            const KernelParams& p, SharedCtl* sc, int ph) {
+__device__ __noinline__ unsigned long long cell_wait(const void* src, unsigned int tag, int ph) {
     const unsigned long long start = global_timer_ns();
     for (unsigned int tries = 1;; ++tries) {
-        __nanosleep(32);
-        ld_cell_pair(src, a, b);
-        if (cell_tag(a) == tag && cell_tag(b) == tag) return;
-        if ((tries & 63u) == 0u && wait_gave_up(p, sc, ph, start)) return;
-    }
-}
-
-__device__ __noinline__ unsigned long long cell_wait(const void* src, unsigned int tag,
-                                                     const KernelParams& p, SharedCtl* sc,
-                                                     int ph) {
-    const unsigned long long start = global_timer_ns();
-    for (unsigned int tries = 1;; ++tries) {
-        __nanosleep(32);
         const unsigned long long v = ld_cell(src);
         if (cell_tag(v) == tag) return v;
-        if ((tries & 63u) == 0u && wait_gave_up(p, sc, ph, start)) return v;
+        if ((tries & 63u) == 0u && wait_gave_up(ph, start)) return v;
     }
 }
 
-// Lock-step within two phases.  A cell buffer is rewritten at the earliest three phases after
-// its last reader (the planner's rule).  So a CTA may enter phase q + 1 only when every CTA has
-// finished phase q - 2 ... the kernel asks for a little more, q - 2 at the END of phase q:
-// Control::finished[q % 4] counts the CTAs that finished phase q, and thread 0 of every CTA
-// checks the counter of phase q - 2 before it reports phase q finished.  `seen` is a value of
-// that counter fetched while the phase ran; in the steady state it is already large enough and
-// nothing waits.
-__device__ __forceinline__ unsigned int finished_target(const KernelParams& p, const SharedCtl* sc,
-                                                        int q) {
+__device__ __forceinline__ unsigned int relay_wait(const void* src, int ph) {
+    const unsigned long long start = global_timer_ns();
+    for (unsigned int tries = 1;; ++tries) {
+        const unsigned int v = ld_relaxed_u32(src);
+        if (v != kUnwritten) return v;
+        if ((tries & 63u) == 0u && wait_gave_up(ph, start)) return 0u;
+    }
+}
+
+// Finished-phase counters, for plans with hand-offs outside the relay arena: the count every CTA
+// has to have reached once phase q of this launch is finished everywhere.
+__device__ __forceinline__ unsigned int finished_target(const SharedCtl* sc, int q) {
     const unsigned int slot = static_cast<unsigned int>(q) & 3u;
     // phases of one launch that count on this slot, and how many of them up to phase q
-    const unsigned int per_launch = (static_cast<unsigned int>(p.n_phases) + 3u - slot) >> 2;
+    const unsigned int per_launch = (static_cast<unsigned int>(sc->n_phases) + 3u - slot) >> 2;
     return gridDim.x * (sc->calls * per_launch + (static_cast<unsigned int>(q) >> 2) + 1u);
 }
 
 // One thread: wait until every CTA has reported phase `q` finished.  The load is an acquire, so
 // what those CTAs stored before a fenced report is visible to this thread afterwards (and,
-// through a CTA barrier, to its CTA).
-__device__ __noinline__ void finished_wait(const KernelParams& p, SharedCtl* sc, int ph, int q) {
-    const unsigned int target = finished_target(p, sc, q);
-    const unsigned int* counter = &p.ctl->finished[q & 3].count;
+// through a warp or CTA barrier, to the others).
+__device__ __noinline__ void finished_wait(int ph, int q) {
+    SharedCtl* sc = ctl_of();
+    const unsigned int target = finished_target(sc, q);
+    const unsigned int* counter = &sc->ctl->finished[q & 3].count;
     const unsigned long long start = global_timer_ns();
     for (unsigned int tries = 1;; ++tries) {
         unsigned int seen;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
         if (static_cast<int>(seen - target) >= 0) return;
-        if ((tries & 63u) == 0u && wait_gave_up(p, sc, ph, start)) return;
+        if ((tries & 63u) == 0u && wait_gave_up(ph, start)) return;
         __nanosleep(40);
     }
 }
 
-// Geometry of one GEMV phase for one CTA; producer and consumers derive it identically.
-// A CTA owns output rows [r0, r1) of the phase's (virtually concatenated) output rows -- whole
-// pairs of rows, so that a lane's two neighbouring results always form one cell -- and streams
-// their weight rows as blocks of `row_tile` rows (8, or 16 = two MMA tiles), each cut into
-// n_chunks stages of k_chunk elements.
-struct GemvGeom {
-    int rows, K, nseg, nmat, n[3], ntotal;
-    int k_chunk, n_chunks, pitch, row_tile;
-    int r0, r1, n_blocks;
-};
+// ---------------------------------------------------------------------------------------
+// Activations written earlier in the launch, eight bf16 values (16 bytes) at a time.
+// ---------------------------------------------------------------------------------------
+enum SourceKind { kPlain = 0, kRelay = 1, kCells = 2 };
 
-__device__ __forceinline__ GemvGeom gemv_geometry(const mb_phase& P, int cta) {
-    GemvGeom g;
-    g.rows = P.i[MB_GV_I_ROWS];
-    g.K = P.i[MB_GV_I_K];
-    g.nseg = P.i[MB_GV_I_NSEG];
-    g.nmat = P.i[MB_GV_I_NMAT];
-    g.n[0] = P.i[MB_GV_I_N0];
-    g.n[1] = g.nseg > 1 ? P.i[MB_GV_I_N0 + 1] : 0;
-    g.n[2] = g.nseg > 2 ? P.i[MB_GV_I_N0 + 2] : 0;
-    g.ntotal = g.n[0] + g.n[1] + g.n[2];
-    g.k_chunk = P.i[MB_GV_I_K_CHUNK];
-    g.n_chunks = (g.K + g.k_chunk - 1) / g.k_chunk;  // small operands: cheap
-    g.pitch = g.k_chunk * 2 + kRowPad;
-    g.row_tile = P.i[MB_GV_I_ROW_TILE];
-    // balanced split precomputed by the host, in pairs of rows: the first `rem` CTAs own one
-    // pair more
-    const int q = P.i[MB_GV_I_SPLIT_Q], rem = P.i[MB_GV_I_SPLIT_R];
-    g.r0 = 2 * (cta * q + min(cta, rem));
-    g.r1 = g.r0 + 2 * (q + (cta < rem ? 1 : 0));
-    g.n_blocks = (g.r1 - g.r0 + g.row_tile - 1) / g.row_tile;
-    return g;
+__device__ __forceinline__ int source_kind(const PhaseEntry* E, bool cells) {
+    return (E->modes & kModeInRelay) ? kRelay : (cells ? kCells : kPlain);
+}
+
+__device__ __forceinline__ bool unwritten(uint4 v) {
+    return v.x == kUnwritten || v.y == kUnwritten || v.z == kUnwritten || v.w == kUnwritten;
+}
+
+// Eight values from four cells.
+__device__ __noinline__ uint4 cells_load(const char* src, unsigned int tag, int ph) {
+    unsigned int v[4];
+    for (int i = 0; i < 4; ++i) {
+        unsigned long long c = ld_cell(src + 8 * i);
+        if (cell_tag(c) != tag) c = cell_wait(src + 8 * i, tag, ph);
+        v[i] = cell_data(c);
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+// Loads the first `count` of N vectors, vector i from `at(i)`, all of them in flight together, again
+// and again until none has a word that is not written yet.  Whole warps only.  (No predicate per
+// lane or vector: callers clamp addresses instead, because on the chain of a phase branches
+// around single loads cost more than the loads.)
+template <int N, typename At>
+__device__ __forceinline__ void gather_source(uint4 (&x)[N], int count, bool relay, At at, int ph) {
+    unsigned long long start = 0;
+#pragma unroll 1
+    for (unsigned int tries = 1;; ++tries) {
+        bool missing = false;
+#pragma unroll
+        for (int i = 0; i < N; i += 2) {
+            if (i >= count) break;
+            x[i] = ld_relaxed_u4(at(i));
+            if (i + 1 < N) x[i + 1] = ld_relaxed_u4(at(i + 1));
+        }
+        if (!relay) return;
+#pragma unroll
+        for (int i = 0; i < N; i += 2) {
+            if (i >= count) break;
+            missing |= unwritten(x[i]);
+            if (i + 1 < N) missing |= unwritten(x[i + 1]);
+        }
+        if (!__any_sync(0xffffffffu, missing)) return;
+        if ((tries & 63u) == 0u) {
+            if (start == 0) start = global_timer_ns();
+            if (__any_sync(0xffffffffu, wait_gave_up(ph, start))) return;  // garbage: the launch has failed
+        }
+    }
+}
+
+// Two neighbouring bf16 results on their way out: 4 bytes, or one cell.
+__device__ __forceinline__ void store_result(char* base, size_t element, unsigned int packed,
+                                             bool cells, unsigned int tag) {
+    if (cells)
+        st_cell(base + element * 4, packed, tag);
+    else
+        st_relaxed_u32(base + element * 2, packed);
 }
 
 // ---------------------------------------------------------------------------------------
-// Producer warp: for every GEMV phase, in phase order, stream this CTA's weight rows into
-// the ring -- stage order is (row block, k chunk), the order the consumers expect.
+// How the key blocks of an attention phase are dealt over the CTAs.  Whole items: CTA c takes
+// (row, kv head) pairs c, c + ctas, ...  Cut: the 16-key blocks of all pairs, in order, are
+// divided into `cut_ctas` runs of equal length (+-1); a CTA's run may end inside a pair, whose
+// parts then meet through the partial buffer.
 // ---------------------------------------------------------------------------------------
-__device__ __noinline__ void producer_loop(const KernelParams& p, SharedCtl* sc, char* ring,
-                                           int lane) {
-    const int cta = blockIdx.x;
-    unsigned int it = 0;
-    // The producer runs phases ahead of the consumers, so it would meet every phase entry
-    // cold in DRAM and chase its fields one dependent load at a time.  Instead: pull the whole
-    // table into L2 once, and per phase fetch the entry with one coalesced 16-byte load per
-    // lane (the next entry's load is already in flight while this one is worked on).
-    {
-        const char* table = reinterpret_cast<const char*>(p.entries);
-        const size_t bytes = sizeof(PhaseEntry) * static_cast<size_t>(p.n_phases);
-        for (size_t off = static_cast<size_t>(lane) * 128; off < bytes; off += 32 * 128)
-            prefetch_l2(table + off);
-    }
-    PhaseEntry* mine = &sc->producer_entry;
-    uint4 next_vector = make_uint4(0u, 0u, 0u, 0u);
-    if (lane < kEntryVectors)
-        next_vector = __ldg(reinterpret_cast<const uint4*>(p.entries) + lane);
-    for (int ph = 0; ph < p.n_phases; ++ph) {
-        __syncwarp();  // everybody is done with the previous entry
-        if (lane < kEntryVectors) {
-            reinterpret_cast<uint4*>(mine)[lane] = next_vector;
-            if (ph + 1 < p.n_phases)
-                next_vector = __ldg(reinterpret_cast<const uint4*>(p.entries + ph + 1) + lane);
+__device__ __forceinline__ int row_length(const KvStream& d, int b) {
+    if (d.len_count <= 1) return d.lens[0];
+    if (d.batch <= 8) return d.lens[b];
+    return __ldg(reinterpret_cast<const int*>(d.lengths) + b);
+}
+
+// Writes segment `which` of this CTA to `out`; false if there are fewer.
+__device__ __noinline__ bool locate_segment(int ph, int which, Segment* out, bool writer) {
+    const KvStream& d = table_of()[ph].kv;
+    const unsigned int cta = blockIdx.x;
+    const unsigned int runs = static_cast<unsigned int>(d.cut_ctas), total = d.total_blocks;
+    int b, h, length, blk0 = 0, blk1, index = 0, parts = 1;
+    if (runs == 0) {
+        const int pair = static_cast<int>(cta) + which * static_cast<int>(gridDim.x);
+        if (pair >= d.batch * d.kv_heads) return false;
+        b = pair / d.kv_heads;
+        h = pair - b * d.kv_heads;
+        length = row_length(d, b);
+        blk1 = (length + 16) >> 4;
+    } else if (d.cut_ctas < 0) {
+        const int length_of_part = -d.cut_ctas;
+        int left = static_cast<int>(cta), nb = 1;
+        if (which > 0) return false;
+        for (b = 0; b < d.batch; ++b) {
+            nb = (row_length(d, b) + 16) >> 4;
+            parts = (nb + length_of_part - 1) / length_of_part;
+            if (left < parts * d.kv_heads) break;
+            left -= parts * d.kv_heads;
         }
-        __syncwarp();
-        patch_dynamic(p, mine, lane);
-        __syncwarp();
-        const PhaseEntry* E = mine;
-        if (E->rec.body == MB_BODY_ATTN_DECODE) {
-            // the few scalars the attention body starts from: pull them into L2 ahead of time
-            if (lane == 0) prefetch_l2(reinterpret_cast<const void*>(entry_address(p, E, MB_AT_S_LEN)));
-            if (lane == 1) prefetch_l2(reinterpret_cast<const void*>(entry_address(p, E, MB_AT_S_POS)));
-            if (lane == 2)
-                prefetch_l2(reinterpret_cast<const void*>(entry_address(p, E, MB_AT_S_INVFREQ)));
+        if (b == d.batch) return false;
+        h = left / parts;
+        index = left - h * parts;
+        length = row_length(d, b);
+        blk0 = index * nb / parts;
+        blk1 = (index + 1) * nb / parts;
+    } else {
+        if (cta >= runs) return false;
+        unsigned int at = cta * total / runs;
+        const unsigned int end = (cta + 1) * total / runs;
+        for (;;) {
+            // which pair block `at` belongs to, and where that pair starts
+            unsigned int start = 0, nb = 1;
+            for (b = 0; b < d.batch; ++b) {
+                nb = static_cast<unsigned int>((row_length(d, b) + 16) >> 4);
+                const unsigned int row_blocks = nb * static_cast<unsigned int>(d.kv_heads);
+                if (at < start + row_blocks) break;
+                start += row_blocks;
+            }
+            if (at >= end || b >= d.batch) return false;
+            h = static_cast<int>((at - start) / nb);
+            start += h * nb;
+            const unsigned int stop = min(start + nb, end);
+            if (which-- == 0) {
+                length = row_length(d, b);
+                blk0 = static_cast<int>(at - start);
+                blk1 = static_cast<int>(stop - start);
+                // run r holds block g iff r = ((g + 1) * runs - 1) / total, rounded down
+                const unsigned int first = ((start + 1) * runs - 1) / total;
+                const unsigned int last = ((start + nb) * runs - 1) / total;
+                index = static_cast<int>(cta - first);
+                parts = static_cast<int>(last - first) + 1;
+                break;
+            }
+            at = stop;
+        }
+    }
+    if (writer) {
+        out->b = b;
+        out->h = h;
+        out->pair = b * d.kv_heads + h;
+        out->length = length;
+        out->blk0 = blk0;
+        out->blk1 = blk1;
+        out->index = index;
+        out->parts = parts;
+    }
+    return true;
+}
+// The same for a consumer warp, into its own record.
+__device__ __forceinline__ bool find_segment(int ph, int which) {
+    __syncwarp();
+    const bool found = locate_segment(ph, which, &ctl_of()->segment[threadIdx.x >> 5], (threadIdx.x & 31) == 0);
+    __syncwarp();
+    return found;
+}
+
+// log2 of the 16-key blocks per stage of a segment: enough that one stage per owning warp -- all of them
+// on their way before the phase begins -- holds it, at most 8 KB of keys.
+__host__ __device__ constexpr int kv_most(int head_dim) { return head_dim == 64 ? 2 : (head_dim == 128 ? 1 : 0); }
+__device__ __forceinline__ int kv_shift(int head_dim, int blocks, int owners) {
+    const int want = blocks > 2 * owners ? 2 : (blocks > owners ? 1 : 0);
+    return min(want, kv_most(head_dim));
+}
+
+// ---------------------------------------------------------------------------------------
+// The weight ring.
+// ---------------------------------------------------------------------------------------
+// What a phase function hands on: the stage to consume next, its parity, and which half of the
+// partial-sum scratch the next batch of rows uses.
+struct Place {
+    unsigned int stage, parity, flip;
+};
+
+// First virtual row of block `b` of this CTA, and the end of the segment it lies in: blocks never
+// straddle two weight matrices.
+__device__ __forceinline__ int block_row(const GemvStream& d, int b, int block_rows, int* end) {
+    int lo = d.r0, hi = min(d.r1, d.n0);
+    int blocks = hi > lo ? (hi - lo + block_rows - 1) / block_rows : 0;
+    if (b >= blocks && hi < d.r1) {
+        b -= blocks;
+        lo = max(d.r0, d.n0);
+        hi = min(d.r1, d.n01);
+        blocks = hi > lo ? (hi - lo + block_rows - 1) / block_rows : 0;
+        if (b >= blocks && hi < d.r1) {
+            b -= blocks;
+            lo = max(d.r0, d.n01);
+            hi = d.r1;
+        }
+    }
+    *end = hi;
+    return lo + b * block_rows;
+}
+__device__ __forceinline__ int count_blocks(const GemvStream& d, int block_rows) {
+    int total = 0;
+    const int bounds[4] = {d.r0, min(max(d.n0, d.r0), d.r1), min(max(d.n01, d.r0), d.r1), d.r1};
+    for (int s = 0; s < 3; ++s)
+        total += (max(bounds[s + 1] - bounds[s], 0) + block_rows - 1) / block_rows;
+    return total;
+}
+
+__device__ __forceinline__ void cp_async16(unsigned int dst_smem, unsigned long long src_gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src_gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(unsigned int dst, const CUtensorMap* map, int row, int group,
+                                            unsigned long long* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(map), "r"(0), "r"(row), "r"(group), "r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d(unsigned int dst, const CUtensorMap* map, int key, int head, int row,
+                                            unsigned long long* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(map), "r"(0), "r"(key), "r"(0), "r"(head), "r"(row), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// Producer: one lane walks the phases and fills stage after stage in the order they are consumed.
+__device__ __noinline__ void producer_loop() {
+    SharedCtl* sc = ctl_of();
+    const StreamDesc* table = table_of();
+    const unsigned int ring = smem_u32(g_smem) + kRingOffset;
+    int stage = 0;
+    unsigned int parity = 1;
+    // the next stage, once every warp has read what it held, armed for `bytes`
+    auto open_stage = [&](int ph, unsigned int bytes) {
+        if (!mbar_wait_bounded(&sc->empty[stage], parity, &sc->abort_flag, 2 * sc->limit_ns)) {
+            if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+            sc->abort_flag = 1;
+            return false;
+        }
+        sc->issued = sc->issued + 1;
+        mbar_arrive_expect_tx(&sc->full[stage], bytes);
+        return true;
+    };
+    auto next_stage = [&] {
+        if (++stage == sc->stages) {
+            stage = 0;
+            parity ^= 1u;
+        }
+    };
+    for (int ph = 0; ph < sc->n_phases; ++ph) {
+        const CUtensorMap* maps = sc->maps + kMapsPerPhase * ph;
+        if (table[ph].kind == kStreamKv) {
+            const int head_dim = table[ph].kv.head_dim;
+            Segment& seg = sc->segment[kWarps];
+            for (int which = 0; locate_segment(ph, which, &seg, true); ++which) {
+                const int shift = kv_shift(head_dim, seg.blk1 - seg.blk0,
+                                           table[ph].kv.exact_keys ? kWarps : min(kWarps, sc->stages));
+                const unsigned int bytes = 32u * static_cast<unsigned int>(head_dim) << shift;  // of the keys
+                for (int blk = seg.blk0; blk < seg.blk1; blk += 1 << shift) {
+                    if (!open_stage(ph, 2 * bytes)) return;
+                    const unsigned int dst = ring + static_cast<unsigned int>(stage) * kRingStage;
+                    tma_load_5d(dst, maps + 2 * shift, blk * 16, seg.h, seg.b, &sc->full[stage]);
+                    tma_load_5d(dst + bytes, maps + 2 * shift + 1, blk * 16, seg.h, seg.b, &sc->full[stage]);
+                    next_stage();
+                }
+            }
             continue;
         }
-        if (E->rec.body != MB_BODY_GEMV) continue;
-        const GemvGeom g = gemv_geometry(E->rec, cta);
-        if (E->rec.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE) {
-            // norm weights are read by every CTA right after the barrier: have them in L2
-            const char* nw = reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_NORM_W));
-            for (int line = lane; line * 128 < g.K * 2; line += 32) prefetch_l2(nw + line * 128);
-        }
-        if (E->rec.slot[MB_GV_S_BIAS0] >= 0 && g.nseg == 1 && lane < 8) {
-            // this CTA's slice of a single-segment bias (a few lines at most per 8 lanes)
-            const char* bias = reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_BIAS0));
-            const int stop = g.r1 * 2;  // byte range [r0 * 2, r1 * 2) of the vector
-            for (int off = (g.r0 * 2 / 128 + lane) * 128; off < stop; off += 8 * 128)
-                prefetch_l2(bias + off);
-        }
-        const char* w0 = reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_W0));
-        const char* w1 = g.nseg > 1
-                             ? reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_W0 + 1))
-                             : nullptr;
-        const char* w2 = g.nseg > 2
-                             ? reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_W0 + 2))
-                             : nullptr;
-        const char* wpair = g.nmat > 1 ? reinterpret_cast<const char*>(
-                                             entry_address(p, E, MB_GV_S_W_PAIR))
-                                       : nullptr;
-        const size_t row_bytes = static_cast<size_t>(g.K) * 2;
-        // ring position: one division per phase, then counted up (a division per stage costs
-        // more than the rest of the stage's bookkeeping)
-        int stage = static_cast<int>(it % static_cast<unsigned int>(p.stages));
-        unsigned int wraps = it / static_cast<unsigned int>(p.stages);
-        for (int blk = 0; blk < g.n_blocks; ++blk) {
-            const int block0 = g.r0 + blk * g.row_tile;
-            const int nrows = min(g.row_tile, g.r1 - block0);
-            // this lane's copy: matrix m, row r of the block (at most 16 copies per stage)
-            const int m = lane / nrows, r = lane - m * nrows;
-            const bool mine = lane < nrows * g.nmat;
-            const char* src_row = nullptr;
-            if (mine) {
-                int local = block0 + r;
-                const char* base;
-                if (m == 1) {
-                    base = wpair;
-                } else if (local < g.n[0]) {
-                    base = w0;
-                } else if (local < g.n[0] + g.n[1]) {
-                    base = w1;
-                    local -= g.n[0];
-                } else {
-                    base = w2;
-                    local -= g.n[0] + g.n[1];
-                }
-                src_row = base + static_cast<size_t>(local) * row_bytes;
+        if (table[ph].kind != kStreamGemv) continue;
+        const GemvStream& d = table[ph].gemv;
+        const bool is_short = (d.shape & kShapeShort) != 0, paired = (d.shape & kShapePaired) != 0;
+        const int block_rows = is_short || paired ? 8 : 16;
+        const int step = is_short ? 32 : 16;  // groups per stage
+        const char* nw = reinterpret_cast<const char*>(d.w_norm);
+        if (nw != nullptr)  // every CTA reads the norm weights right after its wait: have them in L2
+            for (int at = static_cast<int>(blockIdx.x) * 128; at < d.row_bytes; at += 8 * 128)
+                prefetch_l2(nw + at);
+        for (int b = 0; b < d.nblocks; ++b) {
+            int end;
+            int row = block_row(d, b, block_rows, &end);
+            const CUtensorMap* map = maps;
+            if (row >= d.n01) {
+                map = maps + 2;
+                row -= d.n01;
+            } else if (row >= d.n0) {
+                map = maps + 1;
+                row -= d.n0;
             }
-            for (int c = 0; c < g.n_chunks; ++c) {
-                const unsigned int parity = (wraps & 1u) ^ 1u;
-                if (!mbar_wait_bounded(&sc->empty[stage], parity, &sc->abort_flag, sc->limit_ns)) {
-                    if (lane == 0 && !sc->abort_flag) {
-                        record_status(p.ctl, MB_ST_PIPE_TIMEOUT, ph, cta);
-                        sc->abort_flag = 1;
-                    }
-                    return;
-                }
-                const int kc = min(g.k_chunk, g.K - c * g.k_chunk);
-                const unsigned int seg_bytes = static_cast<unsigned int>(kc) * 2u;
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&sc->full[stage], seg_bytes * nrows * g.nmat);
-                    sc->issued = it + 1;
-                }
-                __syncwarp();
-                if (mine) {
-                    char* dst = ring + static_cast<size_t>(stage) * p.stage_bytes +
-                                static_cast<size_t>(m * kRowTile + r) * g.pitch;
-                    bulk_copy_g2s(dst, src_row + static_cast<size_t>(c) * g.k_chunk * 2, seg_bytes,
-                                  &sc->full[stage]);
-                }
-                ++it;
-                if (++stage == p.stages) {
-                    stage = 0;
-                    ++wraps;
-                }
+            for (int g = 0; g < d.groups; g += step) {
+                if (!open_stage(ph, kRingStage)) return;
+                const unsigned int dst = ring + static_cast<unsigned int>(stage) * kRingStage;
+                tma_load_3d(dst, map, row, g, &sc->full[stage]);
+                if (paired) tma_load_3d(dst + kRingStage / 2, maps + 1, row, g, &sc->full[stage]);
+                next_stage();
             }
         }
     }
 }
+// After a fault: never leave while one of this CTA's tensor copies is still in flight.  One thread.
+__device__ __noinline__ void drain_ring() {
+    SharedCtl* sc = ctl_of();
+    const unsigned int stages = sc->stages, issued = sc->issued;
+    for (unsigned int i = issued > stages ? issued - stages : 0u; i < issued; ++i)
+        for (unsigned int tries = 0; tries < kDrainTryLimit; ++tries)
+            if (mbar_try_wait(&sc->full[i % stages], (i / stages) & 1u)) break;
+}
+
+__device__ __forceinline__ uint4 lds128(unsigned int addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+// Waits for a stage.  If the wait runs out the fault is recorded and the values are garbage; the
+// CTA runs through the launch without waiting any more.  (No call: one in the loop of a phase costs
+// more in spilled registers than the wait itself.)
+__device__ __forceinline__ void ring_wait(unsigned int stage, unsigned int parity) {
+    SharedCtl* sc = ctl_of();
+    if (mbar_try_wait(&sc->full[stage], parity)) return;
+    const unsigned long long start = global_timer_ns();
+    for (unsigned int tries = 1; !mbar_try_wait(&sc->full[stage], parity); ++tries) {
+        if ((tries & 127u) != 0u) continue;
+        if (sc->abort_flag) return;
+        if (global_timer_ns() - start > 2 * sc->limit_ns) {
+            record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, 0, blockIdx.x);
+            sc->abort_flag = 1;
+            return;
+        }
+    }
+}
+// Hands the stage back once the warp has its values, and moves on.
+__device__ __forceinline__ void ring_next(Place& s) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(&ctl_of()->empty[s.stage]);
+    if (++s.stage == static_cast<unsigned int>(ctl_of()->stages)) {
+        s.stage = 0;
+        s.parity ^= 1u;
+    }
+}
 
 // ---------------------------------------------------------------------------------------
-// Activation prologue: bring the phase's activation rows into shared memory as bf16,
-// applying the embedding gather and/or RMSNorm.  All consumer threads.
-// xs layout: [rows][K + 32] bf16 (the 64-byte pad spreads rows over banks).
+// Skinny GEMM: out[row, n] = epilogue(prologue(x)[row, :] . W[n, :] + bias[n]), up to 8 rows.
+// mma.sync m16n8k16 with the weight rows as A (16 of them, or 8 gate and 8 up rows) and the
+// activation rows as B (n = row): one instruction takes 512 bytes of weights.  The reduction
+// index is permuted identically in both, so that a lane's operand is 16 contiguous bytes per
+// 32 elements.  The eight warps share a block of rows along K: of every stage a warp takes two
+// groups of 32 elements (four where blocks have 8 rows).
+//
+// A phase is a chain -- activations arrive, norm, products, slices added, results leave -- on
+// which every instruction counts, so whatever does not depend on the activations is done before
+// they arrive.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ const char* activation_row(const PhaseEntry* E, const char* xbase,
-                                                      const long long* ids, int r, int K,
-                                                      bool* bad_token) {
-    if (ids != nullptr) {
-        long long id = ids[r];
+// Element (virtual row) -> segment, and row inside it.
+__device__ __forceinline__ int output_segment(const GemvStream& d, int& local) {
+    if (local >= d.n01) {
+        local -= d.n01;
+        return 2;
+    }
+    if (local >= d.n0) {
+        local -= d.n0;
+        return 1;
+    }
+    return 0;
+}
+// Address of the packed pair that holds an element's residual.
+__device__ __forceinline__ const char* residual_address(const PhaseEntry* E, int local, int tok) {
+    const size_t index = static_cast<size_t>(tok) * E->rec.i[MB_GV_I_N0] + (local & ~1);
+    const bool cells = (E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL) && !(E->modes & kModeResidualRelay);
+    return reinterpret_cast<const char*>(E->addr[MB_GV_S_RESIDUAL]) + index * (cells ? 4 : 2);
+}
+
+__device__ __forceinline__ float dot_self(uint4 v) {  // sum of squares of eight bf16 values
+    const unsigned int w[4] = {v.x, v.y, v.z, v.w};
+    float s = 0.f, t = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        s = __fmaf_rn(lo_bf16(w[q]), lo_bf16(w[q]), s);
+        t = __fmaf_rn(hi_bf16(w[q]), hi_bf16(w[q]), t);
+    }
+    return s + t;
+}
+// RMSNorm of eight values: the same roundings as normalise_vector, with the product of two bf16
+// values -- exact in fp32 -- rounded by the packed multiplication.
+__device__ __forceinline__ uint4 normalise_fast(uint4 x, uint4 w, float inv) {
+    unsigned int xv[4] = {x.x, x.y, x.z, x.w};
+    const unsigned int wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        asm("{\n\t.reg .b32 t;\n\tcvt.rn.bf16x2.f32 t, %1, %2;\n\tmul.rn.bf16x2 %0, t, %3;\n\t}"
+            : "=r"(xv[q])
+            : "f"(hi_bf16(xv[q]) * inv), "f"(lo_bf16(xv[q]) * inv), "r"(wv[q]));
+    }
+    return make_uint4(xv[0], xv[1], xv[2], xv[3]);
+}
+
+// A warp's share of the activations: of every stage the groups it multiplies ("vectors": 32
+// elements of each row), R rows (the batch rounded up to a power of two) of four lanes x 16 bytes
+// each, one after the other in the warp's own 8 KB of shared memory.  A lane brings and normalises the
+// 16 bytes at slot * 512 + lane * 16 -- at small batches a slot holds several vectors, so that
+// no lane works on a row that does not exist -- and reads them as B fragments of m16n8k16.  Reductions
+// longer than 16 slots go chunk by chunk.
+constexpr int kSliceSlots = 16;
+constexpr int kSliceBytes = kSliceSlots * 512;
+static_assert(kSlicesBytes == kWarps * kSliceBytes, "the slices lie in the K/V rings, which GEMV phases do not use");
+struct Slice {
+    int lp, rs;          // log2 of vectors per stage and of R
+    int stages;          // of the whole reduction
+    int chunk;           // stages per chunk
+    int first, vectors, slots;   // of the current chunk
+};
+__device__ __forceinline__ Slice slice_of(const PhaseEntry* E, const GemvStream& d, int c) {
+    Slice v;
+    const int rows = E->rec.i[MB_GV_I_ROWS];
+    v.lp = (d.shape & kShapeShort) ? 2 : 1;
+    v.rs = rows > 2 ? (rows > 4 ? 3 : 2) : rows - 1;
+    v.stages = (d.groups + (8 << v.lp) - 1) >> (3 + v.lp);
+    v.chunk = (kSliceSlots * 8) >> (v.lp + v.rs);
+    v.first = c * v.chunk << v.lp;
+    v.vectors = min(v.chunk, v.stages - c * v.chunk) << v.lp;
+    v.slots = ((v.vectors << v.rs) + 7) >> 3;
+    return v;
+}
+// Group of 32 elements of vector `v` of warp `warp`, possibly past the end of the reduction.
+__device__ __forceinline__ int vector_group(int lp, int warp, int v) {
+    return ((v >> lp) << (3 + lp)) + (warp << lp) + (v & ((1 << lp) - 1));
+}
+__device__ __forceinline__ unsigned int slice_base(int warp) {
+    return smem_u32(g_smem) + kSliceOffset + warp * kSliceBytes;
+}
+// Norm weights of the warp's vectors wait behind the slots where there is room (the usual case).
+__device__ __forceinline__ bool weights_staged(const Slice& v) {
+    return v.stages <= v.chunk && v.slots * 512 + v.vectors * 64 <= kSliceBytes;
+}
+__device__ __forceinline__ void sts128(unsigned int addr, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
+// N slots from `i` on (the last one repeated), all loads in flight together, again and again
+// until no word is left unwritten.
+template <int N>
+__device__ __forceinline__ void fill_slots(const char* x, int lp, int warp, int vec, int step, int groups, int i,
+                                           int slots, unsigned int out, bool relay, int ph) {
+    uint4 v[N];
+    unsigned int at[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+        at[q] = static_cast<unsigned int>(min(vector_group(lp, warp, vec + min(i + q, slots - 1) * step), groups - 1)) * 64u;
+    unsigned long long start = 0;
+#pragma unroll 1
+    for (unsigned int tries = 1;; ++tries) {
+        bool missing = false;
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] = ld_relaxed_u4(x + at[q]);
+        if (!relay) break;
+#pragma unroll
+        for (int q = 0; q < N; ++q) missing |= unwritten(v[q]);
+        if (!__any_sync(0xffffffffu, missing)) break;
+        if ((tries & 63u) == 0u) {
+            if (start == 0) start = global_timer_ns();
+            if (__any_sync(0xffffffffu, wait_gave_up(ph, start))) break;  // garbage: the launch has failed
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q) sts128(out + static_cast<unsigned int>(min(i + q, slots - 1)) * 512u, v[q]);
+}
+
+// Activations kept as flagged cells.
+__device__ __noinline__ void stage_cells(const int ph, const int c) {
+    const SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const GemvStream& d = table_of()[ph].gemv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Slice sl = slice_of(E, d, c);
+    const int row = min((lane >> 2) & ((1 << sl.rs) - 1), E->rec.i[MB_GV_I_ROWS] - 1);
+    const char* x = reinterpret_cast<const char*>(E->addr[MB_GV_S_X]) + (lane & 3) * 32 +
+                    static_cast<size_t>(row) * d.row_bytes * 2;
+    const unsigned int tag = sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_X_SOURCE]) + 1u;
+#pragma unroll 1
+    for (int i = 0; i < sl.slots; ++i) {
+        const int v = sl.first + (lane >> 2 >> sl.rs) + i * (8 >> sl.rs);
+        sts128(slice_base(warp) + lane * 16 + i * 512,
+               cells_load(x + static_cast<size_t>(min(vector_group(sl.lp, warp, v), d.groups - 1)) * 128, tag, ph));
+    }
+}
+
+// Brings chunk `c` of the warp's slice to shared memory, un-normalised, once its producers have
+// written it; `store`: also hand on the gathered rows.  Returns this lane's part of its row's sum of
+// squares when the phase normalises.
+__device__ __forceinline__ float stage_slice(const int ph, const int c, const bool store) {
+    SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const GemvStream& d = table_of()[ph].gemv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tq = lane & 3;
+    const Slice sl = slice_of(E, d, c);
+    const int row = min(gid & ((1 << sl.rs) - 1), E->rec.i[MB_GV_I_ROWS] - 1);
+    const int vec = sl.first + (gid >> sl.rs), step = 8 >> sl.rs;
+    const bool gather = E->rec.i[MB_GV_I_GATHER] != 0;
+    const int flags = E->rec.i[MB_GV_I_CELLS];
+    const bool relay = !gather && (E->modes & kModeInRelay);
+    const bool cells = !gather && !relay && (flags & MB_CELLS_X);
+    const bool norm = E->rec.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
+    const unsigned int out = slice_base(warp) + lane * 16;
+    __syncwarp();
+    if (norm && weights_staged(sl)) {
+        for (int v = gid; v < sl.vectors; v += 8)
+            cp_async16(slice_base(warp) + kSliceBytes - (sl.vectors - v) * 64 + tq * 16,
+                       d.w_norm + min(vector_group(sl.lp, warp, v), d.groups - 1) * 64 + tq * 16);
+    }
+    const char* x = reinterpret_cast<const char*>(E->addr[MB_GV_S_X]) + 16 * tq;
+    if (gather) {
+        long long id = reinterpret_cast<const long long*>(E->addr[MB_GV_S_IDS])[row];
         if (id < 0 || id >= E->rec.i[MB_GV_I_VOCAB]) {
-            *bad_token = true;
+            record_status(sc->ctl, MB_ST_TOKEN_RANGE, ph, blockIdx.x);
             id = 0;
         }
-        return xbase + static_cast<size_t>(id) * K * 2;
-    }
-    return xbase + static_cast<size_t>(r) * K * 2;
-}
-
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)),
-                 "l"(src_gmem)
-                 : "memory");
-}
-// 16 bytes, or 16 zero bytes when `valid` is false (the source is not read then).
-__device__ __forceinline__ void cp_async16_or_zero(void* dst_smem, const void* src_gmem,
-                                                   bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)),
-                 "l"(src_gmem), "r"(valid ? 16 : 0)
-                 : "memory");
-}
-
-// Does this GEMV phase arm the activation mbarrier?  Plain activations come by bulk copy (one
-// per row); so do the norm weights (one more row).  Cell activations with no norm arm nothing.
-__device__ __forceinline__ bool activation_arms(const mb_phase& P) {
-    return !(P.i[MB_GV_I_CELLS] & MB_CELLS_X) || P.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
-}
-
-// Part 1 (activation_issue) starts the bulk copies global -> shared of whatever the phase takes
-// from plain memory: every activation row when they are plain bf16 (one copy per row: the
-// bulk-copy engine takes a row in one instruction, where 16-byte cp.async copies by all threads
-// stalled the issuing warps for about a microsecond on the load/store unit's miss tracking), and
-// the norm weight vector, staged as one extra row.  Part 2 waits for them (activation_finish for
-// plain rows, activation_cells for rows that arrive as flagged cells) and normalises.
-// `round` counts the phases of this CTA that armed the barrier: its parity.
-__device__ __noinline__ void activation_issue(const KernelParams& p, const PhaseEntry* E, int ph,
-                                              SharedCtl* sc, __nv_bfloat16* xs, int tid) {
-    if (tid >= 32) return;
-    const mb_phase& P = E->rec;
-    const int cells = P.i[MB_GV_I_CELLS];
-    const bool waits = (cells & MB_CELLS_X_WAIT) != 0;  // x was written earlier in this launch
-    const int rows = P.i[MB_GV_I_ROWS];
-    const int K = P.i[MB_GV_I_K];
-    const int xpitch = K + 32;
-    const bool gather = P.i[MB_GV_I_GATHER] != 0;
-    const bool normed = P.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
-    const bool plain = !(cells & MB_CELLS_X);
-    const unsigned int row_bytes = static_cast<unsigned int>(K) * 2u;
-    const int lane = tid;
-    if (sc->abort_flag) return;  // a faulted CTA arms nothing (part 2 will not wait)
-    if (activation_arms(P)) {
-        if (lane == 0) {
-            // The destination was last touched by ordinary loads and stores: hand it to the
-            // async proxy.  All bytes of the phase are expected on one barrier phase; the norm
-            // weights (they depend on nothing in this launch) are requested at once, the rows
-            // below when their producers are done.
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive_expect_tx(&sc->act_full,
-                                  row_bytes * static_cast<unsigned int>((plain ? rows : 0) + (normed ? 1 : 0)));
-            if (normed)  // the norm weights travel as row number `rows`
-                bulk_copy_g2s(xs + static_cast<size_t>(rows) * xpitch,
-                              reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_NORM_W)),
-                              row_bytes, &sc->act_full);
-        }
-    }
-    if (waits) {
-        // lane 0 polls one counter until every CTA has reported the producing phase finished
-        if (lane == 0) finished_wait(p, sc, ph, P.i[MB_GV_I_X_SOURCE]);
-        __syncwarp();
-        if (sc->abort_flag) return;
-    }
-    if (!plain) return;
-    const char* xbase = reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_X));
-    const long long* ids =
-        gather ? reinterpret_cast<const long long*>(entry_address(p, E, MB_GV_S_IDS)) : nullptr;
-    bool bad_token = false;
-    const char* src = nullptr;
-    if (lane < rows) src = activation_row(E, xbase, ids, lane, K, &bad_token);
-    // Rows written with ordinary stores by other CTAs earlier in this launch were made visible
-    // by their fence and this warp's acquire; the bulk copies below read them through the async
-    // proxy, which is ordered after that by this fence.
-    if (waits) asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncwarp();
-    if (src != nullptr)
-        bulk_copy_g2s(xs + static_cast<size_t>(lane) * xpitch, src, row_bytes, &sc->act_full);
-    if (__any_sync(0xffffffffu, bad_token) && lane == 0)
-        record_status(p.ctl, MB_ST_TOKEN_RANGE, ph, blockIdx.x);
-}
-
-__device__ __forceinline__ void wait_activation_copies(const KernelParams& p, int ph, SharedCtl* sc,
-                                                       unsigned int round) {
-    if (!mbar_wait_bounded(&sc->act_full, round & 1u, &sc->abort_flag, sc->limit_ns)) {
-        if (!sc->abort_flag) {
-            record_status(p.ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
-            sc->abort_flag = 1;
-        }
-        // fall through: the rows are garbage, the CTA drains at the end of the phase
-    }
-}
-
-// Eight raw bf16 values of the gathered (un-normalised) rows go to the residual stream, as
-// plain bf16 or as four cells.
-__device__ __forceinline__ void store_gathered(char* store, bool cells, unsigned int tag,
-                                               size_t element, uint4 raw) {
-    if (cells) {
-        char* c = store + element * 4;
-        st_cell(c, raw.x, tag);
-        st_cell(c + 8, raw.y, tag);
-        st_cell(c + 16, raw.z, tag);
-        st_cell(c + 24, raw.w, tag);
+        x += static_cast<size_t>(id) * d.row_bytes;
     } else {
-        *reinterpret_cast<uint4*>(store + element * 2) = raw;
+        x += static_cast<size_t>(row) * d.row_bytes;
     }
-}
-
-__device__ __noinline__ void activation_finish(const KernelParams& p, const PhaseEntry* E, int ph,
-                                               SharedCtl* sc, __nv_bfloat16* xs, unsigned int round,
-                                               int tid) {
-    const mb_phase& P = E->rec;
-    const int rows = P.i[MB_GV_I_ROWS];
-    const int K = P.i[MB_GV_I_K];
-    const int xpitch = K + 32;
-    const int pro = P.i[MB_GV_I_PROLOGUE];
-    const bool gather = P.i[MB_GV_I_GATHER] != 0;
-    const float embed_scale = P.f[MB_GV_F_EMBED_SCALE];
-    const bool scaled = gather && embed_scale != 0.f;
-    const bool store_x = gather && P.i[MB_GV_I_STORE_X] && blockIdx.x == 0;
-    const bool store_cells = (P.i[MB_GV_I_CELLS] & MB_CELLS_XSTORE) != 0;
-    const unsigned int tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int vec_per_row = K / 8;  // 16-byte vectors
-    const __nv_bfloat16* wrow = xs + static_cast<size_t>(rows) * xpitch;  // staged norm weights
-    wait_activation_copies(p, ph, sc, round);
-
-    if (rows >= 2 && (pro != MB_PRO_NONE || gather)) {
-        // one warp per row: sum of squares and normalisation of a row need no CTA barrier
-        // between them
-        char* store = store_x ? reinterpret_cast<char*>(entry_address(p, E, MB_GV_S_XSTORE))
-                              : nullptr;
-        for (int r = warp; r < rows; r += kConsumerWarps) {
-            __nv_bfloat16* row = xs + static_cast<size_t>(r) * xpitch;
-            float ss = 0.f;
-            for (int v = lane; v < vec_per_row; v += 32) {
-                uint4* cell = reinterpret_cast<uint4*>(row + v * 8);
-                uint4 raw = *cell;
-                if (scaled) {
-                    raw = scale_vector(raw, embed_scale);
-                    *cell = raw;
-                }
-                ss += sum_squares(raw);
-                if (store_x)
-                    store_gathered(store, store_cells, tag, static_cast<size_t>(r) * K + v * 8, raw);
-            }
-            if (pro != MB_PRO_NONE) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                const float inv = 1.0f / sqrtf(ss / static_cast<float>(K) + P.f[MB_GV_F_EPS]);
-                for (int v = lane; v < vec_per_row; v += 32) {
-                    uint4* cell = reinterpret_cast<uint4*>(row + v * 8);
-                    *cell = normalise_vector(*cell, *reinterpret_cast<const uint4*>(wrow + v * 8),
-                                             inv, pro);
-                }
-            }
+    if (cells) {
+        stage_cells(ph, c);
+        __syncwarp();
+    } else {
+        if (!relay && !gather && (flags & MB_CELLS_X_WAIT)) {
+            if (lane == 0) finished_wait(ph, E->rec.i[MB_GV_I_X_SOURCE]);
+            __syncwarp();
         }
-        named_barrier(kBarConsumers, kConsumerThreads);
-        return;
+        int i = 0;
+#pragma unroll 1
+        for (; sl.slots - i > 4; i += 8)
+            fill_slots<8>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
+        if (sl.slots - i == 1)
+            fill_slots<1>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
+        else if (sl.slots > i)
+            fill_slots<4>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
     }
-
-    if (scaled || store_x || pro != MB_PRO_NONE) {
-        // every thread works on its own vectors in both passes
-        char* store = store_x ? reinterpret_cast<char*>(entry_address(p, E, MB_GV_S_XSTORE))
-                              : nullptr;
-        for (int r = 0; r < rows; ++r) {
-            float ss = 0.f;
-            for (int v = tid; v < vec_per_row; v += kConsumerThreads) {
-                uint4* cell = reinterpret_cast<uint4*>(xs + static_cast<size_t>(r) * xpitch + v * 8);
-                uint4 raw = *cell;
-                if (scaled) {
-                    raw = scale_vector(raw, embed_scale);
-                    *cell = raw;
-                }
-                ss += sum_squares(raw);
-                if (store_x)  // the residual stream needs the un-normalised rows
-                    store_gathered(store, store_cells, tag, static_cast<size_t>(r) * K + v * 8, raw);
+    if (gather) {
+        // embedding scale; the residual stream needs the un-normalised rows
+        const float scale = E->rec.f[MB_GV_F_EMBED_SCALE];
+        char* keep = reinterpret_cast<char*>(E->addr[MB_GV_S_XSTORE]);
+        const bool as_cells = (flags & MB_CELLS_XSTORE) && !(E->modes & kModeStoreRelay);
+        const unsigned int tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
+        const bool mine = store && E->rec.i[MB_GV_I_STORE_X] && blockIdx.x == 0 && row == (gid & ((1 << sl.rs) - 1));
+#pragma unroll 1
+        for (int i = 0; i < sl.slots; ++i) {
+            const int g = vector_group(sl.lp, warp, vec + i * step);
+            uint4 v = lds128(out + i * 512);
+            if (scale != 0.f) {
+                v = scale_vector(v, scale);
+                sts128(out + i * 512, v);
             }
-            if (pro != MB_PRO_NONE) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                if (lane == 0) sc->red[warp][r] = ss;
-            }
-        }
-        if (pro != MB_PRO_NONE) {
-            named_barrier(kBarConsumers, kConsumerThreads);
-            for (int r = 0; r < rows; ++r) {
-                float total = 0.f;
-#pragma unroll
-                for (int w = 0; w < kConsumerWarps; ++w) total += sc->red[w][r];
-                const float inv = 1.0f / sqrtf(total / static_cast<float>(K) + P.f[MB_GV_F_EPS]);
-                for (int v = tid; v < vec_per_row; v += kConsumerThreads) {
-                    uint4* cell =
-                        reinterpret_cast<uint4*>(xs + static_cast<size_t>(r) * xpitch + v * 8);
-                    *cell = normalise_vector(*cell, *reinterpret_cast<const uint4*>(wrow + v * 8),
-                                             inv, pro);
-                }
+            if (mine && g < d.groups) {
+                const size_t e = static_cast<size_t>(row) * (d.row_bytes / 2) + g * 32 + 8 * tq;
+                store_result(keep, e, v.x, as_cells, tag);
+                store_result(keep, e + 2, v.y, as_cells, tag);
+                store_result(keep, e + 4, v.z, as_cells, tag);
+                store_result(keep, e + 6, v.w, as_cells, tag);
             }
         }
     }
-    named_barrier(kBarConsumers, kConsumerThreads);
-}
-
-// Two packed pairs of bf16 values (four elements) through the RMSNorm.
-__device__ __forceinline__ uint2 normalise_quad(uint2 x, uint2 w, float inv, int kind) {
-    unsigned int xv[2] = {x.x, x.y};
-    const unsigned int wv[2] = {w.x, w.y};
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        float a = lo_bf16(xv[q]), b = hi_bf16(xv[q]);
-        const float wa = lo_bf16(wv[q]), wb = hi_bf16(wv[q]);
-        if (kind == MB_PRO_RMS_LLAMA) {
-            a = bf16_round(a * inv) * wa;
-            b = bf16_round(b * inv) * wb;
-        } else {
-            a = (a * inv) * (1.0f + wa);
-            b = (b * inv) * (1.0f + wb);
-        }
-        xv[q] = pack_bf16(a, b);
-    }
-    return make_uint2(xv[0], xv[1]);
-}
-
-// Activation rows that arrive as flagged cells, written by other CTAs earlier in this launch:
-// every thread loads its share of the cells (two per 16-byte load, four loads in flight) and
-// retries the ones that do not yet carry the producing phase's sequence number -- the wait for
-// the producers and the fetch of their data are one round trip through L2.  The values go to
-// shared memory as plain bf16 rows; sums of squares are gathered on the way.
-// A row is shared by `S` warps (8 for one row, 4 for two, 2 for up to four, else 1), each lane
-// works on the same quads in both passes, so RMSNorm needs a CTA barrier only when S > 1.
-__device__ __noinline__ void activation_cells(const KernelParams& p, const PhaseEntry* E, int ph,
-                                              SharedCtl* sc, __nv_bfloat16* xs, unsigned int round,
-                                              int tid) {
-    const mb_phase& P = E->rec;
-    const int rows = P.i[MB_GV_I_ROWS];
-    const int K = P.i[MB_GV_I_K];
-    const int xpitch = K + 32;
-    const int pro = P.i[MB_GV_I_PROLOGUE];
-    const unsigned int tag = sc->tag_base + static_cast<unsigned int>(P.i[MB_GV_I_X_SOURCE]) + 1u;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int quads = K / 4;  // 16-byte loads (two cells, four values) per row
-    const int S = rows >= 5 ? 1 : (rows >= 3 ? 2 : (rows == 2 ? 4 : 8));
-    const int r = warp / S, s = warp - r * S;
-    const bool works = r < rows;
-    const char* src = reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_X)) +
-                      static_cast<size_t>(r) * K * 4;
-    __nv_bfloat16* row = xs + static_cast<size_t>(r) * xpitch;
-    const int first = s * 32 + lane, step = 32 * S;
     float ss = 0.f;
-    // warp 0 has waited for the producers in activation_issue; the others wait for warp 0
-    if (P.i[MB_GV_I_CELLS] & MB_CELLS_X_WAIT) named_barrier(kBarConsumers, kConsumerThreads);
-    if (works) {
-        constexpr int kInFlight = 8;
-        for (int j0 = first; j0 < quads; j0 += kInFlight * step) {
-            unsigned long long c[kInFlight][2];
-#pragma unroll
-            for (int u = 0; u < kInFlight; ++u) {
-                const int j = j0 + u * step;
-                if (j < quads) ld_cell_pair(src + static_cast<size_t>(j) * 16, c[u][0], c[u][1]);
-            }
-#pragma unroll
-            for (int u = 0; u < kInFlight; ++u) {
-                const int j = j0 + u * step;
-                if (j < quads) {
-                    if (cell_tag(c[u][0]) != tag || cell_tag(c[u][1]) != tag)
-                        cell_pair_wait(src + static_cast<size_t>(j) * 16, tag, c[u][0], c[u][1], p,
-                                       sc, ph);
-                    const unsigned int lo = cell_data(c[u][0]), hi = cell_data(c[u][1]);
-                    const float a0 = lo_bf16(lo), a1 = hi_bf16(lo), a2 = lo_bf16(hi), a3 = hi_bf16(hi);
-                    ss += a0 * a0;
-                    ss += a1 * a1;
-                    ss += a2 * a2;
-                    ss += a3 * a3;
-                    *reinterpret_cast<uint2*>(row + 4 * j) = make_uint2(lo, hi);
-                }
-            }
+    if (norm) {
+#pragma unroll 4
+        for (int i = 0; i < sl.slots; ++i) {
+            const float part = dot_self(lds128(out + i * 512));
+            ss += vector_group(sl.lp, warp, vec + i * step) < d.groups ? part : 0.f;
         }
     }
-    if (pro != MB_PRO_NONE) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (S > 1) {
-            if (lane == 0) sc->red[warp][0] = ss;
-            named_barrier(kBarConsumers, kConsumerThreads);
-            ss = 0.f;
-            for (int w = 0; w < S; ++w) ss += sc->red[min(r, rows - 1) * S + w][0];
-        }
-        wait_activation_copies(p, ph, sc, round);  // the norm weights (row number `rows`)
-        if (works) {
-            const float inv = 1.0f / sqrtf(ss / static_cast<float>(K) + P.f[MB_GV_F_EPS]);
-            const __nv_bfloat16* wrow = xs + static_cast<size_t>(rows) * xpitch;
-            for (int j = first; j < quads; j += step) {
-                uint2* cell = reinterpret_cast<uint2*>(row + 4 * j);
-                *cell = normalise_quad(*cell, *reinterpret_cast<const uint2*>(wrow + 4 * j), inv, pro);
-            }
-        }
-    }
-    named_barrier(kBarConsumers, kConsumerThreads);
+    __syncwarp();
+    return ss;
 }
 
-// ---------------------------------------------------------------------------------------
-// Consumer side of a GEMV phase.
-// ---------------------------------------------------------------------------------------
-struct EpilogueCtx {
-    char* out[3];
-    const char* bias[3];
-    const char* residual;
-    int n[3];
-    int epilogue;
-    bool out_cells, res_cells;
-    unsigned int tag, res_tag;
-};
-
-// One lane's pair of neighbouring results: token `gid`, output rows v and v + 1 (v even, both in
-// the same segment because segment sizes are even).  Operands that come from global memory are
-// fetched before the reduction loop so that their latency hides behind it.
-struct PairIO {
-    char* out;             // address of the pair: a cell, or two bf16
-    const char* res;       // address of the residual pair (a cell, or two bf16)
-    unsigned long long residual;  // what was loaded from there
-    unsigned int bias;     // packed bf16 pair, 0 if absent
-    bool live;
-};
-
-__device__ __forceinline__ PairIO locate_pair(const EpilogueCtx& e, int token, int vrow, bool live) {
-    PairIO io;
-    io.live = live;
-    io.out = nullptr;
-    io.res = nullptr;
-    io.residual = 0ull;
-    io.bias = 0u;
-    if (!live) return io;
-    int local = vrow, n = e.n[0];
-    char* out = e.out[0];
-    const char* bias = e.bias[0];
-    if (local >= e.n[0]) {  // segment lookup without dynamically indexed arrays
-        local -= e.n[0];
-        n = e.n[1];
-        out = e.out[1];
-        bias = e.bias[1];
-        if (local >= e.n[1]) {
-            local -= e.n[1];
-            n = e.n[2];
-            out = e.out[2];
-            bias = e.bias[2];
-        }
-    }
-    const size_t index = static_cast<size_t>(token) * n + local;  // even
-    io.out = out + index * (e.out_cells ? 4 : 2);
-    if (bias != nullptr) io.bias = __ldg(reinterpret_cast<const unsigned int*>(bias + local * 2));
-    if (e.epilogue == MB_EPI_RESIDUAL) {
-        io.res = e.residual + index * (e.res_cells ? 4 : 2);
-        io.residual = e.res_cells ? ld_cell(io.res) : static_cast<unsigned long long>(ld_cg_u32(io.res));
-    }
-    return io;
-}
-
-__device__ __forceinline__ void store_pair(const KernelParams& p, SharedCtl* sc, int ph,
-                                           const EpilogueCtx& e, PairIO& io, float acc0, float acc1,
-                                           float pair0, float pair1) {
-    const float y0 = bf16_round(acc0 + lo_bf16(io.bias));
-    const float y1 = bf16_round(acc1 + hi_bf16(io.bias));
-    float r0, r1;
-    switch (e.epilogue) {
-        case MB_EPI_RESIDUAL: {
-            if (e.res_cells && cell_tag(io.residual) != e.res_tag)
-                io.residual = cell_wait(io.res, e.res_tag, p, sc, ph);
-            const unsigned int res = cell_data(io.residual);
-            r0 = lo_bf16(res) + y0;
-            r1 = hi_bf16(res) + y1;
-            break;
-        }
-        case MB_EPI_SILU_MUL:
-            r0 = bf16_round(silu_f32(y0)) * bf16_round(pair0);
-            r1 = bf16_round(silu_f32(y1)) * bf16_round(pair1);
-            break;
-        case MB_EPI_GELU_TANH_MUL:
-            r0 = bf16_round(gelu_tanh_f32(y0)) * bf16_round(pair0);
-            r1 = bf16_round(gelu_tanh_f32(y1)) * bf16_round(pair1);
-            break;
-        default:
-            r0 = y0;
-            r1 = y1;
-            break;
-    }
-    const unsigned int packed = pack_bf16(r0, r1);
-    if (e.out_cells)
-        st_cell(io.out, packed, e.tag);
-    else
-        *reinterpret_cast<unsigned int*>(io.out) = packed;
-}
-
-// All consumer warps work on every stage together, in ring order (so no warp is ever more
-// than one mbarrier phase behind the slot it waits on).  A stage holds SUBS tiles of 8 weight
-// rows x k_chunk elements: the gate and up rows of a paired phase (PAIRED), or 16 consecutive
-// output rows of a plain one (SUBS == 2, rows of at most 1,024 elements: more bytes per stage
-// and so more bytes in flight per SM), or 8 rows.  The 32-element groups of a stage are dealt
-// round-robin to the 8 warps.  A = activations (row = token), B = weights (n = weight row); the
-// reduction index is permuted identically in both so that every lane reads 16 contiguous bytes
-// per group.  Each warp parks its partial sums of a block in shared memory; once a group of
-// blocks is through, one CTA barrier lets warp w add up the eight partials of block w and run
-// that block's epilogue.  That is one barrier pair per 8 (SUBS == 2: 4) blocks instead of a
-// reduction per stage.
-template <int SUBS, bool PAIRED>
-__device__ __noinline__ bool gemv_consume(const KernelParams& p, const PhaseEntry* E, int ph,
-                                          SharedCtl* sc, const __nv_bfloat16* xs, float* red,
-                                          const char* ring, unsigned int& it,
-                                          unsigned int act_round, int tid) {
-    static_assert(!PAIRED || SUBS == 2, "a paired phase stages two tiles");
-    constexpr int NB = SUBS == 1 ? 8 : 4;     // blocks per reduction group
-    constexpr int PV = 2 * SUBS;              // partial values per lane and block
-    constexpr int OUTS = PAIRED ? 1 : SUBS;   // result pairs per lane and block
-    constexpr int RT = 8 * OUTS;              // output rows per block
-    const int cta = blockIdx.x;
-    const GemvGeom g = gemv_geometry(E->rec, cta);
-    trace_stamp(p, ph, 7, tid);
-    const int warp = tid >> 5, lane = tid & 31;
+// Normalises the staged chunk in place.  `ss`: the warp-summed squares are in norm_part.
+__device__ __forceinline__ void normalise_slice(const int ph, const int c) {
+    SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const GemvStream& d = table_of()[ph].gemv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tq = lane & 3;
-    const int xpitch = g.K + 32;
-    const __nv_bfloat16* xrow = xs + static_cast<size_t>(min(gid, g.rows - 1)) * xpitch + 8 * tq;
-    const int cells = E->rec.i[MB_GV_I_CELLS];
-
-    EpilogueCtx e;
-    e.epilogue = E->rec.i[MB_GV_I_EPILOGUE];
-    e.out_cells = (cells & MB_CELLS_OUT) != 0;
-    e.res_cells = (cells & MB_CELLS_RESIDUAL) != 0;
-    e.tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
-    e.res_tag = sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_RES_SOURCE]) + 1u;
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        e.n[s] = g.n[s];
-        e.out[s] = s < g.nseg ? reinterpret_cast<char*>(entry_address(p, E, MB_GV_S_OUT0 + s))
-                              : nullptr;
-        e.bias[s] = (s < g.nseg && E->rec.slot[MB_GV_S_BIAS0 + s] >= 0)
-                        ? reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_BIAS0 + s))
-                        : nullptr;
+    const Slice sl = slice_of(E, d, c);
+    const int row = gid & ((1 << sl.rs) - 1), step = 8 >> sl.rs;
+    const int kind = E->rec.i[MB_GV_I_PROLOGUE];
+    const float4 lo = *reinterpret_cast<const float4*>(&sc->norm_part[row][0]);
+    const float4 hi = *reinterpret_cast<const float4*>(&sc->norm_part[row][4]);
+    const float total = ((lo.x + lo.y) + (lo.z + lo.w)) + ((hi.x + hi.y) + (hi.z + hi.w));
+    const float inv = 1.0f / sqrtf(total / static_cast<float>(d.row_bytes / 2) + E->rec.f[MB_GV_F_EPS]);
+    const unsigned int out = slice_base(warp) + lane * 16;
+    const bool staged = weights_staged(sl);
+    const char* w = staged ? g_smem + kSliceOffset + (warp + 1) * kSliceBytes - sl.vectors * 64
+                           : reinterpret_cast<const char*>(d.w_norm);
+    w += tq * 16;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    const int vec = gid >> sl.rs;
+#pragma unroll 2
+    for (int i = 0; i < sl.slots; ++i) {
+        const int v = vec + i * step;
+        const int at = staged ? min(v, sl.vectors - 1)
+                              : min(vector_group(sl.lp, warp, sl.first + v), d.groups - 1);
+        const uint4 nw = *reinterpret_cast<const uint4*>(w + at * 64);
+        const uint4 x = lds128(out + i * 512);
+        sts128(out + i * 512,
+               kind == MB_PRO_RMS_LLAMA ? normalise_fast(x, nw, inv) : normalise_vector(x, nw, inv, kind));
     }
-    e.residual = e.epilogue == MB_EPI_RESIDUAL
-                     ? reinterpret_cast<const char*>(entry_address(p, E, MB_GV_S_RESIDUAL))
-                     : nullptr;
+    __syncwarp();
+}
 
-    bool dead = false;
-    bool staged = false;  // activation rows not yet waited for / normalised
-    // ring position: one division per phase, then counted up
-    int stage = static_cast<int>(it % static_cast<unsigned int>(p.stages));
-    unsigned int wraps = it / static_cast<unsigned int>(p.stages);
-    for (int group0 = 0; group0 < g.n_blocks; group0 += NB) {
-        const int nb = min(NB, g.n_blocks - group0);
-        // The block this warp finalises, this lane's result pairs in it and their global
-        // epilogue operands: requested now, used after the reduction.
-        PairIO io[OUTS];
-#pragma unroll
-        for (int o = 0; o < OUTS; ++o) {
-            const int v = g.r0 + (group0 + warp) * RT + 8 * o + 2 * tq;
-            io[o] = locate_pair(e, gid, v, warp < nb && gid < g.rows && v < g.r1);
+// The same out of line, for slices of several chunks.
+__device__ __noinline__ float stage_chunk(int ph, int c, bool store) { return stage_slice(ph, c, store); }
+__device__ __noinline__ void normalise_chunk(int ph, int c) { normalise_slice(ph, c); }
+
+// The element of a batch of blocks that a thread finishes.
+struct Result {
+    int vrow, tok;               // virtual row (INT_MAX: none), activation row
+    unsigned int residual;       // the packed pair that holds its residual
+    float bias;
+};
+// `lr`: log2 of the rows of a block, 3 or 4; a block has 8 << lr results.
+__device__ __forceinline__ Result request_result(const PhaseEntry* E, const GemvStream& d, int lr, int block) {
+    const int t = threadIdx.x;
+    Result r;
+    r.vrow = INT_MAX;
+    r.tok = t & 7;
+    r.residual = kUnwritten;
+    r.bias = 0.f;
+    const int b = block + (t >> (3 + lr));
+    if (b < d.nblocks && r.tok < E->rec.i[MB_GV_I_ROWS]) {
+        int end;
+        const int vrow = block_row(d, b, 1 << lr, &end) + (t >> 3 & ((1 << lr) - 1));
+        if (vrow < end) {
+            r.vrow = vrow;
+            int local = vrow;
+            const int seg = output_segment(d, local);
+            const unsigned short* bias = reinterpret_cast<const unsigned short*>(E->addr[MB_GV_S_BIAS0 + seg]);
+            if (bias != nullptr) r.bias = bf16_bits_to_float(__ldg(bias + local));
+            if (E->rec.i[MB_GV_I_EPILOGUE] == MB_EPI_RESIDUAL &&
+                ((E->modes & kModeResidualRelay) || !(E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL)))
+                r.residual = ld_relaxed_u32(residual_address(E, vrow, r.tok));
         }
+    }
+    return r;
+}
 
-        if (!staged) {
-            if (cells & MB_CELLS_X)
-                activation_cells(p, E, ph, sc, const_cast<__nv_bfloat16*>(xs), act_round, tid);
-            else
-                activation_finish(p, E, ph, sc, const_cast<__nv_bfloat16*>(xs), act_round, tid);
-            staged = true;
+// Adds the slices of a thread's element, in slice order, runs the epilogue and stores the result
+// together with its neighbour's (the odd row of a pair sits eight lanes further on).
+__device__ __forceinline__ void finish_result(const PhaseEntry* E, const GemvStream& d, const int ph, const int lr,
+                                              const bool paired, const float* batch, Result r) {
+    const SharedCtl* sc = ctl_of();
+    const int t = threadIdx.x;
+    const float* part = batch + (t >> (3 + lr)) * (kWarps * 128) + (t & ((8 << lr) - 1));
+    float v[kWarps];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) v[w] = part[w * 128];
+    const float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    const bool live = r.vrow != INT_MAX;
+    const int cells = E->rec.i[MB_GV_I_CELLS], epilogue = E->rec.i[MB_GV_I_EPILOGUE];
+    float y = bf16_round(sum + r.bias);
+    if (paired) {
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) v[w] = part[w * 128 + 64];
+        const float up = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        const float act = epilogue == MB_EPI_SILU_MUL ? silu_f32(y) : gelu_tanh_f32(y);
+        y = bf16_round(act) * bf16_round(up);
+    } else if (epilogue == MB_EPI_RESIDUAL) {
+        if (live) {
+            if (E->modes & kModeResidualRelay) {
+                if (r.residual == kUnwritten) r.residual = relay_wait(residual_address(E, r.vrow, r.tok), ph);
+            } else if (cells & MB_CELLS_RESIDUAL) {
+                r.residual = cell_data(cell_wait(
+                    residual_address(E, r.vrow, r.tok),
+                    sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_RES_SOURCE]) + 1u, ph));
+            }
         }
-        for (int b = 0; b < nb; ++b) {
-            // two accumulator sets per tile keep the MMA dependency chains short
-            float acc[SUBS][4][4];
-#pragma unroll
-            for (int m = 0; m < SUBS; ++m)
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[m][u][q] = 0.f;
-            // a plain 16-row block whose second tile is past the CTA's rows multiplies one tile
-            const bool both = PAIRED || SUBS == 1 ||
-                              g.r1 - (g.r0 + (group0 + b) * RT) > kRowTile;
+        y = (r.vrow & 1 ? hi_bf16(r.residual) : lo_bf16(r.residual)) + y;
+    }
+    const float other = __shfl_xor_sync(0xffffffffu, y, 8);
+    if (live && (r.vrow & 1) == 0) {
+        int local = r.vrow;
+        const int seg = output_segment(d, local);
+        store_result(reinterpret_cast<char*>(E->addr[MB_GV_S_OUT0 + seg]),
+                     static_cast<size_t>(r.tok) * E->rec.i[MB_GV_I_N0 + seg] + local, pack_bf16(y, other),
+                     (cells & MB_CELLS_OUT) != 0 && !(E->modes & kModeOutRelay),
+                     sc->tag_base + static_cast<unsigned int>(ph) + 1u);
+    }
+}
 
-            for (int c = 0; c < g.n_chunks; ++c) {
-                const int this_stage = stage;
-                const unsigned int parity = wraps & 1u;
-                ++it;
-                if (++stage == p.stages) {
-                    stage = 0;
-                    ++wraps;
+// SHORT: blocks of 8 rows, 32 groups per stage (a CTA's rows fit one block, or few); else 16 rows,
+// or 8 gate and 8 up rows, 16 groups per stage.
+// WHOLE: the slices fit their place (host rule, kShapeWhole).
+template <bool SHORT, bool WHOLE>
+__device__ __noinline__ Place gemv_phase(const int ph, Place s) {
+    SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const GemvStream& d = table_of()[ph].gemv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nblocks = d.nblocks;
+    const bool paired = !SHORT && (d.shape & kShapePaired);
+    const bool norm = E->rec.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
+    const int lr = SHORT || paired ? 3 : 4;
+    Result result = request_result(E, d, lr, 0);
+
+    const Slice sl = slice_of(E, d, 0);
+    float ss = 0.f;
+    if (WHOLE) {
+        ss = stage_slice(ph, 0, true);
+    } else if (norm) {
+#pragma unroll 1
+        for (int c = 0; c * sl.chunk < sl.stages; ++c) ss += stage_chunk(ph, c, true);
+    }
+    if (norm) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (sl.rs < 3) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+        if (sl.rs < 2) ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+        if (sl.rs < 1) ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+        if ((lane & 3) == 0) sc->norm_part[lane >> 2][warp] = ss;
+        named_barrier(kBarAll, kThreads);
+        if (WHOLE) normalise_slice(ph, 0);
+    }
+    trace_stamp(ph, 1);
+
+    // ---- blocks of rows
+    constexpr int per = SHORT ? 4 : 2;
+    float* batch = scratch_of() + s.flip * (kScratchBytes / 8);
+    const unsigned int piece_step = SHORT || paired ? 512u : 1024u;
+    const unsigned int piece_half = paired ? kRingStage / 2 : 512u;
+    const unsigned int lane_ring = smem_u32(g_smem) + kRingOffset + lane * 16 + warp * per * piece_step;
+    const unsigned int lane_x = slice_base(warp) + (lane & ((4 << sl.rs) - 1)) * 16;
+    const unsigned int x_step = 64u << sl.rs;
+    int in_batch = 0;
+#pragma unroll 1
+    for (int b = 0; b < nblocks; ++b) {
+        float acc[2][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[0][q] = acc[1][q] = 0.f;
+#pragma unroll 1
+        for (int c = 0; WHOLE ? c == 0 : c * sl.chunk < sl.stages; ++c) {
+            if (!WHOLE) {
+                stage_chunk(ph, c, !norm && b == 0);
+                if (norm) normalise_chunk(ph, c);
+            }
+            unsigned int at = lane_x;
+#pragma unroll 1
+            for (int left = WHOLE ? sl.stages : min(sl.chunk, sl.stages - c * sl.chunk); left > 0; --left) {
+                const unsigned int piece = lane_ring + s.stage * kRingStage;
+                uint4 x[per];
+#pragma unroll
+                for (int i = 0; i < per; ++i) x[i] = lds128(at + i * x_step);
+                at += per * x_step;
+                ring_wait(s.stage, s.parity);
+                uint4 a[per], h[SHORT ? 1 : per];
+#pragma unroll
+                for (int i = 0; i < per; ++i) {
+                    a[i] = lds128(piece + i * piece_step);
+                    if (!SHORT) h[SHORT ? 0 : i] = lds128(piece + i * piece_step + piece_half);
                 }
-                if (group0 == 0 && b == 0 && c == 0) trace_stamp(p, ph, 6, tid);
-                // A wait that runs out must not make this warp leave: the others would hang
-                // at the next CTA barrier.  It records the fault, and every warp then falls
-                // through the remaining loops without waiting or computing.
-                // (the bounded wait itself watches the CTA's abort flag while it spins)
-                if (dead || !mbar_wait_bounded(&sc->full[this_stage], parity, &sc->abort_flag,
-                                               sc->limit_ns)) {
-                    if (!dead && !sc->abort_flag) {
-                        record_status(p.ctl, MB_ST_PIPE_TIMEOUT, ph, cta);
-                        sc->abort_flag = 1;
+#pragma unroll
+                for (int i = 0; i < per; ++i) {
+                    if (SHORT) {
+                        mma_bf16_16816(acc[0], a[i].x, 0u, a[i].y, 0u, x[i].x, x[i].y);
+                        mma_bf16_16816(acc[1], a[i].z, 0u, a[i].w, 0u, x[i].z, x[i].w);
+                    } else {
+                        const uint4 g = h[SHORT ? 0 : i];
+                        mma_bf16_16816(acc[0], a[i].x, g.x, a[i].y, g.y, x[i].x, x[i].y);
+                        mma_bf16_16816(acc[1], a[i].z, g.z, a[i].w, g.w, x[i].z, x[i].w);
                     }
-                    dead = true;
-                    continue;
                 }
-                if (group0 == 0 && b == 0 && c == 0) trace_stamp(p, ph, 4, tid);
-                const int kc = min(g.k_chunk, g.K - c * g.k_chunk);
-                const char* wrow = ring + static_cast<size_t>(this_stage) * p.stage_bytes +
-                                   static_cast<size_t>(gid) * g.pitch + 16 * tq;
-                const __nv_bfloat16* xk = xrow + c * g.k_chunk;
-                const int groups = kc >> 5;  // 32 reduction elements per group
-                // groups are taken two at a time onto four independent accumulator sets: the
-                // tensor-core latency of this MMA shape is long, the dependent chain must be short
-                for (int grp = warp; grp < groups; grp += 2 * kConsumerWarps) {
-                    const int grp2 = grp + kConsumerWarps;
-                    const bool second = grp2 < groups;
-                    const uint4 a = *reinterpret_cast<const uint4*>(xk + 32 * grp);
-                    const uint4 a2 = second ? *reinterpret_cast<const uint4*>(xk + 32 * grp2)
-                                            : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                    for (int m = 0; m < SUBS; ++m) {
-                        if (m == 1 && !both) break;
-                        const char* wm = wrow + static_cast<size_t>(m) * kRowTile * g.pitch;
-                        const uint4 w = *reinterpret_cast<const uint4*>(wm + 64 * grp);
-                        const uint4 w2 = second ? *reinterpret_cast<const uint4*>(wm + 64 * grp2)
-                                                : make_uint4(0u, 0u, 0u, 0u);
-                        mma_bf16_16816(acc[m][0], a.x, 0u, a.y, 0u, w.x, w.y);
-                        mma_bf16_16816(acc[m][1], a.z, 0u, a.w, 0u, w.z, w.w);
-                        mma_bf16_16816(acc[m][2], a2.x, 0u, a2.y, 0u, w2.x, w2.y);
-                        mma_bf16_16816(acc[m][3], a2.z, 0u, a2.w, 0u, w2.z, w2.w);
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sc->empty[this_stage]);
-            }
-            float* cell = red + (static_cast<size_t>(b * kConsumerWarps + warp) * 32 + lane) * PV;
-#pragma unroll
-            for (int m = 0; m < SUBS; ++m) {
-                cell[2 * m] = (acc[m][0][0] + acc[m][1][0]) + (acc[m][2][0] + acc[m][3][0]);
-                cell[2 * m + 1] = (acc[m][0][1] + acc[m][1][1]) + (acc[m][2][1] + acc[m][3][1]);
+                ring_next(s);
             }
         }
-        if (group0 == 0) trace_stamp(p, ph, 5, tid);
-        named_barrier(kBarConsumers, kConsumerThreads);
-        if (warp < nb && !dead) {
-            float total[PV];
-#pragma unroll
-            for (int v = 0; v < PV; ++v) total[v] = 0.f;
-#pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) {
-                const float* cell =
-                    red + (static_cast<size_t>(warp * kConsumerWarps + w) * 32 + lane) * PV;
-#pragma unroll
-                for (int v = 0; v < PV; ++v) total[v] += cell[v];
-            }
-            if (PAIRED) {
-                if (io[0].live) store_pair(p, sc, ph, e, io[0], total[0], total[1], total[2], total[3]);
-            } else {
-#pragma unroll
-                for (int o = 0; o < OUTS; ++o)
-                    if (io[o].live)
-                        store_pair(p, sc, ph, e, io[o], total[2 * o], total[2 * o + 1], 0.f, 0.f);
-            }
-        }
-        if (group0 + NB < g.n_blocks) named_barrier(kBarConsumers, kConsumerThreads);
-    }
-    if (!staged) {
-        // No rows here.  Plain activations still run their prologue (CTA 0 may have to store the
-        // gathered rows for the residual stream); cells are simply not read, but a bulk copy
-        // of norm weights this CTA started must land before its shared memory is used again.
-        if (!(cells & MB_CELLS_X)) {
-            activation_finish(p, E, ph, sc, const_cast<__nv_bfloat16*>(xs), act_round, tid);
-        } else if (activation_arms(E->rec)) {
-            wait_activation_copies(p, ph, sc, act_round);
-            named_barrier(kBarConsumers, kConsumerThreads);
+        float* cell = batch + (in_batch * kWarps + warp) * 128 + lane * 2;
+        *reinterpret_cast<float2*>(cell) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+        if (!SHORT)
+            *reinterpret_cast<float2*>(cell + 64) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+        if ((++in_batch << lr) == kThreads / 8 || b + 1 == nblocks) {
+            named_barrier(kBarAll, kThreads);
+            finish_result(E, d, ph, lr, paired, batch, result);
+            if (b + 1 < nblocks) result = request_result(E, d, lr, b + 1);
+            s.flip ^= 1u;
+            batch = scratch_of() + s.flip * (kScratchBytes / 8);
+            in_batch = 0;
         }
     }
-    return !dead && !sc->abort_flag;
+    return s;
 }
 
 // ---------------------------------------------------------------------------------------
-// Decode attention.
-// ---------------------------------------------------------------------------------------
-// Key chunks per (batch row, kv head): pick the count that minimises
-//   waves(items over CTAs) * (rounds of 16-key blocks over the consumer warps + fixed overhead).
-// Evaluated by one warp, two candidates per lane, identical in every CTA.
-__device__ __forceinline__ int choose_chunks(int pairs, int nblocks, int ctas, int max_chunks,
-                                             int lane) {
-    int best_cost = 0x7fffffff, best_nc = 1;
-#pragma unroll
-    for (int rep = 0; rep < 2; ++rep) {
-        const int nc = lane + 1 + 32 * rep;
-        if (nc <= max_chunks && nc <= nblocks) {
-            const int waves = (pairs * nc + ctas - 1) / ctas;
-            const int blocks = (nblocks + nc - 1) / nc;
-            const int rounds = (blocks + kConsumerWarps - 1) / kConsumerWarps;
-            // per wave: block rounds + fixed prologue/merge; plus the last arriver's fold, whose
-            // dependent batches of L2 loads grow with the chunk count
-            const int cost = 4 * waves * (rounds + 3) + nc;
-            if (cost < best_cost) {
-                best_cost = cost;
-                best_nc = nc;
-            }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int oc = __shfl_xor_sync(0xffffffffu, best_cost, o);
-        const int on = __shfl_xor_sync(0xffffffffu, best_nc, o);
-        if (oc < best_cost || (oc == best_cost && on < best_nc)) {
-            best_cost = oc;
-            best_nc = on;
-        }
-    }
-    return best_nc;
-}
-
-// Shared scratch of the attention body (carved from the activation region):
-//   qs       [8][D + 32] bf16   rotated query rows of one kv-head group
-//   kn, vn   [D] bf16 each      the new (rotated) key row and the new value row
-//   cs       [D] fp32           cos (first half) and sin (second half), already bf16-rounded
-//   wstat    [2][8 warps][8] fp32   per-warp row maxima / row sums of the exact mode
-//   fold     [8][64] + [16] fp32    chunk weights and denominators of the cross-CTA fold
-//   merge    [merge_slots][group][D + 2] fp32   per-warp (max, sum, values) states
-//   running  [2][group][D + 2] fp32             CTA state, ping-pong over merge rounds
+// Decode attention.  A CTA works on segments (the key blocks of one (row, kv head) it was dealt),
+// which the producer streams through the weight ring ahead of the phase, `1 << shift` 16-key blocks
+// with their keys and values per stage: the cached rows depend on nothing in the launch.  Stage j of a
+// segment belongs to warp j mod 8 (or the number of stages, if smaller).  Queries (rows = heads of the group) are A and keys are B
+// of the score product, transposed values (ldmatrix) A and the probabilities -- the score fragment as
+// it stands -- B of the value product.  Every warp rotates the queries for itself: element pairs
+// (i, i + D/2) sit in the same lane of two fragments.  The warp that owns the stage with the new key
+// rotates that key, appends both rows to the caches and puts them into the stage.
 //
 // Two softmax modes.  The reference normalises the probabilities in fp32 and rounds them to
 // bf16 *before* the value product (ops/attention.py:82-84).
-//   exact  (contexts of at most `exact_keys` <= 128 keys: one CTA per (row, kv head), one
+//   exact  (contexts of at most `exact_keys` <= 128 keys: one CTA per (row, kv head), at most one
 //          16-key block per warp, scores stay in registers): row max and row sum are
 //          exchanged through shared memory, then bf16(exp / sum) feeds the value product --
 //          the reference's rounding.
-//   split  (longer contexts): online softmax per warp with unnormalised bf16 probabilities,
-//          states merged across warps and, through global partials, across CTAs by the last
-//          chunk to arrive.  With hundreds of keys the rounding of single probabilities
-//          averages out far below one bf16 ulp of the result.
-// The new key/value row is appended to the cache in global memory and, for this launch's own
-// arithmetic, taken from shared memory, so nothing waits on that store.
-// `Lmax` is the largest valid length of the batch (the chunk count is chosen for it); every
-// (row, kv head) item reads its own row's length, so rows may hold different numbers of keys.
-template <int D, bool EXACT>
-__device__ __noinline__ void attention_body(const KernelParams& p, const PhaseEntry* E, int Lmax,
-                                            int ph, SharedCtl* sc, char* scratch, int tid) {
-    constexpr int QP = D + 32;  // bf16 pitch of the rotated query rows
-    constexpr int DC = D / 32;  // 32-element chunks of the head dimension (QK^T)
-    constexpr int DB = D / 64;  // 64-element blocks of the head dimension (PV)
-    constexpr int SW = D + 2;   // floats per head state: max, sum, D values
-    constexpr bool kEarlyKeys = false;      // register prefetch spills at 168 registers: off
-    constexpr bool kEarlyValues = false;    // same for the value tile
-    const mb_phase* P = &E->rec;
-    const int B = P->i[MB_AT_I_BATCH];
-    const int Hq = P->i[MB_AT_I_HEADS];
-    const int Hkv = P->i[MB_AT_I_KV_HEADS];
-    const int merge_slots = P->i[MB_AT_I_MERGE_SLOTS];
-    const int group = Hq / Hkv;  // query heads per kv head, <= 8
-    const float scale = P->f[MB_AT_F_SCALE];
-    const int warp = tid >> 5, lane = tid & 31;
-    const int gid = lane >> 2, tq = lane & 3;
-    const int cta = blockIdx.x, ctas = gridDim.x;
+//   online (longer contexts): online softmax per warp with unnormalised bf16 probabilities,
+//          states merged across warps and, through tagged partials in global memory, across CTAs:
+//          each part of a pair folds its share of the outputs from everybody's partials.  With
+//          hundreds of keys the rounding of single probabilities averages out far below one
+//          bf16 ulp of the result.
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void ldmatrix_x4_trans(unsigned int (&r)[4], unsigned int addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ float cos_of(unsigned int packed) { return lo_bf16(packed); }
+__device__ __forceinline__ float sin_of(unsigned int packed) { return hi_bf16(packed); }
 
-    // Addresses and rarely used scalars are read from the phase entry (shared memory) where
-    // they are needed instead of being kept in registers across the key loop.
-    auto slot = [&](int j) { return entry_address(p, E, j); };
-
-    const int pairs = B * Hkv;
-    constexpr bool exact = EXACT;  // contexts of at most 128 keys: at most 8 blocks
-    const int cells = P->i[MB_AT_I_CELLS];
-    const bool in_cells = (cells & MB_CELLS_X) != 0, out_cells = (cells & MB_CELLS_OUT) != 0;
-    const unsigned int in_tag =
-        sc->tag_base + static_cast<unsigned int>(P->i[MB_AT_I_QKV_SOURCE]) + 1u;
-    const unsigned int out_tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
-    const int* lengths = reinterpret_cast<const int*>(entry_address(p, E, MB_AT_S_LEN));
-    const bool per_row = P->i[MB_AT_I_LEN_COUNT] > 1;
-    // plain q, k and v written earlier in this launch: wait until their phase is finished
-    // everywhere (the named barrier below, or the one before the rotation, publishes it)
-    if ((cells & MB_CELLS_X_WAIT) && tid == 0 && !sc->abort_flag)
-        finished_wait(p, sc, ph, P->i[MB_AT_I_QKV_SOURCE]);
-    if ((cells & MB_CELLS_X_WAIT) && exact) named_barrier(kBarConsumers, kConsumerThreads);
-    int nc = 1;
-    if (!exact) {
-        if (warp == 0) {
-            const int nc_pick = choose_chunks(pairs, (Lmax + 16) >> 4, ctas,
-                                              P->i[MB_AT_I_MAX_CHUNKS], lane);
-            if (lane == 0) sc->bcast[0] = nc_pick;
-        }
-        named_barrier(kBarConsumers, kConsumerThreads);
-        nc = sc->bcast[0];
+// cos / sin of position `pos` for i = first, first + step ... < D/2, rounded to bf16 like the
+// eager tables.
+__device__ __noinline__ void fill_rope_row(unsigned int* table, const PhaseEntry* E, long long pos,
+                                              int half_dim, int first, int step) {
+    const void* invf = reinterpret_cast<const void*>(E->addr[MB_AT_S_INVFREQ]);
+    const float rope_scale = E->rec.f[MB_AT_F_ROPE_SCALE];
+    for (int i = first; i < half_dim; i += step) {
+        const float f = E->rec.i[MB_AT_I_INVFREQ_BF16] != 0
+                            ? bf16_bits_to_float(reinterpret_cast<const unsigned short*>(invf)[i])
+                            : reinterpret_cast<const float*>(invf)[i];
+        float sn, cn;
+        sincosf(static_cast<float>(pos) * f, &sn, &cn);
+        table[i] = pack_bf16(cn * rope_scale, sn * rope_scale);
     }
-    const int items = pairs * nc;
+}
 
-    __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(scratch);
-    __nv_bfloat16* kn = qs + 8 * QP;
-    __nv_bfloat16* vn = kn + D;
-    float* cs = reinterpret_cast<float*>(vn + D);
-    float* wstat = cs + D;                         // [2][kConsumerWarps][8]
-    float* fold = wstat + 2 * kConsumerWarps * 8;  // [8][64] chunk weights + denominators
-    float* merge = fold + kFoldFloats;
-    float* running = merge + static_cast<size_t>(merge_slots) * group * SW;
-    // Split mode with 64-wide heads: every warp streams its 16-key K and V tiles through two
-    // private shared-memory slots with cp.async, one tile ahead of the one it works on, so that
-    // the two dependent global round trips per block leave the critical path.
-    constexpr bool kStaged = D == 64 && !EXACT;
-    constexpr int kKPitch = D * 2 + 64, kVPitch = D * 2 + 16;  // bank-conflict-free fragment reads
-    constexpr int kTileBytes = 16 * (kKPitch + kVPitch);
-    char* staging = reinterpret_cast<char*>(running + 2 * static_cast<size_t>(group) * SW) +
-                    static_cast<size_t>(warp) * 2 * kTileBytes;
-    const size_t key_stride = static_cast<size_t>(Hkv) * D;  // elements between keys
+// Eight elements of the first half of a head and the eight they rotate with, in place.
+__device__ __forceinline__ void rotate_vectors(uint4& lo, uint4& hi, const unsigned int* table,
+                                               float q_scale) {
+    unsigned int a[4] = {lo.x, lo.y, lo.z, lo.w}, b[4] = {hi.x, hi.y, hi.z, hi.w};
+    const bool scaled = q_scale != 0.f && q_scale != 1.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        float r1[2], r2[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float x1 = e ? hi_bf16(a[w]) : lo_bf16(a[w]), x2 = e ? hi_bf16(b[w]) : lo_bf16(b[w]);
+            const unsigned int cs = table[2 * w + e];
+            const float c = cos_of(cs), sn = sin_of(cs);
+            r1[e] = bf16_round(x1 * c) + bf16_round(-x2 * sn);
+            r2[e] = bf16_round(x2 * c) + bf16_round(x1 * sn);
+            if (scaled) {
+                r1[e] = bf16_round(r1[e]) * q_scale;
+                r2[e] = bf16_round(r2[e]) * q_scale;
+            }
+        }
+        a[w] = pack_bf16(r1[0], r1[1]);
+        b[w] = pack_bf16(r2[0], r2[1]);
+    }
+    lo = make_uint4(a[0], a[1], a[2], a[3]);
+    hi = make_uint4(b[0], b[1], b[2], b[3]);
+}
 
-    for (int item = cta; item < items; item += ctas) {
-        const int pair = item / nc, chunk = item - pair * nc;
-        const int b = pair / Hkv, h = pair - b * Hkv;
-        // this row's own length: it may need fewer chunks than the longest row
-        const int L = __ldg(lengths + (per_row ? b : 0));
-        const int nkeys = L + 1;
-        const int nblocks = (nkeys + 15) >> 4;
-        const int row_chunks = min(nc, nblocks);
-        if (chunk >= row_chunks) continue;  // the whole CTA takes this branch together
-        // chunk * nblocks stays far below 2^32: 32-bit division is enough
-        const int blk0 = static_cast<int>(static_cast<unsigned>(chunk) * static_cast<unsigned>(nblocks) /
-                                          static_cast<unsigned>(row_chunks));
-        const int blk1 = static_cast<int>(static_cast<unsigned>(chunk + 1) *
-                                          static_cast<unsigned>(nblocks) /
-                                          static_cast<unsigned>(row_chunks));
-        const size_t cache_row0 =
-            (static_cast<size_t>(b) * P->i[MB_AT_I_CAPACITY] * Hkv + h) * D;  // (b, key 0, h)
-        const unsigned short* kc0 =
-            reinterpret_cast<const unsigned short*>(slot(MB_AT_S_KCACHE)) + cache_row0;
-        const unsigned short* vc0 =
-            reinterpret_cast<const unsigned short*>(slot(MB_AT_S_VCACHE)) + cache_row0;
+template <int D, bool EXACT>
+__device__ __noinline__ Place attention_phase(const int ph, Place s) {
+    constexpr int DC = D / 32;                       // 32-element groups of the head dimension
+    constexpr int DT = D / 16;                       // 16-row tiles of the value product
+    constexpr bool TWO = !EXACT && D < 256;          // two blocks per softmax step
+    constexpr int DR = D < 128 ? D : 128;            // dimensions merged at a time
+    constexpr int PR = DR + 4;                       // floats per dumped head: no bank conflicts
+    static_assert(kSliceBytes >= 8 * PR * 4, "a dumped state fits the warp's slice");
+    SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const KvStream& d = table_of()[ph].kv;
+    unsigned int* rope = rope_of();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gid = lane >> 2, tq = lane & 3;
+    const int Hq = E->rec.i[MB_AT_I_HEADS], Hkv = E->rec.i[MB_AT_I_KV_HEADS];
+    const int group = Hq / Hkv;  // query heads per kv head, <= 8
+    const float scale = E->rec.f[MB_AT_F_SCALE];
+    const int kind = source_kind(E, (E->rec.i[MB_AT_I_CELLS] & MB_CELLS_X) != 0);
+    const unsigned int own_tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
+    const bool out_cells = (E->rec.i[MB_AT_I_CELLS] & MB_CELLS_OUT) != 0 && !(E->modes & kModeOutRelay);
+    char* out = reinterpret_cast<char*>(E->addr[MB_AT_S_OUT]);
+    const bool tabled = d.batch <= kRopeRows;
 
-        // Register tiles of one 16-key block.  kt[j][i]: key kb + 8j + gid, dims 32i + 8tq..+7.
-        // vt[x][q]: key kb + {2tq, 2tq+1, 2tq+8, 2tq+9}[q], dims 64x + 8gid..+7.  Only keys
-        // already in the cache (< L) come from global memory; the new key (== L) is patched in
-        // from shared memory and later keys are zeros (their probabilities are zero too).
-        auto load_keys = [&](int blk, uint4 (&kt)[2][DC]) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int key = (blk << 4) + 8 * j + gid;
-                const bool ok = key < L;
-                const unsigned short* kp = kc0 + static_cast<size_t>(ok ? key : 0) * key_stride;
-#pragma unroll
-                for (int i = 0; i < DC; ++i)
-                    kt[j][i] = ok ? *reinterpret_cast<const uint4*>(kp + 32 * i + 8 * tq)
-                                  : make_uint4(0u, 0u, 0u, 0u);
+    // the slices still belong to the phase before until every warp is here
+    named_barrier(kBarAll, kThreads);
+    if (tabled) {
+        const int shape = d.batch * 4096 + D * 2 + (E->rec.i[MB_AT_I_INVFREQ_BF16] ? 1 : 0);
+        const bool fresh = sc->rope_pos == E->addr[MB_AT_S_POS] &&
+                           sc->rope_freq == E->addr[MB_AT_S_INVFREQ] && sc->rope_shape == shape &&
+                           sc->rope_scale == E->rec.f[MB_AT_F_ROPE_SCALE];
+        if (!fresh) {  // the same for every layer of a model: made once per launch
+            named_barrier(kBarAll, kThreads);
+            const long long* pos = reinterpret_cast<const long long*>(E->addr[MB_AT_S_POS]);
+            for (int b = warp; b < d.batch; b += kWarps)
+                fill_rope_row(rope + b * (D / 2), E, pos[b], D / 2, lane, 32);
+            if (tid == 0) {
+                sc->rope_pos = E->addr[MB_AT_S_POS];
+                sc->rope_freq = E->addr[MB_AT_S_INVFREQ];
+                sc->rope_shape = shape;
+                sc->rope_scale = E->rec.f[MB_AT_F_ROPE_SCALE];
             }
-        };
-        auto load_values = [&](int blk, uint4 (&vt)[DB][4]) {
-            const int k0 = (blk << 4) + 2 * tq;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int key = k0 + (q & 1) + ((q >> 1) << 3);
-                const bool ok = key < L;
-                const unsigned short* vp =
-                    vc0 + static_cast<size_t>(ok ? key : 0) * key_stride + 8 * gid;
-#pragma unroll
-                for (int x = 0; x < DB; ++x)
-                    vt[x][q] = ok ? *reinterpret_cast<const uint4*>(vp + 64 * x)
-                                  : make_uint4(0u, 0u, 0u, 0u);
-            }
-        };
-        // staged variant: this warp's tile `blk` into slot `slot` (rows past the valid length
-        // become zeros: their probabilities are zero, but 0 * stale bits may be NaN)
-        auto issue_tile = [&](int blk, int slot) {
-            char* kdst = staging + slot * kTileBytes;
-            char* vdst = kdst + 16 * kKPitch;
-            constexpr int kChunks = D / 8;  // 16-byte pieces per row
-#pragma unroll
-            for (int t = 0; t < 16 * kChunks / 32; ++t) {
-                const int c = lane + 32 * t, row = c / kChunks, piece = c - row * kChunks;
-                const int key = (blk << 4) + row;
-                const bool ok = key < L;
-                const size_t at = static_cast<size_t>(ok ? key : 0) * key_stride + piece * 8;
-                cp_async16_or_zero(kdst + row * kKPitch + piece * 16, kc0 + at, ok);
-                cp_async16_or_zero(vdst + row * kVPitch + piece * 16, vc0 + at, ok);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        auto staged_keys = [&](int slot, uint4 (&kt)[2][DC]) {
-            const char* kbase = staging + slot * kTileBytes;
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int i = 0; i < DC; ++i)
-                    kt[j][i] = *reinterpret_cast<const uint4*>(kbase + (8 * j + gid) * kKPitch +
-                                                               (32 * i + 8 * tq) * 2);
-        };
-        auto staged_values = [&](int slot, uint4 (&vt)[DB][4]) {
-            const char* vbase = staging + slot * kTileBytes + 16 * kKPitch;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int row = 2 * tq + (q & 1) + ((q >> 1) << 3);
-#pragma unroll
-                for (int x = 0; x < DB; ++x)
-                    vt[x][q] = *reinterpret_cast<const uint4*>(vbase + row * kVPitch +
-                                                               (64 * x + 8 * gid) * 2);
-            }
-        };
-        auto patch_new_row = [&](int blk, uint4 (&kt)[2][DC], uint4 (&vt)[DB][4]) {
-            if ((L >> 4) != blk) return;
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-                if ((blk << 4) + 8 * j + gid == L) {
-#pragma unroll
-                    for (int i = 0; i < DC; ++i)
-                        kt[j][i] = *reinterpret_cast<const uint4*>(kn + 32 * i + 8 * tq);
-                }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if ((blk << 4) + 2 * tq + (q & 1) + ((q >> 1) << 3) == L) {
-#pragma unroll
-                    for (int x = 0; x < DB; ++x)
-                        vt[x][q] = *reinterpret_cast<const uint4*>(vn + 64 * x + 8 * gid);
-                }
-        };
+            named_barrier(kBarAll, kThreads);
+        }
+    }
+    if (kind == kPlain && (E->rec.i[MB_AT_I_CELLS] & MB_CELLS_X_WAIT)) {
+        if (lane == 0) finished_wait(ph, E->rec.i[MB_AT_I_QKV_SOURCE]);
+        __syncwarp();
+    }
 
-        // ---- prologue in one memory round trip.  The raw query rows, the new key row and the
-        // new value row go global -> shared with asynchronous 16-byte copies (no registers are
-        // held across the trigonometry below); cos/sin are computed meanwhile; the first K/V
-        // tiles are requested right after, so they fly during the barrier and the rotation.
-        constexpr int kRowVectors = D / 8;  // 16-byte vectors per head row
-        const int first = blk0 + warp;
-        if (kStaged && in_cells) {
-            // the cache tiles do not depend on this layer's projections: request the first one
-            // before waiting for q, k and v
-            if (first < blk1)
-                issue_tile(first, 0);
-            else
-                asm volatile("cp.async.commit_group;" ::: "memory");
+    const unsigned int stages = static_cast<unsigned int>(sc->stages);
+    const unsigned int ring = smem_u32(g_smem) + kRingOffset;
+    float* dumps = reinterpret_cast<float*>(g_smem + kSliceOffset);
+    const Segment& seg = sc->segment[warp];
+    bool parted = false;  // some segment is one of several parts of its pair
+    for (int which = 0; find_segment(ph, which); ++which) {
+        const int L = seg.length;
+        const int b = seg.b, h = seg.h;
+        const int blocks = seg.blk1 - seg.blk0;
+        const int owners = EXACT ? kWarps : min(kWarps, static_cast<int>(stages));
+        const int shift = kv_shift(D, blocks, EXACT ? kWarps : owners);
+        const int n = (blocks + (1 << shift) - 1) >> shift;  // stages of the segment
+        const bool has = warp < min(n, owners);
+        const unsigned int pitch = 1024u << shift;  // bytes of 32 dimensions of a stage's keys
+        if (!tabled) {
+            named_barrier(kBarAll, kThreads);
+            fill_rope_row(rope, E, reinterpret_cast<const long long*>(E->addr[MB_AT_S_POS])[b], D / 2,
+                          tid, kThreads);
+            named_barrier(kBarAll, kThreads);
         }
-        // cos / sin of this row's position: independent of the projections, so before the wait
-        if (tid < D / 2) {
-            const void* invf = reinterpret_cast<const void*>(slot(MB_AT_S_INVFREQ));
-            const float f =
-                P->i[MB_AT_I_INVFREQ_BF16] != 0
-                    ? bf16_bits_to_float(reinterpret_cast<const unsigned short*>(invf)[tid])
-                    : reinterpret_cast<const float*>(invf)[tid];
-            const float angle =
-                static_cast<float>(reinterpret_cast<const long long*>(slot(MB_AT_S_POS))[b]) * f;
-            const float rope_scale = P->f[MB_AT_F_ROPE_SCALE];
-            float sn, cn;
-            sincosf(angle, &sn, &cn);
-            cs[tid] = bf16_round(cn * rope_scale);
-            cs[D / 2 + tid] = bf16_round(sn * rope_scale);
-        }
-        if (in_cells) {
-            // q, k and v of this (row, kv head) as flagged cells of the projection phase: load,
-            // retry until they carry its sequence number, park the values in shared memory
-            constexpr int kRowQuads = D / 4;  // 16-byte loads (two cells, four values) per row
-            for (int v = tid; v < (group + 2) * kRowQuads; v += kConsumerThreads) {
-                const int row = v / kRowQuads, part = v - row * kRowQuads;
-                const char* src;
-                __nv_bfloat16* dst;
-                if (row < group) {
-                    src = reinterpret_cast<const char*>(slot(MB_AT_S_Q)) +
-                          ((static_cast<size_t>(b) * Hq + h * group + row) * D + part * 4) * 4;
-                    dst = qs + row * QP;
-                } else if (row == group) {
-                    src = reinterpret_cast<const char*>(slot(MB_AT_S_K)) +
-                          ((static_cast<size_t>(b) * Hkv + h) * D + part * 4) * 4;
-                    dst = kn;
-                } else {
-                    src = reinterpret_cast<const char*>(slot(MB_AT_S_V)) +
-                          ((static_cast<size_t>(b) * Hkv + h) * D + part * 4) * 4;
-                    dst = vn;
-                }
-                unsigned long long c0, c1;
-                ld_cell_pair(src, c0, c1);
-                if (cell_tag(c0) != in_tag || cell_tag(c1) != in_tag)
-                    cell_pair_wait(src, in_tag, c0, c1, p, sc, ph);
-                *reinterpret_cast<uint2*>(dst + part * 4) = make_uint2(cell_data(c0), cell_data(c1));
-            }
-        }
-        for (int v = tid; !in_cells && v < (group + 2) * kRowVectors; v += kConsumerThreads) {
-            const int row = v / kRowVectors, part = v - row * kRowVectors;
-            const unsigned short* src;
-            __nv_bfloat16* dst;
-            if (row < group) {
-                src = reinterpret_cast<const unsigned short*>(slot(MB_AT_S_Q)) +
-                      (static_cast<size_t>(b) * Hq + h * group + row) * D;
-                dst = qs + row * QP;
-            } else if (row == group) {
-                src = reinterpret_cast<const unsigned short*>(slot(MB_AT_S_K)) +
-                      (static_cast<size_t>(b) * Hkv + h) * D;
-                dst = kn;
-            } else {
-                src = reinterpret_cast<const unsigned short*>(slot(MB_AT_S_V)) +
-                      (static_cast<size_t>(b) * Hkv + h) * D;
-                dst = vn;
-            }
-            cp_async16(dst + part * 8, src + part * 8);
-        }
-        if (!in_cells) asm volatile("cp.async.commit_group;" ::: "memory");
-        uint4 kt[2][DC];
-        uint4 vt[DB][4];
-        if (first < blk1) {
-            if (kEarlyKeys) load_keys(first, kt);
-            if (kEarlyValues) load_values(first, vt);
-        }
-        if (kStaged) {
-            // the first tile flies during the barrier and the rotation below; an empty group
-            // keeps the group count the same for warps without a tile
-            if (!in_cells) {
-                if (first < blk1)
-                    issue_tile(first, 0);
-                else
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                asm volatile("cp.async.wait_group 1;" ::: "memory");  // the prologue rows only
-            }
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        named_barrier(kBarConsumers, kConsumerThreads);
-        // rotate in place: thread e owns the element pair (i, i + D/2) of row e / (D/2); rows
-        // 0..group-1 are query heads, row `group` is the new key
-        const bool appends = chunk == row_chunks - 1;  // the chunk that holds key L stores the new row
-        const size_t new_row = cache_row0 + static_cast<size_t>(L) * key_stride;
-        const float q_scale = P->f[MB_AT_F_Q_SCALE];
-        unsigned short* kcache = reinterpret_cast<unsigned short*>(slot(MB_AT_S_KCACHE));
-        for (int e = tid; e < (group + 1) * (D / 2); e += kConsumerThreads) {
-            const int gq = e / (D / 2), i = e - gq * (D / 2);
-            __nv_bfloat16* row = gq == group ? kn : qs + gq * QP;
-            const float x1 = __bfloat162float(row[i]), x2 = __bfloat162float(row[i + D / 2]);
-            const float c = cs[i], sn = cs[D / 2 + i];
-            float r1 = bf16_round(bf16_round(x1 * c) + bf16_round(-x2 * sn));
-            float r2 = bf16_round(bf16_round(x2 * c) + bf16_round(x1 * sn));
-            if (gq != group && q_scale != 0.f && q_scale != 1.f) {
-                r1 = bf16_round(r1 * q_scale);
-                r2 = bf16_round(r2 * q_scale);
-            }
-            row[i] = __float2bfloat16_rn(r1);
-            row[i + D / 2] = __float2bfloat16_rn(r2);
-            if (gq == group && appends) {
-                kcache[new_row + i] = float_to_bf16_bits(r1);
-                kcache[new_row + i + D / 2] = float_to_bf16_bits(r2);
-            }
-        }
-        if (appends && tid < D)
-            reinterpret_cast<unsigned short*>(slot(MB_AT_S_VCACHE))[new_row + tid] =
-                reinterpret_cast<unsigned short*>(vn)[tid];
-        named_barrier(kBarConsumers, kConsumerThreads);
-        trace_stamp(p, ph, 4, tid);
+        const unsigned int* row_rope = rope + (tabled ? b * (D / 2) : 0);
 
-        // QK^T: A = rotated queries (row = head of the group), B = keys (n = key).  The head
-        // dimension is permuted identically in both operands so that every lane fetches 16
-        // contiguous bytes of its key per 32-element chunk.
+        // Queries, and in the warp whose stage includes the new key that key and its value: one
+        // round trip for all of them (256-wide heads: one after the other, in as many registers).
         uint4 qf[DC];
+        if (has) {
+            const bool holder = seg.blk1 - 1 == (L >> 4) && (n - 1) % owners == warp;
+            const int elem = kind == kCells ? 4 : 2;
+            const char* qrow = reinterpret_cast<const char*>(E->addr[MB_AT_S_Q]) +
+                               (static_cast<size_t>(b) * Hq + h * group + min(gid, group - 1)) * D * elem +
+                               8 * tq * elem;
+            const size_t kv_row = (static_cast<size_t>(b) * Hkv + h) * D * elem;
+            const char* krow = reinterpret_cast<const char*>(E->addr[MB_AT_S_K]) + kv_row + 8 * tq * elem;
+            const char* vrow = reinterpret_cast<const char*>(E->addr[MB_AT_S_V]) + kv_row +
+                               8 * (lane & (D / 8 - 1)) * elem;
+            if (kind == kCells) {  // one vector at a time, through the warp's slice
+                const unsigned int tag =
+                    sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_AT_I_QKV_SOURCE]) + 1u;
+                const unsigned int keep = slice_base(warp) + lane * 16;
+#pragma unroll 1
+                for (int i = 0; i < (holder ? 2 * DC + 1 : DC); ++i)
+                    sts128(keep + min(i, kSliceSlots - 1) * 512,
+                           cells_load(i < DC ? qrow + 128 * i : (i < 2 * DC ? krow + 128 * (i - DC) : vrow), tag, ph));
+                __syncwarp();
+            }
+            const size_t at = ((static_cast<size_t>(b) * d.capacity + L) * Hkv + h) * D;
+            auto place_new_row = [&](uint4 (&kn)[DC], uint4 vn) {
+                if (gid == 0) {
 #pragma unroll
-        for (int i = 0; i < DC; ++i)
-            qf[i] = gid < group ? *reinterpret_cast<const uint4*>(qs + gid * QP + 32 * i + 8 * tq)
-                                : make_uint4(0u, 0u, 0u, 0u);
-        float m_run = -INFINITY, l_run = 0.f;
-        // PV^T: A = V^T (row = head dim, via byte-permute of per-key vectors), B = P^T, which
-        // is the score fragment as it stands.  acc[x][mt]: dims 64x + 8*gid + 2*mt (+1),
-        // heads 2*tq (+1).
-        float acc[DB][4][4];
+                    for (int i = 0; i < DC / 2; ++i)
+                        rotate_vectors(kn[i], kn[i + DC / 2], row_rope + 32 * i + 8 * tq, 0.f);
+                    unsigned short* cache = reinterpret_cast<unsigned short*>(d.k) + at;
 #pragma unroll
-        for (int x = 0; x < DB; ++x)
+                    for (int i = 0; i < DC; ++i) {
+                        *reinterpret_cast<uint4*>(cache + 32 * i + 8 * tq) = kn[i];
+                        *reinterpret_cast<uint4*>(&sc->new_row[0][32 * i + 8 * tq]) = kn[i];
+                    }
+                }
+                if (lane < D / 8) {
+                    *reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(d.v) + at + 8 * lane) = vn;
+                    *reinterpret_cast<uint4*>(&sc->new_row[1][8 * lane]) = vn;
+                }
+            };
+            if (D < 256 && kind != kCells) {
+                uint4 in[2 * DC + 1], kn[DC];
+                gather_source<2 * DC + 1>(
+                    in, holder ? 2 * DC + 1 : DC, kind == kRelay,
+                    [&](int i) { return i < DC ? qrow + 64 * i : (i < 2 * DC ? krow + 64 * (i - DC) : vrow); }, ph);
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+                for (int i = 0; i < DC; ++i) {
+                    qf[i] = in[i];
+                    kn[i] = in[DC + i];
+                }
+                if (holder) place_new_row(kn, in[2 * DC]);
+            } else {
+                if (holder) {
+                    uint4 in[DC + 1], kn[DC];
+                    const unsigned int kept = slice_base(warp) + lane * 16;
+                    if (kind == kCells) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[x][mt][q] = 0.f;
+                        for (int i = 0; i <= DC; ++i) in[i] = lds128(kept + min(DC + i, kSliceSlots - 1) * 512);
+                        if (2 * DC >= kSliceSlots) {  // the slice holds one vector less: keys 0 .. DC - 2
+                            in[DC] = in[DC - 1];
+                            in[DC - 1] = cells_load(
+                                krow + 128 * (DC - 1),
+                                sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_AT_I_QKV_SOURCE]) + 1u, ph);
+                        }
+                    } else {
+                        gather_source<DC + 1>(
+                            in, DC + 1, kind == kRelay, [&](int i) { return i < DC ? krow + 64 * i : vrow; }, ph);
+                    }
+#pragma unroll
+                    for (int i = 0; i < DC; ++i) kn[i] = in[i];
+                    place_new_row(kn, in[DC]);
+                }
+                if (kind == kCells) {
+#pragma unroll
+                    for (int i = 0; i < DC; ++i) qf[i] = lds128(slice_base(warp) + lane * 16 + i * 512);
+                } else {
+                    gather_source<DC>(qf, DC, kind == kRelay, [&](int i) { return qrow + 64 * i; }, ph);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < DC / 2; ++i)
+                rotate_vectors(qf[i], qf[i + DC / 2], row_rope + 32 * i + 8 * tq, E->rec.f[MB_AT_F_Q_SCALE]);
+            __syncwarp();
+        }
 
-        // scores of one block: sv[2j + q] <-> head gid, key kb + 8j + 2tq + q; bf16-rounded
+        float m_run = -INFINITY, l_run = 0.f;
+        // acc[t]: dims 16t + gid (+8), heads 2*tq (+1)
+        float acc[DT][4];
+#pragma unroll
+        for (int t = 0; t < DT; ++t)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[t][q] = 0.f;
+        // Stage j belongs to warp j mod `owners`: a warp always waits for uses of one slot, in order (a
+        // parity says nothing about a use before the last one).  Exact mode, where eight blocks may
+        // meet a shorter ring: all warps go through all stages.
+        unsigned int slot = s.stage, parity = s.parity;
+        auto advance = [&](unsigned int by) {
+            slot += by;
+            if (slot >= stages) {
+                slot -= stages;
+                parity ^= 1u;
+            }
+        };
+        if (!EXACT) advance(has ? static_cast<unsigned int>(warp) : 0u);
+
+        // The current stage, with the new row in its place and zeros after its value (0 * stale bits
+        // may be NaN) if it is the one.
+        auto open_stage = [&](int first_key, int keys) {
+            ring_wait(slot, parity);
+            const unsigned int base = ring + slot * kRingStage;
+            const int row = L - first_key;
+            if (row >= 0 && row < keys) {
+                constexpr int C = D / 8;  // 16-byte pieces of a row
+                const unsigned int values = base + DC * pitch;
+                const int zero = (15 - (row & 15)) * C;
+                for (int p = lane; p < 2 * C + zero; p += 32) {
+                    const int r = p < 2 * C ? row : row + 1 + (p - 2 * C) / C, c = p & (C - 1);
+                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                    if (p < 2 * C) v = *reinterpret_cast<const uint4*>(&sc->new_row[p < C ? 0 : 1][8 * c]);
+                    const unsigned int at = (c >> 2) * pitch + static_cast<unsigned int>(r) * 64u;
+                    sts128(p < C ? base + at + (c & 3) * 16 : values + at + (((c & 3) ^ ((r >> 1) & 3)) << 4), v);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
+            return base;
+        };
+        auto close_stage = [&](unsigned int by) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive_count(&sc->empty[slot], EXACT ? 1u : kWarps);
+            advance(by);
+        };
+        // scores of block `q` of a stage: sv[2j + e] <-> head gid, key 8j + 2tq + e; bf16-rounded
         // product, scale applied in fp32, keys past the valid length masked
-        auto block_scores = [&](int kb, const uint4 (&kt_)[2][DC], float (&sv)[4]) {
+        auto block_scores = [&](unsigned int base, int q, int first_key, float (&sv)[4]) {
             float frag[2][4], frag2[2][4];  // two independent chains per tile, added at the end
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                frag[j][0] = frag[j][1] = frag[j][2] = frag[j][3] = 0.f;
-                frag2[j][0] = frag2[j][1] = frag2[j][2] = frag2[j][3] = 0.f;
-            }
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int i = 0; i < DC; ++i)
+                for (int e = 0; e < 4; ++e) frag[j][e] = frag2[j][e] = 0.f;
+            unsigned int at = base + static_cast<unsigned int>(q) * 1024u + lane * 16;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    mma_bf16_16816(frag[j], qf[i].x, 0u, qf[i].y, 0u, kt_[j][i].x, kt_[j][i].y);
-                    mma_bf16_16816(frag2[j], qf[i].z, 0u, qf[i].w, 0u, kt_[j][i].z, kt_[j][i].w);
-                }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                frag[j][0] += frag2[j][0];
-                frag[j][1] += frag2[j][1];
+            for (int i = 0; i < DC; ++i, at += pitch) {
+                const uint4 k0 = lds128(at), k1 = lds128(at + 512);
+                mma_bf16_16816(frag[0], qf[i].x, 0u, qf[i].y, 0u, k0.x, k0.y);
+                mma_bf16_16816(frag[1], qf[i].x, 0u, qf[i].y, 0u, k1.x, k1.y);
+                mma_bf16_16816(frag2[0], qf[i].z, 0u, qf[i].w, 0u, k0.z, k0.w);
+                mma_bf16_16816(frag2[1], qf[i].z, 0u, qf[i].w, 0u, k1.z, k1.w);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int key = kb + 8 * j + 2 * tq + q;
-                    const float sval = bf16_round(frag[j][q]) * scale;
-                    sv[2 * j + q] = key < nkeys ? sval : -INFINITY;
+                for (int e = 0; e < 2; ++e) {
+                    const float v = bf16_round(frag[j][e] + frag2[j][e]) * scale;
+                    sv[2 * j + e] = first_key + 16 * q + 8 * j + 2 * tq + e <= L ? v : -INFINITY;
                 }
         };
-        // acc += V^T P^T for one block; pb0/pb1 = probabilities of keys (2tq, 2tq+1) and
-        // (8+2tq, 9+2tq) of head gid, packed bf16
-        auto block_values = [&](const uint4 (&vt_)[DB][4], unsigned int pb0, unsigned int pb1) {
+        // Lane's address for the value fragments of block 0: matrices (keys 0-7, dims 0-7), (keys
+        // 0-7, dims 8-15), then keys 8-15; rows are 64 bytes, their four pieces permuted by the
+        // tensor map so that eight rows touch all banks.
+        const int vr = (lane & 7) + ((lane >> 4) << 3), vc = (lane >> 3) & 1;
+        const unsigned int v_row = DC * pitch + static_cast<unsigned int>(vr) * 64u;
+        const unsigned int v_even = v_row + ((vc ^ ((vr >> 1) & 3)) << 4);  // dims 0-15 of a group
+        const unsigned int v_odd = v_row + (((vc + 2) ^ ((vr >> 1) & 3)) << 4);
+        // acc += V^T P^T for one block; pb0 / pb1 = probabilities of keys (2tq, 2tq + 1) and
+        // (8 + 2tq, 9 + 2tq) of head gid, packed bf16
+        auto block_values = [&](unsigned int base, int q, unsigned int pb0, unsigned int pb1) {
+            unsigned int at = base + static_cast<unsigned int>(q) * 1024u;
 #pragma unroll
-            for (int x = 0; x < DB; ++x) {
-                const unsigned int ra[4] = {vt_[x][0].x, vt_[x][0].y, vt_[x][0].z, vt_[x][0].w};
-                const unsigned int rb[4] = {vt_[x][1].x, vt_[x][1].y, vt_[x][1].z, vt_[x][1].w};
-                const unsigned int rc[4] = {vt_[x][2].x, vt_[x][2].y, vt_[x][2].z, vt_[x][2].w};
-                const unsigned int rd[4] = {vt_[x][3].x, vt_[x][3].y, vt_[x][3].z, vt_[x][3].w};
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    const unsigned int a0 = __byte_perm(ra[mt], rb[mt], 0x5410u);
-                    const unsigned int a1 = __byte_perm(ra[mt], rb[mt], 0x7632u);
-                    const unsigned int a2 = __byte_perm(rc[mt], rd[mt], 0x5410u);
-                    const unsigned int a3 = __byte_perm(rc[mt], rd[mt], 0x7632u);
-                    mma_bf16_16816(acc[x][mt], a0, a1, a2, a3, pb0, pb1);
-                }
+            for (int i = 0; i < DC; ++i, at += pitch) {
+                unsigned int a[4], c[4];
+                ldmatrix_x4_trans(a, at + v_even);
+                ldmatrix_x4_trans(c, at + v_odd);
+                mma_bf16_16816(acc[2 * i], a[0], a[1], a[2], a[3], pb0, pb1);
+                mma_bf16_16816(acc[2 * i + 1], c[0], c[1], c[2], c[3], pb0, pb1);
             }
         };
 
-        if (exact) {
-            // one block per warp at most; warps without a block still join the two exchanges
-            const bool has = first < blk1;
+        if (EXACT) {
+            // one block per warp at most; warps without a block still join the two exchanges.  The
+            // value fragments leave the ring before them, so that a ring shorter than the segment
+            // cannot stall the producer against the barrier.
             float sv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            if (has) {
-                if (!kEarlyKeys) load_keys(first, kt);
-                if (!kEarlyValues) load_values(first, vt);
-                patch_new_row(first, kt, vt);
-                block_scores(first << 4, kt, sv);
+            unsigned int vf[DT][4];
+#pragma unroll 1
+            for (int j = 0; j < n; ++j) {
+                const unsigned int base = open_stage(j * 16, j == warp ? 16 : 0);
+                if (j == warp) {
+                    block_scores(base, 0, j * 16, sv);
+#pragma unroll
+                    for (int i = 0; i < DC; ++i) {
+                        ldmatrix_x4_trans(vf[2 * i], base + i * pitch + v_even);
+                        ldmatrix_x4_trans(vf[2 * i + 1], base + i * pitch + v_odd);
+                    }
+                }
+                close_stage(1);
             }
             float rmax = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
             rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
             rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
-            if (tq == 0) wstat[warp * 8 + gid] = rmax;
-            named_barrier(kBarConsumers, kConsumerThreads);
+            if (tq == 0) sc->exchange[0][warp][gid] = rmax;
+            named_barrier(kBarAll, kThreads);
             float row_max = -INFINITY;
 #pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) row_max = fmaxf(row_max, wstat[w * 8 + gid]);
+            for (int w = 0; w < kWarps; ++w) row_max = fmaxf(row_max, sc->exchange[0][w][gid]);
             float ev[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) ev[q] = expf(sv[q] - row_max);  // 0 for masked keys
             float rsum = (ev[0] + ev[1]) + (ev[2] + ev[3]);
             rsum += __shfl_xor_sync(0xffffffffu, rsum, 1);
             rsum += __shfl_xor_sync(0xffffffffu, rsum, 2);
-            if (tq == 0) wstat[(kConsumerWarps + warp) * 8 + gid] = rsum;
-            named_barrier(kBarConsumers, kConsumerThreads);
+            if (tq == 0) sc->exchange[1][warp][gid] = rsum;
+            named_barrier(kBarAll, kThreads);
             float row_sum = 0.f;
 #pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w)
-                row_sum += wstat[(kConsumerWarps + w) * 8 + gid];
-            if (has)  // normalised probabilities rounded to bf16, as the eager operator does
-                block_values(vt, pack_bf16(ev[0] / row_sum, ev[1] / row_sum),
-                             pack_bf16(ev[2] / row_sum, ev[3] / row_sum));
+            for (int w = 0; w < kWarps; ++w) row_sum += sc->exchange[1][w][gid];
+            if (has) {  // normalised probabilities rounded to bf16, as the eager operator does
+                const unsigned int pb0 = pack_bf16(ev[0] / row_sum, ev[1] / row_sum);
+                const unsigned int pb1 = pack_bf16(ev[2] / row_sum, ev[3] / row_sum);
+#pragma unroll
+                for (int t = 0; t < DT; ++t) mma_bf16_16816(acc[t], vf[t][0], vf[t][1], vf[t][2], vf[t][3], pb0, pb1);
+            }
             // already normalised: merge as plain sums (max 0, total weight 1)
             m_run = 0.f;
             l_run = (warp == 0 && tq == 0) ? 1.f : 0.f;
         } else {
-            // online softmax, one 16-key block per iteration, the next block requested ahead
-            uint4 kt_next[2][DC];
-            uint4 vt_next[DB][4];
-            int slot = 0;
-            for (int blk = first; blk < blk1; blk += kConsumerWarps) {
-                const int kb = blk << 4;
-                const int following = blk + kConsumerWarps;
-                if (kStaged) {
-                    if (following < blk1) {
-                        issue_tile(following, slot ^ 1);
-                        asm volatile("cp.async.wait_group 1;" ::: "memory");
-                    } else {
-                        asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll 1
+            for (int j = has ? warp : n; j < n; j += owners) {
+                const int first_key = (seg.blk0 + (j << shift)) * 16;
+                const int here = min(1 << shift, blocks - (j << shift));  // blocks
+                const unsigned int base = open_stage(first_key, here * 16);
+#pragma unroll 1
+                for (int q = 0; q < here; q += TWO ? 2 : 1) {
+                    const bool two = TWO && q + 1 < here;
+                    float sv[2][4];
+                    block_scores(base, q, first_key, sv[0]);
+                    if (two)
+                        block_scores(base, q + 1, first_key, sv[1]);
+                    else
+                        sv[1][0] = sv[1][1] = sv[1][2] = sv[1][3] = -INFINITY;
+                    float bmax = fmaxf(fmaxf(fmaxf(sv[0][0], sv[0][1]), fmaxf(sv[0][2], sv[0][3])),
+                                       fmaxf(fmaxf(sv[1][0], sv[1][1]), fmaxf(sv[1][2], sv[1][3])));
+                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
+                    if (__any_sync(0xffffffffu, bmax > m_run)) {  // a new maximum: rare after the first blocks
+                        const float m_new = fmaxf(m_run, bmax);
+                        const float alpha = expf(m_run - m_new);
+                        l_run *= alpha;
+                        m_run = m_new;
+                        // rescale factors of the two heads this lane accumulates (columns 2tq, 2tq+1)
+                        const float alpha0 = __shfl_sync(0xffffffffu, alpha, (2 * tq) * 4);
+                        const float alpha1 = __shfl_sync(0xffffffffu, alpha, (2 * tq + 1) * 4);
+#pragma unroll
+                        for (int t = 0; t < DT; ++t) {
+                            acc[t][0] *= alpha0;
+                            acc[t][1] *= alpha1;
+                            acc[t][2] *= alpha0;
+                            acc[t][3] *= alpha1;
+                        }
                     }
-                    __syncwarp();  // every lane's pieces of the current tile have landed
-                    staged_keys(slot, kt);
-                    staged_values(slot, vt);
-                    __syncwarp();  // the slot may be refilled from the next iteration on
-                    slot ^= 1;
-                } else {
-                    if (!kEarlyKeys) load_keys(blk, kt);
-                    if (!kEarlyValues) load_values(blk, vt);
+                    float pv[2][4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        pv[0][e] = expf(sv[0][e] - m_run);
+                        pv[1][e] = TWO ? expf(sv[1][e] - m_run) : 0.f;
+                    }
+                    l_run += ((pv[0][0] + pv[0][1]) + (pv[0][2] + pv[0][3])) +
+                             ((pv[1][0] + pv[1][1]) + (pv[1][2] + pv[1][3]));
+                    block_values(base, q, pack_bf16(pv[0][0], pv[0][1]), pack_bf16(pv[0][2], pv[0][3]));
+                    if (two)
+                        block_values(base, q + 1, pack_bf16(pv[1][0], pv[1][1]), pack_bf16(pv[1][2], pv[1][3]));
                 }
-                if (following < blk1) {
-                    if (kEarlyKeys) load_keys(following, kt_next);
-                    if (kEarlyValues) load_values(following, vt_next);
-                }
-                patch_new_row(blk, kt, vt);
-                float sv[4];
-                block_scores(kb, kt, sv);
-                float bmax = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
-                bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
-                bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
-                const float m_new = fmaxf(m_run, bmax);
-                const float alpha = expf(m_run - m_new);
-                float pv[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) pv[q] = expf(sv[q] - m_new);
-                l_run = l_run * alpha + ((pv[0] + pv[1]) + (pv[2] + pv[3]));
-                m_run = m_new;
-                // rescale factors of the two heads this lane accumulates (columns 2tq, 2tq+1)
-                const float alpha0 = __shfl_sync(0xffffffffu, alpha, (2 * tq) * 4);
-                const float alpha1 = __shfl_sync(0xffffffffu, alpha, (2 * tq + 1) * 4);
-#pragma unroll
-                for (int x = 0; x < DB; ++x)
-#pragma unroll
-                    for (int mt = 0; mt < 4; ++mt) {
-                        acc[x][mt][0] *= alpha0;
-                        acc[x][mt][1] *= alpha1;
-                        acc[x][mt][2] *= alpha0;
-                        acc[x][mt][3] *= alpha1;
-                    }
-                block_values(vt, pack_bf16(pv[0], pv[1]), pack_bf16(pv[2], pv[3]));
-                if (following < blk1) {
-                    if (kEarlyKeys) {
-#pragma unroll
-                        for (int j = 0; j < 2; ++j)
-#pragma unroll
-                            for (int i = 0; i < DC; ++i) kt[j][i] = kt_next[j][i];
-                    }
-                    if (kEarlyValues) {
-#pragma unroll
-                        for (int x = 0; x < DB; ++x)
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) vt[x][q] = vt_next[x][q];
-                    }
-                }
+                close_stage(owners);
             }
         }
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-        trace_stamp(p, ph, 5, tid);
+        {
+            const unsigned int next = s.stage + static_cast<unsigned int>(n);
+            s.parity ^= (next / stages) & 1u;
+            s.stage = next % stages;
+        }
+        trace_stamp(ph, 5);
 
-        // ---- merge the warp states into one CTA state, `merge_slots` warps per round
-        const int rounds = (kConsumerWarps + merge_slots - 1) / merge_slots;
-        for (int round = 0; round < rounds; ++round) {
-            const int lead = round * merge_slots;
-            if (warp >= lead && warp < lead + merge_slots) {
-                float* base = merge + static_cast<size_t>(warp - lead) * group * SW;
-                if (tq == 0 && gid < group) {
-                    base[gid * SW] = m_run;
-                    base[gid * SW + 1] = l_run;
+        // ---- merge the warp states: dumped DR dimensions at a time, added up in warp order
+        if (tq == 0) {
+            sc->stat[warp][gid][0] = m_run;
+            sc->stat[warp][gid][1] = l_run;
+        }
+        if (seg.parts > 1) parted = true;
+#pragma unroll
+        for (int r = 0; r < D / DR; ++r) {
+            if (r > 0) named_barrier(kBarAll, kThreads);
+            __syncwarp();
+            float* dump = dumps + warp * (kSliceBytes / 4) + gid;
+#pragma unroll
+            for (int t = 0; t < DR / 16; ++t) {
+                const float(&v)[4] = acc[r * (DR / 16) + t];
+                if (2 * tq < group) {
+                    dump[(2 * tq) * PR + 16 * t] = v[0];
+                    dump[(2 * tq) * PR + 16 * t + 8] = v[2];
                 }
-                const int h0 = 2 * tq, h1 = 2 * tq + 1;
-#pragma unroll
-                for (int x = 0; x < DB; ++x)
-#pragma unroll
-                    for (int mt = 0; mt < 4; ++mt) {
-                        const int d = 64 * x + 8 * gid + 2 * mt;
-                        if (h0 < group) {
-                            base[h0 * SW + 2 + d] = acc[x][mt][0];
-                            base[h0 * SW + 2 + d + 1] = acc[x][mt][2];
-                        }
-                        if (h1 < group) {
-                            base[h1 * SW + 2 + d] = acc[x][mt][1];
-                            base[h1 * SW + 2 + d + 1] = acc[x][mt][3];
-                        }
-                    }
+                if (2 * tq + 1 < group) {
+                    dump[(2 * tq + 1) * PR + 16 * t] = v[1];
+                    dump[(2 * tq + 1) * PR + 16 * t + 8] = v[3];
+                }
             }
-            named_barrier(kBarConsumers, kConsumerThreads);
-            const int live = min(merge_slots, kConsumerWarps - lead);
-            const float* prev = running + static_cast<size_t>((round & 1) ^ 1) * group * SW;
-            float* next = running + static_cast<size_t>(round & 1) * group * SW;
-            for (int e = tid; e < group * SW; e += kConsumerThreads) {
-                const int gq = e / SW, col = e - gq * SW;
-                float mx = round == 0 ? -INFINITY : prev[gq * SW];
-                for (int w = 0; w < live; ++w)
-                    mx = fmaxf(mx, merge[(static_cast<size_t>(w) * group + gq) * SW]);
-                float sum_l = 0.f, sum_v = 0.f;
-                if (round > 0) {
-                    const float wgt = __expf(prev[gq * SW] - mx);
-                    sum_l = prev[gq * SW + 1] * wgt;
-                    sum_v = prev[gq * SW + col] * wgt;
-                }
-                for (int w = 0; w < live; ++w) {
-                    const float* st = merge + (static_cast<size_t>(w) * group + gq) * SW;
+            named_barrier(kBarAll, kThreads);
+#pragma unroll 1
+            for (int o = tid; o < group * (DR / 2); o += kThreads) {
+                const int head = o / (DR / 2), dim = 2 * (o & (DR / 2 - 1));
+                float m_all = -INFINITY, l_all = 0.f, y0 = 0.f, y1 = 0.f;
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) m_all = fmaxf(m_all, sc->stat[w][head][0]);
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) {
                     // weights between partial softmax states: no rounding point of the operator
                     // sits here, the fast exponential is accurate to 2^-21
-                    const float wgt = __expf(st[0] - mx);  // 0 for a warp that saw no block
-                    sum_l += st[1] * wgt;
-                    sum_v += st[col] * wgt;
+                    const float wgt = __expf(sc->stat[w][head][0] - m_all);  // 0: a warp without a block
+                    const float2 v =
+                        *reinterpret_cast<const float2*>(dumps + w * (kSliceBytes / 4) + head * PR + dim);
+                    l_all += sc->stat[w][head][1] * wgt;
+                    y0 += v.x * wgt;
+                    y1 += v.y * wgt;
                 }
-                next[e] = col == 0 ? mx : (col == 1 ? sum_l : sum_v);
-            }
-            named_barrier(kBarConsumers, kConsumerThreads);
-        }
-        const float* state = running + static_cast<size_t>((rounds - 1) & 1) * group * SW;
-        trace_stamp(p, ph, 6, tid);
-
-        // results leave in pairs of neighbouring elements: one 4-byte store, or one cell
-        char* out = reinterpret_cast<char*>(slot(MB_AT_S_OUT));
-        auto store_out = [&](int gq, int d, float v0, float v1) {
-            const size_t index = (static_cast<size_t>(b) * Hq + h * group + gq) * D + d;
-            const unsigned int packed = pack_bf16(v0, v1);
-            if (out_cells)
-                st_cell(out + index * 4, packed, out_tag);
-            else
-                *reinterpret_cast<unsigned int*>(out + index * 2) = packed;
-        };
-        if (row_chunks == 1) {
-            for (int e = tid; e < group * (D / 2); e += kConsumerThreads) {
-                const int gq = e / (D / 2), d = 2 * (e - gq * (D / 2));
-                const float denom_ = state[gq * SW + 1];
-                store_out(gq, d, state[gq * SW + 2 + d] / denom_, state[gq * SW + 3 + d] / denom_);
-            }
-        } else {
-            float* partial = reinterpret_cast<float*>(slot(MB_AT_S_PARTIAL));
-            int* counter = reinterpret_cast<int*>(slot(MB_AT_S_COUNTER));
-            const int max_chunks = P->i[MB_AT_I_MAX_CHUNKS];
-            float* mine = partial + (static_cast<size_t>(pair) * max_chunks + chunk) * group * SW;
-            for (int e = tid; e < group * SW; e += kConsumerThreads) mine[e] = state[e];
-            __threadfence();
-            named_barrier(kBarConsumers, kConsumerThreads);
-            if (tid == 0) {
-                const int arrived = atomicAdd(counter + pair, 1);
-                __threadfence();
-                sc->bcast[1] = arrived;
-            }
-            named_barrier(kBarConsumers, kConsumerThreads);
-            trace_stamp(p, ph, 7, tid);
-            const int nc_row = row_chunks;
-            if (sc->bcast[1] == nc_row - 1) {
-                // Last chunk of this (row, kv head) to arrive folds all chunks, in chunk order.
-                // Step 1: (max, sum) of every chunk into shared memory, all loads in flight
-                // together, then the per-chunk weights and the denominator.
-                const float* all = partial + static_cast<size_t>(pair) * max_chunks * group * SW;
-                float* weight = fold;          // [group][nc] chunk maxima, then weights
-                float* denom = fold + 8 * 64;  // [group]
-                float* sums = merge;           // [group][nc] chunk sums (merge slots are free)
-                for (int e = tid; e < group * nc_row; e += kConsumerThreads) {
-                    const int gq = e / nc_row, c = e - gq * nc_row;
-                    const float* st = all + (static_cast<size_t>(c) * group + gq) * SW;
-                    weight[e] = ld_cg_f32(st);
-                    sums[e] = ld_cg_f32(st + 1);
-                }
-                named_barrier(kBarConsumers, kConsumerThreads);
-                if (tid < group) {
-                    float mx = -INFINITY;
-                    for (int c = 0; c < nc_row; ++c) mx = fmaxf(mx, weight[tid * nc_row + c]);
-                    float total = 0.f;
-                    for (int c = 0; c < nc_row; ++c) {
-                        const float wgt = expf(weight[tid * nc_row + c] - mx);
-                        weight[tid * nc_row + c] = wgt;
-                        total += sums[tid * nc_row + c] * wgt;
+                const int column = r * DR + dim;
+                if (seg.parts == 1) {
+                    store_result(out, (static_cast<size_t>(b) * Hq + h * group + head) * D + column,
+                                 pack_bf16(y0 / l_all, y1 / l_all), out_cells, own_tag);
+                } else {
+                    // cells of (fp32, tag): maximum, sum, D values per head
+                    char* part = reinterpret_cast<char*>(E->addr[MB_AT_S_PARTIAL]) +
+                                 ((static_cast<size_t>(seg.pair) * d.chunk_cap + seg.index) * group + head) *
+                                     ((D + 2) * 8);
+                    st_cell(part + (2 + column) * 8, __float_as_uint(y0), own_tag);
+                    st_cell(part + (3 + column) * 8, __float_as_uint(y1), own_tag);
+                    if (column == 0) {
+                        st_cell(part, __float_as_uint(m_all), own_tag);
+                        st_cell(part + 8, __float_as_uint(l_all), own_tag);
                     }
-                    denom[tid] = total;
                 }
-                named_barrier(kBarConsumers, kConsumerThreads);
-                // Step 2: weighted sums of the value partials, two neighbouring elements per
-                // thread; loads are independent.
-                for (int e = tid; e < group * (D / 2); e += kConsumerThreads) {
-                    const int gq = e / (D / 2), d = 2 * (e - gq * (D / 2));
-                    const float* col = all + static_cast<size_t>(gq) * SW + 2 + d;
-                    float sum0 = 0.f, sum1 = 0.f;
-                    for (int c0 = 0; c0 < nc_row; c0 += 8) {  // eight loads in flight per batch
-                        float2 part[8];
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            part[u] = c0 + u < nc_row
-                                          ? __ldcg(reinterpret_cast<const float2*>(
-                                                col + static_cast<size_t>(c0 + u) * group * SW))
-                                          : make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            if (c0 + u < nc_row) {
-                                const float wgt = weight[gq * nc_row + c0 + u];
-                                sum0 += part[u].x * wgt;
-                                sum1 += part[u].y * wgt;
-                            }
-                    }
-                    store_out(gq, d, sum0 / denom[gq], sum1 / denom[gq]);
-                }
-                if (tid == 0) counter[pair] = 0;  // ready for the next launch
             }
         }
-        named_barrier(kBarConsumers, kConsumerThreads);  // scratch is reused by the next item
+        named_barrier(kBarAll, kThreads);  // slices and statistics are reused by the next segment
     }
-}
+    trace_stamp(ph, 7);
 
-// Reads the valid lengths (one shared by the batch, or one per row), refuses a full cache --
-// every thread of every CTA sees the same lengths, so all of them take the same branch -- and
-// picks the softmax mode from the longest row.  The two modes are separate functions so that a
-// launch only ever executes one of them: instruction-cache footprint matters more here than
-// code sharing.  The lengths do not change during a launch (they are advanced when it ends).
-template <int D>
-__device__ __forceinline__ void attention_decode(const KernelParams& p, const PhaseEntry* E,
-                                                 int ph, SharedCtl* sc, char* scratch, int tid) {
-    const int* lenp = reinterpret_cast<const int*>(entry_address(p, E, MB_AT_S_LEN));
-    const int count = E->rec.i[MB_AT_I_LEN_COUNT] > 1 ? E->rec.i[MB_AT_I_BATCH] : 1;
-    const int capacity = E->rec.i[MB_AT_I_CAPACITY];
-    int longest = 0, bad = 0, bad_length = 0;
-    for (int r = 0; r < count; ++r) {
-        const int L = __ldg(lenp + r);
-        if (L < 0 || L + 1 > capacity) {
-            bad = 1;
-            bad_length = L;
+    // ---- fold the parts of the pairs this CTA has a part of: its share of their outputs.  Only
+    // after ALL its partials are out, so no chain of CTAs waits for one another's folds.
+    for (int which = 0; parted; ++which) {
+        if (!find_segment(ph, which)) break;
+        if (seg.parts == 1) continue;
+        const int total = group * (D / 2);  // pairs of neighbouring outputs
+        const int lo = seg.index * total / seg.parts, hi = (seg.index + 1) * total / seg.parts;
+        const int width = seg.parts <= 2 ? 2 : (seg.parts <= 4 ? 4 : (seg.parts <= 8 ? 8 : 16));
+        const char* base = reinterpret_cast<const char*>(E->addr[MB_AT_S_PARTIAL]) +
+                           static_cast<size_t>(seg.pair) * d.chunk_cap * group * ((D + 2) * 8);
+        const int j = tid & (width - 1);
+        for (int o0 = lo; o0 < hi; o0 += kThreads / width) {
+            const int o = o0 + tid / width;
+            const int head = min(o, hi - 1) / (D / 2), dim = 2 * (min(o, hi - 1) - head * (D / 2));
+            float m[2], l[2], v0[2], v1[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = j + u * width;
+                m[u] = -INFINITY;
+                l[u] = v0[u] = v1[u] = 0.f;
+                if (c < seg.parts && o < hi) {
+                    const char* part = base + (static_cast<size_t>(c) * group + head) * ((D + 2) * 8);
+                    unsigned long long cm, cl, c0, c1;
+                    ld_cell_pair(part, cm, cl);
+                    ld_cell_pair(part + (2 + dim) * 8, c0, c1);
+                    if (cell_tag(cm) != own_tag) cm = cell_wait(part, own_tag, ph);
+                    if (cell_tag(cl) != own_tag) cl = cell_wait(part + 8, own_tag, ph);
+                    if (cell_tag(c0) != own_tag) c0 = cell_wait(part + (2 + dim) * 8, own_tag, ph);
+                    if (cell_tag(c1) != own_tag) c1 = cell_wait(part + (3 + dim) * 8, own_tag, ph);
+                    m[u] = __uint_as_float(cell_data(cm));
+                    l[u] = __uint_as_float(cell_data(cl));
+                    v0[u] = __uint_as_float(cell_data(c0));
+                    v1[u] = __uint_as_float(cell_data(c1));
+                }
+            }
+            float mx = fmaxf(m[0], m[1]);
+            for (int w = width >> 1; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const float w0 = m[0] == -INFINITY ? 0.f : expf(m[0] - mx);
+            const float w1 = m[1] == -INFINITY ? 0.f : expf(m[1] - mx);
+            float den = l[0] * w0 + l[1] * w1;
+            float s0 = v0[0] * w0 + v0[1] * w1, s1 = v1[0] * w0 + v1[1] * w1;
+            for (int w = width >> 1; w > 0; w >>= 1) {
+                den += __shfl_xor_sync(0xffffffffu, den, w);
+                s0 += __shfl_xor_sync(0xffffffffu, s0, w);
+                s1 += __shfl_xor_sync(0xffffffffu, s1, w);
+            }
+            if (j == 0 && o < hi)
+                store_result(out, (static_cast<size_t>(seg.b) * Hq + seg.h * group + head) * D + dim,
+                             pack_bf16(s0 / den, s1 / den), out_cells, own_tag);
         }
-        longest = max(longest, L);
     }
-    if (bad) {
-        if (tid == 0) {
-            record_status(p.ctl, MB_ST_KV_OVERFLOW, ph, bad_length);
-            sc->abort_flag = 1;
-        }
-        return;
-    }
-    if (longest + 1 <= E->rec.i[MB_AT_I_EXACT_KEYS])
-        attention_body<D, true>(p, E, longest, ph, sc, scratch, tid);
-    else
-        attention_body<D, false>(p, E, longest, ph, sc, scratch, tid);
+    return s;
 }
 
 // ---------------------------------------------------------------------------------------
 // The kernel.
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void prefetch_entry(const PhaseEntry* src, PhaseEntry* dst, int tid) {
-    // 16-byte asynchronous copies global -> shared of one phase entry
-    if (src != nullptr && tid < kEntryVectors) {
-        const unsigned int d = smem_u32(reinterpret_cast<char*>(dst) + 16 * tid);
-        const char* g = reinterpret_cast<const char*>(src) + 16 * tid;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g) : "memory");
+// Completes one stream record in shared memory for this CTA and this launch: its output rows, or
+// the valid lengths and how the keys are dealt.  False: a length (`bad`) does not fit the cache.
+__device__ __forceinline__ bool complete_stream(StreamDesc* desc, int* bad) {
+    if (desc->kind == kStreamGemv) {
+        GemvStream& d = desc->gemv;
+        d.w_norm = resolve_address(d.w_norm);
+        const int cta = blockIdx.x, q = d.r0, rem = d.r1;  // pairs of rows per CTA, and the rest
+        d.r0 = 2 * (cta * q + min(cta, rem));
+        d.r1 = d.r0 + 2 * (q + (cta < rem ? 1 : 0));
+        d.nblocks = count_blocks(d, (d.shape & (kShapeShort | kShapePaired)) ? 8 : 16);
+        return true;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// Thread 0, at the start of phase `ph`: fetch the counter of phase ph - 2 from L2 (not L1: other
-// SMs add to it) into shared memory, in the same group as the entry prefetch, so that the check
-// at the end of the phase finds it there without a round trip of its own.
-__device__ __forceinline__ void prefetch_guard(const KernelParams& p, SharedCtl* sc, int ph) {
-    const unsigned int d = smem_u32(sc->guard);
-    const void* g = &p.ctl->finished[(ph - 2) & 3];
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g) : "memory");
-}
-
-// Every thread waits for its own copies; the 16-byte vectors of one address pair (two slots)
-// were copied by one thread, which then patches them -- no extra barrier is needed before the
-// CTA barrier that publishes the entry.
-__device__ __forceinline__ void wait_entry(const KernelParams& p, PhaseEntry* dst, int tid) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (dst == nullptr) return;
-    constexpr int kFirstAddrVector = offsetof(PhaseEntry, addr) / 16;
-    static_assert(offsetof(PhaseEntry, addr) % 16 == 8, "addr[] starts mid-vector");
-    // vector kFirstAddrVector holds addr[0] in its upper half; vector v > that holds
-    // addr[2 (v - first) - 1] and addr[2 (v - first)]
-    if (tid >= kFirstAddrVector && tid < kEntryVectors) {
-        const int hi = 2 * (tid - kFirstAddrVector), lo = hi - 1;
-        if (lo >= 0 && lo < MB_PHASE_SLOTS) dst->addr[lo] = resolve_dynamic(p, dst->addr[lo]);
-        if (hi < MB_PHASE_SLOTS) dst->addr[hi] = resolve_dynamic(p, dst->addr[hi]);
-    }
-}
-
-__global__ void __launch_bounds__(kThreads, 1)
-decode_kernel(const __grid_constant__ KernelParams p) {
-    extern __shared__ __align__(128) char smem[];
-    SharedCtl* sc = reinterpret_cast<SharedCtl*>(smem);
-    float* red = reinterpret_cast<float*>(smem + kCtlBytes);
-    char* act = smem + kFixedBytes;
-    char* ring = act + p.activation_bytes;
-    const int tid = threadIdx.x;
-
-    if (tid == 0) {
-        for (int s = 0; s < kMaxStages; ++s) {
-            mbar_init(&sc->full[s], 1);
-            mbar_init(&sc->empty[s], kConsumerWarps);
+    if (desc->kind != kStreamKv) return true;
+    KvStream& d = desc->kv;
+    d.k = resolve_address(d.k);
+    d.v = resolve_address(d.v);
+    d.lengths = resolve_address(d.lengths);
+    const int* lengths = reinterpret_cast<const int*>(d.lengths);
+    const int count = d.len_count > 1 ? d.batch : 1;
+    int longest = 0, blocks = 0;
+    bool fits = true;
+    for (int r = 0; r < count; ++r) {
+        const int L = *reinterpret_cast<const volatile int*>(lengths + r);
+        if (L < 0 || L >= d.capacity) {
+            fits = false;
+            *bad = L;
         }
-        mbar_init(&sc->act_full, 1);
-        sc->abort_flag = peek_status(p.ctl) != 0 ? 1 : 0;  // a faulted plan runs nothing
-        sc->issued = 0;
-        sc->limit_ns = static_cast<unsigned long long>(p.wait_limit_us) * 1000ull;
-        // Both words only change after the closing barrier of a launch (or by a host reset).
-        const unsigned int calls = *reinterpret_cast<volatile unsigned int*>(&p.ctl->calls);
-        const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&p.ctl->epoch);
-        sc->tag_base = epoch * static_cast<unsigned int>(p.n_phases);
-        sc->calls = calls;
-        mbar_init_fence();
+        if (r < 8) d.lens[r] = L;
+        longest = max(longest, L);
+        blocks += (L + 16) >> 4;
     }
-    if (tid < kConsumerThreads) {
-        prefetch_entry(p.entries, &sc->entry[0], tid);
-        wait_entry(p, &sc->entry[0], tid);
+    if (!fits) return false;
+    if (count == 1) blocks *= d.batch;
+    blocks *= d.kv_heads;
+    d.exact_keys = longest + 1 <= d.exact_keys ? 1 : 0;
+    d.total_blocks = blocks;
+    d.cut_ctas = 0;
+    const int longest_blocks = (longest + 16) >> 4;
+    if (!d.exact_keys && d.chunk_cap > 1 && longest_blocks > kWholeBlocks) {
+        // parts of a pair: at most nb * runs / total + 2 of them by rounding
+        const int by_cap = static_cast<int>(static_cast<long long>(d.chunk_cap - 1) * blocks / longest_blocks);
+        d.cut_ctas = max(1, min(min(static_cast<int>(gridDim.x), blocks / kRunBlocks), by_cap - 1));
+        if (d.cut_ctas < 2) {
+            d.cut_ctas = 0;
+            return true;
+        }
+        // Parts of one pair per CTA wherever they are not much longer than the even runs: a CTA
+        // with the end of one pair and the start of the next goes through everything but the keys
+        // twice, which takes as long as about kSeamBlocks of them.
+        const int even = (blocks + d.cut_ctas - 1) / d.cut_ctas;
+        for (int t = max(max(even, kRunBlocks), (longest_blocks + d.chunk_cap - 1) / d.chunk_cap);
+             t <= even + kSeamBlocks; ++t) {
+            int ctas = 0;
+            for (int r = 0; r < count; ++r) {
+                const int L = r < 8 ? d.lens[r] : *reinterpret_cast<const volatile int*>(lengths + r);
+                ctas += (((L + 16) >> 4) + t - 1) / t;
+            }
+            if (ctas * (count == 1 ? d.batch : 1) * d.kv_heads <= static_cast<int>(gridDim.x)) {
+                d.cut_ctas = -t;
+                break;
+            }
+        }
+    }
+    return true;
+}
+
+// DIM: the head size of all attention phases of the plan (0: a mix of sizes, every body compiled
+// in).  One kernel per head size keeps the code of a launch within the instruction caches and its
+// loop operands in registers.
+template <int D>
+__device__ __forceinline__ Place attention_call(int ph, Place s) {
+    return table_of()[ph].kv.exact_keys ? attention_phase<D, true>(ph, s) : attention_phase<D, false>(ph, s);
+}
+template <int DIM>
+__device__ __forceinline__ Place run_attention(int ph, Place s) {
+    if constexpr (DIM != 0) {
+        return attention_call<DIM>(ph, s);
+    } else {
+        const int dim = table_of()[ph].kv.head_dim;
+        if (dim == 64) return attention_call<64>(ph, s);
+        if (dim == 128) return attention_call<128>(ph, s);
+        return attention_call<256>(ph, s);
+    }
+}
+
+// Start of a launch, all threads: control block, stream table, ring.  False: a fault is on record
+// (now or from an earlier launch) and nothing may run.
+__device__ __forceinline__ bool begin_launch(const KernelParams& p, const StreamDesc* streams, const void* maps,
+                                             unsigned int tag_base, unsigned int parity,
+                                             unsigned int calls) {
+    SharedCtl* sc = ctl_of();
+    StreamDesc* table = reinterpret_cast<StreamDesc*>(g_smem + table_offset(p.stages));
+    const int tid = threadIdx.x;
+    for (int v = tid; v < p.n_phases * 6; v += kAllThreads)
+        reinterpret_cast<uint4*>(table)[v] = reinterpret_cast<const uint4*>(streams)[v];
+    if (tid == 0) {
+        for (int i = 0; i < p.stages; ++i) {
+            mbar_init(&sc->full[i], 1);
+            mbar_init(&sc->empty[i], kWarps);
+        }
+        mbar_init(&sc->entry_full, 1);
+        sc->issued = 0;
+        mbar_init_fence();
+        sc->abort_flag = peek_status(p.ctl) != 0 ? 1 : 0;  // a faulted plan runs nothing
+        sc->limit_ns = static_cast<unsigned long long>(p.wait_limit_us) * 1000ull;
+        sc->tag_base = tag_base;
+        sc->calls = calls;
+        sc->ctl = p.ctl;
+        sc->trace = p.trace;
+        sc->n_phases = p.n_phases;
+        sc->stages = p.stages;
+        sc->maps = reinterpret_cast<const CUtensorMap*>(maps);
+        sc->entries = p.entries;
+        for (int i = 0; i < MB_MAX_DYNAMIC; ++i) sc->dyn[i] = p.dyn[i];
+        sc->relay_now = p.relay + (parity & 1u) * p.relay_bytes;
+        sc->relay_next = p.relay + ((parity & 1u) ^ 1u) * p.relay_bytes;
+        sc->rope_pos = sc->rope_freq = 0;
+        sc->rope_shape = -1;
     }
     __syncthreads();
-    if (sc->abort_flag) return;
+    if (sc->abort_flag) return false;
+    for (int ph = tid; ph < p.n_phases; ph += kAllThreads) {
+        int bad = 0;
+        if (!complete_stream(table + ph, &bad)) {
+            record_status(p.ctl, MB_ST_KV_OVERFLOW, ph, bad);
+            sc->abort_flag = 1;
+        }
+    }
+    __syncthreads();
+    return sc->abort_flag == 0;
+}
 
-    if (tid >= kConsumerThreads) {
-        producer_loop(p, sc, ring, tid & 31);
-    } else {
-        const unsigned int calls = *reinterpret_cast<volatile unsigned int*>(&p.ctl->calls);
-        const unsigned int base = calls * static_cast<unsigned int>(p.barriers_per_launch);
-        unsigned int it = 0;
-        unsigned int act_round = 0;  // GEMV phases run so far: parity of the activation barrier
-        int barrier_index = 0;
-        bool ok = true;
-        // Optional per-phase trace: thread 0 of every CTA stamps the global timer at phase
-        // start (0), after the activation copies were started (1), after the body (2) and after
-        // the closing grid barrier, if the phase has one (3).
-        auto stamp = [&](int ph, int event) {
-            if (p.trace != nullptr && tid == 0)
-                p.trace[(static_cast<size_t>(blockIdx.x) * p.n_phases + ph) * kTraceEvents + event] =
-                    global_timer_ns();
-        };
-        for (int ph = 0; ph < p.n_phases && ok; ++ph) {
-            // The entry of this phase is in shared memory already; fetch the next one now so
-            // that no phase starts with a dependent chain of global loads.
-            const PhaseEntry* E = &sc->entry[ph & 1];
-            const bool more = ph + 1 < p.n_phases;
-            if (ph >= 2 && tid == 0) prefetch_guard(p, sc, ph);
-            prefetch_entry(more ? p.entries + ph + 1 : nullptr, &sc->entry[(ph + 1) & 1], tid);
-            stamp(ph, 0);
-            switch (E->rec.body) {
-                case MB_BODY_NOP:
-                    break;
-                case MB_BODY_GEMV: {
-                    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(act);
-                    activation_issue(p, E, ph, sc, xs, tid);
-                    stamp(ph, 1);
-                    if (E->rec.i[MB_GV_I_NMAT] == 2)
-                        gemv_consume<2, true>(p, E, ph, sc, xs, red, ring, it, act_round, tid);
-                    else if (E->rec.i[MB_GV_I_ROW_TILE] == 2 * kRowTile)
-                        gemv_consume<2, false>(p, E, ph, sc, xs, red, ring, it, act_round, tid);
-                    else
-                        gemv_consume<1, false>(p, E, ph, sc, xs, red, ring, it, act_round, tid);
-                    if (activation_arms(E->rec)) ++act_round;
-                    break;
-                }
-                case MB_BODY_ATTN_DECODE: {
-                    const int D = E->rec.i[MB_AT_I_HEAD_DIM];
-                    if (D == 64)
-                        attention_decode<64>(p, E, ph, sc, act, tid);
-                    else if (D == 128)
-                        attention_decode<128>(p, E, ph, sc, act, tid);
-                    else
-                        attention_decode<256>(p, E, ph, sc, act, tid);
-                    break;
-                }
-                default:
-                    if (tid == 0) {
-                        record_status(p.ctl, MB_ST_BAD_PHASE, ph, E->rec.body);
-                        sc->abort_flag = 1;
-                    }
-                    break;
-            }
-            // Whether to go on is decided once per CTA, by thread 0 inside the barrier below
-            // (a fault raises the CTA's abort flag; bodies never leave early on their own
-            // except for conditions every thread evaluates identically).
-            stamp(ph, 2);
-            const int flags = E->rec.flags;
-            wait_entry(p, more ? &sc->entry[(ph + 1) & 1] : nullptr, tid);  // published by the barrier below
-            if (ph >= 2 && tid == 0 && !sc->abort_flag) {
-                const unsigned int target = finished_target(p, sc, ph - 2);
-                if (static_cast<int>(sc->guard[0] - target) < 0) finished_wait(p, sc, ph, ph - 2);
-            }
-            if (flags & MB_FLAG_BARRIER) {
-                ++barrier_index;
-                ok = grid_barrier(p.ctl, base + barrier_index, kBarConsumers, kConsumerThreads, tid,
-                                  &sc->abort_flag, &sc->verdict, ph, sc->limit_ns);
-                stamp(ph, 3);
-            } else {
-                // one CTA barrier: every warp is done with the phase's shared memory, and all of
-                // them learn together whether one of them raised the abort flag
-                ok = !named_barrier_or(kBarConsumers, kConsumerThreads, sc->abort_flag != 0);
-            }
-            // This CTA has finished phase `ph` (all its loads of the phase's inputs are done):
-            // counted for the CTAs that are about to leave phase ph + 2.  No ordering is needed
-            // beyond the CTA barrier above.
-            if (ok && tid == 0) {
-                // plain results that a later phase fetches after waiting on this counter: make
-                // the CTA's stores (ordered before this point by the CTA barrier) visible first
+// One 16-byte vector of a phase entry, addresses resolved.  addr[] starts in the upper half of
+// vector kFirst; the last vector's upper half is `modes`.
+__device__ __forceinline__ uint4 resolve_vector(uint4 v, int index) {
+    constexpr int kFirst = offsetof(PhaseEntry, addr) / 16;
+    static_assert(offsetof(PhaseEntry, addr) % 16 == 8 && offsetof(PhaseEntry, modes) % 16 == 8,
+                  "addr[] starts mid-vector and modes ends one");
+    if (index > kFirst) {
+        const unsigned long long a =
+            resolve_address(v.x | (static_cast<unsigned long long>(v.y) << 32));
+        v.x = static_cast<unsigned int>(a);
+        v.y = static_cast<unsigned int>(a >> 32);
+    }
+    if (index >= kFirst && index < kEntryVectors - 1) {
+        const unsigned long long a =
+            resolve_address(v.z | (static_cast<unsigned long long>(v.w) << 32));
+        v.z = static_cast<unsigned int>(a);
+        v.w = static_cast<unsigned int>(a >> 32);
+    }
+    return v;
+}
+
+// Phase entries: at the start of phase ph warp 0 resolves the addresses of record ph + 1, which
+// the barrier inside the phase publishes, and fetches record ph + 2 over that of ph - 2 (no
+// warp can still be there: all have passed the barrier of ph - 1).
+__device__ __noinline__ void fetch_entry(int ph) {
+    SharedCtl* sc = ctl_of();
+    if (ph < sc->n_phases && (threadIdx.x & 31) == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive_expect_tx(&sc->entry_full, sizeof(PhaseEntry));
+        bulk_copy_g2s(&sc->entry[ph & 3], sc->entries + ph, sizeof(PhaseEntry), &sc->entry_full);
+    }
+}
+__device__ __noinline__ void place_entry(int ph) {
+    SharedCtl* sc = ctl_of();
+    const int lane = threadIdx.x & 31;
+    if (ph >= sc->n_phases) return;
+    if (!mbar_wait_bounded(&sc->entry_full, ph & 1, &sc->abort_flag, sc->limit_ns)) {
+        if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+        sc->abort_flag = 1;
+    }
+    if (lane < kEntryVectors) {
+        uint4* v = reinterpret_cast<uint4*>(&sc->entry[ph & 3]) + lane;
+        *v = resolve_vector(*v, lane);
+    }
+    __syncwarp();
+}
+
+// The consumer warps' walk through the phase table.
+template <int DIM>
+__device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned int calls) {
+    SharedCtl* sc = ctl_of();
+    const StreamDesc* table = table_of();
+    const int tid = threadIdx.x, warp = tid >> 5;
+    Place place{0u, 0u, 0u};
+    if (warp == 0) {
+        fetch_entry(0);
+        place_entry(0);
+        fetch_entry(1);
+    }
+    // the other half of the arena becomes blank for the next launch
+    for (unsigned long long at = (static_cast<unsigned long long>(blockIdx.x) * kThreads + tid) * 16;
+         at < p.relay_bytes; at += static_cast<unsigned long long>(gridDim.x) * kThreads * 16)
+        *reinterpret_cast<uint4*>(sc->relay_next + at) =
+            make_uint4(kUnwritten, kUnwritten, kUnwritten, kUnwritten);
+    named_barrier(kBarAll, kThreads);
+
+    const unsigned int barriers = calls * static_cast<unsigned int>(p.barriers_per_launch);
+    int barrier_index = 0;
+    // Optional per-phase trace: thread 0 of every CTA stamps the global timer at phase start (0),
+    // when the first activations are ready (1), after the body (2) and after the closing grid
+    // barrier, if the phase has one (3).
+    for (int ph = 0; ph < p.n_phases; ++ph) {
+        if (warp == 0) {
+            place_entry(ph + 1);
+            fetch_entry(ph + 2);
+        }
+        const PhaseEntry* E = &sc->entry[ph & 3];
+        trace_stamp(ph, 0);
+        const int kind = table[ph].kind;
+        bool meet = true;  // the phase has not had a barrier of all threads
+        if (kind == kStreamGemv) {
+            const GemvStream& d = table[ph].gemv;
+            if (d.shape & kShapeWhole)
+                place = d.shape & kShapeShort ? gemv_phase<true, true>(ph, place) : gemv_phase<false, true>(ph, place);
+            else
+                place = d.shape & kShapeShort ? gemv_phase<true, false>(ph, place) : gemv_phase<false, false>(ph, place);
+            meet = d.nblocks == 0;
+        } else if (kind == kStreamKv) {
+            place = run_attention<DIM>(ph, place);
+            meet = false;
+        }
+        trace_stamp(ph, 2);
+        const int flags = E->rec.flags;
+        if (meet || p.counters) named_barrier(kBarAll, kThreads);
+        if (p.counters && tid == 0) {
+            // This CTA has finished phase `ph`: counted for the CTAs that wait for its plain results
+            // or are about to overwrite what it has read.
+            if (ph >= 2 && !sc->abort_flag) finished_wait(ph, ph - 2);
+            if (!sc->abort_flag) {
                 if (flags & MB_FLAG_FENCE) asm volatile("fence.acq_rel.gpu;" ::: "memory");
                 asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(
                                  &p.ctl->finished[ph & 3].count)
                              : "memory");
             }
         }
-        if (ok) {
-            // Closing barrier: every CTA has read the valid lengths, `calls` and `epoch` and is
-            // done with them; CTA 0 may now advance them.
+        if (flags & MB_FLAG_BARRIER) {
             ++barrier_index;
-            ok = grid_barrier(p.ctl, base + barrier_index, kBarConsumers, kConsumerThreads, tid,
-                              &sc->abort_flag, &sc->verdict, p.n_phases, sc->limit_ns);
-            // a launch that recorded a fault anywhere (a token outside the table ...) leaves the
-            // lengths and the launch counters alone: the host has to reset the plan anyway
-            if (ok && blockIdx.x == 0 && peek_status(p.ctl) == 0) {
-                // valid_length += 1 for every attention phase that asks for it, one thread per
-                // phase (the table is in L2: the producers prefetched it)
-                for (int q = tid; q < p.n_phases; q += kConsumerThreads) {
-                    const PhaseEntry* G = p.entries + q;
-                    if (G->rec.body != MB_BODY_ATTN_DECODE || !(G->rec.flags & MB_FLAG_BUMP_LENGTH))
-                        continue;
-                    int* lenp = reinterpret_cast<int*>(resolve_dynamic(p, G->addr[MB_AT_S_LEN]));
-                    const int count = G->rec.i[MB_AT_I_LEN_COUNT] > 1 ? G->rec.i[MB_AT_I_BATCH] : 1;
-                    for (int r = 0; r < count; ++r) lenp[r] = lenp[r] + 1;
-                }
-                if (tid == 0) {
-                    p.ctl->calls = calls + 1;
-                    p.ctl->epoch = *reinterpret_cast<volatile unsigned int*>(&p.ctl->epoch) + 1u;
-                }
-            }
+            grid_barrier(p.ctl, barriers + barrier_index, kBarAll, kThreads, tid, &sc->abort_flag,
+                         &sc->verdict, ph, sc->limit_ns);
+            trace_stamp(ph, 3);
         }
+    }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kAllThreads, 1)
+decode_kernel(const __grid_constant__ KernelParams p) {
+    SharedCtl* sc = ctl_of();
+    const int tid = threadIdx.x;
+    // Both words only change when the last CTA of a launch closes it (or by a host reset).
+    const unsigned int calls = *reinterpret_cast<volatile unsigned int*>(&p.ctl->calls);
+    const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&p.ctl->epoch);
+    if (!begin_launch(p, p.streams, p.maps, epoch * static_cast<unsigned int>(p.n_phases), epoch, calls)) return;
+    const StreamDesc* table = table_of();
+
+    if (threadIdx.x >= kThreads) {
+        if (threadIdx.x == kThreads) producer_loop();
+    } else {
+        consume_launch<DIM>(p, calls);
     }
 
-    // Drain: never leave while one of this CTA's bulk copies is still in flight.  After an
-    // abort the producer stopped issuing; wait (bounded) for every stage it armed.
+    // End of the launch: the CTA that arrives last knows that every CTA has read the valid lengths,
+    // `calls` and `epoch`, and advances them -- unless a fault was recorded anywhere (a token
+    // outside the table ...): then the host has to reset the plan anyway.
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (sc->abort_flag && tid == 0) {
-        const unsigned int issued = sc->issued;
-        const unsigned int first = issued > static_cast<unsigned int>(p.stages)
-                                       ? issued - p.stages : 0u;
-        for (unsigned int s = first; s < issued; ++s) {
-            const int stage = s % p.stages;
-            const unsigned int parity = (s / p.stages) & 1u;
-            for (unsigned int tries = 0; tries < kDrainTryLimit; ++tries)
-                if (mbar_try_wait(&sc->full[stage], parity)) break;
+    if (sc->abort_flag && tid == 0) drain_ring();
+    if (tid == 0) {
+        __threadfence();
+        const unsigned int before = atomicAdd(&p.ctl->arrived, 1u);
+        __threadfence();
+        const bool last = before == gridDim.x - 1;
+        if (last) p.ctl->arrived = 0;
+        sc->verdict = last && sc->abort_flag == 0 && peek_status(p.ctl) == 0 ? 1 : 0;
+    }
+    __syncthreads();
+    if (sc->verdict) {
+        for (int q = tid; q < p.n_phases; q += kAllThreads) {
+            if (table[q].kind != kStreamKv || !(p.entries[q].rec.flags & MB_FLAG_BUMP_LENGTH)) continue;
+            const KvStream& d = table[q].kv;
+            int* lengths = reinterpret_cast<int*>(d.lengths);
+            const int count = d.len_count > 1 ? d.batch : 1;
+            for (int r = 0; r < count; ++r) lengths[r] += 1;
+        }
+        if (tid == 0) {
+            p.ctl->calls = calls + 1;
+            p.ctl->epoch = epoch + 1;
         }
     }
+}
+
+// Shape of a skinny GEMM: a CTA with at most 8 output rows (o and down projections, q|k|v of small
+// models) takes blocks of 8 rows and twice the reduction per stage, so that no half of a stage and
+// of the MMA runs empty; gate and up rows come eight and eight; everything else sixteen at a time.
+void shape_gemv(const mb_phase& P, int ctas, GemvStream* d) {
+    int total = 0;
+    for (int s = 0; s < P.i[MB_GV_I_NSEG]; ++s) total += P.i[MB_GV_I_N0 + s];
+    d->row_bytes = P.i[MB_GV_I_K] * 2;
+    d->n0 = P.i[MB_GV_I_NSEG] > 1 ? P.i[MB_GV_I_N0] : INT_MAX;
+    d->n01 = P.i[MB_GV_I_NSEG] > 2 ? d->n0 + P.i[MB_GV_I_N0 + 1] : INT_MAX;
+    d->r0 = (total / 2) / ctas;
+    d->r1 = (total / 2) % ctas;
+    d->groups = P.i[MB_GV_I_K] / 32;
+    const int rows = 2 * (d->r0 + (d->r1 > 0 ? 1 : 0));  // of the busiest CTA
+    d->shape = P.i[MB_GV_I_NMAT] == 2 ? kShapePaired : (rows <= 8 ? kShapeShort : 0);
+    // the same arithmetic as slice_of
+    const int batch = P.i[MB_GV_I_ROWS], lp = d->shape == kShapeShort ? 2 : 1;
+    const int rs = batch > 2 ? (batch > 4 ? 3 : 2) : batch - 1;
+    if ((d->groups + (8 << lp) - 1) >> (3 + lp) <= (kSliceSlots * 8) >> (lp + rs)) d->shape |= kShapeWhole;
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+bool encode_map(CUtensorMap* map, unsigned long long base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                const cuuint32_t* box, bool swizzled, bool wide) {
+    static EncodeTiledFn fn = [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult result;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &result) != cudaSuccess ||
+            result != cudaDriverEntryPointSuccess)
+            sym = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(sym);
+    }();
+    const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    return fn != nullptr &&
+           fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank), reinterpret_cast<void*>(base),
+              dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              swizzled ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+              wide ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// [rows, K] bf16 row-major as (32 elements, rows, groups of 32 elements); zeros outside.
+bool encode_weight_map(CUtensorMap* map, unsigned long long base, int rows, int K, int box_rows,
+                       int box_groups) {
+    const cuuint64_t dims[3] = {32, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 32)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, 64};
+    const cuuint32_t box[3] = {32, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_groups)};
+    return encode_map(map, base, 3, dims, strides, box, false, true);
+}
+// A cache [batch, capacity, heads, D] as (32 elements, keys, groups of 32 elements, heads, batch); boxes
+// of `keys` rows of one head.
+bool encode_cache_map(CUtensorMap* map, unsigned long long base, const mb_phase& P, int keys, bool swizzled) {
+    const cuuint64_t D = P.i[MB_AT_I_HEAD_DIM], heads = P.i[MB_AT_I_KV_HEADS], capacity = P.i[MB_AT_I_CAPACITY];
+    const cuuint64_t dims[5] = {32, capacity, D / 32, heads, static_cast<cuuint64_t>(P.i[MB_AT_I_BATCH])};
+    const cuuint64_t strides[4] = {heads * D * 2, 64, D * 2, capacity * heads * D * 2};
+    const cuuint32_t box[5] = {32, static_cast<cuuint32_t>(keys), static_cast<cuuint32_t>(D / 32), 1, 1};
+    return encode_map(map, base, 5, dims, strides, box, swizzled, D > 64);
 }
 
 }  // namespace decode
 
-int decode_threads() { return decode::kThreads; }
-int decode_fixed_smem() { return decode::kFixedBytes; }
+int decode_threads() { return decode::kAllThreads; }
+int decode_fixed_smem() { return decode::kCtlBytes; }
 int decode_stage_bytes() { return decode::kStageBytes; }
-int decode_max_stages() { return decode::kMaxStages; }
 int decode_row_pad() { return decode::kRowPad; }
 int decode_row_tile() { return decode::kRowTile; }
 
-cudaError_t decode_configure(int smem_bytes) {
-    return cudaFuncSetAttribute(decode::decode_kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+int decode_rope_bytes(const mb_phase* phases, unsigned int n) {
+    int bytes = 0;
+    for (unsigned int i = 0; i < n; ++i) {
+        if (phases[i].body != MB_BODY_ATTN_DECODE) continue;
+        const int batch = phases[i].i[MB_AT_I_BATCH];
+        const int rows = batch <= decode::kRopeRows ? batch : 1;
+        const int need = rows * (phases[i].i[MB_AT_I_HEAD_DIM] / 2) * 4;
+        if (need > bytes) bytes = need;
+    }
+    return (bytes + 127) / 128 * 128;
 }
 
-cudaError_t decode_occupancy(int smem_bytes, int* blocks_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, decode::decode_kernel,
-                                                         decode::kThreads, smem_bytes);
+// Shared memory of a plan: fixed part, K/V rings, weight ring, stream table, cos / sin table.
+static long long smem_bytes(int rope_bytes, unsigned int n_phases, int stages) {
+    if (n_phases > 1u << 20) return LLONG_MAX;
+    return static_cast<long long>(decode::rope_offset(stages, n_phases)) + rope_bytes;
+}
+// Stages of the weight ring that fit; fewer than two means the plan does not.
+int decode_ring_stages(int rope_bytes, unsigned int n_phases, int limit) {
+    int stages = decode::kMaxStages;
+    while (stages > 0 && smem_bytes(rope_bytes, n_phases, stages) > limit) --stages;
+    return stages;
+}
+int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int stages) {
+    return static_cast<int>(smem_bytes(rope_bytes, n_phases, stages));
 }
 
-cudaError_t decode_launch(const KernelParams& params, int ctas, int smem_bytes,
+// The static part of a phase's stream record; `addr`: its resolved slots.
+void decode_stream(const mb_phase& P, const unsigned long long* addr, int ctas, StreamDesc* out) {
+    std::memset(out, 0, sizeof(*out));
+    if (P.body == MB_BODY_GEMV) {
+        GemvStream& d = out->gemv;
+        d.kind = kStreamGemv;
+        decode::shape_gemv(P, ctas, &d);
+        if (P.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE) d.w_norm = addr[MB_GV_S_NORM_W];
+    } else if (P.body == MB_BODY_ATTN_DECODE) {
+        KvStream& d = out->kv;
+        d.kind = kStreamKv;
+        d.capacity = P.i[MB_AT_I_CAPACITY];
+        d.k = addr[MB_AT_S_KCACHE];
+        d.v = addr[MB_AT_S_VCACHE];
+        d.lengths = addr[MB_AT_S_LEN];
+        d.batch = P.i[MB_AT_I_BATCH];
+        d.kv_heads = P.i[MB_AT_I_KV_HEADS];
+        d.head_dim = P.i[MB_AT_I_HEAD_DIM];
+        d.len_count = P.i[MB_AT_I_LEN_COUNT];
+        // a partial is kept as (value, tag) pairs, twice the floats the record's buffer counts
+        d.chunk_cap = P.i[MB_AT_I_MAX_CHUNKS] / 2 > 1 ? P.i[MB_AT_I_MAX_CHUNKS] / 2 : 1;
+        d.exact_keys = P.i[MB_AT_I_EXACT_KEYS];
+    }
+}
+
+// The tensor maps of a phase.  GEMV: the weight segments (the second one of a paired phase is the paired
+// matrix); attention: keys and values for boxes of 16, 32 and 64 keys, as far as the head size uses them.
+bool decode_encode_maps(const mb_phase& P, const unsigned long long* addr, int ctas, void* out) {
+    CUtensorMap* maps = static_cast<CUtensorMap*>(out);
+    std::memset(maps, 0, decode::kMapsPerPhase * sizeof(CUtensorMap));
+    if (P.body == MB_BODY_ATTN_DECODE) {
+        for (int shift = 0; shift <= decode::kv_most(P.i[MB_AT_I_HEAD_DIM]); ++shift)
+            if (!decode::encode_cache_map(maps + 2 * shift, addr[MB_AT_S_KCACHE], P, 16 << shift, false) ||
+                !decode::encode_cache_map(maps + 2 * shift + 1, addr[MB_AT_S_VCACHE], P, 16 << shift, true))
+                return false;
+        return true;
+    }
+    if (P.body != MB_BODY_GEMV) return true;
+    GemvStream d;
+    decode::shape_gemv(P, ctas, &d);
+    const bool is_short = (d.shape & kShapeShort) != 0, paired = (d.shape & kShapePaired) != 0;
+    const int box_rows = is_short || paired ? 8 : 16, box_groups = is_short ? 32 : 16;
+    for (int s = 0; s < P.i[MB_GV_I_NSEG]; ++s)
+        if (!decode::encode_weight_map(maps + s, addr[MB_GV_S_W0 + s], P.i[MB_GV_I_N0 + s], P.i[MB_GV_I_K],
+                                       box_rows, box_groups))
+            return false;
+    return !paired || decode::encode_weight_map(maps + 1, addr[MB_GV_S_W_PAIR], P.i[MB_GV_I_N0],
+                                                P.i[MB_GV_I_K], box_rows, box_groups);
+}
+size_t decode_map_bytes() { return decode::kMapsPerPhase * sizeof(CUtensorMap); }
+
+namespace {
+const void* kernel_of(int head_dim) {
+    switch (head_dim) {
+        case 64: return reinterpret_cast<const void*>(&decode::decode_kernel<64>);
+        case 128: return reinterpret_cast<const void*>(&decode::decode_kernel<128>);
+        case 256: return reinterpret_cast<const void*>(&decode::decode_kernel<256>);
+        default: return reinterpret_cast<const void*>(&decode::decode_kernel<0>);
+    }
+}
+}  // namespace
+
+// The one head size of a plan's attention phases (64 if it has none), or 0.
+int decode_head_dim(const mb_phase* phases, unsigned int n) {
+    int dim = -1;
+    for (unsigned int i = 0; i < n; ++i) {
+        if (phases[i].body != MB_BODY_ATTN_DECODE) continue;
+        const int d = phases[i].i[MB_AT_I_HEAD_DIM];
+        if (dim >= 0 && d != dim) return 0;
+        dim = d;
+    }
+    return dim < 0 ? 64 : dim;
+}
+
+cudaError_t decode_configure(int head_dim, int smem_bytes) {
+    return cudaFuncSetAttribute(kernel_of(head_dim), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+}
+
+cudaError_t decode_occupancy(int head_dim, int smem_bytes, int* blocks_per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel_of(head_dim), decode::kAllThreads,
+                                                         smem_bytes);
+}
+
+cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, int smem_bytes,
                           cudaStream_t stream) {
     KernelParams copy = params;
     void* args[] = {&copy};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(decode::decode_kernel), dim3(ctas),
-                                       dim3(decode::kThreads), args,
+    return cudaLaunchCooperativeKernel(kernel_of(head_dim), dim3(ctas), dim3(decode::kAllThreads), args,
                                        static_cast<size_t>(smem_bytes), stream);
 }
 
@@ -1903,64 +2048,53 @@ namespace mb {
 namespace decode {
 
 constexpr size_t kStaticScratchBytes = 4u << 20;
-constexpr size_t kStaticControlBytes = 256;        // status words of Control + "CTAs done" counter
-// The attention body only touches Control::status through the pointer it is given (record_status,
-// peek_status); those words must lie inside the first 128 bytes, before the "done" counter.
-static_assert(offsetof(Control, status) + sizeof(int) * 4 <= 128,
-              "the status words must precede the done counter of the static control area");
+constexpr size_t kStaticControlBytes = 256;        // the head of a Control: status and arrivals
+// The attention body and the end of the launch only touch the words before the finished-phase
+// counters through the pointer they are given.
+static_assert(offsetof(Control, finished) <= kStaticControlBytes, "the static control area is too small");
 constexpr size_t kStaticCounterBytes = 4096;       // arrival counters: up to 1024 (row, kv head)
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// Tags the partials of a call; outside the area that is cleared before every call, so that no
+// partial of an earlier call can be mistaken for one of this call.
+static __device__ unsigned int g_static_epoch;
 
-__global__ void __launch_bounds__(kConsumerThreads, 1)
-attention_static_kernel(const __grid_constant__ PhaseEntry entry, Control* ctl, int* done,
+struct alignas(64) StaticMaps {
+    CUtensorMap map[kMapsPerPhase];
+};
+
+__global__ void __launch_bounds__(kAllThreads, 1)
+attention_static_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ PhaseEntry entry,
+                        const __grid_constant__ StreamDesc stream, const __grid_constant__ StaticMaps maps,
                         int* status_out) {
-    extern __shared__ __align__(128) char smem[];
-    SharedCtl* sc = reinterpret_cast<SharedCtl*>(smem);
-    char* scratch = smem + kCtlBytes;
+    SharedCtl* sc = ctl_of();
     const int tid = threadIdx.x;
+    const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&g_static_epoch);
     if (tid < kEntryVectors)
         reinterpret_cast<uint4*>(&sc->entry[0])[tid] = reinterpret_cast<const uint4*>(&entry)[tid];
-    if (tid == 0) {
-        sc->abort_flag = 0;
-        sc->tag_base = 0;
-        sc->calls = 0;
-        sc->limit_ns = kPipeTimeoutNs;
+    if (begin_launch(p, &stream, &maps, epoch, 0u, 0u)) {
+        if (tid < kThreads)
+            run_attention<0>(0, Place{0u, 0u, 0u});
+        else if (tid == kThreads)
+            producer_loop();
+        __syncthreads();
+        if (sc->abort_flag && tid == 0) drain_ring();
     }
-    __syncthreads();
-    KernelParams p;
-    p.entries = nullptr;
-    p.ctl = ctl;
-    p.trace = nullptr;
-    p.n_phases = 1;
-    p.n_dynamic = 0;
-    p.barriers_per_launch = 0;
-    p.stages = 0;
-    p.stage_bytes = 0;
-    p.activation_bytes = 0;
-    p.wait_limit_us = 2000000u;
-    const PhaseEntry* E = &sc->entry[0];
-    const int D = E->rec.i[MB_AT_I_HEAD_DIM];
-    if (D == 64)
-        attention_decode<64>(p, E, 0, sc, scratch, tid);
-    else if (D == 128)
-        attention_decode<128>(p, E, 0, sc, scratch, tid);
-    else
-        attention_decode<256>(p, E, 0, sc, scratch, tid);
     __syncthreads();
     if (tid == 0) {
         // The valid length may only move once every CTA has read it: the last CTA to finish
         // advances it, reports the status and re-arms the counter for the next call.
         __threadfence();
-        const int finished = atomicAdd(done, 1);
-        if (finished == static_cast<int>(gridDim.x) - 1) {
+        const unsigned int before = atomicAdd(&p.ctl->arrived, 1u);
+        if (before == gridDim.x - 1) {
             __threadfence();
-            const int code = *reinterpret_cast<volatile int*>(&ctl->status[0]);
+            const int code = peek_status(p.ctl);
             if (code == 0) {
-                int* lenp = reinterpret_cast<int*>(E->addr[MB_AT_S_LEN]);
+                int* lenp = reinterpret_cast<int*>(entry.addr[MB_AT_S_LEN]);
                 *lenp = *lenp + 1;
             }
             if (status_out != nullptr) *status_out = code;
-            *done = 0;
+            p.ctl->arrived = 0;
+            g_static_epoch = epoch + 1;
         }
     }
 }
@@ -1968,7 +2102,7 @@ attention_static_kernel(const __grid_constant__ PhaseEntry entry, Control* ctl, 
 struct StaticDevice {
     unsigned char* scratch = nullptr;  // device address of g_static_scratch on this device
     int sm_count = 0;
-    int max_smem = 0;
+    int smem_limit = 0;
     bool ready = false;
 };
 
@@ -1978,13 +2112,6 @@ struct StaticDevice {
 namespace {
 mb::decode::StaticDevice g_static_devices[64];
 std::mutex g_static_mutex;
-
-long long static_attention_smem(int head_dim, int group, int merge_slots) {
-    return mb::decode::kCtlBytes + 8LL * (head_dim + 32) * 2 + 2LL * head_dim * 2 + 4LL * head_dim +
-           4LL * (2 * 8 * 8 + mb::decode::kFoldFloats) +
-           4LL * (head_dim + 2) * group * (merge_slots + 2) +
-           (head_dim == 64 ? 8LL * 2 * 16 * ((head_dim * 2 + 64) + (head_dim * 2 + 16)) : 0);
-}
 }  // namespace
 
 // Declared in include/megabake_b200.h.  The first call on a device performs the one-time
@@ -2018,26 +2145,20 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
             cudaDeviceProp prop;
             if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return MB_ERR_CUDA;
             if (prop.major != 10) return MB_ERR_UNSUPPORTED;
-            dev.max_smem = 160 * 1024;
+            if (!prop.cooperativeLaunch) return MB_ERR_UNSUPPORTED;
             if (cudaFuncSetAttribute(attention_static_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     dev.max_smem) != cudaSuccess)
+                                     static_cast<int>(prop.sharedMemPerBlockOptin)) != cudaSuccess)
                 return MB_ERR_CUDA;
             dev.scratch = static_cast<unsigned char*>(address);
             dev.sm_count = prop.multiProcessorCount;
+            dev.smem_limit = static_cast<int>(prop.sharedMemPerBlockOptin);
             dev.ready = true;
         }
     }
 
     const int group = a->heads / a->kv_heads;
     const int pairs = a->batch * a->kv_heads;
-    int merge_slots = 8;
-    while (merge_slots > 1 &&
-           static_attention_smem(a->head_dim, group, merge_slots) - kCtlBytes -
-                   (a->head_dim == 64 ? 8 * 2 * 16 * ((64 * 2 + 64) + (64 * 2 + 16)) : 0) >
-               48 * 1024)
-        merge_slots /= 2;
-    if (static_attention_smem(a->head_dim, group, merge_slots) > dev.max_smem) return MB_ERR_RESOURCE;
     // What fits the fixed array: arrival counters for every (row, kv head) and at least one
     // key chunk of partials each; more chunks if there is room, up to 32.
     if (static_cast<size_t>(pairs) * 4 > kStaticCounterBytes) return MB_ERR_RESOURCE;
@@ -2059,7 +2180,7 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     entry.rec.i[MB_AT_I_CAPACITY] = a->capacity;
     entry.rec.i[MB_AT_I_INVFREQ_BF16] = a->inv_freq_is_bf16 ? 1 : 0;
     entry.rec.i[MB_AT_I_MAX_CHUNKS] = max_chunks;
-    entry.rec.i[MB_AT_I_MERGE_SLOTS] = merge_slots;
+    entry.rec.i[MB_AT_I_MERGE_SLOTS] = 1;
     entry.rec.i[MB_AT_I_EXACT_KEYS] = a->capacity < 128 ? a->capacity : 128;
     entry.rec.i[MB_AT_I_LEN_COUNT] = 1;
     entry.rec.f[MB_AT_F_SCALE] = 1.0f / sqrtf(static_cast<float>(a->head_dim));
@@ -2085,10 +2206,24 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     // have left them set); the partials are always written before they are read
     if (cudaMemsetAsync(control, 0, kStaticControlBytes + kStaticCounterBytes, s) != cudaSuccess)
         return MB_ERR_CUDA;
-    mb::Control* ctl = reinterpret_cast<mb::Control*>(control);
-    int* done = reinterpret_cast<int*>(control + 128);
-    const int smem = static_cast<int>(static_attention_smem(a->head_dim, group, merge_slots));
-    attention_static_kernel<<<dev.sm_count, kConsumerThreads, smem, s>>>(
-        entry, ctl, done, reinterpret_cast<int*>(a->status));
-    return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_CUDA;
+    mb::StreamDesc desc;
+    mb::decode_stream(entry.rec, entry.addr, dev.sm_count, &desc);
+    mb::KernelParams params;
+    std::memset(&params, 0, sizeof(params));
+    params.ctl = reinterpret_cast<mb::Control*>(control);
+    params.n_phases = 1;
+    params.wait_limit_us = 2000000u;
+    int* status_out = reinterpret_cast<int*>(a->status);
+    // the parts of a split context wait for one another's partials: all CTAs have to be resident
+    const int rope_bytes = mb::decode_rope_bytes(&entry.rec, 1);
+    params.stages = mb::decode_ring_stages(rope_bytes, 1, dev.smem_limit);
+    StaticMaps maps;
+    if (params.stages < 2 || !mb::decode_encode_maps(entry.rec, entry.addr, dev.sm_count, &maps)) return MB_ERR_CUDA;
+    void* args[] = {&params, &entry, &desc, &maps, &status_out};
+    const int smem = mb::decode_smem_bytes(rope_bytes, 1, params.stages);
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&attention_static_kernel),
+                                       dim3(dev.sm_count), dim3(kAllThreads), args,
+                                       static_cast<size_t>(smem), s) == cudaSuccess
+               ? MB_OK
+               : MB_ERR_CUDA;
 }

@@ -18,15 +18,18 @@ constexpr int kBarrierLanes = 8;
 struct Control {
     unsigned int epoch;     // base of the hand-off sequence numbers: grows with every completed
                             // launch and every reset, so that no cell of an earlier launch can
-                            // ever be mistaken for one of this launch
+                            // ever be mistaken for one of this launch; its parity picks the half
+                            // of the relay arena a launch works in
     unsigned int calls;     // completed launches; the barrier targets derive from it
     int status[4];          // code, phase, detail, (unused)
-    unsigned int pad0[26];
+    unsigned int arrived;   // CTAs of the running launch that are through; the last one closes it
+    unsigned int pad0[25];
     // CTAs that finished a phase: a ring of four counters (a line each), phase q counts on
     // counter q % 4.  Every CTA, before it leaves phase q, waits until all CTAs have finished
     // phase q - 2; so no CTA is ever more than two phases ahead of another, a counter never
     // mixes arrivals of two phases, and a cell buffer may be overwritten from the third phase
-    // after its last reader on.
+    // after its last reader on.  Plans whose hand-offs all go through the relay arena do not
+    // count (KernelParams::counters).
     struct Finished {
         unsigned int count;
         unsigned int pad[31];
@@ -42,26 +45,77 @@ struct Control {
 
 // One phase as the kernel reads it: the record plus the device address of every slot it
 // names, resolved by the host at bind time so that the kernel never chases a slot index
-// through a second table.  A per-launch (dynamic) slot holds kDynamicTag | ordinal instead.
-struct PhaseEntry {
+// through a second table.  A per-launch (dynamic) slot holds kDynamicTag | ordinal instead, a
+// tensor handed over inside the relay arena kRelayTag | offset.
+struct alignas(16) PhaseEntry {
     mb_phase rec;
     unsigned long long addr[MB_PHASE_SLOTS];
-    unsigned long long pad;  // keeps sizeof a multiple of 16 (copied in 16-byte vectors)
+    unsigned long long modes;  // kMode* bits; also keeps sizeof a multiple of 16
 };
 static_assert(sizeof(PhaseEntry) % 16 == 0, "PhaseEntry must be a whole number of 16-byte vectors");
 constexpr unsigned long long kDynamicTag = 1ull << 63;
+constexpr unsigned long long kRelayTag = 1ull << 62;
+// operands of a phase that live in the relay arena
+constexpr unsigned long long kModeInRelay = 1, kModeResidualRelay = 2, kModeOutRelay = 4,
+                             kModeStoreRelay = 8;
+// Every 32-bit word of the relay arena that has not been written in this launch holds this
+// pattern.  Conversions to bf16 never produce it: a NaN becomes 0x7fff.
+constexpr unsigned int kUnwritten = 0xffffffffu;
+// The arena starts with one hint counter per phase.
+constexpr unsigned int kHintBytes = 128;
+
+// What a warp needs to stream a phase's global operands ahead of time, one record per phase.
+// The host fills the static part; every CTA completes its copy in shared memory at the start of
+// a launch (its rows; the valid lengths and how the keys are dealt over the CTAs).
+enum StreamKind { kStreamNone = 0, kStreamGemv = 1, kStreamKv = 2 };
+struct GemvStream {
+    int kind;
+    int row_bytes;
+    unsigned long long w_norm;  // norm weights, or 0
+    int n0, n01;                // first virtual row of segments 1 and 2
+    int r0, r1;                 // this CTA's output rows (host: the balanced split)
+    int groups;                 // 32-element groups of the reduction
+    int shape;                  // kShape* bits
+    int nblocks;                // blocks of 16 (8) rows of this CTA
+    int pad[13];
+};
+constexpr int kShapeShort = 1;   // blocks of 8 rows, 32 groups per stage; else 16 rows, 16 groups
+constexpr int kShapeWhole = 4;   // the activations of a warp fit its slice of shared memory
+constexpr int kShapePaired = 2;  // 8 gate rows and the 8 up rows, 16 groups per stage
+struct KvStream {
+    int kind;
+    int capacity;
+    unsigned long long k, v, lengths;
+    int batch, kv_heads, head_dim, len_count;
+    int chunk_cap;       // parts one (row, kv head) may be cut into
+    int exact_keys;      // host: limit; device: 1 if this launch rounds like the eager operator
+    int cut_ctas;        // CTAs that share all key blocks evenly; 0: whole (row, kv head) items
+    int total_blocks;    // 16-key blocks over all (row, kv head)
+    int lens[8];
+};
+union StreamDesc {
+    int kind;
+    GemvStream gemv;
+    KvStream kv;
+    uint4 raw[6];
+};
+static_assert(sizeof(GemvStream) == 96 && sizeof(KvStream) == 96 && sizeof(StreamDesc) == 96,
+              "stream records are copied as six 16-byte vectors");
 
 struct KernelParams {
     const PhaseEntry* entries;
+    const StreamDesc* streams;
+    const void* maps;  // CUtensorMap[n_phases][6]
     Control* ctl;
-    unsigned long long* trace;  // optional [ctas][n_phases][4] global-timer stamps, or null
+    unsigned long long* trace;  // optional [ctas][n_phases][8] global-timer stamps, or null
+    unsigned long long relay;        // two halves of relay_bytes each; a launch writes one of
+    unsigned long long relay_bytes;  // them and makes the other one blank for the next launch
     unsigned long long dyn[MB_MAX_DYNAMIC];
     int n_phases;
     int n_dynamic;
     int barriers_per_launch;
-    int stages;            // weight-ring depth
-    int stage_bytes;       // bytes of one ring stage
-    int activation_bytes;  // shared bytes reserved for activations / attention scratch
+    int stages;            // of the weight ring
+    int counters;          // some hand-off of the plan needs the finished-phase counters
     unsigned int wait_limit_us;  // bound of every device-side wait, microseconds
 };
 
@@ -240,6 +294,18 @@ __device__ __forceinline__ unsigned int ld_relaxed_u32(const void* p) {
     return v;
 }
 
+__device__ __forceinline__ uint4 ld_relaxed_u4(const void* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_u32(void* p, unsigned int v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
                  : "memory");
@@ -249,6 +315,10 @@ __device__ __forceinline__ void mbar_init_fence() {
 }
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_count(unsigned long long* bar, unsigned int count) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
+                 : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar,
                                                       unsigned int bytes) {

@@ -8,16 +8,23 @@
 
 namespace mb {
 struct KernelParams;
+union StreamDesc;
 
 int decode_threads();
 int decode_fixed_smem();
 int decode_stage_bytes();
-int decode_max_stages();
 int decode_row_pad();
 int decode_row_tile();
-cudaError_t decode_configure(int smem_bytes);
-cudaError_t decode_occupancy(int smem_bytes, int* blocks_per_sm);
-cudaError_t decode_launch(const KernelParams& params, int ctas, int smem_bytes,
+int decode_rope_bytes(const mb_phase* phases, unsigned int n);
+int decode_ring_stages(int rope_bytes, unsigned int n_phases, int limit);  // < 2: does not fit
+int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int stages);
+size_t decode_map_bytes();  // of the tensor maps of one phase
+bool decode_encode_maps(const mb_phase& phase, const unsigned long long* addresses, int ctas, void* out);
+void decode_stream(const mb_phase& phase, const unsigned long long* addresses, int ctas, StreamDesc* out);
+int decode_head_dim(const mb_phase* phases, unsigned int n);  // of all attention phases; 0: a mix
+cudaError_t decode_configure(int head_dim, int smem_bytes);
+cudaError_t decode_occupancy(int head_dim, int smem_bytes, int* blocks_per_sm);
+cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, int smem_bytes,
                           cudaStream_t stream);
 
 // Prefill plans (mb_prefill.cu): one kernel launch per phase.

@@ -82,12 +82,13 @@ class PlanLayout:
 class PlannerOptions:
     ctas: int = 148  # CTAs the tile split is planned for (one per SM on B200)
     row_tile: int | None = None  # force the GEMV row tile (tuning sweeps)
-    max_chunks: int = 32
+    max_chunks: int = 64
     merge_slots: int | None = None
     exact_keys: int = EXACT_SOFTMAX_KEYS
     stage_bytes: int | None = None  # force the ring stage size (tuning sweeps)
     cell_limit: int = CELL_LIMIT_BYTES  # largest per-CTA copy of an activation kept as cells
     qkv_cells: bool = True  # q, k and v reach the attention items as flagged cells
+    relay: bool = True  # hand-offs through the plan's relay arena (unless cells are asked for)
     distinct_buffers: bool = False  # every layer gets activation buffers of its own (race check:
     #                                 the results must not depend on the buffers being reused)
 
@@ -373,6 +374,7 @@ def _plan_decode(program: DecoderProgram, options: PlannerOptions, stage_bytes: 
     stream = hidden_a  # the buffer that holds the residual stream at the start of a layer
     hidden_cells, attn_cells, glu_cells = as_cells(H), as_cells(q_dim), as_cells(p.intermediate)
     qkv_cells = options.qkv_cells
+    relay = rt.FLAG_RELAY if options.relay and qkv_cells and options.cell_limit == 0 else 0
     for index, layer in enumerate(p.layers):
         tag = f"layers.{index}."
         first = index == 0
@@ -492,6 +494,8 @@ def _plan_decode(program: DecoderProgram, options: PlannerOptions, stage_bytes: 
         out_cells=False,
     )
 
+    for phase in phases[:-1]:  # everything but the logits stays inside the launch
+        phase.flags |= relay
     activation = _align(activation, 128)
     if fixed_bytes + activation + 2 * stage_bytes > max_smem:
         fail("resource-admission",

@@ -26,7 +26,7 @@ MODE_DECODE, MODE_PREFILL = 0, 1
 (BODY_NOP, BODY_GEMV, BODY_ATTN_DECODE, BODY_EMBED_ROWS, BODY_RMSNORM_ROWS, BODY_GEMM_TC,
  BODY_ROPE_ROWS, BODY_ATTN_PREFILL) = range(8)
 
-FLAG_BARRIER, FLAG_BUMP_LENGTH, FLAG_FENCE = 1, 2, 4
+FLAG_BARRIER, FLAG_BUMP_LENGTH, FLAG_FENCE, FLAG_RELAY = 1, 2, 4, 8
 CELLS_X, CELLS_OUT, CELLS_RESIDUAL, CELLS_XSTORE, CELLS_X_WAIT = 1, 2, 4, 8, 16
 PRO_NONE, PRO_RMS_LLAMA, PRO_RMS_GEMMA = 0, 1, 2
 EPI_NONE, EPI_RESIDUAL, EPI_SILU_MUL, EPI_GELU_TANH_MUL = 0, 1, 2, 3
