@@ -202,10 +202,7 @@ int validate_attention(const mb_plan_desc* d, const mb_phase& P) {
 // written again.
 int lower_relays(mb_plan* plan) {
     plan->relays.assign(plan->phases.size(), Relay());
-    bool any = false;
-    for (const mb_phase& P : plan->phases) any = any || (P.flags & MB_FLAG_RELAY) != 0;
-    plan->relay_bytes = any ? static_cast<unsigned long long>(plan->phases.size()) * mb::kHintBytes : 0;
-    plan->relay_bytes = (plan->relay_bytes + 255) / 256 * 256;
+    plan->relay_bytes = 0;
     std::vector<long long> place(plan->slots.size(), -1);  // slot -> arena offset of its live contents
     auto produce = [&](Relay& r, const mb_phase& P, int s, unsigned long long bytes) {
         const int slot = P.slot[s];

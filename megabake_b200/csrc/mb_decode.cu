@@ -49,14 +49,10 @@ constexpr int kRowPad = 64;          // weight rows in units of these; the kerne
 constexpr int kStageBytes = 34816;   // 16 KB whatever they say
 constexpr int kRingStage = 16384;    // 16 groups of 16 rows, 32 groups of 8, or 2 x 16 groups of 8
 constexpr int kMaxStages = 8;
-constexpr int kMapsPerPhase = 6;     // tensor maps: three weights, or keys and values for three boxes
+constexpr int kMapsPerPhase = 3;     // tensor maps: three weights, or keys and values
 // Partial sums: two halves of 256 results (two blocks of 16 rows x 8 tokens; four blocks of 8) from
 // eight slices each.
 constexpr int kScratchBytes = 2 * 4 * kWarps * 512;
-// Keys are cut over CTAs once a (row, kv head) has more than kWholeBlocks 16-key blocks: up to four
-// rounds of the eight warps cost less than meeting through global memory (about 1.5 us), and
-// a part is never shorter than kRunBlocks.
-constexpr int kWholeBlocks = 32, kRunBlocks = 16, kSeamBlocks = 16;
 constexpr int kBarAll = 1;           // named barrier of the consumer warps
 constexpr int kRopeRows = 8;         // batch rows the cos / sin table holds
 constexpr int kEntryVectors = sizeof(PhaseEntry) / 16;
@@ -269,10 +265,10 @@ __device__ __forceinline__ void store_result(char* base, size_t element, unsigne
 }
 
 // ---------------------------------------------------------------------------------------
-// How the key blocks of an attention phase are dealt over the CTAs.  Whole items: CTA c takes
-// (row, kv head) pairs c, c + ctas, ...  Cut: the 16-key blocks of all pairs, in order, are
-// divided into `cut_ctas` runs of equal length (+-1); a CTA's run may end inside a pair, whose
-// parts then meet through the partial buffer.
+// How the key blocks of an attention phase are dealt over the CTAs: every (row, kv head) pair is cut
+// into `chunks` equal parts, and CTA c takes parts c, c + ctas, ... of all of them; the parts of a pair
+// meet through the partial buffer.  The cut also decides, through the maxima a warp has seen, how the
+// probabilities round.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ int row_length(const KvStream& d, int b) {
     if (d.len_count <= 1) return d.lens[0];
@@ -283,71 +279,26 @@ __device__ __forceinline__ int row_length(const KvStream& d, int b) {
 // Writes segment `which` of this CTA to `out`; false if there are fewer.
 __device__ __noinline__ bool locate_segment(int ph, int which, Segment* out, bool writer) {
     const KvStream& d = table_of()[ph].kv;
-    const unsigned int cta = blockIdx.x;
-    const unsigned int runs = static_cast<unsigned int>(d.cut_ctas), total = d.total_blocks;
-    int b, h, length, blk0 = 0, blk1, index = 0, parts = 1;
-    if (runs == 0) {
-        const int pair = static_cast<int>(cta) + which * static_cast<int>(gridDim.x);
+    const int nc = d.chunks;
+    int b, h, chunk, nblocks, parts;
+    for (int item = blockIdx.x;; item += gridDim.x) {
+        const int pair = item / nc;
         if (pair >= d.batch * d.kv_heads) return false;
+        chunk = item - pair * nc;
         b = pair / d.kv_heads;
         h = pair - b * d.kv_heads;
-        length = row_length(d, b);
-        blk1 = (length + 16) >> 4;
-    } else if (d.cut_ctas < 0) {
-        const int length_of_part = -d.cut_ctas;
-        int left = static_cast<int>(cta), nb = 1;
-        if (which > 0) return false;
-        for (b = 0; b < d.batch; ++b) {
-            nb = (row_length(d, b) + 16) >> 4;
-            parts = (nb + length_of_part - 1) / length_of_part;
-            if (left < parts * d.kv_heads) break;
-            left -= parts * d.kv_heads;
-        }
-        if (b == d.batch) return false;
-        h = left / parts;
-        index = left - h * parts;
-        length = row_length(d, b);
-        blk0 = index * nb / parts;
-        blk1 = (index + 1) * nb / parts;
-    } else {
-        if (cta >= runs) return false;
-        unsigned int at = cta * total / runs;
-        const unsigned int end = (cta + 1) * total / runs;
-        for (;;) {
-            // which pair block `at` belongs to, and where that pair starts
-            unsigned int start = 0, nb = 1;
-            for (b = 0; b < d.batch; ++b) {
-                nb = static_cast<unsigned int>((row_length(d, b) + 16) >> 4);
-                const unsigned int row_blocks = nb * static_cast<unsigned int>(d.kv_heads);
-                if (at < start + row_blocks) break;
-                start += row_blocks;
-            }
-            if (at >= end || b >= d.batch) return false;
-            h = static_cast<int>((at - start) / nb);
-            start += h * nb;
-            const unsigned int stop = min(start + nb, end);
-            if (which-- == 0) {
-                length = row_length(d, b);
-                blk0 = static_cast<int>(at - start);
-                blk1 = static_cast<int>(stop - start);
-                // run r holds block g iff r = ((g + 1) * runs - 1) / total, rounded down
-                const unsigned int first = ((start + 1) * runs - 1) / total;
-                const unsigned int last = ((start + nb) * runs - 1) / total;
-                index = static_cast<int>(cta - first);
-                parts = static_cast<int>(last - first) + 1;
-                break;
-            }
-            at = stop;
-        }
+        nblocks = (row_length(d, b) + 16) >> 4;
+        parts = min(nc, nblocks);
+        if (chunk < parts && which-- == 0) break;
     }
     if (writer) {
         out->b = b;
         out->h = h;
         out->pair = b * d.kv_heads + h;
-        out->length = length;
-        out->blk0 = blk0;
-        out->blk1 = blk1;
-        out->index = index;
+        out->length = row_length(d, b);
+        out->blk0 = static_cast<int>(static_cast<unsigned int>(chunk) * nblocks / parts);
+        out->blk1 = static_cast<int>(static_cast<unsigned int>(chunk + 1) * nblocks / parts);
+        out->index = chunk;
         out->parts = parts;
     }
     return true;
@@ -360,12 +311,31 @@ __device__ __forceinline__ bool find_segment(int ph, int which) {
     return found;
 }
 
-// log2 of the 16-key blocks per stage of a segment: enough that one stage per owning warp -- all of them
-// on their way before the phase begins -- holds it, at most 8 KB of keys.
-__host__ __device__ constexpr int kv_most(int head_dim) { return head_dim == 64 ? 2 : (head_dim == 128 ? 1 : 0); }
-__device__ __forceinline__ int kv_shift(int head_dim, int blocks, int owners) {
-    const int want = blocks > 2 * owners ? 2 : (blocks > owners ? 1 : 0);
-    return min(want, kv_most(head_dim));
+// log2 of the 16-key blocks per stage: 8 KB of keys.
+__host__ __device__ constexpr int kv_shift(int head_dim) { return head_dim == 64 ? 2 : (head_dim == 128 ? 1 : 0); }
+
+// Parts per pair (32 lanes): waves of parts over the CTAs times rounds of 16-key blocks over the eight
+// warps, three rounds' worth of prologue and merge, and the fold, which grows with the parts.
+__device__ __forceinline__ int choose_chunks(int pairs, int nblocks, int max_chunks) {
+    int best_cost = INT_MAX, best = 1;
+    for (int nc = (threadIdx.x & 31) + 1; nc <= min(max_chunks, nblocks); nc += 32) {
+        const int waves = (pairs * nc + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+        const int rounds = ((nblocks + nc - 1) / nc + kWarps - 1) / kWarps;
+        const int cost = 4 * waves * (rounds + 3) + nc;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = nc;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int cost = __shfl_xor_sync(0xffffffffu, best_cost, o), nc = __shfl_xor_sync(0xffffffffu, best, o);
+        if (cost < best_cost || (cost == best_cost && nc < best)) {
+            best_cost = cost;
+            best = nc;
+        }
+    }
+    return best;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -456,14 +426,13 @@ __device__ __noinline__ void producer_loop() {
             const int head_dim = table[ph].kv.head_dim;
             Segment& seg = sc->segment[kWarps];
             for (int which = 0; locate_segment(ph, which, &seg, true); ++which) {
-                const int shift = kv_shift(head_dim, seg.blk1 - seg.blk0,
-                                           table[ph].kv.exact_keys ? kWarps : min(kWarps, sc->stages));
-                const unsigned int bytes = 32u * static_cast<unsigned int>(head_dim) << shift;  // of the keys
+                const int shift = kv_shift(head_dim);
+                const unsigned int bytes = 8192;  // of the keys
                 for (int blk = seg.blk0; blk < seg.blk1; blk += 1 << shift) {
                     if (!open_stage(ph, 2 * bytes)) return;
                     const unsigned int dst = ring + static_cast<unsigned int>(stage) * kRingStage;
-                    tma_load_5d(dst, maps + 2 * shift, blk * 16, seg.h, seg.b, &sc->full[stage]);
-                    tma_load_5d(dst + bytes, maps + 2 * shift + 1, blk * 16, seg.h, seg.b, &sc->full[stage]);
+                    tma_load_5d(dst, maps, blk * 16, seg.h, seg.b, &sc->full[stage]);
+                    tma_load_5d(dst + bytes, maps + 1, blk * 16, seg.h, seg.b, &sc->full[stage]);
                     next_stage();
                 }
             }
@@ -993,12 +962,12 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
 
 // ---------------------------------------------------------------------------------------
 // Decode attention.  A CTA works on segments (the key blocks of one (row, kv head) it was dealt),
-// which the producer streams through the weight ring ahead of the phase, `1 << shift` 16-key blocks
-// with their keys and values per stage: the cached rows depend on nothing in the launch.  Stage j of a
-// segment belongs to warp j mod 8 (or the number of stages, if smaller).  Queries (rows = heads of the group) are A and keys are B
+// which the producer streams through the weight ring ahead of the phase, 8 KB of keys and 8 KB of
+// values per stage: the cached rows depend on nothing in the launch.  16-key block j of a segment belongs
+// to warp j mod 8.  Queries (rows = heads of the group) are A and keys are B
 // of the score product, transposed values (ldmatrix) A and the probabilities -- the score fragment as
 // it stands -- B of the value product.  Every warp rotates the queries for itself: element pairs
-// (i, i + D/2) sit in the same lane of two fragments.  The warp that owns the stage with the new key
+// (i, i + D/2) sit in the same lane of two fragments.  The warp that owns the block with the new key
 // rotates that key, appends both rows to the caches and puts them into the stage.
 //
 // Two softmax modes.  The reference normalises the probabilities in fp32 and rounds them to
@@ -1069,7 +1038,8 @@ template <int D, bool EXACT>
 __device__ __noinline__ Place attention_phase(const int ph, Place s) {
     constexpr int DC = D / 32;                       // 32-element groups of the head dimension
     constexpr int DT = D / 16;                       // 16-row tiles of the value product
-    constexpr bool TWO = !EXACT && D < 256;          // two blocks per softmax step
+    constexpr int PS = 1 << kv_shift(D);             // 16-key blocks per stage
+    constexpr unsigned int pitch = 1024u * PS;       // bytes of 32 dimensions of a stage's keys
     constexpr int DR = D < 128 ? D : 128;            // dimensions merged at a time
     constexpr int PR = DR + 4;                       // floats per dumped head: no bank conflicts
     static_assert(kSliceBytes >= 8 * PR * 4, "a dumped state fits the warp's slice");
@@ -1123,11 +1093,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         const int L = seg.length;
         const int b = seg.b, h = seg.h;
         const int blocks = seg.blk1 - seg.blk0;
-        const int owners = EXACT ? kWarps : min(kWarps, static_cast<int>(stages));
-        const int shift = kv_shift(D, blocks, EXACT ? kWarps : owners);
-        const int n = (blocks + (1 << shift) - 1) >> shift;  // stages of the segment
-        const bool has = warp < min(n, owners);
-        const unsigned int pitch = 1024u << shift;  // bytes of 32 dimensions of a stage's keys
+        const bool has = warp < blocks;
         if (!tabled) {
             named_barrier(kBarAll, kThreads);
             fill_rope_row(rope, E, reinterpret_cast<const long long*>(E->addr[MB_AT_S_POS])[b], D / 2,
@@ -1140,7 +1106,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         // round trip for all of them (256-wide heads: one after the other, in as many registers).
         uint4 qf[DC];
         if (has) {
-            const bool holder = seg.blk1 - 1 == (L >> 4) && (n - 1) % owners == warp;
+            const bool holder = seg.blk1 - 1 == (L >> 4) && ((blocks - 1) & (kWarps - 1)) == warp;
             const int elem = kind == kCells ? 4 : 2;
             const char* qrow = reinterpret_cast<const char*>(E->addr[MB_AT_S_Q]) +
                                (static_cast<size_t>(b) * Hq + h * group + min(gid, group - 1)) * D * elem +
@@ -1229,45 +1195,23 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         for (int t = 0; t < DT; ++t)
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[t][q] = 0.f;
-        // Stage j belongs to warp j mod `owners`: a warp always waits for uses of one slot, in order (a
-        // parity says nothing about a use before the last one).  Exact mode, where eight blocks may
-        // meet a shorter ring: all warps go through all stages.
         unsigned int slot = s.stage, parity = s.parity;
-        auto advance = [&](unsigned int by) {
-            slot += by;
-            if (slot >= stages) {
-                slot -= stages;
-                parity ^= 1u;
+        // The new row in its place and zeros after its value (0 * stale bits may be NaN), if block `q` of
+        // the stage is the one.
+        auto patch = [&](unsigned int base, int q, int first_key) {
+            const int r0 = L - first_key;
+            if (r0 >= 16) return;
+            constexpr int C = D / 8;  // 16-byte pieces of a row
+            const unsigned int keys = base + q * 1024u, values = keys + DC * pitch;
+            for (int p = lane; p < 2 * C + (15 - r0) * C; p += 32) {
+                const int r = p < 2 * C ? r0 : r0 + 1 + (p - 2 * C) / C, c = p & (C - 1);
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (p < 2 * C) v = *reinterpret_cast<const uint4*>(&sc->new_row[p < C ? 0 : 1][8 * c]);
+                const unsigned int at = (c >> 2) * pitch + static_cast<unsigned int>(r) * 64u;
+                sts128(p < C ? keys + at + (c & 3) * 16 : values + at + (((c & 3) ^ ((r >> 1) & 3)) << 4), v);
             }
-        };
-        if (!EXACT) advance(has ? static_cast<unsigned int>(warp) : 0u);
-
-        // The current stage, with the new row in its place and zeros after its value (0 * stale bits
-        // may be NaN) if it is the one.
-        auto open_stage = [&](int first_key, int keys) {
-            ring_wait(slot, parity);
-            const unsigned int base = ring + slot * kRingStage;
-            const int row = L - first_key;
-            if (row >= 0 && row < keys) {
-                constexpr int C = D / 8;  // 16-byte pieces of a row
-                const unsigned int values = base + DC * pitch;
-                const int zero = (15 - (row & 15)) * C;
-                for (int p = lane; p < 2 * C + zero; p += 32) {
-                    const int r = p < 2 * C ? row : row + 1 + (p - 2 * C) / C, c = p & (C - 1);
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (p < 2 * C) v = *reinterpret_cast<const uint4*>(&sc->new_row[p < C ? 0 : 1][8 * c]);
-                    const unsigned int at = (c >> 2) * pitch + static_cast<unsigned int>(r) * 64u;
-                    sts128(p < C ? base + at + (c & 3) * 16 : values + at + (((c & 3) ^ ((r >> 1) & 3)) << 4), v);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-            }
-            return base;
-        };
-        auto close_stage = [&](unsigned int by) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive_count(&sc->empty[slot], EXACT ? 1u : kWarps);
-            advance(by);
         };
         // scores of block `q` of a stage: sv[2j + e] <-> head gid, key 8j + 2tq + e; bf16-rounded
         // product, scale applied in fp32, keys past the valid length masked
@@ -1291,7 +1235,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const float v = bf16_round(frag[j][e] + frag2[j][e]) * scale;
-                    sv[2 * j + e] = first_key + 16 * q + 8 * j + 2 * tq + e <= L ? v : -INFINITY;
+                    sv[2 * j + e] = first_key + 8 * j + 2 * tq + e <= L ? v : -INFINITY;
                 }
         };
         // Lane's address for the value fragments of block 0: matrices (keys 0-7, dims 0-7), (keys
@@ -1315,25 +1259,64 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             }
         };
 
-        if (EXACT) {
-            // one block per warp at most; warps without a block still join the two exchanges.  The
-            // value fragments leave the ring before them, so that a ring shorter than the segment
-            // cannot stall the producer against the barrier.
-            float sv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            unsigned int vf[DT][4];
+        float sv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        unsigned int vf[EXACT ? DT : 1][4];
+        // Block j of the segment is warp j mod 8's, and every warp goes through every stage: the one
+        // parity bit of a wait only tells the last two uses of a slot apart.
 #pragma unroll 1
-            for (int j = 0; j < n; ++j) {
-                const unsigned int base = open_stage(j * 16, j == warp ? 16 : 0);
-                if (j == warp) {
-                    block_scores(base, 0, j * 16, sv);
+        for (int j = 0; j < blocks; j += PS) {
+            ring_wait(slot, parity);
+            const int q = (warp - j) & (kWarps - 1);
+            if (q < PS && j + q < blocks) {
+                const unsigned int base = ring + slot * kRingStage;
+                const int first_key = (seg.blk0 + j + q) * 16;
+                patch(base, q, first_key);
+                block_scores(base, q, first_key, sv);
+                if (EXACT) {
+                    // One block per warp at most.  The value fragments leave the ring before the
+                    // warps meet, so that a ring shorter than the segment cannot stall the producer.
 #pragma unroll
                     for (int i = 0; i < DC; ++i) {
-                        ldmatrix_x4_trans(vf[2 * i], base + i * pitch + v_even);
-                        ldmatrix_x4_trans(vf[2 * i + 1], base + i * pitch + v_odd);
+                        ldmatrix_x4_trans(vf[EXACT ? 2 * i : 0], base + q * 1024u + i * pitch + v_even);
+                        ldmatrix_x4_trans(vf[EXACT ? 2 * i + 1 : 0], base + q * 1024u + i * pitch + v_odd);
                     }
+                } else {
+                    float bmax = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
+                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
+                    if (__any_sync(0xffffffffu, bmax > m_run)) {  // a new maximum: rare after the first blocks
+                        const float m_new = fmaxf(m_run, bmax);
+                        const float alpha = expf(m_run - m_new);
+                        l_run *= alpha;
+                        m_run = m_new;
+                        // rescale factors of the two heads this lane accumulates (columns 2tq, 2tq+1)
+                        const float alpha0 = __shfl_sync(0xffffffffu, alpha, (2 * tq) * 4);
+                        const float alpha1 = __shfl_sync(0xffffffffu, alpha, (2 * tq + 1) * 4);
+#pragma unroll
+                        for (int t = 0; t < DT; ++t) {
+                            acc[t][0] *= alpha0;
+                            acc[t][1] *= alpha1;
+                            acc[t][2] *= alpha0;
+                            acc[t][3] *= alpha1;
+                        }
+                    }
+                    float pv[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) pv[e] = expf(sv[e] - m_run);
+                    l_run += (pv[0] + pv[1]) + (pv[2] + pv[3]);
+                    block_values(base, q, pack_bf16(pv[0], pv[1]), pack_bf16(pv[2], pv[3]));
                 }
-                close_stage(1);
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sc->empty[slot]);
+            if (++slot == stages) {
+                slot = 0;
+                parity ^= 1u;
+            }
+        }
+        s.stage = slot;
+        s.parity = parity;
+        if (EXACT) {
             float rmax = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
             rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
             rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
@@ -1362,63 +1345,9 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             // already normalised: merge as plain sums (max 0, total weight 1)
             m_run = 0.f;
             l_run = (warp == 0 && tq == 0) ? 1.f : 0.f;
-        } else {
-#pragma unroll 1
-            for (int j = has ? warp : n; j < n; j += owners) {
-                const int first_key = (seg.blk0 + (j << shift)) * 16;
-                const int here = min(1 << shift, blocks - (j << shift));  // blocks
-                const unsigned int base = open_stage(first_key, here * 16);
-#pragma unroll 1
-                for (int q = 0; q < here; q += TWO ? 2 : 1) {
-                    const bool two = TWO && q + 1 < here;
-                    float sv[2][4];
-                    block_scores(base, q, first_key, sv[0]);
-                    if (two)
-                        block_scores(base, q + 1, first_key, sv[1]);
-                    else
-                        sv[1][0] = sv[1][1] = sv[1][2] = sv[1][3] = -INFINITY;
-                    float bmax = fmaxf(fmaxf(fmaxf(sv[0][0], sv[0][1]), fmaxf(sv[0][2], sv[0][3])),
-                                       fmaxf(fmaxf(sv[1][0], sv[1][1]), fmaxf(sv[1][2], sv[1][3])));
-                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
-                    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
-                    if (__any_sync(0xffffffffu, bmax > m_run)) {  // a new maximum: rare after the first blocks
-                        const float m_new = fmaxf(m_run, bmax);
-                        const float alpha = expf(m_run - m_new);
-                        l_run *= alpha;
-                        m_run = m_new;
-                        // rescale factors of the two heads this lane accumulates (columns 2tq, 2tq+1)
-                        const float alpha0 = __shfl_sync(0xffffffffu, alpha, (2 * tq) * 4);
-                        const float alpha1 = __shfl_sync(0xffffffffu, alpha, (2 * tq + 1) * 4);
-#pragma unroll
-                        for (int t = 0; t < DT; ++t) {
-                            acc[t][0] *= alpha0;
-                            acc[t][1] *= alpha1;
-                            acc[t][2] *= alpha0;
-                            acc[t][3] *= alpha1;
-                        }
-                    }
-                    float pv[2][4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        pv[0][e] = expf(sv[0][e] - m_run);
-                        pv[1][e] = TWO ? expf(sv[1][e] - m_run) : 0.f;
-                    }
-                    l_run += ((pv[0][0] + pv[0][1]) + (pv[0][2] + pv[0][3])) +
-                             ((pv[1][0] + pv[1][1]) + (pv[1][2] + pv[1][3]));
-                    block_values(base, q, pack_bf16(pv[0][0], pv[0][1]), pack_bf16(pv[0][2], pv[0][3]));
-                    if (two)
-                        block_values(base, q + 1, pack_bf16(pv[1][0], pv[1][1]), pack_bf16(pv[1][2], pv[1][3]));
-                }
-                close_stage(owners);
-            }
         }
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-        {
-            const unsigned int next = s.stage + static_cast<unsigned int>(n);
-            s.parity ^= (next / stages) & 1u;
-            s.stage = next % stages;
-        }
         trace_stamp(ph, 5);
 
         // ---- merge the warp states: dumped DR dimensions at a time, added up in warp order
@@ -1560,7 +1489,7 @@ __device__ __forceinline__ bool complete_stream(StreamDesc* desc, int* bad) {
     d.lengths = resolve_address(d.lengths);
     const int* lengths = reinterpret_cast<const int*>(d.lengths);
     const int count = d.len_count > 1 ? d.batch : 1;
-    int longest = 0, blocks = 0;
+    int longest = 0;
     bool fits = true;
     for (int r = 0; r < count; ++r) {
         const int L = *reinterpret_cast<const volatile int*>(lengths + r);
@@ -1570,40 +1499,11 @@ __device__ __forceinline__ bool complete_stream(StreamDesc* desc, int* bad) {
         }
         if (r < 8) d.lens[r] = L;
         longest = max(longest, L);
-        blocks += (L + 16) >> 4;
     }
     if (!fits) return false;
-    if (count == 1) blocks *= d.batch;
-    blocks *= d.kv_heads;
     d.exact_keys = longest + 1 <= d.exact_keys ? 1 : 0;
-    d.total_blocks = blocks;
-    d.cut_ctas = 0;
-    const int longest_blocks = (longest + 16) >> 4;
-    if (!d.exact_keys && d.chunk_cap > 1 && longest_blocks > kWholeBlocks) {
-        // parts of a pair: at most nb * runs / total + 2 of them by rounding
-        const int by_cap = static_cast<int>(static_cast<long long>(d.chunk_cap - 1) * blocks / longest_blocks);
-        d.cut_ctas = max(1, min(min(static_cast<int>(gridDim.x), blocks / kRunBlocks), by_cap - 1));
-        if (d.cut_ctas < 2) {
-            d.cut_ctas = 0;
-            return true;
-        }
-        // Parts of one pair per CTA wherever they are not much longer than the even runs: a CTA
-        // with the end of one pair and the start of the next goes through everything but the keys
-        // twice, which takes as long as about kSeamBlocks of them.
-        const int even = (blocks + d.cut_ctas - 1) / d.cut_ctas;
-        for (int t = max(max(even, kRunBlocks), (longest_blocks + d.chunk_cap - 1) / d.chunk_cap);
-             t <= even + kSeamBlocks; ++t) {
-            int ctas = 0;
-            for (int r = 0; r < count; ++r) {
-                const int L = r < 8 ? d.lens[r] : *reinterpret_cast<const volatile int*>(lengths + r);
-                ctas += (((L + 16) >> 4) + t - 1) / t;
-            }
-            if (ctas * (count == 1 ? d.batch : 1) * d.kv_heads <= static_cast<int>(gridDim.x)) {
-                d.cut_ctas = -t;
-                break;
-            }
-        }
-    }
+    d.longest = longest;
+    d.chunks = 1;
     return true;
 }
 
@@ -1668,6 +1568,13 @@ __device__ __forceinline__ bool begin_launch(const KernelParams& p, const Stream
             record_status(p.ctl, MB_ST_KV_OVERFLOW, ph, bad);
             sc->abort_flag = 1;
         }
+    }
+    __syncthreads();
+    for (int ph = tid >> 5; ph < p.n_phases; ph += kAllThreads / 32) {
+        if (table[ph].kind != kStreamKv || table[ph].kv.exact_keys) continue;
+        KvStream& d = table[ph].kv;
+        const int chunks = choose_chunks(d.batch * d.kv_heads, (d.longest + 16) >> 4, d.chunk_cap);
+        if ((tid & 31) == 0) d.chunks = chunks;
     }
     __syncthreads();
     return sc->abort_flag == 0;
@@ -1956,15 +1863,15 @@ void decode_stream(const mb_phase& P, const unsigned long long* addr, int ctas, 
 }
 
 // The tensor maps of a phase.  GEMV: the weight segments (the second one of a paired phase is the paired
-// matrix); attention: keys and values for boxes of 16, 32 and 64 keys, as far as the head size uses them.
+// matrix); attention: keys and values.
 bool decode_encode_maps(const mb_phase& P, const unsigned long long* addr, int ctas, void* out) {
     CUtensorMap* maps = static_cast<CUtensorMap*>(out);
     std::memset(maps, 0, decode::kMapsPerPhase * sizeof(CUtensorMap));
     if (P.body == MB_BODY_ATTN_DECODE) {
-        for (int shift = 0; shift <= decode::kv_most(P.i[MB_AT_I_HEAD_DIM]); ++shift)
-            if (!decode::encode_cache_map(maps + 2 * shift, addr[MB_AT_S_KCACHE], P, 16 << shift, false) ||
-                !decode::encode_cache_map(maps + 2 * shift + 1, addr[MB_AT_S_VCACHE], P, 16 << shift, true))
-                return false;
+        const int keys = 16 << decode::kv_shift(P.i[MB_AT_I_HEAD_DIM]);
+        if (!decode::encode_cache_map(maps, addr[MB_AT_S_KCACHE], P, keys, false) ||
+            !decode::encode_cache_map(maps + 1, addr[MB_AT_S_VCACHE], P, keys, true))
+            return false;
         return true;
     }
     if (P.body != MB_BODY_GEMV) return true;

@@ -61,8 +61,6 @@ constexpr unsigned long long kModeInRelay = 1, kModeResidualRelay = 2, kModeOutR
 // Every 32-bit word of the relay arena that has not been written in this launch holds this
 // pattern.  Conversions to bf16 never produce it: a NaN becomes 0x7fff.
 constexpr unsigned int kUnwritten = 0xffffffffu;
-// The arena starts with one hint counter per phase.
-constexpr unsigned int kHintBytes = 128;
 
 // What a warp needs to stream a phase's global operands ahead of time, one record per phase.
 // The host fills the static part; every CTA completes its copy in shared memory at the start of
@@ -89,8 +87,8 @@ struct KvStream {
     int batch, kv_heads, head_dim, len_count;
     int chunk_cap;       // parts one (row, kv head) may be cut into
     int exact_keys;      // host: limit; device: 1 if this launch rounds like the eager operator
-    int cut_ctas;        // CTAs that share all key blocks evenly; 0: whole (row, kv head) items
-    int total_blocks;    // 16-key blocks over all (row, kv head)
+    int chunks;          // parts every (row, kv head) is cut into in this launch
+    int longest;         // valid length of the longest row
     int lens[8];
 };
 union StreamDesc {
@@ -105,7 +103,7 @@ static_assert(sizeof(GemvStream) == 96 && sizeof(KvStream) == 96 && sizeof(Strea
 struct KernelParams {
     const PhaseEntry* entries;
     const StreamDesc* streams;
-    const void* maps;  // CUtensorMap[n_phases][6]
+    const void* maps;  // CUtensorMap[n_phases][3]
     Control* ctl;
     unsigned long long* trace;  // optional [ctas][n_phases][8] global-timer stamps, or null
     unsigned long long relay;        // two halves of relay_bytes each; a launch writes one of
@@ -315,10 +313,6 @@ __device__ __forceinline__ void mbar_init_fence() {
 }
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_count(unsigned long long* bar, unsigned int count) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-                 : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar,
                                                       unsigned int bytes) {
