@@ -151,9 +151,13 @@ __global__ void __launch_bounds__(256) rmsnorm_block_kernel(const unsigned short
     }
 }
 
-// One thread per (row, i): the cos / sin pair of that position and frequency is computed once
-// and applied to element pair (i, i + D/2) of every q and k head of the row, with the rounding
-// points of the eager graph: tables in bf16, every product and the sum rounded to bf16.
+// One thread per (row, group of heads, i): the cos / sin pair of that position and frequency is computed
+// once and applied to element pair (i, i + D/2) of its q and k heads, with the rounding points of the
+// eager graph: tables in bf16, every product and the sum rounded to bf16.  Latency bounds it on
+// short prompts: four heads are loaded before the first is stored, and the groups of four are
+// threads of their own as long as there are few rows (one thread per (row, i) that went through the
+// heads one by one waited for memory once per head).
+constexpr int kRopeHeads = 4;
 struct RopeArgs {
     unsigned short* q;
     unsigned short* k;
@@ -164,6 +168,7 @@ struct RopeArgs {
     int k_tokens, k_capacity;
     int* length;
     int length_value, length_count;
+    int quads;  // threads that share the heads of a (row, i)
 };
 
 // block / blocks: this CTA's index among the CTAs that share the work
@@ -175,15 +180,19 @@ __device__ __forceinline__ void rope_rows_body(const RopeArgs& a, int block, int
     const int rows = a.rows, heads = a.heads, kv_heads = a.kv_heads, D = a.D;
     const int invfreq_bf16 = a.invfreq_bf16, k_tokens = a.k_tokens, k_capacity = a.k_capacity;
     const float rope_scale = a.rope_scale, q_scale = a.q_scale;
-    const int half = D / 2;
-    const long long total = static_cast<long long>(rows) * half;
+    const int half = D / 2, quads = a.quads;
+    const long long total = static_cast<long long>(rows) * quads * half;
     // state handoff: the layer's valid length(s), one shared by the batch or one per row
     if (a.length != nullptr && block == 0 && static_cast<int>(threadIdx.x) < a.length_count)
         a.length[threadIdx.x] = a.length_value;
     for (long long e = block * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
          e += static_cast<long long>(blocks) * blockDim.x) {
-        const int r = static_cast<int>(e / half);
-        const int i = static_cast<int>(e - static_cast<long long>(r) * half);
+        const unsigned int rest = static_cast<unsigned int>(e / half);
+        const int i = static_cast<int>(e - static_cast<long long>(rest) * half);
+        const int r = static_cast<int>(rest / quads), group = static_cast<int>(rest - r * quads);
+        // k rows may live in a KV cache: batch b's rows start at b * capacity
+        const size_t k_row = k_tokens > 0 ? static_cast<size_t>(r / k_tokens) * k_capacity + r % k_tokens
+                                          : static_cast<size_t>(r);
         const float f = invfreq_bf16
                             ? bf16_bits_to_float(reinterpret_cast<const unsigned short*>(inv_freq)[i])
                             : reinterpret_cast<const float*>(inv_freq)[i];
@@ -191,22 +200,30 @@ __device__ __forceinline__ void rope_rows_body(const RopeArgs& a, int block, int
         float sn, cn;
         sincosf(angle, &sn, &cn);
         const float c = bf16_round(cn * rope_scale), s = bf16_round(sn * rope_scale);
-        for (int head = 0; head < heads + kv_heads; ++head) {
-            const bool is_q = head < heads;
-            // k rows may live in a KV cache: batch b's rows start at b * capacity
-            const size_t k_row = k_tokens > 0 ? static_cast<size_t>(r / k_tokens) * k_capacity + r % k_tokens
-                                              : static_cast<size_t>(r);
-            unsigned short* row = is_q ? q + (static_cast<size_t>(r) * heads + head) * D
-                                       : k + (k_row * kv_heads + (head - heads)) * D;
-            const float x1 = bf16_bits_to_float(row[i]), x2 = bf16_bits_to_float(row[i + half]);
-            float r1 = bf16_round(bf16_round(x1 * c) + bf16_round(-x2 * s));
-            float r2 = bf16_round(bf16_round(x2 * c) + bf16_round(x1 * s));
-            if (is_q && q_scale != 0.f && q_scale != 1.f) {
-                r1 = bf16_round(r1 * q_scale);
-                r2 = bf16_round(r2 * q_scale);
+        for (int head0 = group * kRopeHeads; head0 < heads + kv_heads; head0 += quads * kRopeHeads) {
+            unsigned short* row[kRopeHeads];
+            float x1[kRopeHeads], x2[kRopeHeads];
+#pragma unroll
+            for (int n = 0; n < kRopeHeads; ++n) {
+                const int head = min(head0 + n, heads + kv_heads - 1);
+                row[n] = (head < heads ? q + (static_cast<size_t>(r) * heads + head) * D
+                                       : k + (k_row * kv_heads + (head - heads)) * D) + i;
+                x1[n] = bf16_bits_to_float(row[n][0]);
+                x2[n] = bf16_bits_to_float(row[n][half]);
             }
-            row[i] = float_to_bf16_bits(r1);
-            row[i + half] = float_to_bf16_bits(r2);
+#pragma unroll
+            for (int n = 0; n < kRopeHeads; ++n) {
+                const int head = head0 + n;
+                if (head >= heads + kv_heads) break;
+                float r1 = bf16_round(bf16_round(x1[n] * c) + bf16_round(-x2[n] * s));
+                float r2 = bf16_round(bf16_round(x2[n] * c) + bf16_round(x1[n] * s));
+                if (head < heads && q_scale != 0.f && q_scale != 1.f) {
+                    r1 = bf16_round(r1 * q_scale);
+                    r2 = bf16_round(r2 * q_scale);
+                }
+                row[n][0] = float_to_bf16_bits(r1);
+                row[n][half] = float_to_bf16_bits(r2);
+            }
         }
     }
 }
@@ -456,7 +473,21 @@ gemm_tc_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
     tc_fence_after();
     const unsigned int tmem_base = *tmem_slot;
     chain_release();
-    chain_wait();  // nothing above reads or writes global memory
+    // The weights are nobody's output: the first ring of them is on its way while the kernel before
+    // this one drains.
+    auto load_weights = [&](unsigned char* stage, int kx, unsigned long long* bar) {
+        mbar_arrive_expect_tx(bar, kStage);
+        if (a.pair) {
+            tma_load_2d(stage + kStageA, &maps.w[0], kx, n0, bar);
+            tma_load_2d(stage + kStageA + kHalf * kTileK * 2, &maps.w[3], kx, n0, bar);
+        } else {
+            tma_load_2d(stage + kStageA, &maps.w[seg], kx, n0, bar);
+        }
+    };
+    const int ahead = min(nkb, a.stages);
+    if (threadIdx.x == 0)
+        for (int it = 0; it < ahead; ++it) load_weights(smem + it * kStage, (kb0 + it) * kTileK, &full[it]);
+    chain_wait();  // nothing above reads or writes what another kernel writes or reads
     if (threadIdx.x == 0) stamp(1);
 
     if (warp == 0) {
@@ -470,15 +501,9 @@ gemm_tc_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
                     break;
                 }
                 unsigned char* stage = smem + s * kStage;
-                mbar_arrive_expect_tx(&full[s], kStage);
                 const int kx = (kb0 + it) * kTileK;
+                if (it >= ahead) load_weights(stage, kx, &full[s]);
                 tma_load_2d(stage, &maps.a, kx, m0, &full[s]);
-                if (a.pair) {
-                    tma_load_2d(stage + kStageA, &maps.w[0], kx, n0, &full[s]);
-                    tma_load_2d(stage + kStageA + kHalf * kTileK * 2, &maps.w[3], kx, n0, &full[s]);
-                } else {
-                    tma_load_2d(stage + kStageA, &maps.w[seg], kx, n0, &full[s]);
-                }
             }
         }
         __syncwarp();
@@ -715,7 +740,146 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmArgs& a, int seg, int
     }
 }
 
+// Where row `row` of segment `seg` starts.
+__device__ __forceinline__ size_t gemm_row_start(const GemmArgs& a, int seg, int row) {
+    const size_t out_row = (seg >= 1 && a.out_tokens > 0)
+                               ? static_cast<size_t>(row / a.out_tokens) * a.out_capacity + row % a.out_tokens
+                               : static_cast<size_t>(row);
+    return out_row * a.n[seg];
+}
+// Columns at a ragged edge, one by one.
+__device__ __noinline__ void gemm_store_one(const GemmArgs& a, int seg, size_t at, int col, float v, float u) {
+    const unsigned short* bias = a.bias[seg];
+    float y = bf16_round(v + (bias != nullptr ? bf16_bits_to_float(__ldg(bias + col)) : 0.f));
+    if (a.epilogue == MB_EPI_SILU_MUL) y = bf16_round(silu_f32(y)) * bf16_round(u);
+    if (a.epilogue == MB_EPI_GELU_TANH_MUL) y = bf16_round(gelu_tanh_f32(y)) * bf16_round(u);
+    if (a.epilogue == MB_EPI_RESIDUAL) y = bf16_bits_to_float(a.residual[at]) + bf16_round(y);
+    a.out[seg][at] = float_to_bf16_bits(y);
+}
+// Eight columns of an output row from the summed accumulators: the arithmetic of gemm_store_chunk.  (What
+// the epilogue is, is asked once and not per column: the columns' chains have to overlap.)
+__device__ __forceinline__ void gemm_store_eight(const GemmArgs& a, int seg, int row, int col0,
+                                                 const float (&v)[8], const float (&u)[8]) {
+    const int n = a.n[seg];
+    const size_t at = gemm_row_start(a, seg, row) + col0;
+    if (col0 + 8 > n || (n & 7) != 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (col0 + i < n) gemm_store_one(a, seg, at + i, col0 + i, v[i], u[i]);
+        return;
+    }
+    uint4 h = make_uint4(0u, 0u, 0u, 0u), bias = h;
+    if (a.epilogue == MB_EPI_RESIDUAL) h = *reinterpret_cast<const uint4*>(a.residual + at);
+    const unsigned short* b = a.bias[seg];
+    if (b != nullptr) {
+        if ((reinterpret_cast<unsigned long long>(b) & 15ull) == 0) {
+            bias = __ldg(reinterpret_cast<const uint4*>(b + col0));
+        } else {
+            unsigned int w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                w[i] = __ldg(b + col0 + 2 * i) | (static_cast<unsigned int>(__ldg(b + col0 + 2 * i + 1)) << 16);
+            bias = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    const unsigned int bw[4] = {bias.x, bias.y, bias.z, bias.w}, hw[4] = {h.x, h.y, h.z, h.w};
+    float y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = bf16_round(v[i] + (i & 1 ? hi_bf16(bw[i / 2]) : lo_bf16(bw[i / 2])));
+    if (a.epilogue == MB_EPI_SILU_MUL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = bf16_round(silu_f32(y[i])) * bf16_round(u[i]);
+    } else if (a.epilogue == MB_EPI_GELU_TANH_MUL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = bf16_round(gelu_tanh_f32(y[i])) * bf16_round(u[i]);
+    } else if (a.epilogue == MB_EPI_RESIDUAL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = (i & 1 ? hi_bf16(hw[i / 2]) : lo_bf16(hw[i / 2])) + y[i];
+    }
+    *reinterpret_cast<uint4*>(a.out[seg] + at) =
+        make_uint4(pack_bf16_pair(y[0], y[1]), pack_bf16_pair(y[2], y[3]), pack_bf16_pair(y[4], y[5]),
+                   pack_bf16_pair(y[6], y[7]));
+}
+
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same shared-memory address in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned int cluster_address(unsigned int addr, int rank) {
+    unsigned int remote;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ float4 load_cluster(unsigned int addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
+// Clustered slices (kernel below): with few output tiles the reduction of a tile is shared by the CTAs
+// of one cluster, whose partial sums meet in distributed shared memory: every CTA adds up its share of
+// the rows, in slice order, and writes it.  (Through global memory the last slice to arrive went over
+// all of them alone.)  Latency bounds it: a thread asks for all slices of its eight columns at
+// once, neighbouring threads neighbouring columns (remote lines are fetched whole); rows are padded by
+// 16 bytes, so that eight of them being written touch all banks.
+constexpr int kMaxCluster = 8;
 template <int BN>
+__device__ __forceinline__ void gemm_cluster_fold(const GemmArgs& a, unsigned int parts, int seg, int n0, int m0,
+                                                  int z) {
+    constexpr int kHalf = BN / 2, kPitch = BN + 4;
+    const int groups = (a.pair ? kHalf : BN) / 8;
+    const int t = static_cast<int>(threadIdx.x) - 64;
+    if (t < 0) return;
+    const int rows = min(kTileM, a.M - m0);
+    const int first = z * rows / a.split_k, share = (z + 1) * rows / a.split_k - first;
+#pragma unroll 1
+    for (int item = t; item < share * groups; item += 256) {
+        const int g = item % groups, row = first + item / groups;
+        if (n0 + 8 * g >= a.n[seg]) continue;
+        float v[8], u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = u[i] = 0.f;
+#pragma unroll 1
+        for (int half = 0; half < (a.pair ? 2 : 1); ++half) {
+            const unsigned int at = parts + (row * kPitch + half * kHalf + 8 * g) * 4;
+            float4 lo[kMaxCluster], hi[kMaxCluster];
+#pragma unroll
+            for (int sl = 0; sl < kMaxCluster; ++sl) {
+                const unsigned int p = cluster_address(at, min(sl, a.split_k - 1));
+                lo[sl] = load_cluster(p);
+                hi[sl] = load_cluster(p + 16);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                u[i] = v[i];
+                v[i] = 0.f;
+            }
+#pragma unroll
+            for (int sl = 0; sl < kMaxCluster; ++sl) {
+                if (sl >= a.split_k) break;
+                v[0] += lo[sl].x;
+                v[1] += lo[sl].y;
+                v[2] += lo[sl].z;
+                v[3] += lo[sl].w;
+                v[4] += hi[sl].x;
+                v[5] += hi[sl].y;
+                v[6] += hi[sl].z;
+                v[7] += hi[sl].w;
+            }
+        }
+        if (a.pair)  // first half: gate, second: up
+            gemm_store_eight(a, seg, m0 + row, n0 + 8 * g, u, v);
+        else
+            gemm_store_eight(a, seg, m0 + row, n0 + 8 * g, v, u);
+    }
+}
+
+// CLUSTERED is a kernel of its own: the fold's code and registers cost the others up to a third.
+template <int BN, bool CLUSTERED>
 __global__ void __launch_bounds__(kPersistThreads, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a) {
     constexpr int kStageW = BN * kTileK * 2;
@@ -766,7 +930,28 @@ gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs 
     tc_fence_after();
     const unsigned int tmem_base = *tmem_slot;
     chain_release();
-    chain_wait();  // nothing above reads or writes global memory
+    auto load_weights = [&](unsigned char* stage, int kx, int seg, int n0, unsigned long long* bar) {
+        mbar_arrive_expect_tx(bar, kStage);
+        if (a.pair) {
+            tma_load_2d(stage + kStageA, &maps.w[0], kx, n0, bar);
+            tma_load_2d(stage + kStageA + kHalf * kTileK * 2, &maps.w[3], kx, n0, bar);
+        } else {
+            tma_load_2d(stage + kStageA, &maps.w[seg], kx, n0, bar);
+        }
+    };
+    // the weights of the first unit, a ring at most, while the kernel before this one drains (a launch of
+    // several waves gains nothing: the kernel before it needs the bandwidth)
+    int ahead = 0;
+    if (threadIdx.x == 0 && total <= static_cast<int>(gridDim.x)) {
+        const int unit = blockIdx.x, t = unit / a.split_k, z = unit - t * a.split_k, tile = t / a.tiles_m;
+        const int seg = (tile >= a.tile_start[1] ? 1 : 0) + (tile >= a.tile_start[2] ? 1 : 0);
+        const int kb0 = static_cast<int>(static_cast<long long>(z) * a.kblocks / a.split_k);
+        const int kb1 = static_cast<int>(static_cast<long long>(z + 1) * a.kblocks / a.split_k);
+        for (; ahead < min(kb1 - kb0, kStages); ++ahead)
+            load_weights(smem + ahead * kStage, (kb0 + ahead) * kTileK, seg,
+                         (tile - a.tile_start[seg]) * per_tile, &full[ahead]);
+    }
+    chain_wait();  // nothing above reads or writes what another kernel writes or reads
     if (threadIdx.x == 0) stamp(1);
 
     if (warp == 0) {
@@ -789,15 +974,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs 
                         break;
                     }
                     unsigned char* stage = smem + s * kStage;
-                    mbar_arrive_expect_tx(&full[s], kStage);
                     const int kx = kb * kTileK;
+                    if (ahead > 0)
+                        --ahead;
+                    else
+                        load_weights(stage, kx, seg, n0, &full[s]);
                     tma_load_2d(stage, &maps.a, kx, m0, &full[s]);
-                    if (a.pair) {
-                        tma_load_2d(stage + kStageA, &maps.w[0], kx, n0, &full[s]);
-                        tma_load_2d(stage + kStageA + kHalf * kTileK * 2, &maps.w[3], kx, n0, &full[s]);
-                    } else {
-                        tma_load_2d(stage + kStageA, &maps.w[seg], kx, n0, &full[s]);
-                    }
                     if (++s == kStages) {
                         s = 0;
                         ++round;
@@ -881,7 +1063,23 @@ gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs 
             const unsigned int lane_addr =
                 tmem_base + buf * BN + (static_cast<unsigned int>(quarter * 32) << 16);
             const bool row_fast = (n & 7) == 0;
-            if (a.split_k > 1) {
+            if (CLUSTERED) {
+                // the MMAs have read the ring to its end: the partial sums take its place, row by row
+                float* mine = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * (BN + 4);
+                if (ok && mt * kTileM + quarter * 32 < a.M) {
+#pragma unroll 1
+                    for (int c = column_half * (BN / 64); c < (column_half + 1) * (BN / 64); ++c) {
+                        float v[32];
+                        tmem_load32(lane_addr + c * 32, v);
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4)
+                            *reinterpret_cast<float4*>(mine + c * 32 + i) =
+                                make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
+                }
+                break;  // the only unit
+            }
+            if (!CLUSTERED && a.split_k > 1) {
                 // the eight warps meet at barriers below: leave together or not at all
                 if (named_barrier_or(2, 256, !ok)) {
                     *abort_flag = 1;
@@ -964,6 +1162,17 @@ gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs 
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
             if (j == 0 && threadIdx.x == 64) stamp(5);
         }
+    }
+    if (CLUSTERED) {  // uniform over the cluster; every wait before this one is bounded
+        const int unit = blockIdx.x, t = unit / a.split_k, z = unit - t * a.split_k, tile = t / a.tiles_m;
+        const int seg = (tile >= a.tile_start[1] ? 1 : 0) + (tile >= a.tile_start[2] ? 1 : 0);
+        __syncwarp();
+        cluster_meet();
+        if (*abort_flag == 0)
+            gemm_cluster_fold<BN>(a, smem_u32(smem), seg, (tile - a.tile_start[seg]) * per_tile,
+                                  (t % a.tiles_m) * kTileM, z);
+        __syncwarp();
+        cluster_meet();  // nobody leaves while its sums are being read
     }
     tc_fence_before();
     __syncthreads();
@@ -1924,12 +2133,19 @@ int gemm_smem_bytes(int bn, int stages) {
 struct GemmGeometry {
     int bn, stages, tiles_n, tiles_m, split_k, kblocks;
     int persistent;  // 1: gemm_tc_persistent_kernel on `grid` CTAs
+    int clustered;   // ... whose slices of a tile form clusters of `split_k` CTAs
     int grid;
     int tile_start[3];
 };
 
-GemmGeometry gemm_geometry(const mb_phase& P, int sm_count) {
+// How many clusters of 2 .. kMaxCluster CTAs run at once, for 128- and 256-column tiles.
+struct ClusterRoom {
+    int count[2][kMaxCluster + 1] = {};
+};
+
+GemmGeometry gemm_geometry(const mb_phase& P, int sm_count, const ClusterRoom& room) {
     GemmGeometry g;
+    g.clustered = 0;
     const int M = P.i[MB_GV_I_ROWS], K = P.i[MB_GV_I_K];
     const bool pair = P.i[MB_GV_I_NMAT] == 2;
     g.tiles_m = (M + kTileM - 1) / kTileM;
@@ -1980,6 +2196,18 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count) {
                     best = cost;
                     g.bn = bn;
                     persistent_split = split;
+                    g.clustered = 0;
+                }
+                // The slices of a tile as one cluster, if all clusters run at once: two meetings and a
+                // fold, 5 us for 19 live rows of a 128-column tile and about 8 us for all 128, and
+                // twice that for the 256 columns that also leave each CTA twice the sums to store.
+                if (split < 2 || split > kMaxCluster || tiles > room.count[bn == 256][split]) continue;
+                const double joint = stream + (3.0 + 4.0 * (M < kTileM ? M : kTileM) / kTileM) * (bn / 128);
+                if (joint < best - 1e-9) {
+                    best = joint;
+                    g.bn = bn;
+                    persistent_split = split;
+                    g.clustered = 1;
                 }
             }
         }
@@ -2023,9 +2251,10 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count) {
             if (value >= 1 && value <= 16 && value <= g.kblocks) split = value;
         }
     }
+    if (std::getenv("MEGABAKE_B200_GEMM_BN") || std::getenv("MEGABAKE_B200_GEMM_SPLIT")) g.clustered = 0;
     g.split_k = split;
     const int units = g.tiles_n * g.tiles_m * g.split_k;
-    g.grid = units < sm_count ? units : sm_count;
+    g.grid = units < sm_count || g.clustered ? units : sm_count;
     return g;
 }
 
@@ -2139,6 +2368,33 @@ int prefill_validate(const mb_phase& P, unsigned int n_slots, unsigned int n_dyn
     }
 }
 
+namespace {
+cudaError_t cluster_room(prefill::ClusterRoom* room) {
+    using namespace prefill;
+    const void* kernels[2] = {reinterpret_cast<const void*>(&gemm_tc_persistent_kernel<128, true>),
+                              reinterpret_cast<const void*>(&gemm_tc_persistent_kernel<256, true>)};
+    for (int wide = 0; wide < 2; ++wide) {
+        cudaError_t err =
+            cudaFuncSetAttribute(kernels[wide], cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmemBytes);
+        for (int size = 2; size <= kMaxCluster && err == cudaSuccess; ++size) {
+            cudaLaunchConfig_t config = {};
+            config.gridDim = dim3(size);
+            config.blockDim = dim3(kPersistThreads);
+            config.dynamicSmemBytes = kPersistSmemBytes;
+            cudaLaunchAttribute attribute[1];
+            attribute[0].id = cudaLaunchAttributeClusterDimension;
+            attribute[0].val.clusterDim.x = size;
+            attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+            config.attrs = attribute;
+            config.numAttrs = 1;
+            err = cudaOccupancyMaxActiveClusters(&room->count[wide][size], kernels[wide], &config);
+        }
+        if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
+}
+}  // namespace
+
 // Creates the per-plan state: geometry of every GEMM (written back into the phase records so
 // that mb_plan users can read it) and the split-K workspace.
 cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillState** out) {
@@ -2147,6 +2403,12 @@ cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillS
     if (st == nullptr) return cudaErrorMemoryAllocation;
     st->sm_count = sm_count;
     st->launches.resize(phases.size());
+    ClusterRoom room;
+    cudaError_t err = cluster_room(&room);
+    if (err != cudaSuccess) {
+        prefill_destroy(st);
+        return err;
+    }
     size_t floats = 0, counters = 0;
     for (size_t i = 0; i < phases.size(); ++i) {
         mb_phase& P = phases[i];
@@ -2163,18 +2425,17 @@ cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillS
             }
         }
         if (P.body != MB_BODY_GEMM_TC) continue;
-        GemmGeometry g = gemm_geometry(P, sm_count);
+        GemmGeometry g = gemm_geometry(P, sm_count, room);
         st->launches[i].geometry = g;
         P.i[MB_GV_I_SPLIT_K] = g.split_k;
         P.i[MB_GV_I_TILE_N] = g.bn;
         const size_t tiles = static_cast<size_t>(g.tiles_n) * g.tiles_m;
-        if (g.split_k > 1) {
+        if (g.split_k > 1 && !g.clustered) {
             const size_t need = tiles * g.split_k * kTileM * g.bn;
             if (need > floats) floats = need;
             if (tiles > counters) counters = tiles;
         }
     }
-    cudaError_t err = cudaSuccess;
     if (floats > 0) {
         err = cudaMalloc(&st->workspace, floats * sizeof(float));
         if (err == cudaSuccess) err = cudaMalloc(&st->counters, counters * sizeof(int));
@@ -2187,10 +2448,10 @@ cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillS
         err = cudaFuncSetAttribute(gemm_tc_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gemm_smem_bytes(256, 4));
     if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<128>,
+        err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<128, false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmemBytes);
     if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<256>,
+        err = cudaFuncSetAttribute(gemm_tc_persistent_kernel<256, false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistSmemBytes);
     if (err == cudaSuccess)
         err = cudaFuncSetAttribute(attention_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2328,19 +2589,32 @@ namespace {
 // may start while its predecessor drains (every kernel of this file blocks in chain_wait()
 // before it touches global memory).
 template <typename... Params, typename... Args>
-cudaError_t launch_phase(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
-                         cudaStream_t stream, bool chained, Args&&... args) {
+cudaError_t launch_phase_clustered(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                   cudaStream_t stream, bool chained, int cluster, Args&&... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
     config.dynamicSmemBytes = smem;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attribute[2];
     config.attrs = attribute;
-    config.numAttrs = chained ? 1 : 0;
+    if (chained) {
+        attribute[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attribute[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attribute[config.numAttrs].val.clusterDim.x = cluster;
+        attribute[config.numAttrs].val.clusterDim.y = 1;
+        attribute[config.numAttrs++].val.clusterDim.z = 1;
+    }
     return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_phase(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t stream, bool chained, Args&&... args) {
+    return launch_phase_clustered(kernel, grid, block, smem, stream, chained, 1, args...);
 }
 
 prefill::TransposeArgs transpose_args(const prefill::PrefillLaunch& L, int head_dim) {
@@ -2359,18 +2633,15 @@ int transpose_blocks(const prefill::TransposeArgs& t, int batch) {
     return (t.padded / 64) * (t.D / 64) * batch * t.kv_heads;
 }
 
-// Whether the kernels of one prefill are chained by programmatic dependent launch.  Measured
-// on the gemma-2b shape: a launch boundary between two dependent kernels costs about 5 us on a
-// stream (CTA-level stamps of consecutive GEMMs), chaining takes 3-4 % off a step launched
-// kernel by kernel at 128 and 512 tokens, and adds 1-2 % to the same step replayed from a CUDA
-// graph.  So: on for plain stream launches, off while the stream is being captured;
-// MEGABAKE_B200_PREFILL_CHAIN = 0 / 1 forces it (read at every launch, not cached, so that one
-// process can run both ways).
-bool chaining_enabled(cudaStream_t stream) {
-    if (const char* value = std::getenv("MEGABAKE_B200_PREFILL_CHAIN")) return std::atoi(value) != 0;
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) return false;
-    return status == cudaStreamCaptureStatusNone;
+// Whether the kernels of one prefill are chained by programmatic dependent launch.  A launch
+// boundary between two dependent kernels costs 3 - 5 us; chained, a kernel's set-up and the first
+// ring of a GEMM's weights run beside the kernel before it.  Replayed from a CUDA graph that is
+// 1937 -> 1584 us for 19 tokens of the 135M shape and 2499 -> 2369 us for 128 tokens of the 2B shape;
+// 2048 tokens do not care.  MEGABAKE_B200_PREFILL_CHAIN = 0 / 1 forces it (read at every
+// launch, not cached, so that one process can run both ways).
+bool chaining_enabled() {
+    const char* value = std::getenv("MEGABAKE_B200_PREFILL_CHAIN");
+    return value == nullptr || std::atoi(value) != 0;
 }
 
 }  // namespace
@@ -2385,7 +2656,7 @@ cudaError_t prefill_launch(PrefillState* st, const std::vector<mb_phase>& phases
         if (s < 0) return 0ull;
         return static_cast<unsigned int>(s) < n_dynamic ? dyn[s] : slots[s];
     };
-    const bool chain = chaining_enabled(stream);
+    const bool chain = chaining_enabled();
     bool chained = false;  // the first kernel of an invocation follows foreign work: plain launch
     size_t transposed_by = phases.size() + 1;  // the rotary phase that transposed the values, if any
     cudaError_t err = cudaSuccess;
@@ -2423,12 +2694,14 @@ cudaError_t prefill_launch(PrefillState* st, const std::vector<mb_phase>& phases
                 args.trace = trace == nullptr ? nullptr : trace + 8 * i;
                 for (int s = 0; s < args.nseg; ++s)  // outputs may be per-launch tensors (logits)
                     args.out[s] = reinterpret_cast<unsigned short*>(addr(P.slot[MB_GV_S_OUT0 + s]));
-                if (g.persistent && g.bn == 256)
-                    err = launch_phase(gemm_tc_persistent_kernel<256>, dim3(g.grid), dim3(kPersistThreads),
-                                       kPersistSmemBytes, stream, chained, L.maps, args);
-                else if (g.persistent)
-                    err = launch_phase(gemm_tc_persistent_kernel<128>, dim3(g.grid), dim3(kPersistThreads),
-                                       kPersistSmemBytes, stream, chained, L.maps, args);
+                if (g.persistent) {
+                    auto kernel = g.bn == 256 ? (g.clustered ? gemm_tc_persistent_kernel<256, true>
+                                                             : gemm_tc_persistent_kernel<256, false>)
+                                              : (g.clustered ? gemm_tc_persistent_kernel<128, true>
+                                                             : gemm_tc_persistent_kernel<128, false>);
+                    err = launch_phase_clustered(kernel, dim3(g.grid), dim3(kPersistThreads), kPersistSmemBytes,
+                                                 stream, chained, g.clustered ? g.split_k : 1, L.maps, args);
+                }
                 else if (g.bn == 256)
                     err = launch_phase(gemm_tc_kernel<256>, grid, dim3(kGemmThreads),
                                        gemm_smem_bytes(256, g.stages), stream, chained, L.maps, args);
@@ -2438,11 +2711,16 @@ cudaError_t prefill_launch(PrefillState* st, const std::vector<mb_phase>& phases
                 break;
             }
             case MB_BODY_ROPE_ROWS: {
-                const long long work = static_cast<long long>(P.i[MB_RP_I_ROWS]) *
-                                       (P.i[MB_RP_I_HEAD_DIM] / 2);
+                const long long pairs = static_cast<long long>(P.i[MB_RP_I_ROWS]) * (P.i[MB_RP_I_HEAD_DIM] / 2);
+                // half of the machine's threads: more only repeat the sine and cosine
+                const int quads = pairs >= 148 * 1024
+                                      ? 1
+                                      : (P.i[MB_RP_I_HEADS] + P.i[MB_RP_I_KV_HEADS] + kRopeHeads - 1) / kRopeHeads;
+                const long long work = pairs * quads;
                 long long blocks = (work + 255) / 256;
                 if (blocks > 4 * 148 * 8) blocks = 4 * 148 * 8;
                 RopeArgs rope;
+                rope.quads = quads;
                 rope.q = reinterpret_cast<unsigned short*>(addr(P.slot[MB_RP_S_Q]));
                 rope.k = reinterpret_cast<unsigned short*>(addr(P.slot[MB_RP_S_K]));
                 rope.pos = reinterpret_cast<const long long*>(addr(P.slot[MB_RP_S_POS]));
