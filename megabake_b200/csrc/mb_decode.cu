@@ -575,7 +575,7 @@ __device__ __forceinline__ uint4 normalise_fast(uint4 x, uint4 w, float inv) {
 // longer than 16 slots go chunk by chunk.
 constexpr int kSliceSlots = 16;
 constexpr int kSliceBytes = kSliceSlots * 512;
-static_assert(kSlicesBytes == kWarps * kSliceBytes, "the slices lie in the K/V rings, which GEMV phases do not use");
+static_assert(kSlicesBytes == kWarps * kSliceBytes, "eight warps' slices");
 struct Slice {
     int lp, rs;          // log2 of vectors per stage and of R
     int stages;          // of the whole reduction
@@ -1822,7 +1822,7 @@ int decode_rope_bytes(const mb_phase* phases, unsigned int n) {
     return (bytes + 127) / 128 * 128;
 }
 
-// Shared memory of a plan: fixed part, K/V rings, weight ring, stream table, cos / sin table.
+// Shared memory of a plan: fixed part, slices, ring, stream table, cos / sin table.
 static long long smem_bytes(int rope_bytes, unsigned int n_phases, int stages) {
     if (n_phases > 1u << 20) return LLONG_MAX;
     return static_cast<long long>(decode::rope_offset(stages, n_phases)) + rope_bytes;
