@@ -69,6 +69,7 @@ struct mb_plan {
     int threads = 0;
     int smem_bytes = 0;
     int stages = 0;
+    int slots_per_slice = 0;  // decode: of a warp's slice of the activations
     int head_dim = 64;  // decode: of all attention phases, 0 if they differ
     int barriers = 0;
     bool counters = false;
@@ -410,9 +411,11 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     const int limit = static_cast<int>(prop.sharedMemPerBlockOptin);
     const int head_dim = mb::decode_head_dim(desc->phases, desc->n_phases);
     const int rope_bytes = mb::decode_rope_bytes(desc->phases, desc->n_phases);
-    const int stages = mb::decode_ring_stages(rope_bytes, desc->n_phases, limit);
+    const int slots = mb::decode_slice_slots(desc->phases, desc->n_phases,
+                                             desc->ctas == 0 ? prop.multiProcessorCount : static_cast<int>(desc->ctas));
+    const int stages = mb::decode_ring_stages(rope_bytes, desc->n_phases, slots, limit);
     if (stages < 2) return MB_ERR_RESOURCE;
-    const int smem = mb::decode_smem_bytes(rope_bytes, desc->n_phases, stages);
+    const int smem = mb::decode_smem_bytes(rope_bytes, desc->n_phases, slots, stages);
 
     // The attribute belongs to the kernel, not to a plan: set it to the device's opt-in limit so
     // that plans of different sizes (two batch sizes, two models) can be launched in any order.
@@ -445,6 +448,7 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     plan->threads = mb::decode_threads();
     plan->smem_bytes = smem;
     plan->stages = stages;
+    plan->slots_per_slice = slots;
     plan->head_dim = head_dim;
     plan->barriers = barriers;
     if (desc->wait_limit_ms != 0)
@@ -524,7 +528,7 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
             else
                 entries[ph].addr[j] = plan->slots[slot];
         }
-        mb::decode_stream(plan->phases[ph], entries[ph].addr, plan->ctas, &streams[ph]);
+        mb::decode_stream(plan->phases[ph], entries[ph].addr, plan->ctas, plan->slots_per_slice, &streams[ph]);
         if (has_late_map(entries[ph])) {
             plan->late_maps.push_back(ph);
         } else if (!mb::decode_encode_maps(plan->phases[ph], entries[ph].addr, plan->ctas,
@@ -566,6 +570,7 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     params.streams = plan->d_streams;
     params.maps = plan->d_maps;
     params.stages = plan->stages;
+    params.slots = plan->slots_per_slice;
     params.relay = reinterpret_cast<unsigned long long>(plan->d_relay);
     params.relay_bytes = plan->relay_bytes;
     params.ctl = plan->d_ctl;

@@ -83,7 +83,7 @@ struct SharedCtl {
     const PhaseEntry* entries;
     const CUtensorMap* maps;         // kMapsPerPhase per phase
     unsigned long long dyn[MB_MAX_DYNAMIC];
-    int n_phases, stages;
+    int n_phases, stages, slots;
     unsigned long long rope_pos, rope_freq;  // what the cos / sin table was made from
     int rope_shape;
     float rope_scale;
@@ -98,28 +98,29 @@ constexpr int kCtlBytes = 5120;
 constexpr int kFixedBytes = kCtlBytes + kScratchBytes;
 static_assert(sizeof(SharedCtl) <= kCtlBytes, "control block too large");
 
-// Shared activations of GEMV phases, 8 KB per warp; attention dumps its states there.
-constexpr int kSlicesBytes = kWarps * 8 * 1024;
-// After the fixed part: the slices, the ring, the stream table, the cos / sin table.
-// The weight ring starts on a 1024-byte boundary.
-constexpr unsigned int kSliceOffset = kFixedBytes;
-constexpr unsigned int kRingOffset = kSliceOffset + kSlicesBytes;
+// After the fixed part: the ring, the warps' slices (shared activations of GEMV phases; attention dumps
+// its states there), the stream table, the cos / sin table.  Stages start on 1024-byte boundaries.
+constexpr unsigned int kRingOffset = kFixedBytes;
 static_assert(kRingOffset % 1024 == 0, "stages are 1024-byte aligned");
-__host__ __device__ constexpr unsigned int table_offset(int stages) {
+__host__ __device__ constexpr unsigned int slice_offset(int stages) {
     return kRingOffset + static_cast<unsigned int>(stages) * kRingStage;
 }
-__host__ __device__ constexpr unsigned int rope_offset(int stages, unsigned int n_phases) {
-    return table_offset(stages) + (n_phases * static_cast<unsigned int>(sizeof(StreamDesc)) + 127u) / 128u * 128u;
+__host__ __device__ constexpr unsigned int table_offset(int stages, int slots) {
+    return slice_offset(stages) + static_cast<unsigned int>(kWarps * slots) * 512u;
+}
+__host__ __device__ constexpr unsigned int rope_offset(int stages, int slots, unsigned int n_phases) {
+    return table_offset(stages, slots) +
+           (n_phases * static_cast<unsigned int>(sizeof(StreamDesc)) + 127u) / 128u * 128u;
 }
 
 extern __shared__ __align__(1024) char g_smem[];
 __device__ __forceinline__ SharedCtl* ctl_of() { return reinterpret_cast<SharedCtl*>(g_smem); }
 __device__ __forceinline__ float* scratch_of() { return reinterpret_cast<float*>(g_smem + kCtlBytes); }
 __device__ __forceinline__ StreamDesc* table_of() {
-    return reinterpret_cast<StreamDesc*>(g_smem + table_offset(ctl_of()->stages));
+    return reinterpret_cast<StreamDesc*>(g_smem + table_offset(ctl_of()->stages, ctl_of()->slots));
 }
 __device__ __forceinline__ unsigned int* rope_of() {
-    return reinterpret_cast<unsigned int*>(g_smem + rope_offset(ctl_of()->stages, ctl_of()->n_phases));
+    return reinterpret_cast<unsigned int*>(g_smem + rope_offset(ctl_of()->stages, ctl_of()->slots, ctl_of()->n_phases));
 }
 
 __device__ __forceinline__ void trace_stamp(int ph, int event) {
@@ -569,13 +570,15 @@ __device__ __forceinline__ uint4 normalise_fast(uint4 x, uint4 w, float inv) {
 
 // A warp's share of the activations: of every stage the groups it multiplies ("vectors": 32
 // elements of each row), R rows (the batch rounded up to a power of two) of four lanes x 16 bytes
-// each, one after the other in the warp's own 8 KB of shared memory.  A lane brings and normalises the
+// each, one after the other in the warp's own 8 KB (or 10 KB) of shared memory.  A lane brings and normalises the
 // 16 bytes at slot * 512 + lane * 16 -- at small batches a slot holds several vectors, so that
 // no lane works on a row that does not exist -- and reads them as B fragments of m16n8k16.  Reductions
-// longer than 16 slots go chunk by chunk.
-constexpr int kSliceSlots = 16;
-constexpr int kSliceBytes = kSliceSlots * 512;
-static_assert(kSlicesBytes == kWarps * kSliceBytes, "eight warps' slices");
+// longer than the slice go chunk by chunk.
+// A slice has 16 slots, or 20 in plans where that saves the chunks of some phase: five to eight rows
+// of a reduction of 4,097 - 5,120 elements (0.5B shape, 8 rows, 4,096 keys: 1,060 -> 953 us).  The four
+// take one stage from the ring, 1 % of a step where nobody needs them; more would take more.
+constexpr int kSliceSlots = 16, kWideSlots = 20;
+constexpr int kSliceBytes = kSliceSlots * 512;  // at least
 struct Slice {
     int lp, rs;          // log2 of vectors per stage and of R
     int stages;          // of the whole reduction
@@ -588,7 +591,7 @@ __device__ __forceinline__ Slice slice_of(const PhaseEntry* E, const GemvStream&
     v.lp = (d.shape & kShapeShort) ? 2 : 1;
     v.rs = rows > 2 ? (rows > 4 ? 3 : 2) : rows - 1;
     v.stages = (d.groups + (8 << v.lp) - 1) >> (3 + v.lp);
-    v.chunk = (kSliceSlots * 8) >> (v.lp + v.rs);
+    v.chunk = (ctl_of()->slots * 8) >> (v.lp + v.rs);
     v.first = c * v.chunk << v.lp;
     v.vectors = min(v.chunk, v.stages - c * v.chunk) << v.lp;
     v.slots = ((v.vectors << v.rs) + 7) >> 3;
@@ -599,11 +602,11 @@ __device__ __forceinline__ int vector_group(int lp, int warp, int v) {
     return ((v >> lp) << (3 + lp)) + (warp << lp) + (v & ((1 << lp) - 1));
 }
 __device__ __forceinline__ unsigned int slice_base(int warp) {
-    return smem_u32(g_smem) + kSliceOffset + warp * kSliceBytes;
+    return smem_u32(g_smem) + slice_offset(ctl_of()->stages) + warp * ctl_of()->slots * 512;
 }
 // Norm weights of the warp's vectors wait behind the slots where there is room (the usual case).
 __device__ __forceinline__ bool weights_staged(const Slice& v) {
-    return v.stages <= v.chunk && v.slots * 512 + v.vectors * 64 <= kSliceBytes;
+    return v.stages <= v.chunk && v.slots * 512 + v.vectors * 64 <= ctl_of()->slots * 512;
 }
 __device__ __forceinline__ void sts128(unsigned int addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
@@ -679,7 +682,7 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
     __syncwarp();
     if (norm && weights_staged(sl)) {
         for (int v = gid; v < sl.vectors; v += 8)
-            cp_async16(slice_base(warp) + kSliceBytes - (sl.vectors - v) * 64 + tq * 16,
+            cp_async16(slice_base(warp + 1) - (sl.vectors - v) * 64 + tq * 16,
                        d.w_norm + min(vector_group(sl.lp, warp, v), d.groups - 1) * 64 + tq * 16);
     }
     const char* x = reinterpret_cast<const char*>(E->addr[MB_GV_S_X]) + 16 * tq;
@@ -762,7 +765,7 @@ __device__ __forceinline__ void normalise_slice(const int ph, const int c) {
     const float inv = 1.0f / sqrtf(total / static_cast<float>(d.row_bytes / 2) + E->rec.f[MB_GV_F_EPS]);
     const unsigned int out = slice_base(warp) + lane * 16;
     const bool staged = weights_staged(sl);
-    const char* w = staged ? g_smem + kSliceOffset + (warp + 1) * kSliceBytes - sl.vectors * 64
+    const char* w = staged ? g_smem + slice_offset(sc->stages) + (warp + 1) * sc->slots * 512 - sl.vectors * 64
                            : reinterpret_cast<const char*>(d.w_norm);
     w += tq * 16;
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -1086,7 +1089,8 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
 
     const unsigned int stages = static_cast<unsigned int>(sc->stages);
     const unsigned int ring = smem_u32(g_smem) + kRingOffset;
-    float* dumps = reinterpret_cast<float*>(g_smem + kSliceOffset);
+    float* dumps = reinterpret_cast<float*>(g_smem + slice_offset(sc->stages));
+    const int dump_pitch = sc->slots * 128;  // floats
     const Segment& seg = sc->segment[warp];
     bool parted = false;  // some segment is one of several parts of its pair
     for (int which = 0; find_segment(ph, which); ++which) {
@@ -1360,7 +1364,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         for (int r = 0; r < D / DR; ++r) {
             if (r > 0) named_barrier(kBarAll, kThreads);
             __syncwarp();
-            float* dump = dumps + warp * (kSliceBytes / 4) + gid;
+            float* dump = dumps + warp * dump_pitch + gid;
 #pragma unroll
             for (int t = 0; t < DR / 16; ++t) {
                 const float(&v)[4] = acc[r * (DR / 16) + t];
@@ -1386,7 +1390,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
                     // sits here, the fast exponential is accurate to 2^-21
                     const float wgt = __expf(sc->stat[w][head][0] - m_all);  // 0: a warp without a block
                     const float2 v =
-                        *reinterpret_cast<const float2*>(dumps + w * (kSliceBytes / 4) + head * PR + dim);
+                        *reinterpret_cast<const float2*>(dumps + w * dump_pitch + head * PR + dim);
                     l_all += sc->stat[w][head][1] * wgt;
                     y0 += v.x * wgt;
                     y1 += v.y * wgt;
@@ -1532,7 +1536,7 @@ __device__ __forceinline__ bool begin_launch(const KernelParams& p, const Stream
                                              unsigned int tag_base, unsigned int parity,
                                              unsigned int calls) {
     SharedCtl* sc = ctl_of();
-    StreamDesc* table = reinterpret_cast<StreamDesc*>(g_smem + table_offset(p.stages));
+    StreamDesc* table = reinterpret_cast<StreamDesc*>(g_smem + table_offset(p.stages, p.slots));
     const int tid = threadIdx.x;
     for (int v = tid; v < p.n_phases * 6; v += kAllThreads)
         reinterpret_cast<uint4*>(table)[v] = reinterpret_cast<const uint4*>(streams)[v];
@@ -1552,6 +1556,7 @@ __device__ __forceinline__ bool begin_launch(const KernelParams& p, const Stream
         sc->trace = p.trace;
         sc->n_phases = p.n_phases;
         sc->stages = p.stages;
+        sc->slots = p.slots;
         sc->maps = reinterpret_cast<const CUtensorMap*>(maps);
         sc->entries = p.entries;
         for (int i = 0; i < MB_MAX_DYNAMIC; ++i) sc->dyn[i] = p.dyn[i];
@@ -1741,10 +1746,18 @@ decode_kernel(const __grid_constant__ KernelParams p) {
     }
 }
 
+// Slots of a slice that hold a warp's share of a phase's activations: the arithmetic of slice_of.
+int slots_needed(const mb_phase& P, const GemvStream& d) {
+    const int batch = P.i[MB_GV_I_ROWS], lp = (d.shape & kShapeShort) ? 2 : 1;
+    const int rs = batch > 2 ? (batch > 4 ? 3 : 2) : batch - 1;
+    const int stages = (d.groups + (8 << lp) - 1) >> (3 + lp);
+    return ((stages << (lp + rs)) + 7) >> 3;
+}
+
 // Shape of a skinny GEMM: a CTA with at most 8 output rows (o and down projections, q|k|v of small
 // models) takes blocks of 8 rows and twice the reduction per stage, so that no half of a stage and
 // of the MMA runs empty; gate and up rows come eight and eight; everything else sixteen at a time.
-void shape_gemv(const mb_phase& P, int ctas, GemvStream* d) {
+void shape_gemv(const mb_phase& P, int ctas, int slots, GemvStream* d) {
     int total = 0;
     for (int s = 0; s < P.i[MB_GV_I_NSEG]; ++s) total += P.i[MB_GV_I_N0 + s];
     d->row_bytes = P.i[MB_GV_I_K] * 2;
@@ -1755,10 +1768,7 @@ void shape_gemv(const mb_phase& P, int ctas, GemvStream* d) {
     d->groups = P.i[MB_GV_I_K] / 32;
     const int rows = 2 * (d->r0 + (d->r1 > 0 ? 1 : 0));  // of the busiest CTA
     d->shape = P.i[MB_GV_I_NMAT] == 2 ? kShapePaired : (rows <= 8 ? kShapeShort : 0);
-    // the same arithmetic as slice_of
-    const int batch = P.i[MB_GV_I_ROWS], lp = d->shape == kShapeShort ? 2 : 1;
-    const int rs = batch > 2 ? (batch > 4 ? 3 : 2) : batch - 1;
-    if ((d->groups + (8 << lp) - 1) >> (3 + lp) <= (kSliceSlots * 8) >> (lp + rs)) d->shape |= kShapeWhole;
+    if (slots_needed(P, *d) <= slots) d->shape |= kShapeWhole;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -1823,27 +1833,38 @@ int decode_rope_bytes(const mb_phase* phases, unsigned int n) {
 }
 
 // Shared memory of a plan: fixed part, slices, ring, stream table, cos / sin table.
-static long long smem_bytes(int rope_bytes, unsigned int n_phases, int stages) {
+static long long smem_bytes(int rope_bytes, unsigned int n_phases, int stages, int slots) {
     if (n_phases > 1u << 20) return LLONG_MAX;
-    return static_cast<long long>(decode::rope_offset(stages, n_phases)) + rope_bytes;
+    return static_cast<long long>(decode::rope_offset(stages, slots, n_phases)) + rope_bytes;
 }
 // Stages of the weight ring that fit; fewer than two means the plan does not.
-int decode_ring_stages(int rope_bytes, unsigned int n_phases, int limit) {
+int decode_ring_stages(int rope_bytes, unsigned int n_phases, int slots, int limit) {
     int stages = decode::kMaxStages;
-    while (stages > 0 && smem_bytes(rope_bytes, n_phases, stages) > limit) --stages;
+    while (stages > 0 && smem_bytes(rope_bytes, n_phases, stages, slots) > limit) --stages;
     return stages;
 }
-int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int stages) {
-    return static_cast<int>(smem_bytes(rope_bytes, n_phases, stages));
+int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int slots, int stages) {
+    return static_cast<int>(smem_bytes(rope_bytes, n_phases, stages, slots));
+}
+int decode_slice_slots(const mb_phase* phases, unsigned int n, int ctas) {
+    int slots = decode::kSliceSlots;
+    for (unsigned int i = 0; i < n; ++i) {
+        if (phases[i].body != MB_BODY_GEMV) continue;
+        GemvStream d;
+        decode::shape_gemv(phases[i], ctas, 0, &d);
+        const int need = decode::slots_needed(phases[i], d);
+        if (need > decode::kSliceSlots && need <= decode::kWideSlots) slots = decode::kWideSlots;
+    }
+    return slots;
 }
 
 // The static part of a phase's stream record; `addr`: its resolved slots.
-void decode_stream(const mb_phase& P, const unsigned long long* addr, int ctas, StreamDesc* out) {
+void decode_stream(const mb_phase& P, const unsigned long long* addr, int ctas, int slots, StreamDesc* out) {
     std::memset(out, 0, sizeof(*out));
     if (P.body == MB_BODY_GEMV) {
         GemvStream& d = out->gemv;
         d.kind = kStreamGemv;
-        decode::shape_gemv(P, ctas, &d);
+        decode::shape_gemv(P, ctas, slots, &d);
         if (P.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE) d.w_norm = addr[MB_GV_S_NORM_W];
     } else if (P.body == MB_BODY_ATTN_DECODE) {
         KvStream& d = out->kv;
@@ -1876,7 +1897,7 @@ bool decode_encode_maps(const mb_phase& P, const unsigned long long* addr, int c
     }
     if (P.body != MB_BODY_GEMV) return true;
     GemvStream d;
-    decode::shape_gemv(P, ctas, &d);
+    decode::shape_gemv(P, ctas, 0, &d);
     const bool is_short = (d.shape & kShapeShort) != 0, paired = (d.shape & kShapePaired) != 0;
     const int box_rows = is_short || paired ? 8 : 16, box_groups = is_short ? 32 : 16;
     for (int s = 0; s < P.i[MB_GV_I_NSEG]; ++s)
@@ -2114,7 +2135,7 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     if (cudaMemsetAsync(control, 0, kStaticControlBytes + kStaticCounterBytes, s) != cudaSuccess)
         return MB_ERR_CUDA;
     mb::StreamDesc desc;
-    mb::decode_stream(entry.rec, entry.addr, dev.sm_count, &desc);
+    mb::decode_stream(entry.rec, entry.addr, dev.sm_count, kSliceSlots, &desc);
     mb::KernelParams params;
     std::memset(&params, 0, sizeof(params));
     params.ctl = reinterpret_cast<mb::Control*>(control);
@@ -2123,11 +2144,12 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     int* status_out = reinterpret_cast<int*>(a->status);
     // the parts of a split context wait for one another's partials: all CTAs have to be resident
     const int rope_bytes = mb::decode_rope_bytes(&entry.rec, 1);
-    params.stages = mb::decode_ring_stages(rope_bytes, 1, dev.smem_limit);
+    params.slots = kSliceSlots;
+    params.stages = mb::decode_ring_stages(rope_bytes, 1, params.slots, dev.smem_limit);
     StaticMaps maps;
     if (params.stages < 2 || !mb::decode_encode_maps(entry.rec, entry.addr, dev.sm_count, &maps)) return MB_ERR_CUDA;
     void* args[] = {&params, &entry, &desc, &maps, &status_out};
-    const int smem = mb::decode_smem_bytes(rope_bytes, 1, params.stages);
+    const int smem = mb::decode_smem_bytes(rope_bytes, 1, params.slots, params.stages);
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&attention_static_kernel),
                                        dim3(dev.sm_count), dim3(kAllThreads), args,
                                        static_cast<size_t>(smem), s) == cudaSuccess

@@ -113,6 +113,7 @@ struct KernelParams {
     int n_dynamic;
     int barriers_per_launch;
     int stages;            // of the weight ring
+    int slots;             // 512-byte slots of a warp's slice of the activations
     int counters;          // some hand-off of the plan needs the finished-phase counters
     unsigned int wait_limit_us;  // bound of every device-side wait, microseconds
 };

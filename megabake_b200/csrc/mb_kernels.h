@@ -16,11 +16,13 @@ int decode_stage_bytes();
 int decode_row_pad();
 int decode_row_tile();
 int decode_rope_bytes(const mb_phase* phases, unsigned int n);
-int decode_ring_stages(int rope_bytes, unsigned int n_phases, int limit);  // < 2: does not fit
-int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int stages);
+int decode_slice_slots(const mb_phase* phases, unsigned int n, int ctas);
+int decode_ring_stages(int rope_bytes, unsigned int n_phases, int slots, int limit);  // < 2: does not fit
+int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int slots, int stages);
 size_t decode_map_bytes();  // of the tensor maps of one phase
 bool decode_encode_maps(const mb_phase& phase, const unsigned long long* addresses, int ctas, void* out);
-void decode_stream(const mb_phase& phase, const unsigned long long* addresses, int ctas, StreamDesc* out);
+void decode_stream(const mb_phase& phase, const unsigned long long* addresses, int ctas, int slots,
+                   StreamDesc* out);
 int decode_head_dim(const mb_phase* phases, unsigned int n);  // of all attention phases; 0: a mix
 cudaError_t decode_configure(int head_dim, int smem_bytes);
 cudaError_t decode_occupancy(int head_dim, int smem_bytes, int* blocks_per_sm);
