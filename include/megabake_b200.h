@@ -231,7 +231,11 @@ typedef struct mb_phase {
 #define MB_AT_S_POS 6        /* int64 [B]                                                  */
 #define MB_AT_S_INVFREQ 7    /* [D/2]                                                      */
 #define MB_AT_S_OUT 8        /* [B, Hq*D] bf16                                             */
-#define MB_AT_S_PARTIAL 9    /* fp32 [B*Hkv, max_chunks, Hq/Hkv, D+2]                      */
+#define MB_AT_S_PARTIAL 9    /* scratch of fp32 [B*Hkv, max_chunks, Hq/Hkv, D+2], 16-byte aligned:
+                                partial softmax states as 64-bit cells (fp32 value, sequence
+                                number), [B*Hkv, max_chunks / 2, Hq/Hkv, D+2].  mb_plan_bind clears
+                                it when its address is new to the phase; given per launch
+                                instead, it must be zero before its first launch           */
 #define MB_AT_S_COUNTER 10   /* int32 [B*Hkv], zero before the first launch                */
 
 /* ---- prefill bodies (MB_MODE_PREFILL plans: one kernel launch per phase, in order) ----- */

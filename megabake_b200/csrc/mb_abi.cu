@@ -83,6 +83,8 @@ struct mb_plan {
     std::vector<unsigned char> maps;      // the same on the host
     std::vector<size_t> late_maps;        // phases with such an operand that comes with the launch
     std::vector<mb::PhaseEntry> entries;  // as bound
+    std::vector<unsigned long long> partials;  // per phase: split-key buffer that was cleared for it, or 0
+    unsigned int wide_dynamic = 0;        // per-launch slots that must be 16-byte aligned, one bit each
     mb::Control* d_ctl = nullptr;
     unsigned long long trace = 0;
     mb::PrefillState* prefill = nullptr;  // MB_MODE_PREFILL plans only
@@ -286,6 +288,34 @@ cudaError_t blank_relays(const mb_plan* plan) {
     return cudaMemset(plan->d_relay, 0xff, 2 * plan->relay_bytes);
 }
 
+// Bytes of split-key partials an attention phase may poll; 0 if its context is never cut.
+size_t partial_bytes(const mb_phase& P) {
+    if (P.body != MB_BODY_ATTN_DECODE || P.i[MB_AT_I_MAX_CHUNKS] < 4) return 0;
+    if (P.i[MB_AT_I_CAPACITY] <= P.i[MB_AT_I_EXACT_KEYS]) return 0;
+    return static_cast<size_t>(P.i[MB_AT_I_BATCH]) * P.i[MB_AT_I_HEADS] * (P.i[MB_AT_I_MAX_CHUNKS] / 2) *
+           (P.i[MB_AT_I_HEAD_DIM] + 2) * 8;
+}
+
+// The partials are (value, tag) cells, and the tags of every plan start over: what an earlier owner of the
+// memory left there may carry the very tags this plan is going to wait for.  So each buffer is
+// cleared when its address is new to the phase, before any launch can poll it.
+cudaError_t clear_partials(mb_plan* plan, const std::vector<mb::PhaseEntry>& entries) {
+    plan->partials.resize(entries.size(), 0ull);
+    bool cleared = false;
+    for (size_t ph = 0; ph < entries.size(); ++ph) {
+        const size_t bytes = partial_bytes(plan->phases[ph]);
+        const unsigned long long address = entries[ph].addr[MB_AT_S_PARTIAL];
+        if (bytes == 0 || (address & mb::kDynamicTag) || address == plan->partials[ph]) continue;
+        const cudaError_t err = cudaMemset(reinterpret_cast<void*>(address), 0, bytes);
+        if (err != cudaSuccess) return err;
+        for (size_t other = ph; other < entries.size(); ++other)  // the layers of a model share one buffer
+            if (entries[other].addr[MB_AT_S_PARTIAL] == address && partial_bytes(plan->phases[other]) <= bytes)
+                plan->partials[other] = address;
+        cleared = true;
+    }
+    return cleared ? cudaStreamSynchronize(cudaStreamLegacy) : cudaSuccess;  // launches may use any stream
+}
+
 // A prefill plan is a list of kernel launches; it shares the descriptor, the slot table, the
 // status word and the entry points with decode plans.
 int create_prefill_plan(const mb_plan_desc* desc, mb_plan** out) {
@@ -442,6 +472,9 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     }
     plan->slots.assign(desc->n_slots, 0ull);
     plan->n_dynamic = desc->n_dynamic;
+    for (const mb_phase& P : plan->phases)
+        if (P.body == MB_BODY_ATTN_DECODE && static_cast<unsigned int>(P.slot[MB_AT_S_PARTIAL]) < desc->n_dynamic)
+            plan->wide_dynamic |= 1u << P.slot[MB_AT_S_PARTIAL];
     plan->activation_bytes = desc->activation_bytes;
     plan->sm_count = prop.multiProcessorCount;
     plan->ctas = ctas;
@@ -539,6 +572,7 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     }
     DeviceGuard guard(plan->device);
     if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
+    MB_CUDA(clear_partials(plan, entries));
     MB_CUDA(cudaMemcpy(plan->d_entries, entries.data(), sizeof(mb::PhaseEntry) * entries.size(),
                        cudaMemcpyHostToDevice));
     MB_CUDA(cudaMemcpy(plan->d_maps, plan->maps.data(), plan->maps.size(), cudaMemcpyHostToDevice));
@@ -576,7 +610,8 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     params.ctl = plan->d_ctl;
     params.trace = reinterpret_cast<unsigned long long*>(plan->trace);
     for (size_t i = 0; i < n; ++i) {
-        if (dynamic_addresses[i] == 0 || (dynamic_addresses[i] & 7ull) != 0) return MB_ERR_INVALID;
+        const unsigned long long unaligned = (plan->wide_dynamic >> i & 1u) ? 15ull : 7ull;
+        if (dynamic_addresses[i] == 0 || (dynamic_addresses[i] & unaligned) != 0) return MB_ERR_INVALID;
         params.dyn[i] = dynamic_addresses[i];
     }
     params.n_phases = static_cast<int>(plan->phases.size());

@@ -286,7 +286,8 @@ def _plan_decode(program: DecoderProgram, options: PlannerOptions, stage_bytes: 
     glu = slots.buffer(B * p.intermediate * 4, "gated", zero=True)
     max_chunks = max(1, min(options.max_chunks, math.ceil(p.capacity / 16)))
     pairs = B * p.kv_heads
-    partial = slots.buffer(pairs * max_chunks * p.group * (D + 2) * 4, "attention_partials")
+    # polled by tag, like the cells above: what an earlier owner of the memory left must not look valid
+    partial = slots.buffer(pairs * max_chunks * p.group * (D + 2) * 4, "attention_partials", zero=True)
     counters = slots.buffer(_align(pairs * 4, 16), "attention_arrivals", zero=True)
 
     merge_slots = options.merge_slots or CONSUMER_WARPS

@@ -145,3 +145,15 @@ def test_weight_bytes_match_the_roofline_table():
     for name, params in expect.items():
         spec = models.get_spec(name)
         assert spec.parameter_count() == params, name
+
+
+def test_split_key_partials_start_zeroed():
+    """The decode attention polls its partials by tag, and the tags of every plan start over: memory
+    handed on by a plan of the same shape must not carry them into the next one."""
+    layout = planner.plan_decode(models.direct_program(models.get_spec("tiny-qwen2"), 2, 4096))
+    spec, = [s for s in layout.slots if s.name == "attention_partials"]
+    zeroed = dict(layout.zero_ranges)
+    phase = next(p for p in layout.phases if p.body == rt.BODY_ATTN_DECODE)
+    shape = models.get_spec("tiny-qwen2")
+    assert zeroed[spec.offset] == (2 * shape.heads * phase.i[rt.AT_I_MAX_CHUNKS]
+                                   * (shape.head_dim + 2) * 4)

@@ -21,7 +21,7 @@ import torch
 from megabake_b200 import models
 from megabake_b200 import runtime as rt
 from megabake_b200.engine import BoundDecoder
-from megabake_b200.planner import PlannerOptions, plan_decode
+from megabake_b200.planner import PlannerOptions, attention_scratch_bytes, plan_decode
 from tests.helpers import PhaseRunner
 from tests.test_gpu_bodies import _bf16, _gemv_phase, _ref_linear
 
@@ -99,6 +99,79 @@ def test_distinct_buffers_give_identical_results(name, batch, cell_limit):
         assert torch.equal(x, y)
     for x, y in zip(shared[5], own[5]):
         assert torch.equal(x, y)
+
+
+def _split_context(decoder_parts, seed):
+    """Puts 300 cached keys into the state: contexts that are cut over several CTAs."""
+    spec, decoder, args, ids, pos, state = decoder_parts
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    for layer in range(spec.layers):
+        for cache in state[3 * layer: 3 * layer + 2]:
+            cache[:, :300].normal_(0.0, 0.3, generator=g)
+        state[3 * layer + 2].fill_(300)
+    tokens = torch.randint(0, spec.vocab, (decoder.program.batch, 3), generator=g, device="cuda")
+    outputs = []
+    for step in range(3):
+        ids.copy_(tokens[:, step:step + 1])
+        pos.fill_(300 + step)
+        outputs.append(decoder(*args).clone())
+        decoder.check()
+    return outputs + [t.clone() for t in state]
+
+
+def test_a_workspace_of_a_plan_of_the_same_shape(monkeypatch):
+    """A second decoder in the bytes the first one left: its launches wait for the very tags the first
+    one's partials carry, so none of them may still be there."""
+    clean = _split_context(_decoder("tiny-llama", 2, 320, PlannerOptions(), seed=5), seed=7)
+    first = _decoder("tiny-llama", 2, 320, PlannerOptions(), seed=4)
+    _split_context(first, seed=6)
+    left = first[1].workspace.clone()
+    partials, = [s for s in first[1].layout.slots if s.name == "attention_partials"]
+    assert int(left[partials.offset:].view(torch.int32).count_nonzero()) > 0    # contexts were cut
+    empty = torch.empty
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", lambda *a, **k: left.clone() if k.get("dtype") == torch.uint8
+                  else empty(*a, **k))
+        second = _decoder("tiny-llama", 2, 320, PlannerOptions(), seed=5)
+    phase = next(p for p in second[1].layout.phases if p.body == rt.BODY_ATTN_DECODE)
+    size = 2 * second[0].heads * phase.i[rt.AT_I_MAX_CHUNKS] * (second[0].head_dim + 2) * 4
+    assert int(second[1].workspace[partials.offset: partials.offset + size].count_nonzero()) == 0
+    for a, b in zip(clean, _split_context(second, seed=7)):
+        assert torch.equal(a, b)
+
+
+def test_binding_clears_partials_of_another_owner():
+    """The same through the C interface: a buffer that is new to the plan is cleared by the bind, one
+    that it already works in is left alone."""
+    from tests.test_gpu_bodies import _attention_case
+
+    batch, heads, kv_heads, dim, cached, capacity = 1, 4, 2, 64, 300, 320
+    dev = [t.cuda() for t in _attention_case(batch, heads, kv_heads, dim, cached, capacity)]
+    out = torch.zeros(batch, heads * dim, dtype=torch.bfloat16, device="cuda")
+    chunks = 20
+    partial = torch.full((batch * heads * chunks * (dim + 2),), 1.0, device="cuda")
+    phase = rt.Phase.blank(rt.BODY_ATTN_DECODE, 0)
+    for i, value in ((rt.AT_I_BATCH, batch), (rt.AT_I_HEADS, heads), (rt.AT_I_KV_HEADS, kv_heads),
+                     (rt.AT_I_HEAD_DIM, dim), (rt.AT_I_CAPACITY, capacity),
+                     (rt.AT_I_INVFREQ_BF16, 1), (rt.AT_I_MAX_CHUNKS, chunks), (rt.AT_I_MERGE_SLOTS, 8),
+                     (rt.AT_I_EXACT_KEYS, 128)):
+        phase.i[i] = value
+    phase.f[rt.AT_F_SCALE] = dim ** -0.5
+    phase.f[rt.AT_F_ROPE_SCALE] = 1.0
+    q, k, v, kc, vc, inv_freq, pos, length = dev
+    tensors = [q, k, v, kc, vc, length, pos, inv_freq, out, partial,
+               torch.zeros(4, dtype=torch.int32, device="cuda")]
+    for index in range(len(tensors)):
+        phase.slot[index] = index
+    scratch = (attention_scratch_bytes(dim, heads // kv_heads, 8) + 127) // 128 * 128
+    plan = rt.Plan([phase], n_slots=len(tensors), n_dynamic=0, activation_bytes=scratch, device=0)
+    plan.bind([t.data_ptr() for t in tensors])
+    torch.cuda.synchronize()
+    assert int(partial.count_nonzero()) == 0
+    partial.fill_(2.0)
+    plan.bind([t.data_ptr() for t in tensors])
+    torch.cuda.synchronize()
+    assert bool((partial == 2.0).all())
 
 
 def test_a_wait_that_runs_out_returns_a_status():
