@@ -81,6 +81,7 @@ struct mb_plan {
     mb::StreamDesc* d_streams = nullptr;
     void* d_maps = nullptr;               // tensor maps of weights and caches, decode_map_bytes() per phase
     std::vector<unsigned char> maps;      // the same on the host
+    unsigned int maps_written = 0;        // Control::maps_written
     std::vector<size_t> late_maps;        // phases with such an operand that comes with the launch
     std::vector<mb::PhaseEntry> entries;  // as bound
     std::vector<unsigned long long> partials;  // per phase: split-key buffer that was cleared for it, or 0
@@ -576,6 +577,9 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     MB_CUDA(cudaMemcpy(plan->d_entries, entries.data(), sizeof(mb::PhaseEntry) * entries.size(),
                        cudaMemcpyHostToDevice));
     MB_CUDA(cudaMemcpy(plan->d_maps, plan->maps.data(), plan->maps.size(), cudaMemcpyHostToDevice));
+    ++plan->maps_written;
+    MB_CUDA(cudaMemcpy(&plan->d_ctl->maps_written, &plan->maps_written, sizeof(plan->maps_written),
+                       cudaMemcpyHostToDevice));
     MB_CUDA(cudaMemcpy(plan->d_streams, streams.data(), sizeof(mb::StreamDesc) * streams.size(),
                        cudaMemcpyHostToDevice));
     plan->entries = std::move(entries);
@@ -617,6 +621,8 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     params.n_phases = static_cast<int>(plan->phases.size());
     params.n_dynamic = static_cast<int>(plan->n_dynamic);
     params.barriers_per_launch = plan->barriers - 1;
+    params.sm_count = plan->sm_count;
+    params.late_maps = plan->late_maps.empty() ? 0 : 1;
     params.counters = plan->counters ? 1 : 0;
     params.wait_limit_us = plan->wait_limit_us;
     DeviceGuard guard(plan->device);
@@ -675,6 +681,9 @@ int mb_plan_reset(mb_plan* plan) {
     epoch += 1;
     MB_CUDA(cudaMemset(plan->d_ctl, 0, sizeof(mb::Control)));
     MB_CUDA(cudaMemcpy(&plan->d_ctl->epoch, &epoch, sizeof(epoch), cudaMemcpyHostToDevice));
+    ++plan->maps_written;  // not acquired, as far as the cleared block knows
+    MB_CUDA(cudaMemcpy(&plan->d_ctl->maps_written, &plan->maps_written, sizeof(plan->maps_written),
+                       cudaMemcpyHostToDevice));
     MB_CUDA(blank_relays(plan));
     MB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return MB_OK;

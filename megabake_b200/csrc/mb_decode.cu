@@ -379,6 +379,12 @@ __device__ __forceinline__ void cp_async16(unsigned int dst_smem, unsigned long 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src_gmem)
                  : "memory");
 }
+// All threads: orders what was stored to the tensor maps in global memory before this CTA's copies
+// through them, which come after a barrier.
+__device__ __noinline__ void acquire_maps(const CUtensorMap* maps, int count) {
+    for (int m = threadIdx.x; m < count; m += kAllThreads)
+        asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(maps + m) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(unsigned int dst, const CUtensorMap* map, int row, int group,
                                             unsigned long long* bar) {
     asm volatile(
@@ -1704,9 +1710,13 @@ __global__ void __launch_bounds__(kAllThreads, 1)
 decode_kernel(const __grid_constant__ KernelParams p) {
     SharedCtl* sc = ctl_of();
     const int tid = threadIdx.x;
-    // Both words only change when the last CTA of a launch closes it (or by a host reset).
+    // These words only change when the last CTA of a launch closes it (or by a host reset or bind).
     const unsigned int calls = *reinterpret_cast<volatile unsigned int*>(&p.ctl->calls);
     const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&p.ctl->epoch);
+    const unsigned int written = *reinterpret_cast<volatile unsigned int*>(&p.ctl->maps_written);
+    // newer maps than this SM may have cached from their addresses (10 us for those of a model, so not always)
+    if (p.late_maps || *reinterpret_cast<volatile unsigned int*>(&p.ctl->maps_acquired) != written)
+        acquire_maps(static_cast<const CUtensorMap*>(p.maps), p.n_phases * kMapsPerPhase);
     if (!begin_launch(p, p.streams, p.maps, epoch * static_cast<unsigned int>(p.n_phases), epoch, calls)) return;
     const StreamDesc* table = table_of();
 
@@ -1742,6 +1752,8 @@ decode_kernel(const __grid_constant__ KernelParams p) {
         if (tid == 0) {
             p.ctl->calls = calls + 1;
             p.ctl->epoch = epoch + 1;
+            // one CTA of this size fits an SM: a grid of one per SM has been on all of them
+            if (static_cast<int>(gridDim.x) >= p.sm_count) p.ctl->maps_acquired = written;
         }
     }
 }

@@ -23,7 +23,11 @@ struct Control {
     unsigned int calls;     // completed launches; the barrier targets derive from it
     int status[4];          // code, phase, detail, (unused)
     unsigned int arrived;   // CTAs of the running launch that are through; the last one closes it
-    unsigned int pad0[25];
+    // The tensor maps lie in global memory: how often the host has written them, and the last of these
+    // versions that every SM has acquired.  A launch that finds the two different acquires the maps
+    // before it copies through them; until then an SM may hold older maps from the same addresses.
+    unsigned int maps_written, maps_acquired;
+    unsigned int pad0[23];
     // CTAs that finished a phase: a ring of four counters (a line each), phase q counts on
     // counter q % 4.  Every CTA, before it leaves phase q, waits until all CTAs have finished
     // phase q - 2; so no CTA is ever more than two phases ahead of another, a counter never
@@ -114,6 +118,8 @@ struct KernelParams {
     int barriers_per_launch;
     int stages;            // of the weight ring
     int slots;             // 512-byte slots of a warp's slice of the activations
+    int sm_count;
+    int late_maps;         // some tensor map is written for every launch
     int counters;          // some hand-off of the plan needs the finished-phase counters
     unsigned int wait_limit_us;  // bound of every device-side wait, microseconds
 };

@@ -174,6 +174,32 @@ def test_binding_clears_partials_of_another_owner():
     assert bool((partial == 2.0).all())
 
 
+def test_tensor_maps_follow_every_bind():
+    """The tensor maps live in device memory that a bind rewrites, and that a new plan may get from a
+    destroyed one: every launch reads the weights and caches of the latest bind."""
+    rows, k, n = 3, 576, 1536
+    x = _bf16(rows, k, seed=1)
+    weights = [_bf16(n, k, scale=k ** -0.5, seed=10 + i) for i in range(3)]
+    expected = [_ref_linear(x, w) for w in weights]
+    out = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+    plan = None
+    for step in range(12):
+        which = step % 3
+        runner = PhaseRunner()
+        phase = _gemv_phase(runner, x=x, segs=[(weights[which], None, out)], k=k, rows=rows)
+        out.zero_()
+        if plan is None or step % 4 == 0:
+            plan = None     # destroyed here: the next one may work at its addresses
+            plan = runner.run([phase], (rows + 1) * (k + 32) * 2)
+        else:
+            plan.bind([t.data_ptr() for t in runner.tensors])
+            plan.launch([], torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+        assert plan.status().code == 0
+        assert (out != expected[which]).float().mean() < 0.02, step
+        assert float((out.float() - expected[which].float()).abs().max()) <= 0.06
+
+
 def test_a_wait_that_runs_out_returns_a_status():
     """Phase 1 polls cells that phase 0 (a no-op) never writes.  With a 40 ms limit the kernel
     must come back by itself with MB_ST_HANDOFF_TIMEOUT; afterwards another plan runs normally."""
