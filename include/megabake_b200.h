@@ -137,8 +137,9 @@ enum mb_body {
                                   counter: thousands of threads polling their cells would
                                   queue up in front of the very stores they wait for).  With
                                   cell x it is a hint -- the sequence numbers still decide;
-                                  with plain x it is the synchronisation, and the producing
-                                  phase must carry MB_FLAG_FENCE                              */
+                                  with plain x, or a plain residual that an earlier phase wrote,
+                                  it is the synchronisation, and the producing phase must carry
+                                  MB_FLAG_FENCE                                              */
 
 /* GEMV / GEMM prologues (applied to the activation rows) */
 enum mb_prologue {

@@ -239,12 +239,17 @@ int lower_relays(mb_plan* plan) {
                     r.modes |= mb::kModeInRelay;
                 else if (cells & (MB_CELLS_X | MB_CELLS_X_WAIT))
                     plan->counters = true;
+                if ((cells & MB_CELLS_X_WAIT) && !(cells & MB_CELLS_X) && !(r.modes & mb::kModeInRelay))
+                    r.modes |= mb::kModeWait;
             }
             if (P.i[MB_GV_I_EPILOGUE] == MB_EPI_RESIDUAL) {
                 if (consume(r, P, MB_GV_S_RESIDUAL))
                     r.modes |= mb::kModeResidualRelay;
-                else if (cells & MB_CELLS_RESIDUAL)
+                else if (cells & (MB_CELLS_RESIDUAL | MB_CELLS_X_WAIT))
                     plan->counters = true;
+                if ((cells & MB_CELLS_X_WAIT) && !(cells & MB_CELLS_RESIDUAL) &&
+                    !(r.modes & mb::kModeResidualRelay))
+                    r.modes |= mb::kModeWait;  // whatever the activations are
             }
             if (P.i[MB_GV_I_GATHER] && P.i[MB_GV_I_STORE_X]) {
                 if (P.flags & MB_FLAG_RELAY) r.modes |= mb::kModeStoreRelay;

@@ -702,14 +702,14 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
     } else {
         x += static_cast<size_t>(row) * d.row_bytes;
     }
+    if (E->modes & kModeWait) {
+        if (lane == 0) finished_wait(ph, E->rec.i[MB_GV_I_X_SOURCE]);
+        __syncwarp();
+    }
     if (cells) {
         stage_cells(ph, c);
         __syncwarp();
     } else {
-        if (!relay && !gather && (flags & MB_CELLS_X_WAIT)) {
-            if (lane == 0) finished_wait(ph, E->rec.i[MB_GV_I_X_SOURCE]);
-            __syncwarp();
-        }
         int i = 0;
 #pragma unroll 1
         for (; sl.slots - i > 4; i += 8)
@@ -818,8 +818,10 @@ __device__ __forceinline__ Result request_result(const PhaseEntry* E, const Gemv
             const int seg = output_segment(d, local);
             const unsigned short* bias = reinterpret_cast<const unsigned short*>(E->addr[MB_GV_S_BIAS0 + seg]);
             if (bias != nullptr) r.bias = bf16_bits_to_float(__ldg(bias + local));
+            // (a plain one of a phase that waits may not have been written yet: finish_result loads it)
             if (E->rec.i[MB_GV_I_EPILOGUE] == MB_EPI_RESIDUAL &&
-                ((E->modes & kModeResidualRelay) || !(E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL)))
+                ((E->modes & kModeResidualRelay) ||
+                 !((E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL) || (E->modes & kModeWait))))
                 r.residual = ld_relaxed_u32(residual_address(E, vrow, r.tok));
         }
     }
@@ -854,6 +856,8 @@ __device__ __forceinline__ void finish_result(const PhaseEntry* E, const GemvStr
                 r.residual = cell_data(cell_wait(
                     residual_address(E, r.vrow, r.tok),
                     sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_RES_SOURCE]) + 1u, ph));
+            } else if (E->modes & kModeWait) {  // stage_slice has waited for it
+                r.residual = ld_relaxed_u32(residual_address(E, r.vrow, r.tok));
             }
         }
         y = (r.vrow & 1 ? hi_bf16(r.residual) : lo_bf16(r.residual)) + y;

@@ -62,6 +62,8 @@ constexpr unsigned long long kRelayTag = 1ull << 62;
 // operands of a phase that live in the relay arena
 constexpr unsigned long long kModeInRelay = 1, kModeResidualRelay = 2, kModeOutRelay = 4,
                              kModeStoreRelay = 8;
+// GEMV: activations or residual are plain memory of a phase before, guarded by its counter alone
+constexpr unsigned long long kModeWait = 16;
 // Every 32-bit word of the relay arena that has not been written in this launch holds this
 // pattern.  Conversions to bf16 never produce it: a NaN becomes 0x7fff.
 constexpr unsigned int kUnwritten = 0xffffffffu;

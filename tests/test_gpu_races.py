@@ -200,6 +200,60 @@ def test_tensor_maps_follow_every_bind():
         assert float((out.float() - expected[which].float()).abs().max()) <= 0.06
 
 
+def test_a_plain_residual_is_read_after_the_wait():
+    """CTA 0 gathers and stores 8 x 8192 rows in phase 0 while the other CTAs, which own no output row of
+    it, are long through to phase 2, where these rows are the residual: plain memory, ordered by
+    nothing but the wait for phase 1."""
+    rows, k, n = 8, 8192, 8192
+    table, ids = _bf16(16, k, seed=1), torch.arange(3, 3 + rows, dtype=torch.int64, device="cuda")
+    w0, other = _bf16(2, k, scale=k ** -0.5, seed=2), _bf16(rows, 64, seed=3)
+    w1, w2 = _bf16(64, 64, scale=0.125, seed=4), _bf16(n, 64, scale=0.125, seed=5)
+    stored = torch.zeros(rows, k, dtype=torch.bfloat16, device="cuda")
+    o0, o1, out = (torch.zeros(rows, m, dtype=torch.bfloat16, device="cuda") for m in (2, 64, n))
+    runner = PhaseRunner()
+    gather = _gemv_phase(runner, x=table, segs=[(w0, None, o0)], k=k, rows=rows)
+    gather.flags |= rt.FLAG_FENCE
+    gather.i[rt.GV_I_GATHER], gather.i[rt.GV_I_VOCAB], gather.i[rt.GV_I_STORE_X] = 1, 16, 1
+    gather.slot[rt.GV_S_IDS] = runner.slot("ids", ids)
+    gather.slot[rt.GV_S_XSTORE] = runner.slot("stored", stored)
+    runner.names = {}
+    between = _gemv_phase(runner, x=other, segs=[(w1, None, o1)], k=64, rows=rows)
+    between.flags |= rt.FLAG_FENCE
+    runner.names = {}
+    last = _gemv_phase(runner, x=o1, segs=[(w2, None, out)], k=64, rows=rows, residual=stored,
+                       epilogue=rt.EPI_RESIDUAL)
+    last.i[rt.GV_I_CELLS], last.i[rt.GV_I_X_SOURCE] = rt.CELLS_X_WAIT, 1
+    plan = runner.run([gather, between, last], (rows + 1) * (k + 32) * 2)
+    y = _ref_linear(other, w1)
+    expected = table[ids] + _ref_linear(y, w2)
+    for _ in range(5):
+        assert plan.status().code == 0
+        assert torch.equal(stored, table[ids])
+        assert float((out.float() - expected.float()).abs().max()) <= 0.05
+        for t in (stored, o1, out):
+            t.zero_()
+        plan.launch([], torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("name,batch", [("tiny-llama", 1), ("tiny-qwen2", 8), ("tiny-gemma256", 2)])
+@pytest.mark.parametrize("qkv_cells,cell_limit", [(True, 0), (False, 0), (True, 1 << 20), (False, 2048)])
+def test_hand_offs_through_the_workspace_give_the_same_results(name, batch, qkv_cells, cell_limit):
+    """Plain tensors behind fenced counters, flagged cells and mixes of the two against the relay arena:
+    the arithmetic is the same, so are the bits.  One short row: most CTAs have no attention to do."""
+    relayed = _decoder(name, batch, 24, PlannerOptions())
+    plain = _decoder(name, batch, 24, PlannerOptions(relay=False, qkv_cells=qkv_cells,
+                                                     cell_limit=cell_limit))
+    assert any(p.flags & rt.FLAG_RELAY for p in relayed[1].layout.phases)
+    assert not any(p.flags & rt.FLAG_RELAY for p in plain[1].layout.phases)
+    spec = relayed[0]
+    tokens = torch.randint(0, spec.vocab, (batch, 20), generator=torch.Generator().manual_seed(4)).cuda()
+    for a, b in zip(_run_steps(*relayed[1:5], tokens), _run_steps(*plain[1:5], tokens)):
+        assert torch.equal(a, b)
+    for a, b in zip(relayed[5], plain[5]):
+        assert torch.equal(a, b)
+
+
 def test_a_wait_that_runs_out_returns_a_status():
     """Phase 1 polls cells that phase 0 (a no-op) never writes.  With a 40 ms limit the kernel
     must come back by itself with MB_ST_HANDOFF_TIMEOUT; afterwards another plan runs normally."""
