@@ -80,7 +80,6 @@ struct mb_plan {
     mb::PhaseEntry* d_entries = nullptr;
     mb::StreamDesc* d_streams = nullptr;
     void* d_maps = nullptr;               // tensor maps of weights and caches, decode_map_bytes() per phase
-    std::vector<unsigned char> maps;      // the same on the host
     unsigned int maps_written = 0;        // Control::maps_written
     std::vector<size_t> late_maps;        // phases with such an operand that comes with the launch
     std::vector<mb::PhaseEntry> entries;  // as bound
@@ -525,7 +524,8 @@ int mb_plan_query(const mb_plan* plan, mb_plan_info* out) {
     out->stages = plan->stages;
     out->barriers = plan->barriers;
     out->sm_count = plan->sm_count;
-    out->launches = plan->mode == MB_MODE_PREFILL ? mb::prefill_launch_count(plan->prefill) : 1;
+    out->launches = plan->mode == MB_MODE_PREFILL ? mb::prefill_launch_count(plan->prefill)
+                                                  : 1 + static_cast<int>(plan->late_maps.size());
     return MB_OK;
 }
 
@@ -551,7 +551,7 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     // phase and never a second table.
     std::vector<mb::PhaseEntry> entries(plan->phases.size());
     std::vector<mb::StreamDesc> streams(plan->phases.size());
-    plan->maps.assign(plan->phases.size() * mb::decode_map_bytes(), 0);
+    std::vector<unsigned char> maps(plan->phases.size() * mb::decode_map_bytes(), 0);
     plan->late_maps.clear();
     for (size_t ph = 0; ph < plan->phases.size(); ++ph) {
         entries[ph].rec = plan->phases[ph];
@@ -571,7 +571,7 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
         if (has_late_map(entries[ph])) {
             plan->late_maps.push_back(ph);
         } else if (!mb::decode_encode_maps(plan->phases[ph], entries[ph].addr, plan->ctas,
-                                           plan->maps.data() + ph * mb::decode_map_bytes())) {
+                                           maps.data() + ph * mb::decode_map_bytes())) {
             g_last_cuda_error = "tensor map encoding failed";
             return MB_ERR_CUDA;
         }
@@ -581,7 +581,7 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     MB_CUDA(clear_partials(plan, entries));
     MB_CUDA(cudaMemcpy(plan->d_entries, entries.data(), sizeof(mb::PhaseEntry) * entries.size(),
                        cudaMemcpyHostToDevice));
-    MB_CUDA(cudaMemcpy(plan->d_maps, plan->maps.data(), plan->maps.size(), cudaMemcpyHostToDevice));
+    MB_CUDA(cudaMemcpy(plan->d_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
     ++plan->maps_written;
     MB_CUDA(cudaMemcpy(&plan->d_ctl->maps_written, &plan->maps_written, sizeof(plan->maps_written),
                        cudaMemcpyHostToDevice));
@@ -627,22 +627,19 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
     params.n_dynamic = static_cast<int>(plan->n_dynamic);
     params.barriers_per_launch = plan->barriers - 1;
     params.sm_count = plan->sm_count;
-    params.late_maps = plan->late_maps.empty() ? 0 : 1;
     params.counters = plan->counters ? 1 : 0;
     params.wait_limit_us = plan->wait_limit_us;
     DeviceGuard guard(plan->device);
     if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
+    // Weights and caches that come with the launch: their maps travel as parameters of a kernel before it, so
+    // that a captured launch keeps its own and the host may go on to the next one at once.
     for (size_t ph : plan->late_maps) {
         mb::PhaseEntry entry = plan->entries[ph];
         for (unsigned long long& a : entry.addr)
             if (a & mb::kDynamicTag) a = dynamic_addresses[a & (MB_MAX_DYNAMIC - 1)];
-        unsigned char* maps = plan->maps.data() + ph * mb::decode_map_bytes();
-        if (!mb::decode_encode_maps(plan->phases[ph], entry.addr, plan->ctas, maps)) {
-            g_last_cuda_error = "tensor map encoding failed";
-            return MB_ERR_CUDA;
-        }
-        MB_CUDA(cudaMemcpyAsync(static_cast<unsigned char*>(plan->d_maps) + ph * mb::decode_map_bytes(), maps,
-                                mb::decode_map_bytes(), cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)));
+        MB_CUDA(mb::decode_store_maps(plan->phases[ph], entry.addr, plan->ctas,
+                                      static_cast<unsigned char*>(plan->d_maps) + ph * mb::decode_map_bytes(),
+                                      plan->d_ctl, static_cast<cudaStream_t>(stream)));
     }
     MB_CUDA(mb::decode_launch(params, plan->head_dim, plan->ctas, plan->smem_bytes,
                               static_cast<cudaStream_t>(stream)));

@@ -1719,7 +1719,7 @@ decode_kernel(const __grid_constant__ KernelParams p) {
     const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&p.ctl->epoch);
     const unsigned int written = *reinterpret_cast<volatile unsigned int*>(&p.ctl->maps_written);
     // newer maps than this SM may have cached from their addresses (10 us for those of a model, so not always)
-    if (p.late_maps || *reinterpret_cast<volatile unsigned int*>(&p.ctl->maps_acquired) != written)
+    if (*reinterpret_cast<volatile unsigned int*>(&p.ctl->maps_acquired) != written)
         acquire_maps(static_cast<const CUtensorMap*>(p.maps), p.n_phases * kMapsPerPhase);
     if (!begin_launch(p, p.streams, p.maps, epoch * static_cast<unsigned int>(p.n_phases), epoch, calls)) return;
     const StreamDesc* table = table_of();
@@ -1923,6 +1923,26 @@ bool decode_encode_maps(const mb_phase& P, const unsigned long long* addr, int c
     return !paired || decode::encode_weight_map(maps + 1, addr[MB_GV_S_W_PAIR], P.i[MB_GV_I_N0],
                                                 P.i[MB_GV_I_K], box_rows, box_groups);
 }
+namespace decode {
+struct alignas(64) PhaseMaps {
+    CUtensorMap map[kMapsPerPhase];
+};
+// One warp: the maps of one phase of the launch that follows, which finds them newer than those acquired.
+__global__ void store_maps_kernel(const __grid_constant__ PhaseMaps maps, uint4* out, Control* ctl) {
+    for (unsigned int v = threadIdx.x; v < sizeof(PhaseMaps) / 16; v += 32)
+        out[v] = reinterpret_cast<const uint4*>(&maps)[v];
+    asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
+    if (threadIdx.x == 0) ctl->maps_written += 1;
+}
+}  // namespace decode
+
+cudaError_t decode_store_maps(const mb_phase& P, const unsigned long long* addr, int ctas, void* out, Control* ctl,
+                              cudaStream_t stream) {
+    decode::PhaseMaps maps;
+    if (!decode_encode_maps(P, addr, ctas, &maps)) return cudaErrorInvalidValue;
+    decode::store_maps_kernel<<<1, 32, 0, stream>>>(maps, static_cast<uint4*>(out), ctl);
+    return cudaGetLastError();
+}
 size_t decode_map_bytes() { return decode::kMapsPerPhase * sizeof(CUtensorMap); }
 
 namespace {
@@ -2002,13 +2022,9 @@ static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBy
 // partial of an earlier call can be mistaken for one of this call.
 static __device__ unsigned int g_static_epoch;
 
-struct alignas(64) StaticMaps {
-    CUtensorMap map[kMapsPerPhase];
-};
-
 __global__ void __launch_bounds__(kAllThreads, 1)
 attention_static_kernel(const __grid_constant__ KernelParams p, const __grid_constant__ PhaseEntry entry,
-                        const __grid_constant__ StreamDesc stream, const __grid_constant__ StaticMaps maps,
+                        const __grid_constant__ StreamDesc stream, const __grid_constant__ PhaseMaps maps,
                         int* status_out) {
     SharedCtl* sc = ctl_of();
     const int tid = threadIdx.x;
@@ -2162,7 +2178,7 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     const int rope_bytes = mb::decode_rope_bytes(&entry.rec, 1);
     params.slots = kSliceSlots;
     params.stages = mb::decode_ring_stages(rope_bytes, 1, params.slots, dev.smem_limit);
-    StaticMaps maps;
+    PhaseMaps maps;
     if (params.stages < 2 || !mb::decode_encode_maps(entry.rec, entry.addr, dev.sm_count, &maps)) return MB_ERR_CUDA;
     void* args[] = {&params, &entry, &desc, &maps, &status_out};
     const int smem = mb::decode_smem_bytes(rope_bytes, 1, params.slots, params.stages);

@@ -23,7 +23,7 @@ struct Control {
     unsigned int calls;     // completed launches; the barrier targets derive from it
     int status[4];          // code, phase, detail, (unused)
     unsigned int arrived;   // CTAs of the running launch that are through; the last one closes it
-    // The tensor maps lie in global memory: how often the host has written them, and the last of these
+    // The tensor maps lie in global memory: how often they have been written, and the last of these
     // versions that every SM has acquired.  A launch that finds the two different acquires the maps
     // before it copies through them; until then an SM may hold older maps from the same addresses.
     unsigned int maps_written, maps_acquired;
@@ -121,7 +121,6 @@ struct KernelParams {
     int stages;            // of the weight ring
     int slots;             // 512-byte slots of a warp's slice of the activations
     int sm_count;
-    int late_maps;         // some tensor map is written for every launch
     int counters;          // some hand-off of the plan needs the finished-phase counters
     unsigned int wait_limit_us;  // bound of every device-side wait, microseconds
 };

@@ -8,6 +8,7 @@
 
 namespace mb {
 struct KernelParams;
+struct Control;
 union StreamDesc;
 
 int decode_threads();
@@ -21,6 +22,9 @@ int decode_ring_stages(int rope_bytes, unsigned int n_phases, int slots, int lim
 int decode_smem_bytes(int rope_bytes, unsigned int n_phases, int slots, int stages);
 size_t decode_map_bytes();  // of the tensor maps of one phase
 bool decode_encode_maps(const mb_phase& phase, const unsigned long long* addresses, int ctas, void* out);
+// The same for one launch: encoded now, written to `out` on the device in stream order.
+cudaError_t decode_store_maps(const mb_phase& phase, const unsigned long long* addresses, int ctas, void* out,
+                              Control* ctl, cudaStream_t stream);
 void decode_stream(const mb_phase& phase, const unsigned long long* addresses, int ctas, int slots,
                    StreamDesc* out);
 int decode_head_dim(const mb_phase* phases, unsigned int n);  // of all attention phases; 0: a mix
@@ -31,7 +35,6 @@ cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, in
 
 // Prefill plans (mb_prefill.cu): one kernel launch per phase.
 struct PrefillState;
-struct Control;
 int prefill_validate(const mb_phase& phase, unsigned int n_slots, unsigned int n_dynamic);
 cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillState** out);
 int prefill_launch_count(const PrefillState* state);  // kernels one prefill_launch enqueues

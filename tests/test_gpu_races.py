@@ -13,6 +13,7 @@
   stays usable and the next plan runs.
 """
 
+import math
 import time
 
 import pytest
@@ -252,6 +253,69 @@ def test_hand_offs_through_the_workspace_give_the_same_results(name, batch, qkv_
         assert torch.equal(a, b)
     for a, b in zip(relayed[5], plain[5]):
         assert torch.equal(a, b)
+
+
+def test_weights_of_a_captured_launch_stay_its_own():
+    """Weights and caches given per launch are read through tensor maps made for that launch.  A captured
+    launch replays with its own, whatever later launches of the plan were given."""
+    from tests.test_gpu_bodies import _attention_case
+
+    rows, k, n, heads, kv_heads, dim, cached, capacity = 2, 256, 512, 4, 2, 64, 200, 220
+    x = _bf16(rows, k, seed=1)
+    weights = [_bf16(n, k, scale=k ** -0.5, seed=10 + i) for i in range(3)]
+    q, key, value, kc, vc, inv_freq, pos, length = (
+        t.cuda() for t in _attention_case(rows, heads, kv_heads, dim, cached, capacity))
+    caches = [(kc, vc), (kc.flip(1).contiguous(), vc.flip(1).contiguous()), (kc * 0.5, vc * 2)]
+    linear = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+    mixed = torch.zeros(rows, heads * dim, dtype=torch.bfloat16, device="cuda")
+    chunks = math.ceil(capacity / 16)
+    runner = PhaseRunner()
+    for name, tensor in (("w0", weights[0]), ("kc", kc), ("vc", vc)):
+        runner.slot(name, tensor)                       # slots 0 .. 2 come with the launch
+    gemv = _gemv_phase(runner, x=x, segs=[(weights[0], None, linear)], k=k, rows=rows)
+    attention = rt.Phase.blank(rt.BODY_ATTN_DECODE, 0)  # (the lengths stay: every launch sees the same keys)
+    for i, v in ((rt.AT_I_BATCH, rows), (rt.AT_I_HEADS, heads), (rt.AT_I_KV_HEADS, kv_heads),
+                 (rt.AT_I_HEAD_DIM, dim), (rt.AT_I_CAPACITY, capacity), (rt.AT_I_INVFREQ_BF16, 1),
+                 (rt.AT_I_MAX_CHUNKS, chunks), (rt.AT_I_MERGE_SLOTS, 8), (rt.AT_I_EXACT_KEYS, 128)):
+        attention.i[i] = v
+    attention.f[rt.AT_F_SCALE], attention.f[rt.AT_F_ROPE_SCALE] = dim ** -0.5, 1.0
+    for index, (name, tensor) in enumerate([
+        ("q", q), ("k", key), ("v", value), ("kc", kc), ("vc", vc), ("len", length), ("pos", pos),
+        ("invf", inv_freq), ("out", mixed),
+        ("partial", torch.zeros(rows * heads * chunks * (dim + 2), device="cuda")),
+        ("cnt", torch.zeros(8, dtype=torch.int32, device="cuda")),
+    ]):
+        attention.slot[index] = runner.slot(name, tensor)
+    scratch = max((rows + 1) * (k + 32) * 2, attention_scratch_bytes(dim, heads // kv_heads, 8))
+    plan = rt.Plan([gemv, attention], n_slots=len(runner.tensors), n_dynamic=3,
+                   activation_bytes=(scratch + 127) // 128 * 128, device=0)
+    plan.bind([t.data_ptr() for t in runner.tensors])
+
+    def launch(which):
+        plan.launch([weights[which].data_ptr(), *(t.data_ptr() for t in caches[which])],
+                    torch.cuda.current_stream().cuda_stream)
+
+    def results(run):
+        linear.zero_(), mixed.zero_()
+        run()
+        torch.cuda.synchronize()
+        assert plan.status().code == 0
+        return linear.clone(), mixed.clone()
+
+    alone = [results(lambda: launch(which)) for which in range(3)]
+    for which, (product, _) in enumerate(alone):
+        assert (product != _ref_linear(x, weights[which])).float().mean() < 0.02
+    assert not torch.equal(alone[0][1], alone[1][1])
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        launch(0)
+        launch(1)
+    for which in (2, 1, 0):
+        for a, b in zip(results(lambda: launch(which)), alone[which]):
+            assert torch.equal(a, b)
+        for a, b in zip(results(graph.replay), alone[1]):
+            assert torch.equal(a, b)
 
 
 def test_a_wait_that_runs_out_returns_a_status():
