@@ -72,6 +72,7 @@ struct SharedCtl {
     unsigned long long empty[kMaxStages];  // all consumer warps have read it
     unsigned long long entry_full;         // the next phase record has landed
     volatile unsigned int issued;          // stages the producer armed
+    volatile unsigned int fetched;         // phase records requested
     unsigned long long limit_ns;           // bound of every wait of this launch
     unsigned long long relay_now, relay_next;  // this launch's half of the arena, the other half
     volatile int abort_flag;
@@ -140,7 +141,8 @@ __device__ __forceinline__ unsigned long long resolve_address(unsigned long long
 // ---------------------------------------------------------------------------------------
 // Bounded waits.  A wait gives up when the launch's limit has run out (status
 // MB_ST_HANDOFF_TIMEOUT) or when this CTA or any other has recorded a fault; the caller goes on
-// with whatever it has and the CTA drains at the next barrier all its threads meet at.
+// with whatever it has, without waiting any more, and the CTA leaves before the next phase or the one
+// after that (next_entry).
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ bool wait_gave_up(int ph, unsigned long long start) {
     SharedCtl* sc = ctl_of();
@@ -475,13 +477,16 @@ __device__ __noinline__ void producer_loop() {
         }
     }
 }
-// After a fault: never leave while one of this CTA's tensor copies is still in flight.  One thread.
+// After a fault: never leave while one of this CTA's copies is still in flight.  One thread.
 __device__ __noinline__ void drain_ring() {
     SharedCtl* sc = ctl_of();
     const unsigned int stages = sc->stages, issued = sc->issued;
     for (unsigned int i = issued > stages ? issued - stages : 0u; i < issued; ++i)
         for (unsigned int tries = 0; tries < kDrainTryLimit; ++tries)
             if (mbar_try_wait(&sc->full[i % stages], (i / stages) & 1u)) break;
+    const unsigned int records = sc->fetched;
+    for (unsigned int tries = 0; records > 0 && tries < kDrainTryLimit; ++tries)
+        if (mbar_try_wait(&sc->entry_full, (records - 1) & 1u)) break;
 }
 
 __device__ __forceinline__ uint4 lds128(unsigned int addr) {
@@ -1557,6 +1562,7 @@ __device__ __forceinline__ bool begin_launch(const KernelParams& p, const Stream
         }
         mbar_init(&sc->entry_full, 1);
         sc->issued = 0;
+        sc->fetched = 0;
         mbar_init_fence();
         sc->abort_flag = peek_status(p.ctl) != 0 ? 1 : 0;  // a faulted plan runs nothing
         sc->limit_ns = static_cast<unsigned long long>(p.wait_limit_us) * 1000ull;
@@ -1618,28 +1624,38 @@ __device__ __forceinline__ uint4 resolve_vector(uint4 v, int index) {
 
 // Phase entries: at the start of phase ph warp 0 resolves the addresses of record ph + 1, which
 // the barrier inside the phase publishes, and fetches record ph + 2 over that of ph - 2 (no
-// warp can still be there: all have passed the barrier of ph - 1).
+// warp can still be there: all have passed the barrier of ph - 1).  Once a fault is on record in this
+// CTA it ends the walk at ph + 1 instead, through the kind of that phase, which the same barrier
+// publishes: every warp leaves there, and nobody looks at a record whose copy has not landed.
 __device__ __noinline__ void fetch_entry(int ph) {
     SharedCtl* sc = ctl_of();
     if (ph < sc->n_phases && (threadIdx.x & 31) == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive_expect_tx(&sc->entry_full, sizeof(PhaseEntry));
         bulk_copy_g2s(&sc->entry[ph & 3], sc->entries + ph, sizeof(PhaseEntry), &sc->entry_full);
+        sc->fetched = ph + 1;
     }
 }
-__device__ __noinline__ void place_entry(int ph) {
+__device__ __noinline__ void next_entry(int ph) {
     SharedCtl* sc = ctl_of();
     const int lane = threadIdx.x & 31;
     if (ph >= sc->n_phases) return;
-    if (!mbar_wait_bounded(&sc->entry_full, ph & 1, &sc->abort_flag, sc->limit_ns)) {
-        if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
-        sc->abort_flag = 1;
+    const bool landed = mbar_wait_bounded(&sc->entry_full, ph & 1, &sc->abort_flag, sc->limit_ns);
+    if (__any_sync(0xffffffffu, !landed || sc->abort_flag != 0)) {
+        if (lane == 0) {
+            if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+            sc->abort_flag = 1;
+            table_of()[ph].kind = kStreamStop;
+        }
+        __syncwarp();
+        return;
     }
     if (lane < kEntryVectors) {
         uint4* v = reinterpret_cast<uint4*>(&sc->entry[ph & 3]) + lane;
         *v = resolve_vector(*v, lane);
     }
     __syncwarp();
+    fetch_entry(ph + 1);
 }
 
 // The consumer warps' walk through the phase table.
@@ -1651,8 +1667,7 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
     Place place{0u, 0u, 0u};
     if (warp == 0) {
         fetch_entry(0);
-        place_entry(0);
-        fetch_entry(1);
+        next_entry(0);
     }
     // the other half of the arena becomes blank for the next launch
     for (unsigned long long at = (static_cast<unsigned long long>(blockIdx.x) * kThreads + tid) * 16;
@@ -1667,13 +1682,11 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
     // when the first activations are ready (1), after the body (2) and after the closing grid
     // barrier, if the phase has one (3).
     for (int ph = 0; ph < p.n_phases; ++ph) {
-        if (warp == 0) {
-            place_entry(ph + 1);
-            fetch_entry(ph + 2);
-        }
+        const int kind = table[ph].kind;
+        if (kind == kStreamStop) break;
+        if (warp == 0) next_entry(ph + 1);
         const PhaseEntry* E = &sc->entry[ph & 3];
         trace_stamp(ph, 0);
-        const int kind = table[ph].kind;
         bool meet = true;  // the phase has not had a barrier of all threads
         if (kind == kStreamGemv) {
             const GemvStream& d = table[ph].gemv;
@@ -1702,8 +1715,9 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
         }
         if (flags & MB_FLAG_BARRIER) {
             ++barrier_index;
-            grid_barrier(p.ctl, barriers + barrier_index, kBarAll, kThreads, tid, &sc->abort_flag,
-                         &sc->verdict, ph, sc->limit_ns);
+            if (!grid_barrier(p.ctl, barriers + barrier_index, kBarAll, kThreads, tid, &sc->abort_flag,
+                              &sc->verdict, ph, sc->limit_ns))
+                break;  // the same for all threads
             trace_stamp(ph, 3);
         }
     }

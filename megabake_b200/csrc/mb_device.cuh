@@ -71,7 +71,8 @@ constexpr unsigned int kUnwritten = 0xffffffffu;
 // What a warp needs to stream a phase's global operands ahead of time, one record per phase.
 // The host fills the static part; every CTA completes its copy in shared memory at the start of
 // a launch (its rows; the valid lengths and how the keys are dealt over the CTAs).
-enum StreamKind { kStreamNone = 0, kStreamGemv = 1, kStreamKv = 2 };
+enum StreamKind { kStreamNone = 0, kStreamGemv = 1, kStreamKv = 2,
+                  kStreamStop = 3 };  // set by a CTA that has seen a fault: it goes no further
 struct GemvStream {
     int kind;
     int row_bytes;

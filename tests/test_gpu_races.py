@@ -349,6 +349,38 @@ def test_a_wait_that_runs_out_returns_a_status():
     assert (out != ref).float().mean() < 0.05
 
 
+def test_a_fault_ends_the_walk_through_the_phases():
+    """Every CTA's wait in phase 1 runs out; it leaves the launch at the end of phase 2 at the latest, so
+    the phases behind never run and their outputs stay as they were.  Then the plan runs again."""
+    rows, k, n = 2, 256, 512
+    x_cells = torch.zeros(rows * k // 2, dtype=torch.int64, device="cuda")
+    x, w = _bf16(rows, k, seed=1), _bf16(n, k, scale=0.05, seed=2)
+    runner = PhaseRunner()
+    waits = _gemv_phase(runner, x=x_cells, segs=[(w, None, torch.zeros(rows, n, dtype=torch.bfloat16,
+                                                                       device="cuda"))], k=k, rows=rows)
+    waits.i[rt.GV_I_CELLS], waits.i[rt.GV_I_X_SOURCE] = rt.CELLS_X, 0
+    phases, outputs = [rt.Phase.blank(rt.BODY_NOP, 0), waits], []
+    for _ in range(6):
+        runner.names = {}
+        outputs.append(torch.full((rows, n), 7.0, dtype=torch.bfloat16, device="cuda"))
+        phases.append(_gemv_phase(runner, x=x, segs=[(w, None, outputs[-1])], k=k, rows=rows))
+    phases[4].flags |= rt.FLAG_BARRIER
+    plan = runner.run(phases, rows * (k + 32) * 2, wait_limit_ms=40)
+    status = plan.status()
+    assert status.code == 7 and status.phase == 1 and status.calls == 0
+    for out in outputs[1:]:
+        assert bool((out == 7.0).all())
+    plan.reset()
+    # the same records with the wait satisfied: cells of the epoch after the reset
+    tag = 1 * len(phases) + 0 + 1
+    x_cells.copy_((x.view(torch.int32).to(torch.int64).flatten() & 0xFFFFFFFF) | (tag << 32))
+    plan.launch([], torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert plan.status().code == 0
+    for out in outputs:
+        assert (out != _ref_linear(x, w)).float().mean() < 0.05
+
+
 def test_a_faulted_launch_leaves_the_state_alone():
     """A token outside the embedding table is recorded in phase 0.  Waits that are still spinning
     see the status and drain; CTAs that get through reach the end of the launch, where the valid
