@@ -216,6 +216,9 @@ __device__ __forceinline__ bool unwritten(uint4 v) {
     return v.x == kUnwritten || v.y == kUnwritten || v.z == kUnwritten || v.w == kUnwritten;
 }
 
+// A pair of values as the arena may hold it: two NaNs that look like the blank pattern become two others.
+__device__ __forceinline__ unsigned int as_written(unsigned int v) { return v == kUnwritten ? 0x7fff7fffu : v; }
+
 // Eight values from four cells.
 __device__ __noinline__ uint4 cells_load(const char* src, unsigned int tag, int ph) {
     unsigned int v[4];
@@ -739,6 +742,8 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
                 v = scale_vector(v, scale);
                 sts128(out + i * 512, v);
             }
+            if (E->modes & kModeStoreRelay)  // rows of the table as they are: the one thing not converted
+                v = make_uint4(as_written(v.x), as_written(v.y), as_written(v.z), as_written(v.w));
             if (mine && g < d.groups) {
                 const size_t e = static_cast<size_t>(row) * (d.row_bytes / 2) + g * 32 + 8 * tq;
                 store_result(keep, e, v.x, as_cells, tag);

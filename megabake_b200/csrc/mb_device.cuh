@@ -65,7 +65,8 @@ constexpr unsigned long long kModeInRelay = 1, kModeResidualRelay = 2, kModeOutR
 // GEMV: activations or residual are plain memory of a phase before, guarded by its counter alone
 constexpr unsigned long long kModeWait = 16;
 // Every 32-bit word of the relay arena that has not been written in this launch holds this
-// pattern.  Conversions to bf16 never produce it: a NaN becomes 0x7fff.
+// pattern.  Conversions to bf16 never produce it: a NaN becomes 0x7fff.  (Gathered embedding rows are not
+// converted; as_written keeps the pattern out.)
 constexpr unsigned int kUnwritten = 0xffffffffu;
 
 // What a warp needs to stream a phase's global operands ahead of time, one record per phase.

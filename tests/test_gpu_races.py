@@ -381,6 +381,26 @@ def test_a_fault_ends_the_walk_through_the_phases():
         assert (out != _ref_linear(x, w)).float().mean() < 0.05
 
 
+def test_an_embedding_row_of_all_ones():
+    """bf16 0xffff is a NaN, and a pair of them the pattern of a word nobody has written yet: such a row
+    gives NaN logits for its batch row, no fault, and leaves the other row alone."""
+    spec, decoder, args, ids, pos, state = _decoder("tiny-llama", 2, 8, PlannerOptions())
+    table = next(a for a in args if isinstance(a, torch.Tensor) and a.shape == (spec.vocab, spec.hidden))
+    ids.copy_(torch.tensor([[3], [5]]))
+    clean = decoder(*args).clone()
+    decoder.check()
+    table[5].view(torch.int16).fill_(-1)
+    for layer in range(spec.layers):
+        state[3 * layer + 2].zero_()
+    got = decoder(*args)
+    decoder.check()
+    assert bool(got[1].isnan().all())
+    changed = torch.tensor([5])                  # the table is the LM head too: only logit 5 of row 0
+    keep = torch.ones(spec.vocab, dtype=torch.bool)
+    keep[changed] = False
+    assert torch.equal(got[0, 0].cpu()[keep], clean[0, 0].cpu()[keep])
+
+
 def test_a_faulted_launch_leaves_the_state_alone():
     """A token outside the embedding table is recorded in phase 0.  Waits that are still spinning
     see the status and drain; CTAs that get through reach the end of the launch, where the valid
