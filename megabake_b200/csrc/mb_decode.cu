@@ -2139,14 +2139,14 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     const int group = a->heads / a->kv_heads;
     const int pairs = a->batch * a->kv_heads;
     // What fits the fixed array: arrival counters for every (row, kv head) and at least one
-    // key chunk of partials each; more chunks if there is room, up to 32.
+    // part of partials each; more parts if there is room, up to 32.
     if (static_cast<size_t>(pairs) * 4 > kStaticCounterBytes) return MB_ERR_RESOURCE;
     const size_t per_chunk = static_cast<size_t>(pairs) * group * (a->head_dim + 2) * 4;
     const size_t room = kStaticScratchBytes - kStaticControlBytes - kStaticCounterBytes;
     if (per_chunk > room) return MB_ERR_RESOURCE;  // shapes beyond the 4 MiB scratch
-    int max_chunks = static_cast<int>(room / per_chunk);
-    if (max_chunks > 32) max_chunks = 32;
-    const int by_capacity = (a->capacity + 15) / 16;
+    int max_chunks = static_cast<int>(room / per_chunk);  // two for every part: cells take twice the room
+    if (max_chunks > 64) max_chunks = 64;
+    const int by_capacity = 2 * ((a->capacity + 15) / 16);
     if (max_chunks > by_capacity) max_chunks = by_capacity;
 
     mb::PhaseEntry entry;

@@ -40,7 +40,7 @@ def _inputs(batch, heads, kv_heads, dim, cached, capacity, seed):
 def _static_max_chunks(batch, heads, kv_heads, dim, capacity):
     per_chunk = batch * heads * (dim + 2) * 4
     room = STATIC_SCRATCH_BYTES - STATIC_RESERVED_BYTES
-    return max(1, min(32, room // per_chunk, math.ceil(capacity / 16)))
+    return max(1, min(64, room // per_chunk, 2 * math.ceil(capacity / 16)))
 
 
 def _plan_step(tensors, batch, heads, kv_heads, dim, capacity):
@@ -105,6 +105,7 @@ def _oracle_step(tensors, batch, heads, kv_heads, dim):
     (2, 14, 2, 64, 700),     # split keys: partials and arrival counters in the static array
     (1, 32, 8, 64, 40),      # short context: exact softmax, no partials
     (2, 4, 2, 128, 2500),
+    (1, 8, 1, 128, 20000),   # one kv head: as many parts as there are, 32
     (1, 8, 1, 256, 300),     # 256-wide heads, eight query heads on one kv head
     (2, 4, 2, 64, 126),      # the two calls cross from the exact softmax (<= 128 keys) ...
     (2, 4, 2, 64, 127),      # ... to the split one
