@@ -1632,7 +1632,7 @@ __device__ __forceinline__ uint4 resolve_vector(uint4 v, int index) {
 // warp can still be there: all have passed the barrier of ph - 1).  Once a fault is on record in this
 // CTA it ends the walk at ph + 1 instead, through the kind of that phase, which the same barrier
 // publishes: every warp leaves there, and nobody looks at a record whose copy has not landed.
-__device__ __noinline__ void fetch_entry(int ph) {
+__device__ __forceinline__ void fetch_entry(int ph) {
     SharedCtl* sc = ctl_of();
     if (ph < sc->n_phases && (threadIdx.x & 31) == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
