@@ -18,7 +18,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("k,mid,n", [
     (64, 32, 2),            # less than a stage of either shape, one pair of rows in all
     (576, 1536, 576),       # blocks of eight rows
-    (896, 4864, 896),       # a slice that needs two chunks from three rows on
+    (896, 4864, 896),       # 20 slots of a slice from five rows on: the wide slices
+    (896, 6016, 896),       # more than a wide slice from five rows on: two chunks
     (2048, 8192, 2560),     # blocks of sixteen rows, several per CTA
 ])
 def test_results_handed_over_inside_the_launch(rows, k, mid, n):

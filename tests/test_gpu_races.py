@@ -1,13 +1,14 @@
 """Race, reuse and wait-limit evidence that needs no sanitizer.
 
-* Poisoned workspace: every byte of the plan's workspace that is not declared "starts at zero",
-  and the logits buffer, are filled with 0xE5 before a launch; the results must not change (the
-  reference poisons its workspace the same way, ``src/megabake/compiler.py:1972-1973``,
-  ``tests/gpu/test_task29_transformer_block.py:116-124``).
+* Poisoned workspace: every byte of the plan's workspace and the logits buffer are filled with 0xE5
+  before a launch; the results must not change (the reference poisons its workspace the same way,
+  ``src/megabake/compiler.py:1972-1973``, ``tests/gpu/test_task29_transformer_block.py:116-124``).
+  Short contexts, and contexts that are cut over several CTAs.
 * Distinct buffers: the same model planned with activation buffers of its own for every layer
   against the normal plan that reuses one set: bit-identical logits and KV state (reference
   ``src/megabake/compiler.py:227-241``).  A phase that read a buffer too early or wrote it too
-  late shows up as a difference.
+  late shows up as a difference.  (In plans that hand over through the workspace; in the relay arena
+  no place is used twice in a launch.)
 * Wait limit: a consumer whose producer never stores (a flag nothing sets) gives up after the
   plan's limit, the kernel RETURNS ``MB_ST_HANDOFF_TIMEOUT`` through the status word, the context
   stays usable and the next plan runs.
@@ -41,11 +42,20 @@ def _decoder(name, batch, capacity, options, seed=3):
     return spec, BoundDecoder(layout, args), args, ids, pos, state
 
 
-def _run_steps(decoder, args, ids, pos, tokens, poison=None):
+def _fill_caches(spec, state, cached, seed=9):
+    """``cached`` random keys and values in every row."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    for layer in range(spec.layers):
+        for cache in state[3 * layer: 3 * layer + 2]:
+            cache[:, :cached].normal_(0.0, 0.3, generator=g)
+        state[3 * layer + 2].fill_(cached)
+
+
+def _run_steps(decoder, args, ids, pos, tokens, poison=None, first=0):
     outputs = []
     for step in range(tokens.shape[1]):
         ids.copy_(tokens[:, step:step + 1])
-        pos.fill_(step)
+        pos.fill_(first + step)
         if poison is not None:
             poison(decoder)
         logits = torch.empty(decoder.program.batch, 1, decoder.program.vocab, dtype=torch.bfloat16,
@@ -58,39 +68,47 @@ def _run_steps(decoder, args, ids, pos, tokens, poison=None):
     return outputs
 
 
-@pytest.mark.parametrize("name,batch,cell_limit", [
-    ("tiny-llama", 3, 0), ("tiny-qwen2", 8, 0), ("tiny-gemma", 2, 0), ("tiny-qwen2", 4, 1 << 20),
+# Hand-offs through the relay arena (the default), through plain tensors behind counters with q, k and
+# v as cells or plain too, and everything as cells: only the last three work in the workspace.
+HAND_OFFS = {
+    "relay": {},
+    "plain": {"relay": False},
+    "all-plain": {"relay": False, "qkv_cells": False},
+    "cells": {"relay": False, "cell_limit": 1 << 20},
+}
+
+
+@pytest.mark.parametrize("hand_offs", HAND_OFFS)
+@pytest.mark.parametrize("name,batch,cached", [
+    ("tiny-llama", 3, 0), ("tiny-qwen2", 8, 0), ("tiny-gemma", 2, 0), ("tiny-qwen2", 4, 300),
 ])
-def test_poisoned_workspace_changes_nothing(name, batch, cell_limit):
-    options = PlannerOptions(cell_limit=cell_limit)
-    spec, clean, args, ids, pos, state = _decoder(name, batch, 16, options)
+def test_poisoned_workspace_changes_nothing(name, batch, cached, hand_offs):
+    options = PlannerOptions(**HAND_OFFS[hand_offs])
+    spec, clean, args, ids, pos, state = _decoder(name, batch, cached + 16, options)
     tokens = torch.randint(0, spec.vocab, (batch, 5), generator=torch.Generator().manual_seed(2)).cuda()
-    expected = _run_steps(clean, args, ids, pos, tokens)
+    _fill_caches(spec, state, cached)
+    expected = _run_steps(clean, args, ids, pos, tokens, first=cached)
     expected_state = [t.clone() for t in state]
-    spec, dirty, args, ids, pos, state = _decoder(name, batch, 16, options)
-    keep = dirty.layout.zero_ranges  # only the attention arrival counters must start at zero ...
-    counters = [s for s in dirty.layout.slots if s.name == "attention_arrivals"]
-    assert len(counters) == 1
+    spec, dirty, args, ids, pos, state = _decoder(name, batch, cached + 16, options)
+    _fill_caches(spec, state, cached)
+    # cells and partials start zeroed; later on their sequence numbers decide, so poison is harmless
+    assert dirty.layout.zero_ranges
 
-    def poison(decoder):
-        saved = decoder.workspace[counters[0].offset: counters[0].offset + 256].clone()
-        decoder.workspace.fill_(0xE5)
-        decoder.workspace[counters[0].offset: counters[0].offset + 256] = saved
-
-    got = _run_steps(dirty, args, ids, pos, tokens, poison=poison)
+    got = _run_steps(dirty, args, ids, pos, tokens, first=cached,
+                     poison=lambda decoder: decoder.workspace.fill_(0xE5))
     for a, b in zip(expected, got):
         assert torch.equal(a, b)
     for a, b in zip(expected_state, state):
         assert torch.equal(a, b)
-    assert keep  # (the cell buffers are zeroed at creation too; poisoning them later is harmless)
 
 
-@pytest.mark.parametrize("name,batch,cell_limit", [
-    ("tiny-llama", 2, 0), ("tiny-qwen2", 8, 0), ("tiny-mha", 4, 1 << 20),
+@pytest.mark.parametrize("name,batch,hand_offs", [
+    ("tiny-llama", 2, "plain"), ("tiny-qwen2", 8, "all-plain"), ("tiny-mha", 4, "cells"),
+    ("tiny-qwen2", 8, "relay"),
 ])
-def test_distinct_buffers_give_identical_results(name, batch, cell_limit):
-    shared = _decoder(name, batch, 16, PlannerOptions(cell_limit=cell_limit))
-    own = _decoder(name, batch, 16, PlannerOptions(cell_limit=cell_limit, distinct_buffers=True))
+def test_distinct_buffers_give_identical_results(name, batch, hand_offs):
+    shared = _decoder(name, batch, 16, PlannerOptions(**HAND_OFFS[hand_offs]))
+    own = _decoder(name, batch, 16, PlannerOptions(**HAND_OFFS[hand_offs], distinct_buffers=True))
     assert own[1].layout.workspace_bytes > shared[1].layout.workspace_bytes
     spec = shared[0]
     tokens = torch.randint(0, spec.vocab, (batch, 6), generator=torch.Generator().manual_seed(4)).cuda()
@@ -105,11 +123,8 @@ def test_distinct_buffers_give_identical_results(name, batch, cell_limit):
 def _split_context(decoder_parts, seed):
     """Puts 300 cached keys into the state: contexts that are cut over several CTAs."""
     spec, decoder, args, ids, pos, state = decoder_parts
-    g = torch.Generator(device="cuda").manual_seed(seed)
-    for layer in range(spec.layers):
-        for cache in state[3 * layer: 3 * layer + 2]:
-            cache[:, :300].normal_(0.0, 0.3, generator=g)
-        state[3 * layer + 2].fill_(300)
+    _fill_caches(spec, state, 300, seed)
+    g = torch.Generator(device="cuda").manual_seed(seed + 1)
     tokens = torch.randint(0, spec.vocab, (decoder.program.batch, 3), generator=g, device="cuda")
     outputs = []
     for step in range(3):
