@@ -5,8 +5,9 @@
  * table of fixed-size phase records plus a table of device addresses ("slots") and hands
  * both to this library.  One call of mb_plan_launch() is one cooperative persistent
  * kernel launch that executes every phase in order.  Phases hand their activations to one
- * another either through flagged cells (below) that the consumers poll -- no barrier at all --
- * or, where a record asks for one, across a grid barrier.
+ * another through memory of the plan's own (MB_FLAG_RELAY) or flagged cells (below) that the consumers
+ * poll -- no barrier at all --, through plain tensors behind a counter (MB_CELLS_X_WAIT) or,
+ * where a record asks for one, across a grid barrier.
  *
  * Flagged cells.  An activation tensor [rows, N] of bf16 that one phase produces and a later
  * phase of the same launch consumes can be kept as [rows, N / 2] 64-bit cells: two bf16 values
@@ -43,7 +44,8 @@
  * plans are independent.  No function synchronises the device except mb_plan_create,
  * mb_plan_bind, mb_plan_status, mb_plan_reset and mb_plan_destroy.  mb_plan_launch
  * performs no allocation and no host synchronisation and always passes the same kernel
- * parameters for the same dynamic addresses, so it can be captured in a CUDA graph.
+ * parameters for the same dynamic addresses, so it can be captured in a CUDA graph.  (Weights and
+ * caches in per-launch slots cost one small launch per phase that reads them.)
  */
 #ifndef MEGABAKE_B200_H
 #define MEGABAKE_B200_H
@@ -77,7 +79,7 @@ enum mb_status_code {
     MB_ST_TOKEN_RANGE = 4,     /* an input id outside [0, vocab)                         */
     MB_ST_BAD_PHASE = 5,       /* unknown body id in the phase table                     */
     MB_ST_TMEM = 6,            /* tensor-memory allocation failed                        */
-    MB_ST_HANDOFF_TIMEOUT = 7  /* a flagged cell never showed the expected sequence number */
+    MB_ST_HANDOFF_TIMEOUT = 7  /* an activation of an earlier phase never arrived          */
 };
 
 typedef struct mb_status {
@@ -99,7 +101,8 @@ enum mb_body {
      * matrices are paired (gate|up) for a gated-activation epilogue.                      */
     MB_BODY_GEMV = 1,
     /* One-token attention over the KV cache: RoPE of q and the new k, append of k/v at
-     * valid_length, split-key flash decoding with an online softmax, last-arriver merge.  */
+     * valid_length, split-key flash decoding with an online softmax; every part of a context
+     * folds its share of the outputs.                                                     */
     MB_BODY_ATTN_DECODE = 2,
     /* ---- prefill bodies ---- */
     MB_BODY_EMBED_ROWS = 3,   /* gather embedding rows (+ scalar scale)                    */
@@ -177,10 +180,10 @@ typedef struct mb_phase {
 #define MB_GV_I_NMAT 6     /* 1, or 2 for a paired gate/up phase (then NSEG == 1)         */
 #define MB_GV_I_PROLOGUE 7
 #define MB_GV_I_EPILOGUE 8
-#define MB_GV_I_ROW_TILE 9 /* output rows per pipeline stage: 8 (always for a paired phase)
-                              or 16 (two 8-row tiles per stage: rows of at most 1,024
-                              elements, so that a stage still carries ~30 KB)              */
-#define MB_GV_I_K_CHUNK 10 /* reduction elements per pipeline stage, multiple of 16       */
+#define MB_GV_I_ROW_TILE 9 /* 8 (always for a paired phase) or 16; with K_CHUNK checked by
+                              mb_plan_create against stage_bytes, without effect on the
+                              decode kernel, whose stages are 16 KB of a shape of its own  */
+#define MB_GV_I_K_CHUNK 10 /* multiple of 32, at most K                                   */
 #define MB_GV_I_GATHER 11  /* 1: activation rows are gathered from an embedding table     */
 #define MB_GV_I_VOCAB 12   /* rows of that table (range check)                            */
 #define MB_GV_I_STORE_X 13 /* 1: CTA 0 also stores the un-normalised rows at S_XSTORE     */
@@ -210,8 +213,9 @@ typedef struct mb_phase {
 #define MB_AT_I_HEAD_DIM 3   /* 64, 128 or 256                                            */
 #define MB_AT_I_CAPACITY 4
 #define MB_AT_I_INVFREQ_BF16 5 /* 1 if the inv_freq buffer is bf16, 0 if fp32             */
-#define MB_AT_I_MAX_CHUNKS 6 /* key chunks per (batch, kv head) the workspace is sized for */
-#define MB_AT_I_MERGE_SLOTS 7 /* per-warp states that fit the shared scratch at once      */
+#define MB_AT_I_MAX_CHUNKS 6 /* size of MB_AT_S_PARTIAL, 1..64: a context is cut into at most half
+                                as many parts                                             */
+#define MB_AT_I_MERGE_SLOTS 7 /* 1..8; part of the admission check, without effect        */
 #define MB_AT_I_EXACT_KEYS 8 /* contexts up to this many keys (<= 128, 0 = never) use the
                                 softmax that rounds normalised probabilities to bf16
                                 like the eager operator                                */
@@ -237,7 +241,7 @@ typedef struct mb_phase {
                                 number), [B*Hkv, max_chunks / 2, Hq/Hkv, D+2].  mb_plan_bind clears
                                 it when its address is new to the phase; given per launch
                                 instead, it must be zero before its first launch           */
-#define MB_AT_S_COUNTER 10   /* int32 [B*Hkv], zero before the first launch                */
+#define MB_AT_S_COUNTER 10   /* int32 [B*Hkv]; has to be given, is not touched               */
 
 /* ---- prefill bodies (MB_MODE_PREFILL plans: one kernel launch per phase, in order) ----- */
 /* MB_BODY_EMBED_ROWS: out[r, :] = table[ids[r], :] (x scale, rounded to bf16)              */
@@ -310,17 +314,18 @@ typedef struct mb_plan_desc {
     uint32_t abi_version;     /* MB_ABI_VERSION                                           */
     int32_t device;           /* CUDA device ordinal                                      */
     int32_t mode;             /* enum mb_mode                                             */
-    uint32_t n_phases;
+    uint32_t n_phases;        /* decode: each takes 96 B of shared memory, MB_ERR_RESOURCE from
+                                 about 950 on                                             */
     const mb_phase* phases;
     uint32_t n_slots;         /* size of the address table                                */
     uint32_t n_dynamic;       /* slots [0, n_dynamic) are given per launch, <= 8          */
-    uint32_t activation_bytes;/* shared memory for activations / attention scratch        */
+    uint32_t activation_bytes;/* what the records' activations and scratch are checked against;
+                                 the kernels size their shared memory themselves          */
     uint32_t ctas;            /* 0 = one per SM                                           */
-    uint32_t stage_bytes;     /* decode: bytes of one weight-ring stage, a multiple of 1024 up
-                                 to mb_stage_bytes(); 0 = mb_stage_bytes().  Small stages give
-                                 a deeper ring when the reduction length is short            */
-    uint32_t wait_limit_ms;   /* bound of every device-side wait (hand-off cells, pipeline
-                                 stages, grid barrier) in milliseconds; 0 = 2000.  When a wait
+    uint32_t stage_bytes;     /* decode: what ROW_TILE and K_CHUNK are checked against, a multiple
+                                 of 1024 up to mb_stage_bytes(); 0 = mb_stage_bytes()      */
+    uint32_t wait_limit_ms;   /* bound of every device-side wait (hand-offs, grid barrier; twice it
+                                 for pipeline stages) in milliseconds; 0 = 2000.  When a wait
                                  runs out the kernel records a status, drains and returns   */
     uint32_t reserved[2];
 } mb_plan_desc;
@@ -330,7 +335,7 @@ typedef struct mb_plan_info {
     int32_t threads;          /* threads per CTA                                          */
     int32_t smem_bytes;       /* dynamic shared memory per CTA                            */
     int32_t stages;           /* weight-ring stages                                       */
-    int32_t barriers;         /* grid barriers per launch                                 */
+    int32_t barriers;         /* grid barriers per launch (records with MB_FLAG_BARRIER)   */
     int32_t sm_count;
     int32_t launches;         /* kernel launches one mb_plan_launch enqueues              */
     int32_t reserved[1];
@@ -359,7 +364,7 @@ void mb_plan_destroy(mb_plan* plan);
  * at start-up, a region where cudaMalloc would synchronise the device): the same decode
  * attention as MB_BODY_ATTN_DECODE -- RoPE of q and the new k, append at valid_length,
  * valid_length += 1, attention over every valid key -- with its scratch (split-key partials,
- * arrival counters, status) in a fixed 4 MiB array inside the library's device image instead
+ * status) in a fixed 4 MiB array inside the library's device image instead
  * of allocated memory.  It calls no cudaMalloc/cudaFree or allocating library routine.
  *
  * Limits: batch * kv_heads <= 1024 and batch * heads * (head_dim + 2) * 4 B must fit the array

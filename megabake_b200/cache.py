@@ -23,7 +23,9 @@ per model shape and device, after the reference's ``bodies/cuda/sm100/tuning.py:
      "choices": {"896:4864:151936:8": {"stage_bytes": 30720, "max_chunks": 32}}}
 
 The key is ``hidden:intermediate:vocab:batch``; a choice may set ``stage_bytes``, ``max_chunks``,
-``merge_slots`` and ``cell_limit``.  A file whose fingerprint does not match the device is an
+``merge_slots`` and ``cell_limit``.  (A context is cut into at most half of ``max_chunks`` parts;
+``stage_bytes`` and ``merge_slots`` only change what a plan is checked against; a ``cell_limit``
+plans without the relay arena.)  A file whose fingerprint does not match the device is an
 error, as in the reference.
 """
 

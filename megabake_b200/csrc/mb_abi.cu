@@ -92,7 +92,8 @@ struct mb_plan {
 
 namespace {
 
-// Shared-memory scratch the decode attention body carves from the activation region.
+// What activation_bytes is checked against for an attention phase.  (The kernel's own scratch does not
+// depend on it; the check stays as callers know it.)
 long long attention_scratch_bytes(int head_dim, int group, int merge_slots) {
     const long long qs = 8LL * (head_dim + 32) * 2;
     const long long new_rows = 2LL * head_dim * 2;
@@ -418,7 +419,7 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
         desc->stage_bytes > static_cast<unsigned int>(mb::decode_stage_bytes()))
         return MB_ERR_INVALID;
 
-    int barriers = 1;  // the last arrival closes the launch
+    int barriers = 1;  // one more than the records ask for: the end of the launch
     for (unsigned int i = 0; i < desc->n_phases; ++i) {
         const mb_phase& P = desc->phases[i];
         int rc = MB_OK;
@@ -522,7 +523,7 @@ int mb_plan_query(const mb_plan* plan, mb_plan_info* out) {
     out->threads = plan->threads;
     out->smem_bytes = plan->smem_bytes;
     out->stages = plan->stages;
-    out->barriers = plan->barriers;
+    out->barriers = plan->mode == MB_MODE_PREFILL ? 0 : plan->barriers - 1;
     out->sm_count = plan->sm_count;
     out->launches = plan->mode == MB_MODE_PREFILL ? mb::prefill_launch_count(plan->prefill)
                                                   : 1 + static_cast<int>(plan->late_maps.size());

@@ -18,8 +18,8 @@
 // the activations it needs, in fragment layout, until they are there.  Data and "ready" are one L2
 // round trip; there is no fence and no grid barrier.  (Records may also ask for plain
 // tensors behind a counter, flagged cells, or a grid barrier.)  A warp multiplies a slice of the
-// reduction for all rows of the CTA, keeps its activations in registers, and the slices are added
-// in shared memory in a fixed order.
+// reduction for all rows of the CTA, with its slice of the activations in shared memory of its own,
+// and the slices' products are added in shared memory in a fixed order.
 //
 // Replaces, for decode, the reference's generated persistent kernel
 // (src/megabake/codegen.py:1634-1703), its sm100 swapAB GEMM bodies
@@ -2014,7 +2014,7 @@ cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, in
 // runs inside a fixed amount of memory handed out at start-up, a caller inside a region where
 // cudaMalloc would synchronise the device.  For them this entry point runs the same
 // attention body as the plan path, but everything the plan path keeps in allocated memory
-// (phase table, control block, split-key partials, arrival counters) lives either in the
+// (phase table, control block, split-key partials) lives either in the
 // kernel parameters or in one fixed-size array inside this library's device image.
 //
 // The array is a file-scope `static __device__` object of kStaticScratchBytes (4 MiB); every
@@ -2022,10 +2022,10 @@ cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, in
 // a host-side stand-in, not a device address: the address the kernel gets is asked for once
 // per device with cudaGetSymbolAddress, with that device current.
 //
-// All calls share the array.  The arrival counters and the control words are cleared on the
-// stream before every launch; the partials need no clearing (they are written before they
-// are read).  Two calls that overlap on the GPU (different streams, no dependency) race on
-// it -- callers serialise them.
+// All calls share the array.  The control words are cleared on the stream before every launch.  The
+// partials need no clearing: they are cells tagged with the call's number, which is kept outside the
+// cleared part and never repeats.  Two calls that overlap on the GPU (different streams, no
+// dependency) race on the array -- callers serialise them.
 // =======================================================================================
 namespace mb {
 namespace decode {
@@ -2035,7 +2035,8 @@ constexpr size_t kStaticControlBytes = 256;        // the head of a Control: sta
 // The attention body and the end of the launch only touch the words before the finished-phase
 // counters through the pointer they are given.
 static_assert(offsetof(Control, finished) <= kStaticControlBytes, "the static control area is too small");
-constexpr size_t kStaticCounterBytes = 4096;       // arrival counters: up to 1024 (row, kv head)
+constexpr size_t kStaticCounterBytes = 4096;       // a word for each of up to 1024 (row, kv head): unused,
+                                                   // but part of the size limits callers know
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 // Tags the partials of a call; outside the area that is cleared before every call, so that no
 // partial of an earlier call can be mistaken for one of this call.
@@ -2138,7 +2139,7 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
 
     const int group = a->heads / a->kv_heads;
     const int pairs = a->batch * a->kv_heads;
-    // What fits the fixed array: arrival counters for every (row, kv head) and at least one
+    // What fits the fixed array: a word for every (row, kv head) and at least one
     // part of partials each; more parts if there is room, up to 32.
     if (static_cast<size_t>(pairs) * 4 > kStaticCounterBytes) return MB_ERR_RESOURCE;
     const size_t per_chunk = static_cast<size_t>(pairs) * group * (a->head_dim + 2) * 4;
@@ -2181,8 +2182,7 @@ extern "C" int mb_attention_decode_static(const mb_attention_args* a, void* stre
     entry.addr[MB_AT_S_COUNTER] = reinterpret_cast<unsigned long long>(counters);
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // control words + arrival counters start every call at zero (a faulted earlier call may
-    // have left them set); the partials are always written before they are read
+    // control words start every call at zero (a faulted earlier call may have left them set)
     if (cudaMemsetAsync(control, 0, kStaticControlBytes + kStaticCounterBytes, s) != cudaSuccess)
         return MB_ERR_CUDA;
     mb::StreamDesc desc;

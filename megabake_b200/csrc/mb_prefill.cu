@@ -2199,8 +2199,9 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count, const ClusterRoom& r
                     g.clustered = 0;
                 }
                 // The slices of a tile as one cluster, if all clusters run at once: two meetings and a
-                // fold, 5 us for 19 live rows of a 128-column tile and about 8 us for all 128, and
+                // fold, taken as 3.6 us for 19 live rows of a 128-column tile and 7 us for all 128, and
                 // twice that for the 256 columns that also leave each CTA twice the sums to store.
+                // (Stamps inside a step read up to 9 us for 128 rows, skew of the slices included.)
                 if (split < 2 || split > kMaxCluster || tiles > room.count[bn == 256][split]) continue;
                 const double joint = stream + (3.0 + 4.0 * (M < kTileM ? M : kTileM) / kTileM) * (bn / 128);
                 if (joint < best - 1e-9) {
@@ -2634,11 +2635,13 @@ int transpose_blocks(const prefill::TransposeArgs& t, int batch) {
 }
 
 // Whether the kernels of one prefill are chained by programmatic dependent launch.  A launch
-// boundary between two dependent kernels costs 3 - 5 us; chained, a kernel's set-up and the first
-// ring of a GEMM's weights run beside the kernel before it.  Replayed from a CUDA graph that is
-// 1937 -> 1584 us for 19 tokens of the 135M shape and 2499 -> 2369 us for 128 tokens of the 2B shape;
-// 2048 tokens do not care.  MEGABAKE_B200_PREFILL_CHAIN = 0 / 1 forces it (read at every
-// launch, not cached, so that one process can run both ways).
+// boundary between two dependent kernels costs 3 - 5 us; chained, a kernel's set-up and, in GEMMs of
+// one wave, the first ring of weights run beside the kernel before it.  Replayed from CUDA graphs,
+// unchained -> chained: 135M shape 1859 -> 1612 us for 19 tokens and 4419 -> 4123 for 2048; 0.5B 1733 ->
+// 1585 and 5202 -> 5040; 1B 1508 -> 1329 and 7368 -> 7087; 2B 2055 -> 1882, 3109 -> 3023 for 256 tokens and
+// 11678 -> 11626; the one size of 40 that did not gain is 128 tokens of the 2B shape, 2476 -> 2495.
+// MEGABAKE_B200_PREFILL_CHAIN = 0 / 1 forces it (read at every launch, not cached, so that one process
+// can run both ways).
 bool chaining_enabled() {
     const char* value = std::getenv("MEGABAKE_B200_PREFILL_CHAIN");
     return value == nullptr || std::atoi(value) != 0;

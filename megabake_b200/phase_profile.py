@@ -2,10 +2,10 @@
 
 The counterpart of the reference's phase profiler (``tools/phase_profile.py:104-238`` on top of
 the ``MEGABAKE_PHASE_TIMER`` stamps, ``src/megabake/runtime.py:22-47``): thread 0 of every CTA
-records the time at phase start, after the activation copies were started, after the body and,
+records the time at phase start, when the activations are staged and normalised, after the body and,
 where a phase ends in a grid barrier, after that barrier.  From those this module derives, per
-phase, how long the critical CTA worked and how long the others waited; with flagged-cell
-hand-offs (no barrier) a phase's wait shows up inside the next phase's body, as the time its
+phase, how long the critical CTA worked and how long the others waited; where phases hand over without
+a barrier (the default) the wait for a phase shows up in the next one's prologue, as the time its
 consumers spent polling.
 """
 
@@ -29,7 +29,7 @@ class PhaseTiming:
     prologue_us: float   # median over CTAs
     work_us: float       # median body time over CTAs
     slowest_us: float    # slowest CTA: phase start -> body done
-    wait_us: float       # median time spent in the closing barrier
+    wait_us: float       # median time spent in the phase's grid barrier, if it has one
     release_us: float    # last arrival -> median barrier exit
 
 

@@ -1,9 +1,10 @@
 """Execution planner: packs a ``DecoderProgram`` into phases and emits the phase records +
 address-table layout of the C ABI.
 
-Decode packing (five phases per layer; the activations between them travel as flagged cells,
-so no grid barrier separates them -- a consumer polls the very cells it needs and starts on
-them as soon as their producers have stored them):
+Decode packing (five phases per layer).  By default every phase but the last carries FLAG_RELAY: its
+results live in an arena of the plan's own, consumers poll the very words they need, and the
+buffers, cells and counters below are not used.  What the table and the next paragraph name is how
+plans without the arena hand over (``relay=False``, or a ``cell_limit`` / ``qkv_cells`` of one's own):
 
     [embed gather (layer 0) . rmsnorm . q|k|v (+bias)]          -> q, k, v cells
     [rope(q, new k) . kv append . split-key attention . merge]   -> attention cells
@@ -46,7 +47,8 @@ N_DYNAMIC = 3
 CONSUMER_WARPS = 8
 EXACT_SOFTMAX_KEYS = 128  # contexts up to here use the reference-rounding softmax (one CTA)
 MAX_GEMV_ROWS = 8
-# Activations that EVERY CTA reads whole (the input rows of a skinny GEMM) stay plain bf16: their
+# In plans without the relay arena: activations that EVERY CTA reads whole (the input rows of a skinny
+# GEMM) stay plain bf16: their
 # producers fence and report the phase finished, a consumer waits on that one counter and fetches
 # the rows with bulk copies -- measured on B200, the copy engine brings 14-78 KB per CTA into
 # shared memory in about a microsecond, where polling as many flagged cells with ordinary loads
@@ -254,9 +256,8 @@ def _check_program(p: DecoderProgram) -> None:
 
 
 def plan_decode(program: DecoderProgram, options: PlannerOptions | None = None) -> PlanLayout:
-    """Plan one decode step.  The ring stage size is the library's largest unless forced:
-    measured on B200, smaller stages (a deeper ring) never paid -- the consumers' per-stage
-    work, not the bytes in flight, bounds the weight stream."""
+    """Plan one decode step.  ``stage_bytes`` and ``row_tile`` shape the records that
+    ``mb_plan_create`` checks; the kernel's ring stages do not depend on them."""
     options = options or PlannerOptions.resolve(program)
     largest = rt.load_library().mb_stage_bytes(rt.MODE_DECODE)
     return _plan_decode(program, options, options.stage_bytes or largest)
@@ -503,7 +504,7 @@ def _plan_decode(program: DecoderProgram, options: PlannerOptions, stage_bytes: 
              f"activations need {activation} B of shared memory; with {fixed_bytes} B fixed and two "
              f"{stage_bytes} B weight stages that exceeds {max_smem} B",
              requirement="batch * max(hidden, intermediate) * 2 B must leave room for the ring")
-    # grid barriers per launch: none between phases, one closes the launch
+    # stretches of phases between grid barriers: the whole launch, unless a record asks for one
     intervals = sum(1 for phase in phases if phase.flags & rt.FLAG_BARRIER) + 1
     return PlanLayout(
         program=p,
