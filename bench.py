@@ -231,6 +231,22 @@ def algorithmic_bytes(spec, program, batch: int, mean_keys: float) -> float:
     return program.weight_bytes() + batch * mean_keys * program.kv_bytes_per_key()
 
 
+def greedy_ties(got, ref) -> dict:
+    """Rows whose pick differs from the reference's, and how far the reference's logit of that pick lies
+    below its best one, in bf16 steps of the best.  Up to two steps the pick is a tie of random
+    weights that the order of the fp32 sums decides, the rule the tests judge picks by."""
+    import math
+
+    gaps = []
+    for mine, theirs in zip(got, ref):
+        best, pick = int(theirs.argmax()), int(mine.argmax())
+        if pick != best:
+            step = 2.0 ** (math.floor(math.log2(abs(float(theirs[best])) or 1.0)) - 7)
+            gaps.append(float(theirs[best] - theirs[pick]) / step)
+    return {"greedy_rows_differing": len(gaps), "greedy_gaps_bf16_steps": gaps,
+            "greedy_picks_ok": all(gap <= 2.0 for gap in gaps)}
+
+
 def parity_check(spec, weights, inv_freq, state, ids, position, decoder, ids_dev, pos_dev,
                  logits) -> dict:
     """One decode step by the kernel against the CPU oracle on copies of the same state."""
@@ -262,6 +278,7 @@ def parity_check(spec, weights, inv_freq, state, ids, position, decoder, ids_dev
     return {
         "max_abs": float((got - ref).abs().max()), "cosine": cos(got, ref),
         "greedy_ids_equal": bool(torch.equal(got[:, -1].argmax(-1), ref[:, -1].argmax(-1))),
+        **greedy_ties(got[:, -1], ref[:, -1]),
         "kernel_vs_fp32_max_abs": float((got - wide).abs().max()),
         "eager_vs_fp32_max_abs": float((ref - wide).abs().max()),
         "kernel_vs_fp32_cosine": cos(got, wide), "eager_vs_fp32_cosine": cos(ref, wide),
@@ -728,7 +745,7 @@ def _report(args, spec, program, layout, batch, keys, steps, warmup, device_ms, 
             "data": "synthetic",
             "config": decode_config(args.workload, world, args.cache_fill),
             "plan": {"tokens_per_s": whole_job_rate(batch, world, ms_per_step * 1e-3),
-                     "phases": len(layout.phases), "grid_barriers": layout.intervals,
+                     "phases": len(layout.phases), "grid_barriers": layout.intervals - 1,
                      "ctas": plan_info["ctas"], "ring_stages": plan_info["ring_stages"]},
             "roofline": {
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
