@@ -231,20 +231,21 @@ def algorithmic_bytes(spec, program, batch: int, mean_keys: float) -> float:
     return program.weight_bytes() + batch * mean_keys * program.kv_bytes_per_key()
 
 
-def greedy_ties(got, ref) -> dict:
-    """Rows whose pick differs from the reference's, and how far the reference's logit of that pick lies
-    below its best one, in bf16 steps of the best.  Up to two steps the pick is a tie of random
-    weights that the order of the fp32 sums decides, the rule the tests judge picks by."""
+def greedy_gaps(got, ref, wide) -> dict:
+    """Rows whose pick differs from the reference's, and how far that pick lies below the reference's
+    best logit, in bf16 steps of the best: by the reference's eager bf16 forward, and by the same
+    forward in fp32 (negative: fp32 prefers the kernel's pick).  With random weights the best logits
+    are a few steps apart, less than either bf16 forward is away from fp32."""
     import math
 
-    gaps = []
-    for mine, theirs in zip(got, ref):
+    eager, exact = [], []
+    for mine, theirs, full in zip(got, ref, wide):
         best, pick = int(theirs.argmax()), int(mine.argmax())
         if pick != best:
             step = 2.0 ** (math.floor(math.log2(abs(float(theirs[best])) or 1.0)) - 7)
-            gaps.append(float(theirs[best] - theirs[pick]) / step)
-    return {"greedy_rows_differing": len(gaps), "greedy_gaps_bf16_steps": gaps,
-            "greedy_picks_ok": all(gap <= 2.0 for gap in gaps)}
+            eager.append(float(theirs[best] - theirs[pick]) / step)
+            exact.append(float(full[best] - full[pick]) / step)
+    return {"greedy_gaps_bf16_steps": eager, "greedy_gaps_in_fp32_bf16_steps": exact}
 
 
 def parity_check(spec, weights, inv_freq, state, ids, position, decoder, ids_dev, pos_dev,
@@ -278,7 +279,7 @@ def parity_check(spec, weights, inv_freq, state, ids, position, decoder, ids_dev
     return {
         "max_abs": float((got - ref).abs().max()), "cosine": cos(got, ref),
         "greedy_ids_equal": bool(torch.equal(got[:, -1].argmax(-1), ref[:, -1].argmax(-1))),
-        **greedy_ties(got[:, -1], ref[:, -1]),
+        **greedy_gaps(got[:, -1], ref[:, -1], wide[:, -1].float()),
         "kernel_vs_fp32_max_abs": float((got - wide).abs().max()),
         "eager_vs_fp32_max_abs": float((ref - wide).abs().max()),
         "kernel_vs_fp32_cosine": cos(got, wide), "eager_vs_fp32_cosine": cos(ref, wide),
