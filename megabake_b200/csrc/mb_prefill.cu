@@ -1,5 +1,6 @@
 // Prefill path: one kernel launch per phase of an MB_MODE_PREFILL plan, enqueued in order on
-// the caller's stream (and captured as a whole by a CUDA graph when the caller does so).
+// the caller's stream (and captured as a whole by a CUDA graph when the caller does so).  Short prompts
+// are one launch instead (mb_prompt.cu).
 //
 //   embed_rows_kernel      gather of embedding rows (+ Gemma's bf16 scalar scale)
 //   rmsnorm_block_kernel   row-wise RMSNorm, Llama and Gemma spellings, one CTA per row
@@ -32,6 +33,7 @@
 
 #include "mb_device.cuh"
 #include "mb_kernels.h"
+#include "mb_tensor.cuh"
 
 namespace mb {
 namespace prefill {
@@ -47,20 +49,6 @@ __device__ __forceinline__ void chain_release() {
 }
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-// Two floats to a bf16 pair in one instruction (same bits as two cvt.rn.bf16.f32, checked over
-// every finite float): the attention's softmax warps and the GEMM epilogue are bound by the
-// instructions they issue, and packing was four of them per pair.
-__device__ __forceinline__ float exp2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ unsigned int pack_bf16_pair(float lo, float hi) {
-    unsigned int packed;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
-    return packed;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -235,101 +223,9 @@ __global__ void __launch_bounds__(256) rope_rows_kernel(const RopeArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------
-// tcgen05 / TMA wrappers
-// ---------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int x, int y,
-                                            unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst_smem)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(unsigned int* slot_smem, unsigned int columns) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(slot_smem)),
-                 "r"(columns)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(unsigned int base, unsigned int columns) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns)
-                 : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// The mbarrier gets one arrival once every tcgen05.mma this thread issued before has finished.
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
-}
-// D[tmem] (+)= A[smem] . B[smem]^T, bf16 operands, fp32 accumulate, M = 128.
-__device__ __forceinline__ void umma_bf16(unsigned int tmem_d, unsigned long long desc_a,
-                                          unsigned long long desc_b, unsigned int idesc,
-                                          unsigned int accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Shared-memory operand descriptor: K-major tile of 128-byte rows, 128-byte swizzle, groups of
-// 8 rows 1024 bytes apart (the layout TMA writes with CU_TENSOR_MAP_SWIZZLE_128B).
-__device__ __forceinline__ unsigned long long umma_desc(unsigned int smem_addr) {
-    unsigned long long d = 0;
-    d |= static_cast<unsigned long long>((smem_addr & 0x3ffffu) >> 4);  // start address
-    d |= 1ull << 16;                                                     // leading byte offset (unused)
-    d |= static_cast<unsigned long long>(1024 >> 4) << 32;               // stride byte offset
-    d |= 1ull << 46;                                                     // descriptor version
-    d |= 2ull << 61;                                                     // SWIZZLE_128B
-    return d;
-}
-// 32 consecutive fp32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_load32(unsigned int taddr, float (&v)[32]) {
-    unsigned int r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 16 consecutive fp32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_load16(unsigned int taddr, float (&v)[16]) {
-    unsigned int r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// ---------------------------------------------------------------------------------------
 // The GEMM
 // ---------------------------------------------------------------------------------------
 constexpr int kTileM = 128;
-constexpr int kTileK = 64;  // bf16 elements = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: epilogue
 constexpr int kStageA = kTileM * kTileK * 2;
 
@@ -954,88 +850,88 @@ gemm_tc_persistent_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs 
     chain_wait();  // nothing above reads or writes what another kernel writes or reads
     if (threadIdx.x == 0) stamp(1);
 
+    // The producer's and the MMA warp's lanes stay together, and one elected lane issues (elect_one says why).
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0, round = 0;  // ring position; `round` counts wraps
-            bool ok = true;
-            for (int unit = blockIdx.x; unit < total && ok; unit += gridDim.x) {
-                const int t = unit / a.split_k, z = unit - t * a.split_k;
-                const int mt = t % a.tiles_m, tile = t / a.tiles_m;
-                const int seg = (tile >= a.tile_start[1] ? 1 : 0) + (tile >= a.tile_start[2] ? 1 : 0);
-                const int n0 = (tile - a.tile_start[seg]) * per_tile;
-                const int m0 = mt * kTileM;
-                const int kb0 = static_cast<int>(static_cast<long long>(z) * a.kblocks / a.split_k);
-                const int kb1 = static_cast<int>(static_cast<long long>(z + 1) * a.kblocks / a.split_k);
-                for (int kb = kb0; kb < kb1; ++kb) {
-                    if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1, abort_flag)) {
-                        record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 1);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    unsigned char* stage = smem + s * kStage;
-                    const int kx = kb * kTileK;
-                    if (ahead > 0)
-                        --ahead;
-                    else
-                        load_weights(stage, kx, seg, n0, &full[s]);
+        ahead = __shfl_sync(0xffffffffu, ahead, 0);
+        int s = 0, round = 0;  // ring position; `round` counts wraps
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < total && ok; unit += gridDim.x) {
+            const int t = unit / a.split_k, z = unit - t * a.split_k;
+            const int mt = t % a.tiles_m, tile = t / a.tiles_m;
+            const int seg = (tile >= a.tile_start[1] ? 1 : 0) + (tile >= a.tile_start[2] ? 1 : 0);
+            const int n0 = (tile - a.tile_start[seg]) * per_tile;
+            const int m0 = mt * kTileM;
+            const int kb0 = static_cast<int>(static_cast<long long>(z) * a.kblocks / a.split_k);
+            const int kb1 = static_cast<int>(static_cast<long long>(z + 1) * a.kblocks / a.split_k);
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (round > 0 && !mbar_wait_warp(&empty[s], (round - 1) & 1, abort_flag)) {
+                    record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 1);
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                unsigned char* stage = smem + s * kStage;
+                const int kx = kb * kTileK;
+                if (elect_one()) {
+                    if (ahead == 0) load_weights(stage, kx, seg, n0, &full[s]);
                     tma_load_2d(stage, &maps.a, kx, m0, &full[s]);
-                    if (++s == kStages) {
-                        s = 0;
-                        ++round;
-                    }
+                }
+                __syncwarp();
+                if (ahead > 0) --ahead;
+                if (++s == kStages) {
+                    s = 0;
+                    ++round;
                 }
             }
         }
-        __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            // instruction descriptor: fp32 accumulate, bf16 x bf16, both operands K-major,
-            // N = BN, M = 128
-            const unsigned int idesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                       (static_cast<unsigned int>(BN >> 3) << 17) |
-                                       (static_cast<unsigned int>(kTileM >> 4) << 24);
-            int s = 0, round = 0, j = 0;
-            bool ok = true;
-            for (int unit = blockIdx.x; unit < total && ok; unit += gridDim.x, ++j) {
-                const int buf = j & 1;
-                const int z = unit % a.split_k;
-                const int kb0 = static_cast<int>(static_cast<long long>(z) * a.kblocks / a.split_k);
-                const int kb1 = static_cast<int>(static_cast<long long>(z + 1) * a.kblocks / a.split_k);
-                // the epilogue must have drained this buffer's previous tile
-                if (j >= 2 && !mbar_wait_bounded(&acc_empty[buf], ((j >> 1) - 1) & 1, abort_flag)) {
-                    record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 4);
+        // instruction descriptor: fp32 accumulate, bf16 x bf16, both operands K-major,
+        // N = BN, M = 128
+        const unsigned int idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                   (static_cast<unsigned int>(BN >> 3) << 17) |
+                                   (static_cast<unsigned int>(kTileM >> 4) << 24);
+        int s = 0, round = 0, j = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < total && ok; unit += gridDim.x, ++j) {
+            const int buf = j & 1;
+            const int z = unit % a.split_k;
+            const int kb0 = static_cast<int>(static_cast<long long>(z) * a.kblocks / a.split_k);
+            const int kb1 = static_cast<int>(static_cast<long long>(z + 1) * a.kblocks / a.split_k);
+            // the epilogue must have drained this buffer's previous tile
+            if (j >= 2 && !mbar_wait_warp(&acc_empty[buf], ((j >> 1) - 1) & 1, abort_flag)) {
+                record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 4);
+                *abort_flag = 1;
+                break;
+            }
+            tc_fence_after();
+            const unsigned int acc = tmem_base + buf * BN;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait_warp(&full[s], round & 1, abort_flag)) {
+                    record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 2);
                     *abort_flag = 1;
+                    ok = false;
                     break;
                 }
                 tc_fence_after();
-                const unsigned int acc = tmem_base + buf * BN;
-                for (int kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait_bounded(&full[s], round & 1, abort_flag)) {
-                        record_status(a.ctl, MB_ST_PIPE_TIMEOUT, a.phase, 2);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    if (j == 0 && kb == kb0) stamp(2);
-                    const unsigned int base = smem_u32(smem + s * kStage);
-                    const unsigned long long da = umma_desc(base);
-                    const unsigned long long db = umma_desc(base + kStageA);
+                if (j == 0 && kb == kb0 && lane == 0) stamp(2);
+                const unsigned int base = smem_u32(smem + s * kStage);
+                const unsigned long long da = umma_desc(base);
+                const unsigned long long db = umma_desc(base + kStageA);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < kTileK / 16; ++k)  // 32 bytes along K per step: +2 encoded
                         umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
                     umma_commit(&empty[s]);  // the stage is free once these MMAs have read it
-                    if (++s == kStages) {
-                        s = 0;
-                        ++round;
-                    }
+                    if (kb == kb1 - 1) umma_commit(&acc_full[buf]);
                 }
-                if (ok) umma_commit(&acc_full[buf]);
-                if (j == 0) stamp(3);
+                __syncwarp();
+                if (++s == kStages) {
+                    s = 0;
+                    ++round;
+                }
             }
+            if (j == 0 && lane == 0) stamp(3);
         }
-        __syncwarp();
     } else {
         const int quarter = warp & 3;        // the TMEM lanes a warp may read: 32 * (warp % 4) ...
         const int column_half = (warp - 2) >> 2;
@@ -1216,21 +1112,6 @@ struct AttnArgs {
 constexpr int kAttnWhole = 0, kAttnStats = 1, kAttnValues = 2;
 
 constexpr int kAttnKeys = 64;  // keys per block
-
-__device__ __forceinline__ void ldmatrix_x4(unsigned int (&r)[4], const void* smem_ptr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smem_u32(smem_ptr)));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(unsigned int (&r)[4], const void* smem_ptr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smem_u32(smem_ptr)));
-}
-__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src)
-                 : "memory");
-}
 
 // `rows` rows of D bf16 each into a tile with pitch D + 8; rows past `limit` repeat the last one
 template <int D, int THREADS>
@@ -2093,38 +1974,6 @@ inline AttnParts attention_parts(int batch, int tokens, int heads, int D, bool c
 // Host side: validation, tile / split-K geometry, tensor maps, launches.
 // ---------------------------------------------------------------------------------------
 namespace {
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    if (fn == nullptr) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult result;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &result) ==
-                cudaSuccess &&
-            result == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-    }
-    return fn;
-}
-
-// [rows, K] bf16 row-major, boxes of `box_rows` x 64 elements, 128-byte swizzle, zero fill
-// outside the tensor.
-bool make_map(CUtensorMap* map, unsigned long long base, int rows, int K, int box_rows) {
-    EncodeTiledFn fn = encode_tiled();
-    if (fn == nullptr) return false;
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kTileK), static_cast<cuuint32_t>(box_rows)};
-    const cuuint32_t elem[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, reinterpret_cast<void*>(base), dims,
-              strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 int gemm_smem_bytes(int bn, int stages) {
     return stages * (kStageA + bn * kTileK * 2) + 256 + 1024;  // ring + barriers + alignment slack
