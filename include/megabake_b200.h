@@ -243,7 +243,9 @@ typedef struct mb_phase {
                                 instead, it must be zero before its first launch           */
 #define MB_AT_S_COUNTER 10   /* int32 [B*Hkv]; has to be given, is not touched               */
 
-/* ---- prefill bodies (MB_MODE_PREFILL plans: one kernel launch per phase, in order) ----- */
+/* ---- prefill bodies (MB_MODE_PREFILL plans: one kernel launch per phase, in order; the list of a
+ * whole decoder prefill of a short prompt runs as one launch, mb_plan_info.launches == 1, and then
+ * writes of the intermediate tensors only those its own steps pass on) -------------------- */
 /* MB_BODY_EMBED_ROWS: out[r, :] = table[ids[r], :] (x scale, rounded to bf16)              */
 #define MB_EM_I_ROWS 0
 #define MB_EM_I_K 1
@@ -353,7 +355,9 @@ int mb_plan_reset(mb_plan* plan);
  * src/megabake/runtime.py:22-47, is the same idea): `device_address` points at
  * ctas * n_phases * 8 uint64 the kernel fills with global-timer stamps (0 phase start,
  * 1 prologue done, 2 body done, 3 barrier passed, 4..7 body-specific) on every later
- * launch; 0 switches it off. */
+ * launch; 0 switches it off.  Prefill: 8 uint64 per phase (CTA 0 of each GEMM); a prompt that runs as
+ * one launch stamps its steps instead (CTA 0: 2 step done, 3 step before complete, 4 first operands
+ * there, 5 products issued, 6 accumulators complete). */
 int mb_plan_set_trace(mb_plan* plan, uint64_t device_address, size_t bytes);
 void mb_plan_destroy(mb_plan* plan);
 

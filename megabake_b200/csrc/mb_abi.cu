@@ -87,7 +87,8 @@ struct mb_plan {
     unsigned int wide_dynamic = 0;        // per-launch slots that must be 16-byte aligned, one bit each
     mb::Control* d_ctl = nullptr;
     unsigned long long trace = 0;
-    mb::PrefillState* prefill = nullptr;  // MB_MODE_PREFILL plans only
+    mb::PrefillState* prefill = nullptr;  // MB_MODE_PREFILL plans only, one of the two:
+    mb::PromptState* prompt = nullptr;    // a short prompt in one launch
 };
 
 namespace {
@@ -349,7 +350,9 @@ int create_prefill_plan(const mb_plan_desc* desc, mb_plan** out) {
     plan->ctas = prop.multiProcessorCount;
     cudaError_t err = cudaMalloc(&plan->d_ctl, sizeof(mb::Control));
     if (err == cudaSuccess) err = cudaMemset(plan->d_ctl, 0, sizeof(mb::Control));
-    if (err == cudaSuccess) err = mb::prefill_create(plan->phases, plan->sm_count, &plan->prefill);
+    if (err == cudaSuccess) err = mb::prompt_create(plan->phases, plan->n_dynamic, plan->sm_count, &plan->prompt);
+    if (err == cudaSuccess && plan->prompt == nullptr)
+        err = mb::prefill_create(plan->phases, plan->sm_count, &plan->prefill);
     if (err != cudaSuccess) {
         cuda_fail(err, "prefill plan allocation");
         mb_plan_destroy(plan);
@@ -525,8 +528,9 @@ int mb_plan_query(const mb_plan* plan, mb_plan_info* out) {
     out->stages = plan->stages;
     out->barriers = plan->mode == MB_MODE_PREFILL ? 0 : plan->barriers - 1;
     out->sm_count = plan->sm_count;
-    out->launches = plan->mode == MB_MODE_PREFILL ? mb::prefill_launch_count(plan->prefill)
-                                                  : 1 + static_cast<int>(plan->late_maps.size());
+    out->launches = plan->prompt != nullptr           ? 1
+                    : plan->mode == MB_MODE_PREFILL ? mb::prefill_launch_count(plan->prefill)
+                                                    : 1 + static_cast<int>(plan->late_maps.size());
     return MB_OK;
 }
 
@@ -540,7 +544,9 @@ int mb_plan_bind(mb_plan* plan, const uint64_t* slot_addresses, size_t n) {
     if (plan->mode == MB_MODE_PREFILL) {
         DeviceGuard guard(plan->device);
         if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
-        const int rc = mb::prefill_bind(plan->prefill, plan->phases, plan->slots, plan->d_ctl);
+        const int rc = plan->prompt != nullptr
+                           ? mb::prompt_bind(plan->prompt, plan->slots, plan->d_ctl)
+                           : mb::prefill_bind(plan->prefill, plan->phases, plan->slots, plan->d_ctl);
         if (rc != MB_OK) {
             g_last_cuda_error = "tensor map encoding failed";
             return rc;
@@ -602,6 +608,13 @@ int mb_plan_launch(mb_plan* plan, const uint64_t* dynamic_addresses, size_t n, v
             if (dynamic_addresses[i] == 0 || (dynamic_addresses[i] & 7ull) != 0) return MB_ERR_INVALID;
         DeviceGuard guard(plan->device);
         if (guard.error != cudaSuccess) return cuda_fail(guard.error, "cudaSetDevice");
+        if (plan->prompt != nullptr) {
+            MB_CUDA(mb::prompt_launch(plan->prompt, plan->slots,
+                                      reinterpret_cast<const unsigned long long*>(dynamic_addresses),
+                                      reinterpret_cast<unsigned long long*>(plan->trace),
+                                      static_cast<cudaStream_t>(stream)));
+            return MB_OK;
+        }
         MB_CUDA(mb::prefill_launch(plan->prefill, plan->phases, plan->slots, plan->n_dynamic,
                                    reinterpret_cast<const unsigned long long*>(dynamic_addresses),
                                    plan->d_ctl, reinterpret_cast<unsigned long long*>(plan->trace),
@@ -688,6 +701,7 @@ int mb_plan_reset(mb_plan* plan) {
     MB_CUDA(cudaMemcpy(&plan->d_ctl->maps_written, &plan->maps_written, sizeof(plan->maps_written),
                        cudaMemcpyHostToDevice));
     MB_CUDA(blank_relays(plan));
+    MB_CUDA(mb::prompt_reset(plan->prompt));
     MB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return MB_OK;
 }
@@ -702,6 +716,7 @@ void mb_plan_destroy(mb_plan* plan) {
         if (plan->d_relay) cudaFree(plan->d_relay);
         if (plan->d_ctl) cudaFree(plan->d_ctl);
         mb::prefill_destroy(plan->prefill);
+        mb::prompt_destroy(plan->prompt);
     }
     delete plan;
 }

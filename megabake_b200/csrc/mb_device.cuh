@@ -226,6 +226,37 @@ __device__ __forceinline__ float gelu_tanh_f32(float x) {
     return 0.5f * x * (1.0f + tanhf(inner));
 }
 
+// Both as x times a sigmoid, with the device's fast exponential and reciprocal; the graph rounds the result to bf16
+// next.  Over all bf16 x, silu then has the same bits as above but for three results below 1e-36; GELU differs
+// at 150, at each of which it is closer to the exact value: 0.5 (1 + tanh u) cancels where tanh u nears -1,
+// the sigmoid of 2 u does not.
+__device__ __forceinline__ float gelu_exponent(float x) {
+    return 1.5957691216057308f * (x + 0.044715f * (x * x * x));  // 2 sqrt(2 / pi) (x + 0.044715 x^3)
+}
+__device__ __forceinline__ float sigmoid_product(float x, float t) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return x * r;
+}
+// Two bf16 values at a time: products and sums of bf16 operands rounded once, which is what rounding the fp32 result
+// gives (a product of two is exact in fp32; a sum is either exact there or too uneven for its tail to matter).
+__device__ __forceinline__ unsigned int mul_bf16_pair(unsigned int a, unsigned int b) {
+    unsigned int d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned int add_bf16_pair(unsigned int a, unsigned int b) {
+    unsigned int d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned int sub_bf16_pair(unsigned int a, unsigned int b) {
+    unsigned int d;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
 // ---------------------------------------------------------------------------------------
 // Loads that bypass L1 for data another CTA produced earlier in the same launch.
 // ---------------------------------------------------------------------------------------

@@ -45,4 +45,16 @@ cudaError_t prefill_launch(PrefillState* state, const std::vector<mb_phase>& pha
                            const std::vector<unsigned long long>& slots, unsigned int n_dynamic,
                            const unsigned long long* dynamic_addresses, Control* ctl,
                            unsigned long long* trace, cudaStream_t stream);
+
+// Short prompts (mb_prompt.cu): the whole of a prefill plan as one launch.  The state stays null where the phases are
+// no such prompt.
+struct PromptState;
+cudaError_t prompt_create(const std::vector<mb_phase>& phases, unsigned int n_dynamic, int sm_count,
+                          PromptState** out);
+void prompt_destroy(PromptState* state);
+cudaError_t prompt_reset(PromptState* state);
+int prompt_bind(PromptState* state, const std::vector<unsigned long long>& slots, Control* ctl);
+cudaError_t prompt_launch(const PromptState* state, const std::vector<unsigned long long>& slots,
+                          const unsigned long long* dynamic_addresses, unsigned long long* trace,
+                          cudaStream_t stream);
 }  // namespace mb
