@@ -856,7 +856,7 @@ __device__ __forceinline__ void finish_result(const PhaseEntry* E, const GemvStr
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) v[w] = part[w * 128 + 64];
         const float up = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-        const float act = epilogue == MB_EPI_SILU_MUL ? silu_f32(y) : gelu_tanh_f32(y);
+        const float act = sigmoid_product(y, epilogue == MB_EPI_SILU_MUL ? y : gelu_exponent(y));
         y = bf16_round(act) * bf16_round(up);
     } else if (epilogue == MB_EPI_RESIDUAL) {
         if (live) {
@@ -1011,8 +1011,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned int (&r)[4], unsigned
                  : "r"(addr)
                  : "memory");
 }
-__device__ __forceinline__ float cos_of(unsigned int packed) { return lo_bf16(packed); }
-__device__ __forceinline__ float sin_of(unsigned int packed) { return hi_bf16(packed); }
 
 // cos / sin of position `pos` for i = first, first + step ... < D/2, rounded to bf16 like the
 // eager tables.
@@ -1034,24 +1032,21 @@ __device__ __noinline__ void fill_rope_row(unsigned int* table, const PhaseEntry
 __device__ __forceinline__ void rotate_vectors(uint4& lo, uint4& hi, const unsigned int* table,
                                                float q_scale) {
     unsigned int a[4] = {lo.x, lo.y, lo.z, lo.w}, b[4] = {hi.x, hi.y, hi.z, hi.w};
-    const bool scaled = q_scale != 0.f && q_scale != 1.f;
+    const uint4 t0 = *reinterpret_cast<const uint4*>(table), t1 = *reinterpret_cast<const uint4*>(table + 4);
+    const unsigned int t[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-        float r1[2], r2[2];
+        const unsigned int c = __byte_perm(t[2 * w], t[2 * w + 1], 0x5410), x1 = a[w];
+        const unsigned int sn = __byte_perm(t[2 * w], t[2 * w + 1], 0x7632), x2 = b[w];
+        a[w] = sub_bf16_pair(mul_bf16_pair(x1, c), mul_bf16_pair(x2, sn));
+        b[w] = add_bf16_pair(mul_bf16_pair(x2, c), mul_bf16_pair(x1, sn));
+    }
+    if (q_scale != 0.f && q_scale != 1.f) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const float x1 = e ? hi_bf16(a[w]) : lo_bf16(a[w]), x2 = e ? hi_bf16(b[w]) : lo_bf16(b[w]);
-            const unsigned int cs = table[2 * w + e];
-            const float c = cos_of(cs), sn = sin_of(cs);
-            r1[e] = bf16_round(x1 * c) + bf16_round(-x2 * sn);
-            r2[e] = bf16_round(x2 * c) + bf16_round(x1 * sn);
-            if (scaled) {
-                r1[e] = bf16_round(r1[e]) * q_scale;
-                r2[e] = bf16_round(r2[e]) * q_scale;
-            }
+        for (int w = 0; w < 4; ++w) {
+            a[w] = pack_bf16(lo_bf16(a[w]) * q_scale, hi_bf16(a[w]) * q_scale);
+            b[w] = pack_bf16(lo_bf16(b[w]) * q_scale, hi_bf16(b[w]) * q_scale);
         }
-        a[w] = pack_bf16(r1[0], r1[1]);
-        b[w] = pack_bf16(r2[0], r2[1]);
     }
     lo = make_uint4(a[0], a[1], a[2], a[3]);
     hi = make_uint4(b[0], b[1], b[2], b[3]);
@@ -1444,48 +1439,73 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         if (seg.parts == 1) continue;
         const int total = group * (D / 2);  // pairs of neighbouring outputs
         const int lo = seg.index * total / seg.parts, hi = (seg.index + 1) * total / seg.parts;
-        const int width = seg.parts <= 2 ? 2 : (seg.parts <= 4 ? 4 : (seg.parts <= 8 ? 8 : 16));
         const char* base = reinterpret_cast<const char*>(E->addr[MB_AT_S_PARTIAL]) +
                            static_cast<size_t>(seg.pair) * d.chunk_cap * group * ((D + 2) * 8);
-        const int j = tid & (width - 1);
-        for (int o0 = lo; o0 < hi; o0 += kThreads / width) {
-            const int o = o0 + tid / width;
+        // A thread takes up to eight parts of an output pair, four threads up to 32: the cells of all of
+        // them are in flight together, again and again until none carries an older tag.  (One part a
+        // thread, its four cells waited for one after the other, took 4.6 us on the 0.5B shape
+        // and 9.7 on the 2B, after the last part was out.)
+        const int lanes = seg.parts > 8 ? 4 : 1, j = tid & (lanes - 1);
+        for (int o0 = lo; o0 < hi; o0 += kThreads / lanes) {
+            const int o = o0 + tid / lanes;
             const int head = min(o, hi - 1) / (D / 2), dim = 2 * (min(o, hi - 1) - head * (D / 2));
-            float m[2], l[2], v0[2], v1[2];
+            const char* first = base + static_cast<size_t>(head) * ((D + 2) * 8);
+            unsigned long long cm[8], cl[8], c0[8], c1[8];
+            unsigned long long start = 0;
+#pragma unroll 1
+            for (unsigned int tries = 1;; ++tries) {
+                bool missing = false;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int c = j + u * width;
-                m[u] = -INFINITY;
-                l[u] = v0[u] = v1[u] = 0.f;
-                if (c < seg.parts && o < hi) {
-                    const char* part = base + (static_cast<size_t>(c) * group + head) * ((D + 2) * 8);
-                    unsigned long long cm, cl, c0, c1;
-                    ld_cell_pair(part, cm, cl);
-                    ld_cell_pair(part + (2 + dim) * 8, c0, c1);
-                    if (cell_tag(cm) != own_tag) cm = cell_wait(part, own_tag, ph);
-                    if (cell_tag(cl) != own_tag) cl = cell_wait(part + 8, own_tag, ph);
-                    if (cell_tag(c0) != own_tag) c0 = cell_wait(part + (2 + dim) * 8, own_tag, ph);
-                    if (cell_tag(c1) != own_tag) c1 = cell_wait(part + (3 + dim) * 8, own_tag, ph);
-                    m[u] = __uint_as_float(cell_data(cm));
-                    l[u] = __uint_as_float(cell_data(cl));
-                    v0[u] = __uint_as_float(cell_data(c0));
-                    v1[u] = __uint_as_float(cell_data(c1));
+                for (int i = 0; i < 8; ++i) {
+                    // slot 8, 16 or 24 of these parts does not exist: the last one again, with no weight below
+                    const int c = min(lanes == 1 ? i : j + 4 * (i & 3) + 16 * (i >> 2), seg.parts - 1);
+                    const char* part = first + static_cast<size_t>(c) * group * ((D + 2) * 8);
+                    ld_cell_pair(part, cm[i], cl[i]);
+                    ld_cell_pair(part + (2 + dim) * 8, c0[i], c1[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    missing |= cell_tag(cm[i]) != own_tag || cell_tag(cl[i]) != own_tag ||
+                               cell_tag(c0[i]) != own_tag || cell_tag(c1[i]) != own_tag;
+                if (!__any_sync(0xffffffffu, missing)) break;
+                if ((tries & 63u) == 0u) {
+                    if (start == 0) start = global_timer_ns();
+                    if (__any_sync(0xffffffffu, wait_gave_up(ph, start))) break;  // garbage: the launch has failed
                 }
             }
-            float mx = fmaxf(m[0], m[1]);
-            for (int w = width >> 1; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-            const float w0 = m[0] == -INFINITY ? 0.f : expf(m[0] - mx);
-            const float w1 = m[1] == -INFINITY ? 0.f : expf(m[1] - mx);
-            float den = l[0] * w0 + l[1] * w1;
-            float s0 = v0[0] * w0 + v0[1] * w1, s1 = v1[0] * w0 + v1[1] * w1;
-            for (int w = width >> 1; w > 0; w >>= 1) {
-                den += __shfl_xor_sync(0xffffffffu, den, w);
-                s0 += __shfl_xor_sync(0xffffffffu, s0, w);
-                s1 += __shfl_xor_sync(0xffffffffu, s1, w);
+            float m[8], mx = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int c = lanes == 1 ? i : j + 4 * (i & 3) + 16 * (i >> 2);
+                m[i] = c < seg.parts ? __uint_as_float(cell_data(cm[i])) : -INFINITY;
+                mx = fmaxf(mx, m[i]);
+            }
+            for (int w = lanes >> 1; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            float den[8], s0[8], s1[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float weight = m[i] == -INFINITY ? 0.f : expf(m[i] - mx);
+                den[i] = __uint_as_float(cell_data(cl[i])) * weight;
+                s0[i] = __uint_as_float(cell_data(c0[i])) * weight;
+                s1[i] = __uint_as_float(cell_data(c1[i])) * weight;
+            }
+            // part c meets part c + 16, then c + 8, + 4, + 2, + 1, whoever holds them
+#pragma unroll
+            for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+                for (int i = 0; i < w; ++i) {
+                    den[i] += den[i + w];
+                    s0[i] += s0[i + w];
+                    s1[i] += s1[i + w];
+                }
+            for (int w = lanes >> 1; w > 0; w >>= 1) {
+                den[0] += __shfl_xor_sync(0xffffffffu, den[0], w);
+                s0[0] += __shfl_xor_sync(0xffffffffu, s0[0], w);
+                s1[0] += __shfl_xor_sync(0xffffffffu, s1[0], w);
             }
             if (j == 0 && o < hi)
                 store_result(out, (static_cast<size_t>(seg.b) * Hq + seg.h * group + head) * D + dim,
-                             pack_bf16(s0 / den, s1 / den), out_cells, own_tag);
+                             pack_bf16(s0[0] / den[0], s1[0] / den[0]), out_cells, own_tag);
         }
     }
     return s;
