@@ -1,5 +1,5 @@
 // Decode megakernel: one cooperative persistent launch runs every phase of a one-token
-// decoder step.  One CTA per SM, nine warps:
+// decoder step.  One CTA per SM, ten warps:
 //
 //   warp 8       streams weight rows through a ring of 16 KB stages in shared memory, one
 //                tensor-map copy per stage, a ring length ahead of the others and across phase
@@ -10,6 +10,7 @@
 //                address arithmetic.  (Measured with nothing but the copies: 6.6 TB/s; 16-byte
 //                copies by one producer warp reach 3.4 TB/s and by all warps 6.9, but then every
 //                warp spends about as many instructions on copying as on everything else.)
+//   warp 9       copies the phase records and resolves their addresses, up to four phases ahead.
 //   warps 0..7   consumers: activation prologues (RMSNorm, embedding gather), the skinny GEMM on
 //                mma.sync, epilogues, decode attention.
 //
@@ -43,7 +44,7 @@ namespace decode {
 
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;        // consumers
-constexpr int kAllThreads = kThreads + 32;   // and the producer warp
+constexpr int kAllThreads = kThreads + 64;   // and two more: weights, keys and values; phase records
 constexpr int kRowTile = 8;          // ROW_TILE and K_CHUNK of a record describe the staging of
 constexpr int kRowPad = 64;          // weight rows in units of these; the kernel's own stages are
 constexpr int kStageBytes = 34816;   // 16 KB whatever they say
@@ -70,9 +71,9 @@ struct Segment {
 struct SharedCtl {
     unsigned long long full[kMaxStages];   // a stage's copies have landed
     unsigned long long empty[kMaxStages];  // all consumer warps have read it
-    unsigned long long entry_full;         // the next phase record has landed
+    unsigned long long entry_ready[4];     // a phase record is there, its addresses resolved
+    unsigned long long entry_done[4];      // all consumer warps are through with it
     volatile unsigned int issued;          // stages the producer armed
-    volatile unsigned int fetched;         // phase records requested
     unsigned long long limit_ns;           // bound of every wait of this launch
     unsigned long long relay_now, relay_next;  // this launch's half of the arena, the other half
     volatile int abort_flag;
@@ -487,9 +488,6 @@ __device__ __noinline__ void drain_ring() {
     for (unsigned int i = issued > stages ? issued - stages : 0u; i < issued; ++i)
         for (unsigned int tries = 0; tries < kDrainTryLimit; ++tries)
             if (mbar_try_wait(&sc->full[i % stages], (i / stages) & 1u)) break;
-    const unsigned int records = sc->fetched;
-    for (unsigned int tries = 0; records > 0 && tries < kDrainTryLimit; ++tries)
-        if (mbar_try_wait(&sc->entry_full, (records - 1) & 1u)) break;
 }
 
 __device__ __forceinline__ uint4 lds128(unsigned int addr) {
@@ -516,6 +514,21 @@ __device__ __forceinline__ void ring_wait(unsigned int stage, unsigned int parit
             return;
         }
     }
+}
+// The record of phase ph; it is there but for the first phases of a launch.  False: it will not come, and must not
+// be looked at.
+__device__ __forceinline__ bool entry_wait(int ph) {
+    SharedCtl* sc = ctl_of();
+    if (mbar_try_wait(&sc->entry_ready[ph & 3], (ph >> 2) & 1)) return true;
+    const unsigned long long start = global_timer_ns();
+    for (unsigned int tries = 1; !mbar_try_wait(&sc->entry_ready[ph & 3], (ph >> 2) & 1); ++tries) {
+        if ((tries & 127u) == 0u && global_timer_ns() - start > 2 * sc->limit_ns) {
+            record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+            sc->abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
 }
 // Hands the stage back once the warp has its values, and moves on.
 __device__ __forceinline__ void ring_next(Place& s) {
@@ -1585,9 +1598,11 @@ __device__ __forceinline__ bool begin_launch(const KernelParams& p, const Stream
             mbar_init(&sc->full[i], 1);
             mbar_init(&sc->empty[i], kWarps);
         }
-        mbar_init(&sc->entry_full, 1);
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&sc->entry_ready[i], 1);
+            mbar_init(&sc->entry_done[i], kWarps);
+        }
         sc->issued = 0;
-        sc->fetched = 0;
         mbar_init_fence();
         sc->abort_flag = peek_status(p.ctl) != 0 ? 1 : 0;  // a faulted plan runs nothing
         sc->limit_ns = static_cast<unsigned long long>(p.wait_limit_us) * 1000ull;
@@ -1647,40 +1662,25 @@ __device__ __forceinline__ uint4 resolve_vector(uint4 v, int index) {
     return v;
 }
 
-// Phase entries: at the start of phase ph warp 0 resolves the addresses of record ph + 1, which
-// the barrier inside the phase publishes, and fetches record ph + 2 over that of ph - 2 (no
-// warp can still be there: all have passed the barrier of ph - 1).  Once a fault is on record in this
-// CTA it ends the walk at ph + 1 instead, through the kind of that phase, which the same barrier
-// publishes: every warp leaves there, and nobody looks at a record whose copy has not landed.
-__device__ __forceinline__ void fetch_entry(int ph) {
-    SharedCtl* sc = ctl_of();
-    if (ph < sc->n_phases && (threadIdx.x & 31) == 0) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive_expect_tx(&sc->entry_full, sizeof(PhaseEntry));
-        bulk_copy_g2s(&sc->entry[ph & 3], sc->entries + ph, sizeof(PhaseEntry), &sc->entry_full);
-        sc->fetched = ph + 1;
-    }
-}
-__device__ __noinline__ void next_entry(int ph) {
+// Phase entries: a warp of its own copies the records and resolves their addresses, up to four phases ahead of
+// the consumers.  (Warp 0 did it at the start of each phase: 2,500 cycles on the chain of every phase of
+// the 135M shape with a bulk copy, whose proxy fence waited for the results the warp had just stored, 1,700
+// without, most of them instructions that are not in the cache after a phase.)
+__device__ __noinline__ void entry_loop() {
     SharedCtl* sc = ctl_of();
     const int lane = threadIdx.x & 31;
-    if (ph >= sc->n_phases) return;
-    const bool landed = mbar_wait_bounded(&sc->entry_full, ph & 1, &sc->abort_flag, sc->limit_ns);
-    if (__any_sync(0xffffffffu, !landed || sc->abort_flag != 0)) {
-        if (lane == 0) {
-            if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
-            sc->abort_flag = 1;
-            table_of()[ph].kind = kStreamStop;
+#pragma unroll 1
+    for (int ph = 0; ph < sc->n_phases; ++ph) {
+        if (ph >= 4 && !__all_sync(0xffffffffu, mbar_wait_bounded(&sc->entry_done[ph & 3], ((ph >> 2) - 1) & 1,
+                                                                 &sc->abort_flag, 8 * sc->limit_ns)))
+            return;  // a fault is on record, or soon will be: the consumers have limits of their own
+        if (lane < kEntryVectors) {
+            uint4* v = reinterpret_cast<uint4*>(&sc->entry[ph & 3]) + lane;
+            *v = resolve_vector(ld_cg_u4(reinterpret_cast<const uint4*>(sc->entries + ph) + lane), lane);
         }
         __syncwarp();
-        return;
+        if (lane == 0) mbar_arrive(&sc->entry_ready[ph & 3]);
     }
-    if (lane < kEntryVectors) {
-        uint4* v = reinterpret_cast<uint4*>(&sc->entry[ph & 3]) + lane;
-        *v = resolve_vector(*v, lane);
-    }
-    __syncwarp();
-    fetch_entry(ph + 1);
 }
 
 // The consumer warps' walk through the phase table.
@@ -1688,12 +1688,8 @@ template <int DIM>
 __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned int calls) {
     SharedCtl* sc = ctl_of();
     const StreamDesc* table = table_of();
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
     Place place{0u, 0u, 0u};
-    if (warp == 0) {
-        fetch_entry(0);
-        next_entry(0);
-    }
     // the other half of the arena becomes blank for the next launch
     for (unsigned long long at = (static_cast<unsigned long long>(blockIdx.x) * kThreads + tid) * 16;
          at < p.relay_bytes; at += static_cast<unsigned long long>(gridDim.x) * kThreads * 16)
@@ -1709,7 +1705,10 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
     for (int ph = 0; ph < p.n_phases; ++ph) {
         const int kind = table[ph].kind;
         if (kind == kStreamStop) break;
-        if (warp == 0) next_entry(ph + 1);
+        if (!entry_wait(ph)) break;
+        // Once a fault is on record in this CTA the walk ends at ph + 1, through the kind of that phase, which
+        // the barrier inside this one publishes: every warp leaves there.
+        if (tid == 0 && sc->abort_flag != 0 && ph + 1 < p.n_phases) table_of()[ph + 1].kind = kStreamStop;
         const PhaseEntry* E = &sc->entry[ph & 3];
         trace_stamp(ph, 0);
         bool meet = true;  // the phase has not had a barrier of all threads
@@ -1745,6 +1744,8 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
                 break;  // the same for all threads
             trace_stamp(ph, 3);
         }
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(&sc->entry_done[ph & 3]);
     }
 }
 
@@ -1765,6 +1766,7 @@ decode_kernel(const __grid_constant__ KernelParams p) {
 
     if (threadIdx.x >= kThreads) {
         if (threadIdx.x == kThreads) producer_loop();
+        if (threadIdx.x >= kThreads + 32) entry_loop();
     } else {
         consume_launch<DIM>(p, calls);
     }
