@@ -595,6 +595,24 @@ __device__ __forceinline__ uint4 normalise_fast(uint4 x, uint4 w, float inv) {
     return make_uint4(xv[0], xv[1], xv[2], xv[3]);
 }
 
+// What the code on a phase's chain needs of its record, read before the activations arrive.  (Every asm statement
+// that touches memory makes the compiler read a record again.)
+struct Recipe {
+    int rows, prologue, epilogue, cells;
+    unsigned int modes;
+    bool gather;
+};
+__device__ __forceinline__ Recipe recipe_of(const PhaseEntry* E) {
+    Recipe r;
+    r.rows = E->rec.i[MB_GV_I_ROWS];
+    r.prologue = E->rec.i[MB_GV_I_PROLOGUE];
+    r.epilogue = E->rec.i[MB_GV_I_EPILOGUE];
+    r.cells = E->rec.i[MB_GV_I_CELLS];
+    r.modes = static_cast<unsigned int>(E->modes);
+    r.gather = E->rec.i[MB_GV_I_GATHER] != 0;
+    return r;
+}
+
 // A warp's share of the activations: of every stage the groups it multiplies ("vectors": 32
 // elements of each row), R rows (the batch rounded up to a power of two) of four lanes x 16 bytes
 // each, one after the other in the warp's own 8 KB (or 10 KB) of shared memory.  A lane brings and normalises the
@@ -612,9 +630,8 @@ struct Slice {
     int chunk;           // stages per chunk
     int first, vectors, slots;   // of the current chunk
 };
-__device__ __forceinline__ Slice slice_of(const PhaseEntry* E, const GemvStream& d, int c) {
+__device__ __forceinline__ Slice slice_of(int rows, const GemvStream& d, int c) {
     Slice v;
-    const int rows = E->rec.i[MB_GV_I_ROWS];
     v.lp = (d.shape & kShapeShort) ? 2 : 1;
     v.rs = rows > 2 ? (rows > 4 ? 3 : 2) : rows - 1;
     v.stages = (d.groups + (8 << v.lp) - 1) >> (3 + v.lp);
@@ -675,7 +692,7 @@ __device__ __noinline__ void stage_cells(const int ph, const int c) {
     const PhaseEntry* E = &sc->entry[ph & 3];
     const GemvStream& d = table_of()[ph].gemv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const Slice sl = slice_of(E, d, c);
+    const Slice sl = slice_of(E->rec.i[MB_GV_I_ROWS], d, c);
     const int row = min((lane >> 2) & ((1 << sl.rs) - 1), E->rec.i[MB_GV_I_ROWS] - 1);
     const char* x = reinterpret_cast<const char*>(E->addr[MB_GV_S_X]) + (lane & 3) * 32 +
                     static_cast<size_t>(row) * d.row_bytes * 2;
@@ -691,26 +708,29 @@ __device__ __noinline__ void stage_cells(const int ph, const int c) {
 // Brings chunk `c` of the warp's slice to shared memory, un-normalised, once its producers have
 // written it; `store`: also hand on the gathered rows.  Returns this lane's part of its row's sum of
 // squares when the phase normalises.
-__device__ __forceinline__ float stage_slice(const int ph, const int c, const bool store) {
+__device__ __forceinline__ float stage_slice(const int ph, const int c, const bool store, const Recipe& rc,
+                                             const Slice& sl, const unsigned int base, const int groups,
+                                             const int row_bytes) {
     SharedCtl* sc = ctl_of();
     const PhaseEntry* E = &sc->entry[ph & 3];
     const GemvStream& d = table_of()[ph].gemv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tq = lane & 3;
-    const Slice sl = slice_of(E, d, c);
-    const int row = min(gid & ((1 << sl.rs) - 1), E->rec.i[MB_GV_I_ROWS] - 1);
+    const int row = min(gid & ((1 << sl.rs) - 1), rc.rows - 1);
     const int vec = sl.first + (gid >> sl.rs), step = 8 >> sl.rs;
-    const bool gather = E->rec.i[MB_GV_I_GATHER] != 0;
-    const int flags = E->rec.i[MB_GV_I_CELLS];
-    const bool relay = !gather && (E->modes & kModeInRelay);
+    const bool gather = rc.gather;
+    const int flags = rc.cells;
+    const bool relay = !gather && (rc.modes & kModeInRelay);
     const bool cells = !gather && !relay && (flags & MB_CELLS_X);
-    const bool norm = E->rec.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
-    const unsigned int out = slice_base(warp) + lane * 16;
+    const bool norm = rc.prologue != MB_PRO_NONE;
+    const unsigned int out = base + lane * 16;
     __syncwarp();
     if (norm && weights_staged(sl)) {
+        const unsigned long long w_norm = d.w_norm;
+        const unsigned int end = base + sc->slots * 512;
         for (int v = gid; v < sl.vectors; v += 8)
-            cp_async16(slice_base(warp + 1) - (sl.vectors - v) * 64 + tq * 16,
-                       d.w_norm + min(vector_group(sl.lp, warp, v), d.groups - 1) * 64 + tq * 16);
+            cp_async16(end - (sl.vectors - v) * 64 + tq * 16,
+                       w_norm + min(vector_group(sl.lp, warp, v), groups - 1) * 64 + tq * 16);
     }
     const char* x = reinterpret_cast<const char*>(E->addr[MB_GV_S_X]) + 16 * tq;
     if (gather) {
@@ -719,11 +739,11 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
             record_status(sc->ctl, MB_ST_TOKEN_RANGE, ph, blockIdx.x);
             id = 0;
         }
-        x += static_cast<size_t>(id) * d.row_bytes;
+        x += static_cast<size_t>(id) * row_bytes;
     } else {
-        x += static_cast<size_t>(row) * d.row_bytes;
+        x += static_cast<size_t>(row) * row_bytes;
     }
-    if (E->modes & kModeWait) {
+    if (rc.modes & kModeWait) {
         if (lane == 0) finished_wait(ph, E->rec.i[MB_GV_I_X_SOURCE]);
         __syncwarp();
     }
@@ -734,17 +754,17 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
         int i = 0;
 #pragma unroll 1
         for (; sl.slots - i > 4; i += 8)
-            fill_slots<8>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
+            fill_slots<8>(x, sl.lp, warp, vec, step, groups, i, sl.slots, out, relay, ph);
         if (sl.slots - i == 1)
-            fill_slots<1>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
+            fill_slots<1>(x, sl.lp, warp, vec, step, groups, i, sl.slots, out, relay, ph);
         else if (sl.slots > i)
-            fill_slots<4>(x, sl.lp, warp, vec, step, d.groups, i, sl.slots, out, relay, ph);
+            fill_slots<4>(x, sl.lp, warp, vec, step, groups, i, sl.slots, out, relay, ph);
     }
     if (gather) {
         // embedding scale; the residual stream needs the un-normalised rows
         const float scale = E->rec.f[MB_GV_F_EMBED_SCALE];
         char* keep = reinterpret_cast<char*>(E->addr[MB_GV_S_XSTORE]);
-        const bool as_cells = (flags & MB_CELLS_XSTORE) && !(E->modes & kModeStoreRelay);
+        const bool as_cells = (flags & MB_CELLS_XSTORE) && !(rc.modes & kModeStoreRelay);
         const unsigned int tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
         const bool mine = store && E->rec.i[MB_GV_I_STORE_X] && blockIdx.x == 0 && row == (gid & ((1 << sl.rs) - 1));
 #pragma unroll 1
@@ -755,10 +775,10 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
                 v = scale_vector(v, scale);
                 sts128(out + i * 512, v);
             }
-            if (E->modes & kModeStoreRelay)  // rows of the table as they are: the one thing not converted
+            if (rc.modes & kModeStoreRelay)  // rows of the table as they are: the one thing not converted
                 v = make_uint4(as_written(v.x), as_written(v.y), as_written(v.z), as_written(v.w));
-            if (mine && g < d.groups) {
-                const size_t e = static_cast<size_t>(row) * (d.row_bytes / 2) + g * 32 + 8 * tq;
+            if (mine && g < groups) {
+                const size_t e = static_cast<size_t>(row) * (row_bytes / 2) + g * 32 + 8 * tq;
                 store_result(keep, e, v.x, as_cells, tag);
                 store_result(keep, e + 2, v.y, as_cells, tag);
                 store_result(keep, e + 4, v.z, as_cells, tag);
@@ -771,7 +791,7 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
 #pragma unroll 4
         for (int i = 0; i < sl.slots; ++i) {
             const float part = dot_self(lds128(out + i * 512));
-            ss += vector_group(sl.lp, warp, vec + i * step) < d.groups ? part : 0.f;
+            ss += vector_group(sl.lp, warp, vec + i * step) < groups ? part : 0.f;
         }
     }
     __syncwarp();
@@ -779,23 +799,20 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
 }
 
 // Normalises the staged chunk in place.  `ss`: the warp-summed squares are in norm_part.
-__device__ __forceinline__ void normalise_slice(const int ph, const int c) {
+__device__ __forceinline__ void normalise_slice(const int ph, const int kind, const Slice& sl, const unsigned int base,
+                                                const int groups, const int row_bytes, const float eps) {
     SharedCtl* sc = ctl_of();
-    const PhaseEntry* E = &sc->entry[ph & 3];
-    const GemvStream& d = table_of()[ph].gemv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tq = lane & 3;
-    const Slice sl = slice_of(E, d, c);
     const int row = gid & ((1 << sl.rs) - 1), step = 8 >> sl.rs;
-    const int kind = E->rec.i[MB_GV_I_PROLOGUE];
     const float4 lo = *reinterpret_cast<const float4*>(&sc->norm_part[row][0]);
     const float4 hi = *reinterpret_cast<const float4*>(&sc->norm_part[row][4]);
     const float total = ((lo.x + lo.y) + (lo.z + lo.w)) + ((hi.x + hi.y) + (hi.z + hi.w));
-    const float inv = 1.0f / sqrtf(total / static_cast<float>(d.row_bytes / 2) + E->rec.f[MB_GV_F_EPS]);
-    const unsigned int out = slice_base(warp) + lane * 16;
+    const float inv = 1.0f / sqrtf(total / static_cast<float>(row_bytes / 2) + eps);
+    const unsigned int out = base + lane * 16;
     const bool staged = weights_staged(sl);
     const char* w = staged ? g_smem + slice_offset(sc->stages) + (warp + 1) * sc->slots * 512 - sl.vectors * 64
-                           : reinterpret_cast<const char*>(d.w_norm);
+                           : reinterpret_cast<const char*>(table_of()[ph].gemv.w_norm);
     w += tq * 16;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
@@ -804,7 +821,7 @@ __device__ __forceinline__ void normalise_slice(const int ph, const int c) {
     for (int i = 0; i < sl.slots; ++i) {
         const int v = vec + i * step;
         const int at = staged ? min(v, sl.vectors - 1)
-                              : min(vector_group(sl.lp, warp, sl.first + v), d.groups - 1);
+                              : min(vector_group(sl.lp, warp, sl.first + v), groups - 1);
         const uint4 nw = *reinterpret_cast<const uint4*>(w + at * 64);
         const uint4 x = lds128(out + i * 512);
         sts128(out + i * 512,
@@ -814,25 +831,37 @@ __device__ __forceinline__ void normalise_slice(const int ph, const int c) {
 }
 
 // The same out of line, for slices of several chunks.
-__device__ __noinline__ float stage_chunk(int ph, int c, bool store) { return stage_slice(ph, c, store); }
-__device__ __noinline__ void normalise_chunk(int ph, int c) { normalise_slice(ph, c); }
+__device__ __noinline__ float stage_chunk(int ph, int c, bool store) {
+    const GemvStream& d = table_of()[ph].gemv;
+    const Recipe rc = recipe_of(&ctl_of()->entry[ph & 3]);
+    return stage_slice(ph, c, store, rc, slice_of(rc.rows, d, c), slice_base(threadIdx.x >> 5), d.groups, d.row_bytes);
+}
+__device__ __noinline__ void normalise_chunk(int ph, int c) {
+    const GemvStream& d = table_of()[ph].gemv;
+    const PhaseEntry* E = &ctl_of()->entry[ph & 3];
+    normalise_slice(ph, E->rec.i[MB_GV_I_PROLOGUE], slice_of(E->rec.i[MB_GV_I_ROWS], d, c),
+                    slice_base(threadIdx.x >> 5), d.groups, d.row_bytes, E->rec.f[MB_GV_F_EPS]);
+}
 
 // The element of a batch of blocks that a thread finishes.
 struct Result {
     int vrow, tok;               // virtual row (INT_MAX: none), activation row
     unsigned int residual;       // the packed pair that holds its residual
     float bias;
+    char* out;                   // where an even row's pair goes
 };
 // `lr`: log2 of the rows of a block, 3 or 4; a block has 8 << lr results.
-__device__ __forceinline__ Result request_result(const PhaseEntry* E, const GemvStream& d, int lr, int block) {
+__device__ __forceinline__ Result request_result(const PhaseEntry* E, const GemvStream& d, const Recipe& rc, int lr,
+                                                 int block) {
     const int t = threadIdx.x;
     Result r;
     r.vrow = INT_MAX;
     r.tok = t & 7;
     r.residual = kUnwritten;
     r.bias = 0.f;
+    r.out = nullptr;
     const int b = block + (t >> (3 + lr));
-    if (b < d.nblocks && r.tok < E->rec.i[MB_GV_I_ROWS]) {
+    if (b < d.nblocks && r.tok < rc.rows) {
         int end;
         const int vrow = block_row(d, b, 1 << lr, &end) + (t >> 3 & ((1 << lr) - 1));
         if (vrow < end) {
@@ -842,20 +871,32 @@ __device__ __forceinline__ Result request_result(const PhaseEntry* E, const Gemv
             const unsigned short* bias = reinterpret_cast<const unsigned short*>(E->addr[MB_GV_S_BIAS0 + seg]);
             if (bias != nullptr) r.bias = bf16_bits_to_float(__ldg(bias + local));
             // (a plain one of a phase that waits may not have been written yet: finish_result loads it)
-            if (E->rec.i[MB_GV_I_EPILOGUE] == MB_EPI_RESIDUAL &&
-                ((E->modes & kModeResidualRelay) ||
-                 !((E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL) || (E->modes & kModeWait))))
+            if (rc.epilogue == MB_EPI_RESIDUAL &&
+                ((rc.modes & kModeResidualRelay) || !((rc.cells & MB_CELLS_RESIDUAL) || (rc.modes & kModeWait))))
                 r.residual = ld_relaxed_u32(residual_address(E, vrow, r.tok));
+            const bool out_cells = (rc.cells & MB_CELLS_OUT) != 0 && !(rc.modes & kModeOutRelay);
+            r.out = reinterpret_cast<char*>(E->addr[MB_GV_S_OUT0 + seg]) +
+                    (static_cast<size_t>(r.tok) * E->rec.i[MB_GV_I_N0 + seg] + local) * (out_cells ? 4 : 2);
         }
     }
     return r;
 }
 
+// The residual where it was not there when it was asked for.  (Out of line: it is there by then.)
+__device__ __noinline__ unsigned int late_residual(int ph, int vrow, int tok) {
+    const SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const char* at = residual_address(E, vrow, tok);
+    if (E->modes & kModeResidualRelay) return relay_wait(at, ph);
+    if (E->rec.i[MB_GV_I_CELLS] & MB_CELLS_RESIDUAL)
+        return cell_data(cell_wait(at, sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_RES_SOURCE]) + 1u, ph));
+    return ld_relaxed_u32(at);  // plain, of a phase that waits: stage_slice has waited for it
+}
+
 // Adds the slices of a thread's element, in slice order, runs the epilogue and stores the result
 // together with its neighbour's (the odd row of a pair sits eight lanes further on).
-__device__ __forceinline__ void finish_result(const PhaseEntry* E, const GemvStream& d, const int ph, const int lr,
-                                              const bool paired, const float* batch, Result r) {
-    const SharedCtl* sc = ctl_of();
+__device__ __forceinline__ void finish_result(const Recipe& rc, const int ph, const int lr, const bool paired,
+                                              const float* batch, Result r) {
     const int t = threadIdx.x;
     const float* part = batch + (t >> (3 + lr)) * (kWarps * 128) + (t & ((8 << lr) - 1));
     float v[kWarps];
@@ -863,41 +904,33 @@ __device__ __forceinline__ void finish_result(const PhaseEntry* E, const GemvStr
     for (int w = 0; w < kWarps; ++w) v[w] = part[w * 128];
     const float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     const bool live = r.vrow != INT_MAX;
-    const int cells = E->rec.i[MB_GV_I_CELLS], epilogue = E->rec.i[MB_GV_I_EPILOGUE];
     float y = bf16_round(sum + r.bias);
     if (paired) {
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) v[w] = part[w * 128 + 64];
         const float up = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-        const float act = sigmoid_product(y, epilogue == MB_EPI_SILU_MUL ? y : gelu_exponent(y));
+        const float act = sigmoid_product(y, rc.epilogue == MB_EPI_SILU_MUL ? y : gelu_exponent(y));
         y = bf16_round(act) * bf16_round(up);
-    } else if (epilogue == MB_EPI_RESIDUAL) {
-        if (live) {
-            if (E->modes & kModeResidualRelay) {
-                if (r.residual == kUnwritten) r.residual = relay_wait(residual_address(E, r.vrow, r.tok), ph);
-            } else if (cells & MB_CELLS_RESIDUAL) {
-                r.residual = cell_data(cell_wait(
-                    residual_address(E, r.vrow, r.tok),
-                    sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_GV_I_RES_SOURCE]) + 1u, ph));
-            } else if (E->modes & kModeWait) {  // stage_slice has waited for it
-                r.residual = ld_relaxed_u32(residual_address(E, r.vrow, r.tok));
-            }
-        }
+    } else if (rc.epilogue == MB_EPI_RESIDUAL) {
+        const bool asked = (rc.modes & kModeResidualRelay) || !((rc.cells & MB_CELLS_RESIDUAL) || (rc.modes & kModeWait));
+        // in the relay arena the blank pattern says that it was not there yet; elsewhere it may be a value
+        if (live && (!asked || (r.residual == kUnwritten && (rc.modes & kModeResidualRelay))))
+            r.residual = late_residual(ph, r.vrow, r.tok);
         y = (r.vrow & 1 ? hi_bf16(r.residual) : lo_bf16(r.residual)) + y;
     }
     const float other = __shfl_xor_sync(0xffffffffu, y, 8);
     if (live && (r.vrow & 1) == 0) {
-        int local = r.vrow;
-        const int seg = output_segment(d, local);
-        store_result(reinterpret_cast<char*>(E->addr[MB_GV_S_OUT0 + seg]),
-                     static_cast<size_t>(r.tok) * E->rec.i[MB_GV_I_N0 + seg] + local, pack_bf16(y, other),
-                     (cells & MB_CELLS_OUT) != 0 && !(E->modes & kModeOutRelay),
-                     sc->tag_base + static_cast<unsigned int>(ph) + 1u);
+        const unsigned int both = pack_bf16(y, other);
+        if ((rc.cells & MB_CELLS_OUT) != 0 && !(rc.modes & kModeOutRelay))
+            st_cell(r.out, both, ctl_of()->tag_base + static_cast<unsigned int>(ph) + 1u);
+        else
+            st_relaxed_u32(r.out, both);
     }
 }
 
 // SHORT: blocks of 8 rows, 32 groups per stage (a CTA's rows fit one block, or few); else 16 rows,
-// or 8 gate and 8 up rows, 16 groups per stage.
+// or 8 gate and 8 up rows, 16 groups per stage.  (One body for all three shapes, told apart at run time, is 37 KB
+// less code and slower: 1B 673 -> 695 us, 1.7B with 8 rows 3,520 -> 3,700.)
 // WHOLE: the slices fit their place (host rule, kShapeWhole).
 template <bool SHORT, bool WHOLE>
 __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
@@ -907,14 +940,18 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nblocks = d.nblocks;
     const bool paired = !SHORT && (d.shape & kShapePaired);
-    const bool norm = E->rec.i[MB_GV_I_PROLOGUE] != MB_PRO_NONE;
+    const Recipe rc = recipe_of(E);
+    const bool norm = rc.prologue != MB_PRO_NONE;
     const int lr = SHORT || paired ? 3 : 4;
-    Result result = request_result(E, d, lr, 0);
+    const int groups = d.groups, row_bytes = d.row_bytes;
+    const float eps = E->rec.f[MB_GV_F_EPS];
+    const unsigned int base = slice_base(warp);
+    Result result = request_result(E, d, rc, lr, 0);
 
-    const Slice sl = slice_of(E, d, 0);
+    const Slice sl = slice_of(rc.rows, d, 0);
     float ss = 0.f;
     if (WHOLE) {
-        ss = stage_slice(ph, 0, true);
+        ss = stage_slice(ph, 0, true, rc, sl, base, groups, row_bytes);
     } else if (norm) {
 #pragma unroll 1
         for (int c = 0; c * sl.chunk < sl.stages; ++c) ss += stage_chunk(ph, c, true);
@@ -927,7 +964,7 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
         if (sl.rs < 1) ss += __shfl_xor_sync(0xffffffffu, ss, 4);
         if ((lane & 3) == 0) sc->norm_part[lane >> 2][warp] = ss;
         named_barrier(kBarAll, kThreads);
-        if (WHOLE) normalise_slice(ph, 0);
+        if (WHOLE) normalise_slice(ph, rc.prologue, sl, base, groups, row_bytes, eps);
     }
     trace_stamp(ph, 1);
 
@@ -937,7 +974,7 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
     const unsigned int piece_step = SHORT || paired ? 512u : 1024u;
     const unsigned int piece_half = paired ? kRingStage / 2 : 512u;
     const unsigned int lane_ring = smem_u32(g_smem) + kRingOffset + lane * 16 + warp * per * piece_step;
-    const unsigned int lane_x = slice_base(warp) + (lane & ((4 << sl.rs) - 1)) * 16;
+    const unsigned int lane_x = base + (lane & ((4 << sl.rs) - 1)) * 16;
     const unsigned int x_step = 64u << sl.rs;
     int in_batch = 0;
 #pragma unroll 1
@@ -986,8 +1023,8 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
             *reinterpret_cast<float2*>(cell + 64) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
         if ((++in_batch << lr) == kThreads / 8 || b + 1 == nblocks) {
             named_barrier(kBarAll, kThreads);
-            finish_result(E, d, ph, lr, paired, batch, result);
-            if (b + 1 < nblocks) result = request_result(E, d, lr, b + 1);
+            finish_result(rc, ph, lr, paired, batch, result);
+            if (b + 1 < nblocks) result = request_result(E, d, rc, lr, b + 1);
             s.flip ^= 1u;
             batch = scratch_of() + s.flip * (kScratchBytes / 8);
             in_batch = 0;
