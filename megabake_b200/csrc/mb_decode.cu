@@ -409,22 +409,26 @@ __device__ __forceinline__ void tma_load_5d(unsigned int dst, const CUtensorMap*
         : "memory");
 }
 
-// Producer: one lane walks the phases and fills stage after stage in the order they are consumed.
+// Producer: a warp walks the phases and fills stage after stage in the order they are consumed; its lanes stay
+// together and one elected lane issues (elect_one says why).
 __device__ __noinline__ void producer_loop() {
     SharedCtl* sc = ctl_of();
     const StreamDesc* table = table_of();
     const unsigned int ring = smem_u32(g_smem) + kRingOffset;
+    const int lane = threadIdx.x & 31;
     int stage = 0;
-    unsigned int parity = 1;
-    // the next stage, once every warp has read what it held, armed for `bytes`
-    auto open_stage = [&](int ph, unsigned int bytes) {
-        if (!mbar_wait_bounded(&sc->empty[stage], parity, &sc->abort_flag, 2 * sc->limit_ns)) {
-            if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
-            sc->abort_flag = 1;
+    unsigned int parity = 1, issued = 0;
+    // the next stage, once every warp has read what it held
+    auto open_stage = [&](int ph) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sc->empty[stage], parity, &sc->abort_flag, 2 * sc->limit_ns))) {
+            if (lane == 0) {
+                if (!sc->abort_flag) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+                sc->abort_flag = 1;
+            }
             return false;
         }
-        sc->issued = sc->issued + 1;
-        mbar_arrive_expect_tx(&sc->full[stage], bytes);
+        ++issued;
+        if (lane == 0) sc->issued = issued;
         return true;
     };
     auto next_stage = [&] {
@@ -438,16 +442,23 @@ __device__ __noinline__ void producer_loop() {
         if (table[ph].kind == kStreamKv) {
             const int head_dim = table[ph].kv.head_dim;
             Segment& seg = sc->segment[kWarps];
-            for (int which = 0; locate_segment(ph, which, &seg, true); ++which) {
+            for (int which = 0; locate_segment(ph, which, &seg, lane == 0); ++which) {
+                __syncwarp();
                 const int shift = kv_shift(head_dim);
                 const unsigned int bytes = 8192;  // of the keys
-                for (int blk = seg.blk0; blk < seg.blk1; blk += 1 << shift) {
-                    if (!open_stage(ph, 2 * bytes)) return;
+                const int blk0 = seg.blk0, blk1 = seg.blk1, h = seg.h, b = seg.b;
+                for (int blk = blk0; blk < blk1; blk += 1 << shift) {
+                    if (!open_stage(ph)) return;
                     const unsigned int dst = ring + static_cast<unsigned int>(stage) * kRingStage;
-                    tma_load_5d(dst, maps, blk * 16, seg.h, seg.b, &sc->full[stage]);
-                    tma_load_5d(dst + bytes, maps + 1, blk * 16, seg.h, seg.b, &sc->full[stage]);
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&sc->full[stage], 2 * bytes);
+                        tma_load_5d(dst, maps, blk * 16, h, b, &sc->full[stage]);
+                        tma_load_5d(dst + bytes, maps + 1, blk * 16, h, b, &sc->full[stage]);
+                    }
+                    __syncwarp();
                     next_stage();
                 }
+                __syncwarp();
             }
             continue;
         }
@@ -458,7 +469,7 @@ __device__ __noinline__ void producer_loop() {
         const int step = is_short ? 32 : 16;  // groups per stage
         const char* nw = reinterpret_cast<const char*>(d.w_norm);
         if (nw != nullptr)  // every CTA reads the norm weights right after its wait: have them in L2
-            for (int at = static_cast<int>(blockIdx.x) * 128; at < d.row_bytes; at += 8 * 128)
+            for (int at = (static_cast<int>(blockIdx.x) + 8 * lane) * 128; at < d.row_bytes; at += 8 * 32 * 128)
                 prefetch_l2(nw + at);
         for (int b = 0; b < d.nblocks; ++b) {
             int end;
@@ -472,10 +483,14 @@ __device__ __noinline__ void producer_loop() {
                 row -= d.n0;
             }
             for (int g = 0; g < d.groups; g += step) {
-                if (!open_stage(ph, kRingStage)) return;
+                if (!open_stage(ph)) return;
                 const unsigned int dst = ring + static_cast<unsigned int>(stage) * kRingStage;
-                tma_load_3d(dst, map, row, g, &sc->full[stage]);
-                if (paired) tma_load_3d(dst + kRingStage / 2, maps + 1, row, g, &sc->full[stage]);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sc->full[stage], kRingStage);
+                    tma_load_3d(dst, map, row, g, &sc->full[stage]);
+                    if (paired) tma_load_3d(dst + kRingStage / 2, maps + 1, row, g, &sc->full[stage]);
+                }
+                __syncwarp();
                 next_stage();
             }
         }
@@ -1802,8 +1817,10 @@ decode_kernel(const __grid_constant__ KernelParams p) {
     const StreamDesc* table = table_of();
 
     if (threadIdx.x >= kThreads) {
-        if (threadIdx.x == kThreads) producer_loop();
-        if (threadIdx.x >= kThreads + 32) entry_loop();
+        if (threadIdx.x < kThreads + 32)
+            producer_loop();
+        else
+            entry_loop();
     } else {
         consume_launch<DIM>(p, calls);
     }
@@ -2113,7 +2130,7 @@ attention_static_kernel(const __grid_constant__ KernelParams p, const __grid_con
     if (begin_launch(p, &stream, &maps, epoch, 0u, 0u)) {
         if (tid < kThreads)
             run_attention<0>(0, Place{0u, 0u, 0u});
-        else if (tid == kThreads)
+        else if (tid < kThreads + 32)
             producer_loop();
         __syncthreads();
         if (sc->abort_flag && tid == 0) drain_ring();
