@@ -1173,6 +1173,9 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
     const int dump_pitch = sc->slots * 128;  // floats
     const Segment& seg = sc->segment[warp];
     bool parted = false;  // some segment is one of several parts of its pair
+    // One item a CTA at most, the usual case: its record still holds it when its parts are folded (a search takes
+    // 1,000 cycles).
+    const bool single = d.batch * d.kv_heads * d.chunks <= static_cast<int>(gridDim.x);
     for (int which = 0; find_segment(ph, which); ++which) {
         const int L = seg.length;
         const int b = seg.b, h = seg.h;
@@ -1458,17 +1461,35 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
                 }
             }
             named_barrier(kBarAll, kThreads);
+            // Several outputs a thread (256-wide heads): the warps' weights are worked out once.
+            constexpr bool kShared = D > DR;
+            if (kShared && r == 0) {
+                const int w = tid >> 3, head = tid & 7;
+                if (tid < 8 * kWarps) {
+                    float m_all = -INFINITY;
+#pragma unroll
+                    for (int q = 0; q < kWarps; ++q) m_all = fmaxf(m_all, sc->stat[q][head][0]);
+                    sc->exchange[0][w][head] = __expf(sc->stat[w][head][0] - m_all);
+                    if (w == 0) sc->exchange[1][0][head] = m_all;
+                }
+                named_barrier(kBarAll, kThreads);
+            }
 #pragma unroll 1
             for (int o = tid; o < group * (DR / 2); o += kThreads) {
                 const int head = o / (DR / 2), dim = 2 * (o & (DR / 2 - 1));
                 float m_all = -INFINITY, l_all = 0.f, y0 = 0.f, y1 = 0.f;
+                if (kShared) {
+                    m_all = sc->exchange[1][0][head];
+                } else {
 #pragma unroll
-                for (int w = 0; w < kWarps; ++w) m_all = fmaxf(m_all, sc->stat[w][head][0]);
+                    for (int w = 0; w < kWarps; ++w) m_all = fmaxf(m_all, sc->stat[w][head][0]);
+                }
 #pragma unroll
                 for (int w = 0; w < kWarps; ++w) {
                     // weights between partial softmax states: no rounding point of the operator
                     // sits here, the fast exponential is accurate to 2^-21
-                    const float wgt = __expf(sc->stat[w][head][0] - m_all);  // 0: a warp without a block
+                    const float wgt = kShared ? sc->exchange[0][w][head]
+                                              : __expf(sc->stat[w][head][0] - m_all);  // 0: a warp without a block
                     const float2 v =
                         *reinterpret_cast<const float2*>(dumps + w * dump_pitch + head * PR + dim);
                     l_all += sc->stat[w][head][1] * wgt;
@@ -1500,7 +1521,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
     // ---- fold the parts of the pairs this CTA has a part of: its share of their outputs.  Only
     // after ALL its partials are out, so no chain of CTAs waits for one another's folds.
     for (int which = 0; parted; ++which) {
-        if (!find_segment(ph, which)) break;
+        if (single ? which > 0 : !find_segment(ph, which)) break;
         if (seg.parts == 1) continue;
         const int total = group * (D / 2);  // pairs of neighbouring outputs
         const int lo = seg.index * total / seg.parts, hi = (seg.index + 1) * total / seg.parts;
@@ -1509,29 +1530,36 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         // A thread takes up to eight parts of an output pair, four threads up to 32: the cells of all of
         // them are in flight together, again and again until none carries an older tag.  (One part a
         // thread, its four cells waited for one after the other, took 4.6 us on the 0.5B shape
-        // and 9.7 on the 2B, after the last part was out.)
+        // and 9.7 on the 2B, after the last part was out; now 1.9 and 2.7.)
+        // Only what is needed is asked for: a poll of all threads for eight parts each is 64 KB per CTA.
         const int lanes = seg.parts > 8 ? 4 : 1, j = tid & (lanes - 1);
-        for (int o0 = lo; o0 < hi; o0 += kThreads / lanes) {
+        const int slots = seg.parts > 16 ? 8 : (seg.parts > 8 ? 4 : seg.parts);
+        for (int o0 = lo; o0 + (tid & ~31) / lanes < hi; o0 += kThreads / lanes) {
             const int o = o0 + tid / lanes;
             const int head = min(o, hi - 1) / (D / 2), dim = 2 * (min(o, hi - 1) - head * (D / 2));
             const char* first = base + static_cast<size_t>(head) * ((D + 2) * 8);
             unsigned long long cm[8], cl[8], c0[8], c1[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cm[i] = cl[i] = c0[i] = c1[i] = 0ull;
             unsigned long long start = 0;
 #pragma unroll 1
             for (unsigned int tries = 1;; ++tries) {
                 bool missing = false;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    // slot 8, 16 or 24 of these parts does not exist: the last one again, with no weight below
+                    if (i >= slots) break;
+                    // a part that does not exist: the last one again, with no weight below
                     const int c = min(lanes == 1 ? i : j + 4 * (i & 3) + 16 * (i >> 2), seg.parts - 1);
                     const char* part = first + static_cast<size_t>(c) * group * ((D + 2) * 8);
                     ld_cell_pair(part, cm[i], cl[i]);
                     ld_cell_pair(part + (2 + dim) * 8, c0[i], c1[i]);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < 8; ++i) {
+                    if (i >= slots) break;
                     missing |= cell_tag(cm[i]) != own_tag || cell_tag(cl[i]) != own_tag ||
                                cell_tag(c0[i]) != own_tag || cell_tag(c1[i]) != own_tag;
+                }
                 if (!__any_sync(0xffffffffu, missing)) break;
                 if ((tries & 63u) == 0u) {
                     if (start == 0) start = global_timer_ns();
