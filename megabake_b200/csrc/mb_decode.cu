@@ -145,7 +145,7 @@ __device__ __forceinline__ unsigned long long resolve_address(unsigned long long
 // with whatever it has, without waiting any more, and the CTA leaves before the next phase or the one
 // after that (next_entry).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ bool wait_gave_up(int ph, unsigned long long start) {
+__device__ __noinline__ bool wait_gave_up(int ph, unsigned long long start) {
     SharedCtl* sc = ctl_of();
     if (sc->abort_flag) return true;
     if (peek_status(sc->ctl) != 0) {
@@ -720,6 +720,46 @@ __device__ __noinline__ void stage_cells(const int ph, const int c) {
     }
 }
 
+// Gathered rows, in the slice as they are in the table: the embedding scale, and the copy that the residual stream
+// needs.  (Out of line: one phase of a launch.)
+__device__ __noinline__ void finish_gather(const int ph, const int c, const bool store) {
+    const SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const GemvStream& d = table_of()[ph].gemv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tq = lane & 3;
+    const Recipe rc = recipe_of(E);
+    const Slice sl = slice_of(rc.rows, d, c);
+    const int row = min(gid & ((1 << sl.rs) - 1), rc.rows - 1);
+    const int vec = sl.first + (gid >> sl.rs), step = 8 >> sl.rs;
+    const int groups = d.groups, row_bytes = d.row_bytes, flags = rc.cells;
+    const unsigned int out = slice_base(warp) + lane * 16;
+    // embedding scale; the residual stream needs the un-normalised rows
+    const float scale = E->rec.f[MB_GV_F_EMBED_SCALE];
+    char* keep = reinterpret_cast<char*>(E->addr[MB_GV_S_XSTORE]);
+    const bool as_cells = (flags & MB_CELLS_XSTORE) && !(rc.modes & kModeStoreRelay);
+    const unsigned int tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
+    const bool mine = store && E->rec.i[MB_GV_I_STORE_X] && blockIdx.x == 0 && row == (gid & ((1 << sl.rs) - 1));
+#pragma unroll 1
+    for (int i = 0; i < sl.slots; ++i) {
+        const int g = vector_group(sl.lp, warp, vec + i * step);
+        uint4 v = lds128(out + i * 512);
+        if (scale != 0.f) {
+            v = scale_vector(v, scale);
+            sts128(out + i * 512, v);
+        }
+        if (rc.modes & kModeStoreRelay)  // rows of the table as they are: the one thing not converted
+            v = make_uint4(as_written(v.x), as_written(v.y), as_written(v.z), as_written(v.w));
+        if (mine && g < groups) {
+            const size_t e = static_cast<size_t>(row) * (row_bytes / 2) + g * 32 + 8 * tq;
+            store_result(keep, e, v.x, as_cells, tag);
+            store_result(keep, e + 2, v.y, as_cells, tag);
+            store_result(keep, e + 4, v.z, as_cells, tag);
+            store_result(keep, e + 6, v.w, as_cells, tag);
+        }
+    }
+}
+
 // Brings chunk `c` of the warp's slice to shared memory, un-normalised, once its producers have
 // written it; `store`: also hand on the gathered rows.  Returns this lane's part of its row's sum of
 // squares when the phase normalises.
@@ -776,30 +816,7 @@ __device__ __forceinline__ float stage_slice(const int ph, const int c, const bo
             fill_slots<4>(x, sl.lp, warp, vec, step, groups, i, sl.slots, out, relay, ph);
     }
     if (gather) {
-        // embedding scale; the residual stream needs the un-normalised rows
-        const float scale = E->rec.f[MB_GV_F_EMBED_SCALE];
-        char* keep = reinterpret_cast<char*>(E->addr[MB_GV_S_XSTORE]);
-        const bool as_cells = (flags & MB_CELLS_XSTORE) && !(rc.modes & kModeStoreRelay);
-        const unsigned int tag = sc->tag_base + static_cast<unsigned int>(ph) + 1u;
-        const bool mine = store && E->rec.i[MB_GV_I_STORE_X] && blockIdx.x == 0 && row == (gid & ((1 << sl.rs) - 1));
-#pragma unroll 1
-        for (int i = 0; i < sl.slots; ++i) {
-            const int g = vector_group(sl.lp, warp, vec + i * step);
-            uint4 v = lds128(out + i * 512);
-            if (scale != 0.f) {
-                v = scale_vector(v, scale);
-                sts128(out + i * 512, v);
-            }
-            if (rc.modes & kModeStoreRelay)  // rows of the table as they are: the one thing not converted
-                v = make_uint4(as_written(v.x), as_written(v.y), as_written(v.z), as_written(v.w));
-            if (mine && g < groups) {
-                const size_t e = static_cast<size_t>(row) * (row_bytes / 2) + g * 32 + 8 * tq;
-                store_result(keep, e, v.x, as_cells, tag);
-                store_result(keep, e + 2, v.y, as_cells, tag);
-                store_result(keep, e + 4, v.z, as_cells, tag);
-                store_result(keep, e + 6, v.w, as_cells, tag);
-            }
-        }
+        finish_gather(ph, c, store);
     }
     float ss = 0.f;
     if (norm) {
@@ -832,7 +849,7 @@ __device__ __forceinline__ void normalise_slice(const int ph, const int kind, co
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     const int vec = gid >> sl.rs;
-#pragma unroll 2
+#pragma unroll 1
     for (int i = 0; i < sl.slots; ++i) {
         const int v = vec + i * step;
         const int at = staged ? min(v, sl.vectors - 1)
@@ -895,6 +912,12 @@ __device__ __forceinline__ Result request_result(const PhaseEntry* E, const Gemv
         }
     }
     return r;
+}
+
+// The same out of line, for the blocks after the first.
+__device__ __noinline__ Result next_result(int ph, int lr, int block) {
+    const PhaseEntry* E = &ctl_of()->entry[ph & 3];
+    return request_result(E, table_of()[ph].gemv, recipe_of(E), lr, block);
 }
 
 // The residual where it was not there when it was asked for.  (Out of line: it is there by then.)
@@ -1039,7 +1062,7 @@ __device__ __noinline__ Place gemv_phase(const int ph, Place s) {
         if ((++in_batch << lr) == kThreads / 8 || b + 1 == nblocks) {
             named_barrier(kBarAll, kThreads);
             finish_result(rc, ph, lr, paired, batch, result);
-            if (b + 1 < nblocks) result = request_result(E, d, rc, lr, b + 1);
+            if (b + 1 < nblocks) result = next_result(ph, lr, b + 1);
             s.flip ^= 1u;
             batch = scratch_of() + s.flip * (kScratchBytes / 8);
             in_batch = 0;
@@ -1463,7 +1486,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             named_barrier(kBarAll, kThreads);
             // Several outputs a thread (256-wide heads): the warps' weights are worked out once.
             constexpr bool kShared = D > DR;
-            if (kShared && r == 0) {
+            if (kShared && !EXACT && r == 0) {
                 const int w = tid >> 3, head = tid & 7;
                 if (tid < 8 * kWarps) {
                     float m_all = -INFINITY;
@@ -1478,7 +1501,9 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             for (int o = tid; o < group * (DR / 2); o += kThreads) {
                 const int head = o / (DR / 2), dim = 2 * (o & (DR / 2 - 1));
                 float m_all = -INFINITY, l_all = 0.f, y0 = 0.f, y1 = 0.f;
-                if (kShared) {
+                if (EXACT) {  // normalised already: every weight is 1, and so is their sum
+                    m_all = 0.f;
+                } else if (kShared) {
                     m_all = sc->exchange[1][0][head];
                 } else {
 #pragma unroll
@@ -1488,18 +1513,18 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
                 for (int w = 0; w < kWarps; ++w) {
                     // weights between partial softmax states: no rounding point of the operator
                     // sits here, the fast exponential is accurate to 2^-21
-                    const float wgt = kShared ? sc->exchange[0][w][head]
+                    const float wgt = EXACT ? 1.f : kShared ? sc->exchange[0][w][head]
                                               : __expf(sc->stat[w][head][0] - m_all);  // 0: a warp without a block
                     const float2 v =
                         *reinterpret_cast<const float2*>(dumps + w * dump_pitch + head * PR + dim);
-                    l_all += sc->stat[w][head][1] * wgt;
+                    if (!EXACT) l_all += sc->stat[w][head][1] * wgt;
                     y0 += v.x * wgt;
                     y1 += v.y * wgt;
                 }
                 const int column = r * DR + dim;
                 if (seg.parts == 1) {
                     store_result(out, (static_cast<size_t>(b) * Hq + h * group + head) * D + column,
-                                 pack_bf16(y0 / l_all, y1 / l_all), out_cells, own_tag);
+                                 EXACT ? pack_bf16(y0, y1) : pack_bf16(y0 / l_all, y1 / l_all), out_cells, own_tag);
                 } else {
                     // cells of (fp32, tag): maximum, sum, D values per head
                     char* part = reinterpret_cast<char*>(E->addr[MB_AT_S_PARTIAL]) +
