@@ -216,20 +216,10 @@ __device__ __forceinline__ uint4 normalise_vector(uint4 x, uint4 w, float inv, i
     return make_uint4(xv[0], xv[1], xv[2], xv[3]);
 }
 
-// x / (1 + exp(-x)) with the operation order of the decomposed graph.
-__device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)); }
-// 0.5 * x * (1 + tanh(sqrt(2/pi) * (x + 0.044715 x^3)))
-__device__ __forceinline__ float gelu_tanh_f32(float x) {
-    const float kBeta = 0.7978845608028654f;
-    const float kKappa = 0.044715f;
-    float inner = kBeta * (x + kKappa * (x * x * x));
-    return 0.5f * x * (1.0f + tanhf(inner));
-}
-
-// Both as x times a sigmoid, with the device's fast exponential and reciprocal; the graph rounds the result to bf16
-// next.  Over all bf16 x, silu then has the same bits as above but for three results below 1e-36; GELU differs
-// at 150, at each of which it is closer to the exact value: 0.5 (1 + tanh u) cancels where tanh u nears -1,
-// the sigmoid of 2 u does not.
+// Both gated activations as x times a sigmoid, with the device's fast exponential and reciprocal; the graph rounds the
+// result to bf16 next.  Over all bf16 x, silu then has the bits of x / (1 + expf(-x)) but for three results below
+// 1e-36; GELU differs from 0.5 x (1 + tanhf u) at 150, at each of which it is closer to the exact value: that form
+// cancels where tanh u nears -1, the sigmoid of 2 u does not.
 __device__ __forceinline__ float gelu_exponent(float x) {
     return 1.5957691216057308f * (x + 0.044715f * (x * x * x));  // 2 sqrt(2 / pi) (x + 0.044715 x^3)
 }
