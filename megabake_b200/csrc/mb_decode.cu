@@ -1116,6 +1116,24 @@ __device__ __noinline__ void fill_rope_row(unsigned int* table, const PhaseEntry
     }
 }
 
+// The table of a launch's positions: the same for every layer of a model, made once.  All consumer threads.
+__device__ __noinline__ void make_rope_table(int ph, int D, int shape) {
+    SharedCtl* sc = ctl_of();
+    const PhaseEntry* E = &sc->entry[ph & 3];
+    const int batch = table_of()[ph].kv.batch;
+    named_barrier(kBarAll, kThreads);
+    const long long* pos = reinterpret_cast<const long long*>(E->addr[MB_AT_S_POS]);
+    for (int b = threadIdx.x >> 5; b < batch; b += kWarps)
+        fill_rope_row(rope_of() + b * (D / 2), E, pos[b], D / 2, threadIdx.x & 31, 32);
+    if (threadIdx.x == 0) {
+        sc->rope_pos = E->addr[MB_AT_S_POS];
+        sc->rope_freq = E->addr[MB_AT_S_INVFREQ];
+        sc->rope_shape = shape;
+        sc->rope_scale = E->rec.f[MB_AT_F_ROPE_SCALE];
+    }
+    named_barrier(kBarAll, kThreads);
+}
+
 // Eight elements of the first half of a head and the eight they rotate with, in place.
 __device__ __forceinline__ void rotate_vectors(uint4& lo, uint4& hi, const unsigned int* table,
                                                float q_scale) {
@@ -1138,6 +1156,20 @@ __device__ __forceinline__ void rotate_vectors(uint4& lo, uint4& hi, const unsig
     }
     lo = make_uint4(a[0], a[1], a[2], a[3]);
     hi = make_uint4(b[0], b[1], b[2], b[3]);
+}
+
+// Queries (and the new key and value) kept as cells: one vector at a time, into the warp's slice.
+__device__ __noinline__ void gather_cells(int ph, const char* qrow, const char* krow, const char* vrow, int groups,
+                                          bool holder) {
+    const SharedCtl* sc = ctl_of();
+    const unsigned int tag =
+        sc->tag_base + static_cast<unsigned int>(sc->entry[ph & 3].rec.i[MB_AT_I_QKV_SOURCE]) + 1u;
+    const unsigned int keep = slice_base(threadIdx.x >> 5) + (threadIdx.x & 31) * 16;
+#pragma unroll 1
+    for (int i = 0; i < (holder ? 2 * groups + 1 : groups); ++i)
+        sts128(keep + min(i, kSliceSlots - 1) * 512,
+               cells_load(i < groups ? qrow + 128 * i : (i < 2 * groups ? krow + 128 * (i - groups) : vrow), tag, ph));
+    __syncwarp();
 }
 
 template <int D, bool EXACT>
@@ -1171,19 +1203,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
         const bool fresh = sc->rope_pos == E->addr[MB_AT_S_POS] &&
                            sc->rope_freq == E->addr[MB_AT_S_INVFREQ] && sc->rope_shape == shape &&
                            sc->rope_scale == E->rec.f[MB_AT_F_ROPE_SCALE];
-        if (!fresh) {  // the same for every layer of a model: made once per launch
-            named_barrier(kBarAll, kThreads);
-            const long long* pos = reinterpret_cast<const long long*>(E->addr[MB_AT_S_POS]);
-            for (int b = warp; b < d.batch; b += kWarps)
-                fill_rope_row(rope + b * (D / 2), E, pos[b], D / 2, lane, 32);
-            if (tid == 0) {
-                sc->rope_pos = E->addr[MB_AT_S_POS];
-                sc->rope_freq = E->addr[MB_AT_S_INVFREQ];
-                sc->rope_shape = shape;
-                sc->rope_scale = E->rec.f[MB_AT_F_ROPE_SCALE];
-            }
-            named_barrier(kBarAll, kThreads);
-        }
+        if (__builtin_expect(!fresh, 0)) make_rope_table(ph, D, shape);
     }
     if (kind == kPlain && (E->rec.i[MB_AT_I_CELLS] & MB_CELLS_X_WAIT)) {
         if (lane == 0) finished_wait(ph, E->rec.i[MB_AT_I_QKV_SOURCE]);
@@ -1225,16 +1245,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             const char* krow = reinterpret_cast<const char*>(E->addr[MB_AT_S_K]) + kv_row + 8 * tq * elem;
             const char* vrow = reinterpret_cast<const char*>(E->addr[MB_AT_S_V]) + kv_row +
                                8 * (lane & (D / 8 - 1)) * elem;
-            if (kind == kCells) {  // one vector at a time, through the warp's slice
-                const unsigned int tag =
-                    sc->tag_base + static_cast<unsigned int>(E->rec.i[MB_AT_I_QKV_SOURCE]) + 1u;
-                const unsigned int keep = slice_base(warp) + lane * 16;
-#pragma unroll 1
-                for (int i = 0; i < (holder ? 2 * DC + 1 : DC); ++i)
-                    sts128(keep + min(i, kSliceSlots - 1) * 512,
-                           cells_load(i < DC ? qrow + 128 * i : (i < 2 * DC ? krow + 128 * (i - DC) : vrow), tag, ph));
-                __syncwarp();
-            }
+            if (__builtin_expect(kind == kCells, 0)) gather_cells(ph, qrow, krow, vrow, DC, holder);
             const size_t at = ((static_cast<size_t>(b) * d.capacity + L) * Hkv + h) * D;
             auto place_new_row = [&](uint4 (&kn)[DC], uint4 vn) {
                 if (gid == 0) {
@@ -1797,6 +1808,30 @@ __device__ __noinline__ void entry_loop() {
     }
 }
 
+// The end of a phase in plans with hand-offs outside the relay arena: counters and the grid barrier.  False: the
+// barrier failed.
+__device__ __noinline__ bool close_phase(Control* ctl, int ph, int flags, bool meet, bool counters,
+                                         unsigned int generation) {
+    SharedCtl* sc = ctl_of();
+    const int tid = threadIdx.x;
+    if (meet || counters) named_barrier(kBarAll, kThreads);
+    if (counters && tid == 0) {
+        // This CTA has finished phase `ph`: counted for the CTAs that wait for its plain results
+        // or are about to overwrite what it has read.
+        if (ph >= 2 && !sc->abort_flag) finished_wait(ph, ph - 2);
+        if (!sc->abort_flag) {
+            if (flags & MB_FLAG_FENCE) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->finished[ph & 3].count) : "memory");
+        }
+    }
+    if (flags & MB_FLAG_BARRIER) {
+        if (!grid_barrier(ctl, generation, kBarAll, kThreads, tid, &sc->abort_flag, &sc->verdict, ph, sc->limit_ns))
+            return false;
+        trace_stamp(ph, 3);
+    }
+    return true;
+}
+
 // The consumer warps' walk through the phase table.
 template <int DIM>
 __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned int calls) {
@@ -1839,24 +1874,11 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
         }
         trace_stamp(ph, 2);
         const int flags = E->rec.flags;
-        if (meet || p.counters) named_barrier(kBarAll, kThreads);
-        if (p.counters && tid == 0) {
-            // This CTA has finished phase `ph`: counted for the CTAs that wait for its plain results
-            // or are about to overwrite what it has read.
-            if (ph >= 2 && !sc->abort_flag) finished_wait(ph, ph - 2);
-            if (!sc->abort_flag) {
-                if (flags & MB_FLAG_FENCE) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-                asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(
-                                 &p.ctl->finished[ph & 3].count)
-                             : "memory");
-            }
-        }
-        if (flags & MB_FLAG_BARRIER) {
-            ++barrier_index;
-            if (!grid_barrier(p.ctl, barriers + barrier_index, kBarAll, kThreads, tid, &sc->abort_flag,
-                              &sc->verdict, ph, sc->limit_ns))
-                break;  // the same for all threads
-            trace_stamp(ph, 3);
+        if (__builtin_expect(p.counters || (flags & MB_FLAG_BARRIER) != 0, 0)) {
+            if (flags & MB_FLAG_BARRIER) ++barrier_index;
+            if (!close_phase(p.ctl, ph, flags, meet, p.counters != 0, barriers + barrier_index)) break;  // all threads
+        } else if (meet) {
+            named_barrier(kBarAll, kThreads);
         }
         __syncwarp();
         if ((tid & 31) == 0) mbar_arrive(&sc->entry_done[ph & 3]);

@@ -111,7 +111,7 @@ struct Params {
     int norm_kind, activation, invfreq_bf16, capacity, length_value, length_count;
     float eps, embed_scale, rope_scale, q_scale, softmax_scale;
     int attn_units, attn_blocks;  // units of the attention step; query blocks of a (row, head)
-    int steps, rows_at_once;
+    int steps, small;
 };
 
 enum Step { kQkv = 0, kAttention, kOut, kRowsMid, kGated, kDown, kRowsEnd, kStepsPerLayer };
@@ -920,7 +920,8 @@ __device__ __forceinline__ Place place_of(const Params& p, int i) {
     return x;
 }
 
-template <int D>
+// SMALL: at most one block of keys and one row of tokens a CTA.
+template <int D, bool SMALL>
 __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_constant__ Params p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ float sums[16];  // [2 turns][8 warps]
@@ -1005,20 +1006,14 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
                 const Gemm& g = p.gemm[mid ? kProjOut : kProjDown];
                 const unsigned short* bias = mid ? layer.bias[3] : layer.bias[4];
                 const int slices = step == 0 ? 0 : g.slices;
-                ok = p.rows_at_once > 1
-                         ? row_step<4>(p, sh, tid, lane, sums, norm, bias, slices, step, g.units)
-                         : row_step<1>(p, sh, tid, lane, sums, norm, bias, slices, step, g.units);
+                ok = row_step<SMALL ? 1 : 4>(p, sh, tid, lane, sums, norm, bias, slices, step, g.units);
             } else if (kind == kAttention) {
                 if (attn_here > 0) {
                     ok = workers_await(p, sh, tid, step - 1, p.gemm[kProjQkv].units);
                     if (tid == 0) stamp_at(p, step, 3);
                     if (ok) {
-                        for (int u = blockIdx.x; u < p.attn_units; u += gridDim.x) {
-                            if (p.tokens <= kOneBlock)
-                                attention_unit<D, true>(p, sh.ring, u, tid, wid, lane);
-                            else
-                                attention_unit<D, false>(p, sh.ring, u, tid, wid, lane);
-                        }
+                        for (int u = blockIdx.x; u < p.attn_units; u += gridDim.x)
+                            attention_unit<D, SMALL>(p, sh.ring, u, tid, wid, lane);
                         // weights are copied to where the operands were
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         ok = workers_done(p, sh, tid, step, attn_here, true);
@@ -1057,11 +1052,14 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
     }
 }
 
-const void* kernel_of(int head_dim) {
-    return head_dim == 64    ? reinterpret_cast<const void*>(&prompt_kernel<64>)
-           : head_dim == 128 ? reinterpret_cast<const void*>(&prompt_kernel<128>)
-                             : reinterpret_cast<const void*>(&prompt_kernel<256>);
+template <bool SMALL>
+const void* kernel_for(int head_dim) {
+    return head_dim == 64    ? reinterpret_cast<const void*>(&prompt_kernel<64, SMALL>)
+           : head_dim == 128 ? reinterpret_cast<const void*>(&prompt_kernel<128, SMALL>)
+                             : reinterpret_cast<const void*>(&prompt_kernel<256, SMALL>);
 }
+// One kernel per head size and form: neither carries the other's code.
+const void* kernel_of(const Params& p) { return p.small ? kernel_for<true>(p.head_dim) : kernel_for<false>(p.head_dim); }
 
 // ---------------------------------------------------------------------------------------
 // Host: does a list of phases describe such a prefill, and how is each projection cut?
@@ -1302,7 +1300,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     p.length_count = rope.i[MB_RP_I_LEN_COUNT] > 1 ? rope.i[MB_RP_I_LEN_COUNT] : 1;
     p.attn_blocks = (p.tokens + kAttnRows - 1) / kAttnRows;
     p.attn_units = p.batch * p.heads * p.attn_blocks;
-    p.rows_at_once = p.rows > sm_count ? 4 : 1;
+    p.small = p.rows <= sm_count && p.tokens <= kOneBlock ? 1 : 0;
 
     const int M = p.rows, H = p.hidden_size, grid = st->grid;
     const int half = p.head_dim / 2, pairs[3] = {p.heads * half, p.kv_heads * half, p.kv_heads * half};
@@ -1327,7 +1325,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
         p.counters = reinterpret_cast<unsigned int*>(st->scratch + qkv + parts + rotary);
         err = cudaMemset(p.counters, 0, counters);
     }
-    const void* kernel = kernel_of(p.head_dim);
+    const void* kernel = kernel_of(p);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     int per_sm = 0;
     if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, kSmemBytes);
@@ -1412,7 +1410,7 @@ cudaError_t prompt_launch(const PromptState* st, const std::vector<unsigned long
     p.logits = reinterpret_cast<unsigned short*>(addr(st->phases.back().slot[MB_GV_S_OUT0]));
     p.trace = trace;
     void* args[] = {&p};
-    return cudaLaunchCooperativeKernel(kernel_of(p.head_dim), dim3(st->grid), dim3(kThreads), args, kSmemBytes,
+    return cudaLaunchCooperativeKernel(kernel_of(p), dim3(st->grid), dim3(kThreads), args, kSmemBytes,
                                        stream);
 }
 
