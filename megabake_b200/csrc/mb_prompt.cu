@@ -1067,7 +1067,8 @@ const void* kernel_of(const Params& p) { return p.small ? kernel_for<true>(p.hea
 // Cost of a cut in microseconds.  An SM takes 72 bytes a nanosecond from L2 while all of them stream; weights up to a ring come before
 // the step begins; a product of 16 elements takes 27 cycles to issue and works through two columns a cycle; a
 // stage costs 250 cycles of barriers around its products; the last unit's accumulators are drained
-// with nothing beside them.
+// with nothing beside them; a further unit of the same CTA costs half a microsecond of refilling (1B, logits of 19
+// tokens: 106 us in units of 56 features, 80 in units of 128).
 struct Cut {
     Gemm gemm;
     double cost;
@@ -1110,7 +1111,7 @@ Cut best_cut(const int* n, int segments, bool pair, bool sliced, int half, int K
                 double cost = load > product ? load : product;
                 if (cost < hbm) cost = hbm;
                 if (cost < waves * drain) cost = waves * drain;
-                cost += drain;
+                cost += drain + 0.5 * (waves - 1);
                 if (sliced) cost += slices * 8.0 * M * hidden / 5.0e6 + 0.05 * slices;
                 if (cost >= best.cost - 1e-9) continue;
                 best.cost = cost;
