@@ -2017,12 +2017,12 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count, const ClusterRoom& r
     int persistent_split = 1;
     const char* persistent_env = std::getenv("MEGABAKE_B200_GEMM_PERSISTENT");
     if (persistent_env == nullptr || std::atoi(persistent_env) != 0) {
-        // Tile width and number of reduction slices by a cost model in microseconds, fitted to
-        // a sweep of both over the twelve GEMM shapes of the gemma-2b prefill (128 / 512 / 2048
-        // rows): a CTA takes a k-block every 0.44 us (256 columns) or 0.30 us (128) when every
-        // SM streams operands; the weights cannot arrive faster than HBM delivers them; a wave
-        // of sliced tiles pays 4 us (2 us) for parking its partial sums and the last slice
-        // 2 us (1 us) per slice for its pass over them, a chain of L2 round trips.
+        // Tile width and number of reduction slices by a cost model in microseconds, fitted to a sweep of both over
+        // the GEMM shapes of four models at 300 to 2048 rows: a CTA takes a k-block every 0.385 us (256 columns)
+        // or 0.305 us (128); the weights cannot arrive faster than HBM delivers them; parking partial sums
+        // and the last slice's pass over them, a chain of L2 round trips, take 4.8 us (3.4 us) a slice for one
+        // wave of tiles and 70 % (80 %) of that for each further one.  (2048 -> 2048, 300 rows: one slice 13.9 us,
+        // two 16.4, clustered 17.9; 8192 -> 2048, 1332 rows, 256 columns: 51.0, two 65.3, three 58.2.)
         g.persistent = 1;
         double best = 1e30;
         const double weight_bytes = 2.0 * K * (pair ? 2 : 1) * [&] {
@@ -2037,11 +2037,13 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count, const ClusterRoom& r
                 const int units = tiles * split;
                 const int waves = (units + sm_count - 1) / sm_count;
                 const int per_unit = (g.kblocks + split - 1) / split;
-                double stream = waves * per_unit * (bn == 256 ? 0.44 : 0.30);
+                double stream = waves * per_unit * (bn == 256 ? 0.385 : 0.305);
                 const double hbm = weight_bytes / 6.0e6;
                 if (stream < hbm) stream = hbm;
                 const double slices =
-                    split > 1 ? (bn == 256 ? 4.0 : 2.0) * waves + (bn == 256 ? 2.0 : 1.0) * split : 0.0;
+                    split == 1 ? 0.0
+                    : bn == 256 ? 4.8 * split * (0.3 + 0.7 * waves)
+                                : 3.4 * split * (0.2 + 0.8 * waves);
                 const double cost = stream + slices;
                 if (cost < best - 1e-9) {
                     best = cost;
@@ -2050,11 +2052,10 @@ GemmGeometry gemm_geometry(const mb_phase& P, int sm_count, const ClusterRoom& r
                     g.clustered = 0;
                 }
                 // The slices of a tile as one cluster, if all clusters run at once: two meetings and a
-                // fold, taken as 3.6 us for 19 live rows of a 128-column tile and 7 us for all 128, and
+                // fold, taken as 4 us for 19 live rows of a 128-column tile and 9.5 us for all 128, and
                 // twice that for the 256 columns that also leave each CTA twice the sums to store.
-                // (Stamps inside a step read up to 9 us for 128 rows, skew of the slices included.)
                 if (split < 2 || split > kMaxCluster || tiles > room.count[bn == 256][split]) continue;
-                const double joint = stream + (3.0 + 4.0 * (M < kTileM ? M : kTileM) / kTileM) * (bn / 128);
+                const double joint = stream + (3.0 + 6.5 * (M < kTileM ? M : kTileM) / kTileM) * (bn / 128);
                 if (joint < best - 1e-9) {
                     best = joint;
                     g.bn = bn;
