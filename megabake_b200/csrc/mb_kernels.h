@@ -33,7 +33,7 @@ cudaError_t decode_occupancy(int head_dim, int smem_bytes, int* blocks_per_sm);
 cudaError_t decode_launch(const KernelParams& params, int head_dim, int ctas, int smem_bytes,
                           cudaStream_t stream);
 
-// Prefill plans (mb_prefill.cu): one kernel launch per phase.
+// Prefill plans (mb_prefill.cu): one kernel launch per phase; mb_prompt.cu below takes short prompts.
 struct PrefillState;
 int prefill_validate(const mb_phase& phase, unsigned int n_slots, unsigned int n_dynamic);
 cudaError_t prefill_create(std::vector<mb_phase>& phases, int sm_count, PrefillState** out);

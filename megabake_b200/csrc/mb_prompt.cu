@@ -44,14 +44,16 @@ using namespace prefill;
 constexpr int kWorkers = 256;
 constexpr int kThreads = 128 + kWorkers;
 constexpr int kMaxLayers = 30;     // what fits the parameters of one launch
-// Tokens over all rows of the batch up to which one launch is the faster form.  What it saves is launches; what it
-// costs grows with the tokens (tiles of 128 tokens take more operand bytes than mb_prefill.cu's, attention
-// without tcgen05).  Launches of their own / one launch, us: 135M shape 1,565 / 955 for 19 tokens, 2,017 /
-// 1,374 for 256, 2,135 / 1,712 for 512, 2,650 / 2,971 for 1,024; 0.5B 1,628 / 1,041 for 64, 2,561 / 2,201 for 512;
-// 1B 1,274 / 1,062 for 19, 2,065 / 1,835 for 256, 2,610 / 2,648 for 400; 2B 2,491 / 1,857 for 128, 3,049 /
-// 2,815 for 256, 3,888 / 4,288 for 400.
-constexpr int kMaxRows = 256, kMaxRowsSmall = 640;
-constexpr long long kSmallLayer = 16ll << 20;  // weights of a layer
+// Tokens over all rows of the batch up to which one launch is the faster form, by the weights of a layer.  What it
+// saves is launches; what it costs grows with the tokens and the weights (tiles of 128 tokens take more operand
+// bytes than mb_prefill.cu's, attention does without tcgen05).  Launches of their own / one launch, us: 135M shape
+// (3.5 M weights a layer) 1,239 / 947 for 19 tokens, 1,847 / 1,360 for 256, 1,998 / 1,718 for 512, 2,120 / 2,106 for
+// 640; 0.5B (15 M) 1,427 / 1,018 for 64, 1,849 / 1,604 for 256, 2,124 / 2,031 for 400, 2,136 / 2,193 for 512; 1B (61 M)
+// 1,194 / 973 for 19, 1,489 / 1,339 for 128, 1,648 / 1,579 for 160, 1,655 / 1,674 for 176; 2B (110 M) 1,731 / 1,472 for
+// 19, 2,175 / 1,831 for 128, 2,442 / 2,459 for 130, 2,647 / 2,810 for 256.
+inline int most_rows(long long layer_weights) {
+    return layer_weights <= 4ll << 20 ? 640 : layer_weights <= 16ll << 20 ? 400 : layer_weights <= 64ll << 20 ? 160 : 128;
+}
 constexpr int kAttnRows = 32;      // query rows of an attention unit
 constexpr int kSmemBytes = 232448 - 1024;  // 1 KB for what the kernel declares itself
 // A 128-row MMA reads 16 KB of weights from wherever a tile starts, also where the tile has fewer rows
@@ -1172,7 +1174,7 @@ bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
     const long long weights = static_cast<long long>(H) * (one[1].i[MB_GV_I_N0] + one[1].i[MB_GV_I_N0 + 1] +
                                                            one[1].i[MB_GV_I_N0 + 2] + one[4].i[MB_GV_I_K] +
                                                            3ll * one[6].i[MB_GV_I_N0]);
-    if (M > (weights <= kSmallLayer ? kMaxRowsSmall : kMaxRows)) return false;
+    if (M > most_rows(weights)) return false;
     for (int l = 0; l < layers; ++l) {
         const mb_phase* P = &f[1 + l * kPhasesPerLayer];
         if (!is_norm(P[0], one[0]) || !is_norm(P[5], one[0])) return false;

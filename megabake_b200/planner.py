@@ -523,7 +523,8 @@ def _plan_decode(program: DecoderProgram, options: PlannerOptions, stage_bytes: 
 
 def plan_prefill(program: DecoderProgram, options: PlannerOptions | None = None,
                  mask=None) -> PlanLayout:
-    """Prefill packing: one kernel launch per phase, in stream order (no grid barriers).
+    """Prefill packing: one kernel launch per phase, in stream order (no grid barriers); the library runs
+    the whole list of a short prompt as one launch.
 
         [embed rows]                                   (layer 0)
         [rmsnorm rows] [q|k|v GEMM (+bias)] [rope rows] [attention] [o GEMM + residual]
@@ -670,5 +671,5 @@ def plan_prefill(program: DecoderProgram, options: PlannerOptions | None = None,
     return PlanLayout(
         program=p, phases=phases, slots=slots.specs,
         workspace_bytes=_align(slots.workspace, 256), zero_ranges=[], activation_bytes=0,
-        intervals=len(phases), notes=[f"{len(phases)} kernel launches per prefill"],
+        intervals=len(phases), notes=[f"{len(phases)} phases: one kernel launch each, or one launch for all of a short prompt"],
         mode=rt.MODE_PREFILL, constants=constants)
