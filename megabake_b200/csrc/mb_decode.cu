@@ -1593,7 +1593,7 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     if (i >= slots) break;
-                    // a part that does not exist: the last one again, with no weight below
+                    // a part that does not exist: the last one again, left out below
                     const int c = min(lanes == 1 ? i : j + 4 * (i & 3) + 16 * (i >> 2), seg.parts - 1);
                     const char* part = first + static_cast<size_t>(c) * group * ((D + 2) * 8);
                     ld_cell_pair(part, cm[i], cl[i]);
@@ -1622,10 +1622,12 @@ __device__ __noinline__ Place attention_phase(const int ph, Place s) {
             float den[8], s0[8], s1[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
+                // (not by a weight of zero: an infinity times zero is a NaN)
+                const bool there = (lanes == 1 ? i : j + 4 * (i & 3) + 16 * (i >> 2)) < seg.parts;
                 const float weight = m[i] == -INFINITY ? 0.f : expf(m[i] - mx);
-                den[i] = __uint_as_float(cell_data(cl[i])) * weight;
-                s0[i] = __uint_as_float(cell_data(c0[i])) * weight;
-                s1[i] = __uint_as_float(cell_data(c1[i])) * weight;
+                den[i] = there ? __uint_as_float(cell_data(cl[i])) * weight : 0.f;
+                s0[i] = there ? __uint_as_float(cell_data(c0[i])) * weight : 0.f;
+                s1[i] = there ? __uint_as_float(cell_data(c1[i])) * weight : 0.f;
             }
             // part c meets part c + 16, then c + 8, + 4, + 2, + 1, whoever holds them
 #pragma unroll
