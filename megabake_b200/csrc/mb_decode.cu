@@ -94,7 +94,7 @@ struct SharedCtl {
     float stat[kWarps][8][2];        // attention: (maximum, sum) per warp and head
     float exchange[2][kWarps][8];    // attention, exact mode: maxima and sums of the warps
     __align__(16) unsigned short new_row[2][256];  // rotated new key and new value of an item
-    __align__(16) PhaseEntry entry[4];  // phase records ph - 1 .. ph + 2
+    __align__(16) PhaseEntry entry[4];  // phase records ph .. ph + 3
 };
 constexpr int kCtlBytes = 5120;
 constexpr int kFixedBytes = kCtlBytes + kScratchBytes;
@@ -143,7 +143,7 @@ __device__ __forceinline__ unsigned long long resolve_address(unsigned long long
 // Bounded waits.  A wait gives up when the launch's limit has run out (status
 // MB_ST_HANDOFF_TIMEOUT) or when this CTA or any other has recorded a fault; the caller goes on
 // with whatever it has, without waiting any more, and the CTA leaves before the next phase or the one
-// after that (next_entry).
+// after that (consume_launch).
 // ---------------------------------------------------------------------------------------
 __device__ __noinline__ bool wait_gave_up(int ph, unsigned long long start) {
     SharedCtl* sc = ctl_of();
@@ -530,20 +530,19 @@ __device__ __forceinline__ void ring_wait(unsigned int stage, unsigned int parit
         }
     }
 }
-// The record of phase ph; it is there but for the first phases of a launch.  False: it will not come, and must not
-// be looked at.
-__device__ __forceinline__ bool entry_wait(int ph) {
+// The record of phase ph; it is there but for the first phases of a launch.  One thread, whose verdict all warps take
+// (consume_launch).  False: a fault is on record in this CTA, or the record has not come in time.
+__device__ __noinline__ bool await_record(int ph) {
     SharedCtl* sc = ctl_of();
-    if (mbar_try_wait(&sc->entry_ready[ph & 3], (ph >> 2) & 1)) return true;
-    const unsigned long long start = global_timer_ns();
-    for (unsigned int tries = 1; !mbar_try_wait(&sc->entry_ready[ph & 3], (ph >> 2) & 1); ++tries) {
-        if ((tries & 127u) == 0u && global_timer_ns() - start > 2 * sc->limit_ns) {
-            record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
-            sc->abort_flag = 1;
-            return false;
-        }
-    }
-    return true;
+    if (sc->abort_flag != 0) return false;
+    if (mbar_wait_bounded(&sc->entry_ready[ph & 3], (ph >> 2) & 1, &sc->abort_flag, 2 * sc->limit_ns)) return true;
+    if (sc->abort_flag == 0) record_status(sc->ctl, MB_ST_PIPE_TIMEOUT, ph, blockIdx.x);
+    sc->abort_flag = 1;
+    return false;
+}
+__device__ __forceinline__ bool record_ready(int ph) {
+    SharedCtl* sc = ctl_of();
+    return (sc->abort_flag == 0 && mbar_try_wait(&sc->entry_ready[ph & 3], (ph >> 2) & 1)) || await_record(ph);
 }
 // Hands the stage back once the warp has its values, and moves on.
 __device__ __forceinline__ void ring_next(Place& s) {
@@ -1846,6 +1845,7 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
          at < p.relay_bytes; at += static_cast<unsigned long long>(gridDim.x) * kThreads * 16)
         *reinterpret_cast<uint4*>(sc->relay_next + at) =
             make_uint4(kUnwritten, kUnwritten, kUnwritten, kUnwritten);
+    if (tid == 0 && !record_ready(0)) table_of()[0].kind = kStreamStop;
     named_barrier(kBarAll, kThreads);
 
     const unsigned int barriers = calls * static_cast<unsigned int>(p.barriers_per_launch);
@@ -1856,10 +1856,11 @@ __device__ __forceinline__ void consume_launch(const KernelParams& p, unsigned i
     for (int ph = 0; ph < p.n_phases; ++ph) {
         const int kind = table[ph].kind;
         if (kind == kStreamStop) break;
-        if (!entry_wait(ph)) break;
-        // Once a fault is on record in this CTA the walk ends at ph + 1, through the kind of that phase, which
-        // the barrier inside this one publishes: every warp leaves there.
-        if (tid == 0 && sc->abort_flag != 0 && ph + 1 < p.n_phases) table_of()[ph + 1].kind = kStreamStop;
+        // Whether there will be a phase ph + 1 -- its record has come, no fault is on record in this CTA -- is one
+        // thread's verdict, through the kind of that phase, which the barrier inside this one publishes: all warps
+        // leave there or none does, and that barrier also orders the record before their reads of it.  (Each
+        // warp waiting for itself could leave some of them alone at the next barrier, which has no limit.)
+        if (tid == 0 && ph + 1 < p.n_phases && !record_ready(ph + 1)) table_of()[ph + 1].kind = kStreamStop;
         const PhaseEntry* E = &sc->entry[ph & 3];
         trace_stamp(ph, 0);
         bool meet = true;  // the phase has not had a barrier of all threads
