@@ -301,7 +301,9 @@ __device__ __forceinline__ bool produce_activations(const Params& p, const Share
                 stamp_at(p, step, 3);
             }
             if (!__all_sync(0xffffffffu, ready)) return false;
-            // the step before wrote through the generic proxy, TMA reads through the async proxy
+            // What lane 0 acquired holds for whichever lane issues the copies: a vote says nothing about memory, this
+            // does.  Then the proxies: the step before wrote through the generic one, TMA reads through the async one.
+            __syncwarp();
             asm volatile("fence.proxy.async;" ::: "memory");
             waited = true;
         }
