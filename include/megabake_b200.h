@@ -328,7 +328,8 @@ typedef struct mb_plan_desc {
                                  of 1024 up to mb_stage_bytes(); 0 = mb_stage_bytes()      */
     uint32_t wait_limit_ms;   /* bound of every device-side wait (hand-offs, grid barrier; twice it
                                  for pipeline stages) in milliseconds; 0 = 2000.  When a wait
-                                 runs out the kernel records a status, drains and returns   */
+                                 runs out the kernel records a status, drains and returns.  Prefill
+                                 of more than one launch: always 2000, within a launch       */
     uint32_t reserved[2];
 } mb_plan_desc;
 

@@ -323,6 +323,11 @@ cudaError_t clear_partials(mb_plan* plan, const std::vector<mb::PhaseEntry>& ent
     return cleared ? cudaStreamSynchronize(cudaStreamLegacy) : cudaSuccess;  // launches may use any stream
 }
 
+unsigned int wait_limit_us(const mb_plan_desc* desc) {
+    if (desc->wait_limit_ms == 0) return 2000000u;
+    return desc->wait_limit_ms > 4000000u ? 4000000000u : desc->wait_limit_ms * 1000u;
+}
+
 // A prefill plan is a list of kernel launches; it shares the descriptor, the slot table, the
 // status word and the entry points with decode plans.
 int create_prefill_plan(const mb_plan_desc* desc, mb_plan** out) {
@@ -350,7 +355,8 @@ int create_prefill_plan(const mb_plan_desc* desc, mb_plan** out) {
     plan->ctas = prop.multiProcessorCount;
     cudaError_t err = cudaMalloc(&plan->d_ctl, sizeof(mb::Control));
     if (err == cudaSuccess) err = cudaMemset(plan->d_ctl, 0, sizeof(mb::Control));
-    if (err == cudaSuccess) err = mb::prompt_create(plan->phases, plan->n_dynamic, plan->sm_count, &plan->prompt);
+    if (err == cudaSuccess)
+        err = mb::prompt_create(plan->phases, plan->n_dynamic, plan->sm_count, wait_limit_us(desc), &plan->prompt);
     if (err == cudaSuccess && plan->prompt == nullptr)
         err = mb::prefill_create(plan->phases, plan->sm_count, &plan->prefill);
     if (err != cudaSuccess) {
@@ -493,8 +499,7 @@ int mb_plan_create(const mb_plan_desc* desc, mb_plan** out) {
     plan->slots_per_slice = slots;
     plan->head_dim = head_dim;
     plan->barriers = barriers;
-    if (desc->wait_limit_ms != 0)
-        plan->wait_limit_us = desc->wait_limit_ms > 4000000u ? 4000000000u : desc->wait_limit_ms * 1000u;
+    plan->wait_limit_us = wait_limit_us(desc);
 
     const int lowered = lower_relays(plan);
     if (lowered != MB_OK) {

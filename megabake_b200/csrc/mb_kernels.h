@@ -50,7 +50,7 @@ cudaError_t prefill_launch(PrefillState* state, const std::vector<mb_phase>& pha
 // no such prompt.
 struct PromptState;
 cudaError_t prompt_create(const std::vector<mb_phase>& phases, unsigned int n_dynamic, int sm_count,
-                          PromptState** out);
+                          unsigned int wait_limit_us, PromptState** out);
 void prompt_destroy(PromptState* state);
 cudaError_t prompt_reset(PromptState* state);
 int prompt_bind(PromptState* state, const std::vector<unsigned long long>& slots, Control* ctl);

@@ -114,6 +114,7 @@ struct Params {
     float eps, embed_scale, rope_scale, q_scale, softmax_scale;
     int attn_units, attn_blocks;  // units of the attention step; query blocks of a (row, head)
     int steps, small;
+    unsigned long long limit_ns;  // of a hand-off between steps; twice as much for the pipeline within a CTA
 };
 
 enum Step { kQkv = 0, kAttention, kOut, kRowsMid, kGated, kDown, kRowsEnd, kStepsPerLayer };
@@ -133,7 +134,8 @@ struct Shared {
 // twice in a row.  So a body has one place in the code, waits that do not succeed at once continue
 // out of line, and loops stay rolled.
 // ---------------------------------------------------------------------------------------
-__device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, volatile int* abort_flag) {
+__device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, volatile int* abort_flag,
+                                       unsigned long long limit_ns) {
     const unsigned long long start = global_timer_ns();
     for (unsigned int tries = 1;; ++tries) {
         unsigned int done;
@@ -145,13 +147,14 @@ __device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, vo
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((tries & 127u) == 0u && (*abort_flag || global_timer_ns() - start > kPipeTimeoutNs)) return false;
+        if ((tries & 127u) == 0u && (*abort_flag || global_timer_ns() - start > limit_ns)) return false;
     }
 }
 // All lanes of a warp; the compiler knows the result to be the same in all of them.
-__device__ __forceinline__ bool wait_warp(unsigned long long* bar, unsigned int parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool wait_warp(const Params& p, const Shared& sh, unsigned long long* bar,
+                                          unsigned int parity) {
     bool done = mbar_try_wait(bar, parity);
-    if (!__all_sync(0xffffffffu, done)) done = wait_long(smem_u32(bar), parity, abort_flag);
+    if (!__all_sync(0xffffffffu, done)) done = wait_long(smem_u32(bar), parity, sh.abort_flag, 2 * p.limit_ns);
     return __all_sync(0xffffffffu, done) != 0;
 }
 
@@ -172,7 +175,8 @@ __device__ __forceinline__ void give_up(const Params& p, const Shared& sh, int c
 
 // Waits until `units` units of `step` are complete; one thread.
 __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned int units, const unsigned int* mark,
-                                         volatile int* abort_flag, Control* ctl, int step) {
+                                         volatile int* abort_flag, Control* ctl, int step,
+                                         unsigned long long limit_ns) {
     unsigned long long start = 0;
     for (unsigned int tries = 1;; ++tries) {
         unsigned int seen;
@@ -185,7 +189,7 @@ __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned i
                 *abort_flag = 1;
                 return false;
             }
-            if (global_timer_ns() - start > kBarrierTimeoutNs) {
+            if (global_timer_ns() - start > limit_ns) {
                 record_fault(ctl, const_cast<unsigned int*>(mark), abort_flag, MB_ST_HANDOFF_TIMEOUT, step,
                              static_cast<int>(blockIdx.x));
                 return false;
@@ -194,7 +198,7 @@ __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned i
     }
 }
 __device__ __forceinline__ bool await_step(const Params& p, const Shared& sh, int step, unsigned int units) {
-    return await_count(p.counters + step, units, fault_mark(p), sh.abort_flag, p.ctl, step);
+    return await_count(p.counters + step, units, fault_mark(p), sh.abort_flag, p.ctl, step, p.limit_ns);
 }
 
 // The workers of this CTA have finished `units` units of `step`.  False: some wait ran out.
@@ -265,7 +269,7 @@ __device__ __forceinline__ bool produce_weights(const Params& p, const Shared& s
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x) {
         const Unit x = unit_of(g, u);
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (at.round > 0 && !wait_warp(&sh.empty[at.s], (at.round - 1) & 1, sh.abort_flag)) {
+            if (at.round > 0 && !wait_warp(p, sh, &sh.empty[at.s], (at.round - 1) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 1);
                 return false;
             }
@@ -308,7 +312,7 @@ __device__ __forceinline__ bool produce_activations(const Params& p, const Share
             waited = true;
         }
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (at.round > 0 && !wait_warp(&sh.empty[at.s], (at.round - 1) & 1, sh.abort_flag)) {
+            if (at.round > 0 && !wait_warp(p, sh, &sh.empty[at.s], (at.round - 1) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 2);
                 return false;
             }
@@ -331,14 +335,14 @@ __device__ __forceinline__ bool issue_products(const Params& p, const Shared& sh
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x, ++turn) {
         const Unit x = unit_of(g, u);
         const int buf = turn & 1;
-        if (turn >= 2 && !wait_warp(&sh.acc_empty[buf], ((turn >> 1) - 1) & 1, sh.abort_flag)) {
+        if (turn >= 2 && !wait_warp(p, sh, &sh.acc_empty[buf], ((turn >> 1) - 1) & 1)) {
             give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 3);
             return false;
         }
         tc_fence_after();
         const unsigned int acc = tmem + buf * 256;
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (!wait_warp(&sh.full[at.s], at.round & 1, sh.abort_flag)) {
+            if (!wait_warp(p, sh, &sh.full[at.s], at.round & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 4);
                 return false;
             }
@@ -446,7 +450,7 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x, ++turn) {
         const Unit x = unit_of(g, u);
         const int buf = turn & 1;
-        if (!wait_warp(&sh.acc_full[buf], (turn >> 1) & 1, sh.abort_flag)) {
+        if (!wait_warp(p, sh, &sh.acc_full[buf], (turn >> 1) & 1)) {
             if (lane == 0) give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 5);
             return false;
         }
@@ -967,7 +971,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
         bool ok = true;
         for (int i = 0; ok && i < projections; ++i) {
             const Place x = place_of(p, i);
-            if (x.proj == kProjOut && attn_here > 0 && !wait_warp(sh.attn_done, (i >> 2) & 1, sh.abort_flag)) {
+            if (x.proj == kProjOut && attn_here > 0 && !wait_warp(p, sh, sh.attn_done, (i >> 2) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, x.step, 6);
                 break;
             }
@@ -1261,7 +1265,8 @@ cudaError_t prompt_reset(PromptState* st) {
 }
 
 // *out stays null where the phases are not a short prompt: they run as launches of their own.
-cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic, int sm_count, PromptState** out) {
+cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic, int sm_count,
+                          unsigned int wait_limit_us, PromptState** out) {
     using namespace prompt;
     *out = nullptr;
     const char* env = std::getenv("MEGABAKE_B200_PREFILL_ONE_LAUNCH");
@@ -1281,6 +1286,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     std::memset(&p, 0, sizeof(p));
     const mb_phase* one = &f[1];
     const mb_phase &attn = one[3], &rope = one[2], &head = f.back();
+    p.limit_ns = wait_limit_us * 1000ull;
     p.layers = (static_cast<int>(f.size()) - 3) / kPhasesPerLayer;
     p.steps = 2 + p.layers * kStepsPerLayer;
     p.rows = f[0].i[MB_EM_I_ROWS];

@@ -1,0 +1,45 @@
+"""Short prompts as one launch: its limits, its SMs and the tensors it leaves behind."""
+
+from dataclasses import replace
+
+import pytest
+import torch
+
+from megabake_b200 import models
+from megabake_b200 import runtime as rt
+from megabake_b200.diagnostics import CompilerError
+from megabake_b200.engine import BoundDecoder
+from megabake_b200.planner import plan_prefill
+
+pytestmark = [pytest.mark.gpu, pytest.mark.timeout(300)]
+
+SWITCH = "MEGABAKE_B200_PREFILL_ONE_LAUNCH"
+
+
+def _arguments(spec, tokens, batch=1, seed=1, weights=None):
+    if weights is None:
+        weights = {k: v.cuda() for k, v in models.init_weights(spec, seed).items()}
+    ids = torch.randint(0, spec.vocab, (batch, tokens), generator=torch.Generator().manual_seed(tokens)).cuda()
+    return models.direct_prefill_arguments(spec, weights, models.inv_freq_buffer(spec).cuda(), ids)
+
+
+def test_a_hand_over_that_takes_longer_than_the_limit_ends_the_launch():
+    """A gated projection of eight million features and the sum over them keep the device busy for milliseconds, and
+    whoever waits for either does so for one (CTAs without work there), or for two (inside their own
+    pipeline): the launch ends with a status and leaves the device and the plan usable."""
+    spec = models.get_spec("tiny-llama", hidden=64, layers=1, heads=1, kv_heads=1, intermediate=1 << 23, vocab=20000)
+    weights = {name: torch.zeros(shape, dtype=torch.bfloat16, device="cuda")
+               for name, shape in models.parameter_shapes(spec)}
+    args = _arguments(spec, 128, weights=weights)
+    layout = plan_prefill(models.direct_prefill_program(spec, 1, 128))
+    short = BoundDecoder(layout, args, wait_limit_ms=1)
+    assert short.plan.launches == 1
+    for _ in range(2):
+        short(*args)
+        torch.cuda.synchronize()
+        assert short.plan.status().code in (2, 7)   # MB_ST_PIPE_TIMEOUT, MB_ST_HANDOFF_TIMEOUT: whose limit was first
+        with pytest.raises(CompilerError):
+            short.check()                      # and makes it usable again
+    patient = BoundDecoder(layout, args)
+    assert not patient(*args).any()
+    patient.check()
