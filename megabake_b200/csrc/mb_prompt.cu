@@ -928,7 +928,7 @@ __device__ __forceinline__ Place place_of(const Params& p, int i) {
     return x;
 }
 
-// SMALL: at most one block of keys and one row of tokens a CTA.
+// SMALL: at most one block of keys and one row of tokens a CTA.  Any number of CTAs works that run at once.
 template <int D, bool SMALL>
 __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_constant__ Params p) {
     extern __shared__ unsigned char smem_raw[];
@@ -1058,6 +1058,41 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
             for (int s = 0; s < p.steps + 2; ++s) p.counters[s] = 0u;
         }
     }
+}
+
+// SMs that a launch on `stream` may use: fewer than the device has in a green context, which is the current context's
+// or the stream's.
+int usable_sms(cudaStream_t stream, int device_sms) {
+    typedef CUresult (*CurrentFn)(CUcontext*);
+    typedef CUresult (*ContextResourceFn)(CUcontext, CUdevResource*, CUdevResourceType);
+    typedef CUresult (*StreamGreenFn)(CUstream, CUgreenCtx*);
+    typedef CUresult (*GreenResourceFn)(CUgreenCtx, CUdevResource*, CUdevResourceType);
+    static const auto entry = [](const char* name) -> void* {
+        void* symbol = nullptr;
+        cudaDriverEntryPointQueryResult result;
+        return cudaGetDriverEntryPoint(name, &symbol, cudaEnableDefault, &result) == cudaSuccess &&
+                       result == cudaDriverEntryPointSuccess
+                   ? symbol
+                   : nullptr;
+    };
+    static const auto current = reinterpret_cast<CurrentFn>(entry("cuCtxGetCurrent"));
+    static const auto of_context = reinterpret_cast<ContextResourceFn>(entry("cuCtxGetDevResource"));
+    static const auto green_of = reinterpret_cast<StreamGreenFn>(entry("cuStreamGetGreenCtx"));
+    static const auto of_green = reinterpret_cast<GreenResourceFn>(entry("cuGreenCtxGetDevResource"));
+    int sms = device_sms;
+    auto at_most = [&](const CUdevResource& room) {
+        if (room.sm.smCount > 0 && static_cast<int>(room.sm.smCount) < sms) sms = static_cast<int>(room.sm.smCount);
+    };
+    CUdevResource room;
+    CUcontext context = nullptr;
+    CUgreenCtx green = nullptr;
+    if (current != nullptr && of_context != nullptr && current(&context) == CUDA_SUCCESS && context != nullptr &&
+        of_context(context, &room, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+        at_most(room);
+    if (green_of != nullptr && of_green != nullptr && stream != nullptr && green_of(stream, &green) == CUDA_SUCCESS &&
+        green != nullptr && of_green(green, &room, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+        at_most(room);
+    return sms;
 }
 
 template <bool SMALL>
@@ -1277,6 +1312,10 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
                              "MEGABAKE_B200_PREFILL_CHAIN"})
         if (std::getenv(name) != nullptr) return cudaSuccess;
     if (!describes_prompt(f, n_dynamic)) return cudaSuccess;
+    int device = 0, cooperative = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
+    if (err != cudaSuccess || cooperative == 0) return err;
     PromptState* st = new (std::nothrow) PromptState();
     if (st == nullptr) return cudaErrorMemoryAllocation;
     st->phases = f;
@@ -1328,7 +1367,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
     const size_t qkv = room(static_cast<size_t>(M) * pitch * 2), parts = room(static_cast<size_t>(slices) * M * H * 4),
                  rotary = room(static_cast<size_t>(M) * (p.head_dim / 2) * 4), counters = room((p.steps + 2) * 4);
-    cudaError_t err = cudaMalloc(&st->scratch, qkv + parts + rotary + counters);
+    err = cudaMalloc(&st->scratch, qkv + parts + rotary + counters);
     if (err == cudaSuccess) {
         p.qkv = reinterpret_cast<unsigned short*>(st->scratch);
         p.parts = reinterpret_cast<float*>(st->scratch + qkv);
@@ -1336,10 +1375,15 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
         p.counters = reinterpret_cast<unsigned int*>(st->scratch + qkv + parts + rotary);
         err = cudaMemset(p.counters, 0, counters);
     }
-    const void* kernel = kernel_of(p);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    int per_sm = 0;
-    if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, kSmemBytes);
+    // the form a launch takes, and the one it takes where it has fewer SMs
+    const void* kernels[2] = {kernel_of(p), kernel_for<false>(p.head_dim)};
+    int per_sm = 1;
+    for (const void* kernel : kernels) {
+        int room = 0;
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&room, kernel, kThreads, kSmemBytes);
+        per_sm = room < per_sm ? room : per_sm;
+    }
     if (err == cudaSuccess) err = cudaStreamSynchronize(cudaStreamLegacy);
     if (err != cudaSuccess || per_sm < 1) {
         prompt_destroy(st);
@@ -1420,9 +1464,14 @@ cudaError_t prompt_launch(const PromptState* st, const std::vector<unsigned long
     p.pos = reinterpret_cast<const long long*>(addr(st->phases[3].slot[MB_RP_S_POS]));
     p.logits = reinterpret_cast<unsigned short*>(addr(st->phases.back().slot[MB_GV_S_OUT0]));
     p.trace = trace;
+    // All CTAs have to run at once.  What the projections are cut into does not depend on how many there are.
+    const int grid = usable_sms(stream, st->grid);
+    if (grid < st->grid) {
+        p.gemm[kProjOut].first = p.attn_units % grid;
+        if (p.rows > grid) p.small = 0;
+    }
     void* args[] = {&p};
-    return cudaLaunchCooperativeKernel(kernel_of(p), dim3(st->grid), dim3(kThreads), args, kSmemBytes,
-                                       stream);
+    return cudaLaunchCooperativeKernel(kernel_of(p), dim3(grid), dim3(kThreads), args, kSmemBytes, stream);
 }
 
 }  // namespace mb

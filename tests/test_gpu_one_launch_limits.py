@@ -43,3 +43,28 @@ def test_a_hand_over_that_takes_longer_than_the_limit_ends_the_launch():
     patient = BoundDecoder(layout, args)
     assert not patient(*args).any()
     patient.check()
+
+
+@pytest.mark.parametrize("name,batch,tokens,sms", [
+    ("tiny-llama", 1, 24, 72), ("tiny-qwen2", 1, 100, 72), ("tiny-gemma256", 1, 257, 40), ("tiny-mha", 5, 9, 16),
+])
+def test_fewer_sms_give_the_same_bits(name, batch, tokens, sms):
+    """Under a context that has a part of the device's SMs the launch takes that many CTAs."""
+    from torch.cuda.green_contexts import GreenContext
+
+    spec = models.get_spec(name)
+    args = _arguments(spec, tokens, batch)
+    bound = BoundDecoder(plan_prefill(models.direct_prefill_program(spec, batch, tokens)), args)
+    assert bound.plan.launches == 1
+    expect = bound(*args)
+    bound.check()
+    part = GreenContext.create(num_sms=sms, device_id=0)
+    part.set_context()
+    try:
+        got = bound(*args)
+        bound.check()
+    finally:
+        part.pop_context()
+    assert torch.equal(got, expect)
+    assert torch.equal(bound(*args), expect)
+    bound.check()
