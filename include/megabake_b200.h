@@ -244,8 +244,8 @@ typedef struct mb_phase {
 #define MB_AT_S_COUNTER 10   /* int32 [B*Hkv]; has to be given, is not touched               */
 
 /* ---- prefill bodies (MB_MODE_PREFILL plans: one kernel launch per phase, in order; the list of a
- * whole decoder prefill of a short prompt runs as one launch, mb_plan_info.launches == 1, and then
- * writes of the intermediate tensors only those its own steps pass on) -------------------- */
+ * whole decoder prefill of a short prompt runs as one launch, mb_plan_info.launches == 1, and leaves
+ * the same tensors behind, scratch apart) ------------------------------------------------- */
 /* MB_BODY_EMBED_ROWS: out[r, :] = table[ids[r], :] (x scale, rounded to bf16)              */
 #define MB_EM_I_ROWS 0
 #define MB_EM_I_K 1

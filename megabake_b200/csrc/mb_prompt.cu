@@ -83,7 +83,7 @@ struct LayerArgs {
     CUtensorMap w[7];  // q, k, v, o, gate, up, down
     const unsigned short* norm[2];  // before attention, before the gated projections
     const unsigned short* bias[5];  // q, k, v, o, down
-    unsigned short* cache[2];       // keys and values handed over, or null
+    unsigned short* kv[2];          // keys and values: one pair of tensors for all layers, or caches of the layer's own
     int* length;
 };
 
@@ -100,7 +100,7 @@ struct Params {
     const void* inv_freq;
     unsigned short* hidden;
     unsigned short* normed;
-    unsigned short* qkv;
+    unsigned short* q;
     unsigned short* attn;
     unsigned short* glu;
     unsigned short* logits;
@@ -110,7 +110,7 @@ struct Params {
     Control* ctl;
     unsigned long long* trace;
     int layers, rows, tokens, batch, hidden_size, vocab_in, heads, kv_heads, head_dim, intermediate;
-    int norm_kind, activation, invfreq_bf16, capacity, length_value, length_count;
+    int norm_kind, activation, invfreq_bf16, kv_rows, length_value, length_count;  // kv_rows: per batch row
     float eps, embed_scale, rope_scale, q_scale, softmax_scale;
     int attn_units, attn_blocks;  // units of the attention step; query blocks of a (row, head)
     int steps, small;
@@ -423,8 +423,7 @@ __device__ __forceinline__ void gate_pairs(unsigned int (&out)[4], const float (
 // tokens, an odd lane those of the odd ones (4 bytes a store instead of 2).  Tokens from `left` on, and
 // every `period` further, are `jump` elements further away.
 __device__ __forceinline__ void store_pairs(unsigned short* dst, int pitch, const unsigned int (&v)[4], int lane,
-                                            bool mine, int count, int left = 0x7fffffff, int period = 1,
-                                            size_t jump = 0) {
+                                            bool mine, int count, int left, int period, size_t jump) {
     const int odd = lane & 1;
     unsigned short* at = dst - odd;
 #pragma unroll
@@ -470,7 +469,6 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
             int pitch, head = 0, i0 = 0;
             const unsigned short* bias = nullptr;
             const unsigned int* rotary = nullptr;
-            unsigned short* cache = nullptr;
             if (proj == kProjGated) {
                 pitch = p.intermediate;
                 out = p.glu + feature;
@@ -482,17 +480,15 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
                 // pairs of elements i and i + D / 2 of a head; q's and k's are turned by the row's angle
                 head = feature / g.half;
                 i0 = feature - head * g.half;
-                const int q_dim = 2 * g.n[0], kv_dim = 2 * g.n[1];
-                pitch = q_dim + 2 * kv_dim;
-                out = p.qkv + (x.seg > 0 ? q_dim : 0) + (x.seg > 1 ? kv_dim : 0) + 2 * head * g.half + i0;
+                pitch = 2 * n;
+                out = (x.seg == 0 ? p.q : layer.kv[x.seg - 1]) + 2 * head * g.half + i0;
                 bias = layer.bias[x.seg];
                 if (x.seg < 2) rotary = p.rotary + static_cast<size_t>(t0) * g.half + i0;
-                if (x.seg > 0) cache = layer.cache[x.seg - 1];
             } else {
                 pitch = p.hidden_size;
                 sum = p.parts + (static_cast<size_t>(x.slice) * p.rows + t0) * pitch + feature;
             }
-            if (out != nullptr) out += static_cast<size_t>(t0) * pitch;
+            const bool kv = proj == kProjQkv && x.seg > 0 && p.kv_rows != p.tokens;
             float b1 = 0.f, b2 = 0.f;
             if (mine && bias != nullptr) {
                 b1 = bf16_bits_to_float(__ldg(bias + (proj == kProjQkv ? 2 * head * g.half + i0 : feature)));
@@ -546,18 +542,13 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
                     }
                     ask_angles(col + 16);
                 }
-                unsigned short* dst = out + static_cast<size_t>(col) * pitch;
-                store_pairs(dst, pitch, v2, lane, mine, count);
-                if (proj == kProjQkv) store_pairs(dst + g.half, pitch, w2, lane, mine, count);
-                if (cache != nullptr) {  // keys and values handed over: the same, where the caller keeps them
-                    const int kv_dim = 2 * g.n[1];
-                    const int r = t0 + col, b = r / p.tokens, left = (b + 1) * p.tokens - r;
-                    unsigned short* to =
-                        cache + (static_cast<size_t>(b) * p.capacity + r - b * p.tokens) * kv_dim + 2 * head * g.half + i0;
-                    const size_t jump = static_cast<size_t>(p.capacity - p.tokens) * kv_dim;
-                    store_pairs(to, kv_dim, v2, lane, mine, count, left, p.tokens, jump);
-                    store_pairs(to + g.half, kv_dim, w2, lane, mine, count, left, p.tokens, jump);
-                }
+                // caches of keys and values have kv_rows rows for each prompt of the batch
+                const int r = t0 + col, b = kv ? r / p.tokens : 0;
+                const int left = kv ? (b + 1) * p.tokens - r : 0x7fffffff;
+                const size_t gap = kv ? static_cast<size_t>(p.kv_rows - p.tokens) * pitch : 0;
+                unsigned short* dst = out + static_cast<size_t>(r) * pitch + b * gap;
+                store_pairs(dst, pitch, v2, lane, mine, count, left, p.tokens, gap);
+                if (proj == kProjQkv) store_pairs(dst + g.half, pitch, w2, lane, mine, count, left, p.tokens, gap);
             }
         }
         tc_fence_before();
@@ -726,8 +717,8 @@ __device__ __forceinline__ void copies_wait() {
 }
 
 template <int D, bool ONE>
-__device__ __forceinline__ void attention_unit(const Params& p, unsigned char* smem, int u, int tid, int warp,
-                                               int lane) {
+__device__ __forceinline__ void attention_unit(const Params& p, const LayerArgs& layer, unsigned char* smem, int u,
+                                               int tid, int warp, int lane) {
     constexpr int P = D + 8, KB = attention_block(D, ONE), KW = KB / 4, NT = KW / 8, PP = KB + 8;
     constexpr int kBuffers = ONE ? 1 : 2;
     const int T = p.tokens, group = p.heads / p.kv_heads;
@@ -743,18 +734,18 @@ __device__ __forceinline__ void attention_unit(const Params& p, unsigned char* s
     unsigned short* Ps = Vs + kBuffers * KB * P;  // [32][PP]
     float* stats = reinterpret_cast<float*>(Ps + kAttnRows * PP);  // [2][4 groups][32 rows]
     const int q_dim = p.heads * D, kv_dim = p.kv_heads * D;
-    const size_t pitch = q_dim + 2 * kv_dim;
-    const unsigned short* base = p.qkv + static_cast<size_t>(b) * T * pitch;
-    const unsigned short *keys = base + q_dim + kvh * D, *values = keys + kv_dim;
+    const size_t kv_at = static_cast<size_t>(b) * p.kv_rows * kv_dim + kvh * D;
+    const unsigned short *queries_at = p.q + static_cast<size_t>(b * T + q0) * q_dim + head * D;
+    const unsigned short *keys = layer.kv[0] + kv_at, *values = layer.kv[1] + kv_at;
     const int rg = warp & 1, kg = warp >> 1, gid = lane >> 2, tq = lane & 3;
     constexpr float kLog2e = 1.4426950408889634f;
 
     auto copy_keys = [&](int j) {
-        copy_rows<D>(Ks + (j & 1) * KB * P, keys + static_cast<size_t>(j) * KB * pitch, pitch,
+        copy_rows<D>(Ks + (j & 1) * KB * P, keys + static_cast<size_t>(j) * KB * kv_dim, kv_dim,
                      min(KB, (seen - j * KB + 31) / 32 * 32), seen - j * KB, tid);
     };
     auto copy_values = [&](int j) {
-        copy_rows<D>(Vs + (j & 1) * KB * P, values + static_cast<size_t>(j) * KB * pitch, pitch,
+        copy_rows<D>(Vs + (j & 1) * KB * P, values + static_cast<size_t>(j) * KB * kv_dim, kv_dim,
                      min(KB, (seen - j * KB + 31) / 32 * 32), seen - j * KB, tid);
     };
     // scores of this warp's 16 rows and KW keys of block j, with the operator's rounding points
@@ -791,7 +782,7 @@ __device__ __forceinline__ void attention_unit(const Params& p, unsigned char* s
             }
     };
 
-    copy_rows<D>(Qs, base + q0 * pitch + head * D, pitch, kAttnRows, queries, tid);
+    copy_rows<D>(Qs, queries_at, q_dim, kAttnRows, queries, tid);
     copy_keys(0);
     copies_commit();
     if (nblocks == 1) copy_values(0);
@@ -1021,7 +1012,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
                     if (tid == 0) stamp_at(p, step, 3);
                     if (ok) {
                         for (int u = blockIdx.x; u < p.attn_units; u += gridDim.x)
-                            attention_unit<D, SMALL>(p, sh.ring, u, tid, wid, lane);
+                            attention_unit<D, SMALL>(p, layer, sh.ring, u, tid, wid, lane);
                         // weights are copied to where the operands were
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         ok = workers_done(p, sh, tid, step, attn_here, true);
@@ -1242,7 +1233,8 @@ bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
             if (attn.slot[MB_AP_S_Q + s] != qkv.slot[MB_GV_S_OUT0 + s]) return false;
         if (rope.slot[MB_RP_S_Q] != qkv.slot[MB_GV_S_OUT0] || rope.slot[MB_RP_S_K] != qkv.slot[MB_GV_S_OUT0 + 1])
             return false;
-        if (attn.slot[MB_AP_S_OUT] != one[3].slot[MB_AP_S_OUT]) return false;
+        if (attn.slot[MB_AP_S_OUT] != one[3].slot[MB_AP_S_OUT] || attn.slot[MB_AP_S_Q] != one[3].slot[MB_AP_S_Q])
+            return false;
         // keys and values of their own per layer (caches the caller reads): all three records say so
         const int capacity = attn.i[MB_AP_I_KV_CAPACITY];
         if (capacity > 0) {
@@ -1337,7 +1329,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     p.heads = attn.i[MB_AP_I_HEADS];
     p.kv_heads = attn.i[MB_AP_I_KV_HEADS];
     p.head_dim = attn.i[MB_AP_I_HEAD_DIM];
-    p.capacity = attn.i[MB_AP_I_KV_CAPACITY];
+    p.kv_rows = attn.i[MB_AP_I_KV_CAPACITY] > 0 ? attn.i[MB_AP_I_KV_CAPACITY] : p.tokens;
     p.softmax_scale = attn.f[MB_AP_F_SCALE];
     p.intermediate = one[6].i[MB_GV_I_N0];
     p.activation = one[6].i[MB_GV_I_EPILOGUE];
@@ -1361,18 +1353,16 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     p.gemm[kProjHead] = best_cut(&head.i[MB_GV_I_N0], 1, false, false, 0, H, M, H, grid).gemm;
     // CTAs with attention units cannot have their weights of the next projection ahead: others come first
     p.gemm[kProjOut].first = p.attn_units % grid;
-    const int pitch = (p.heads + 2 * p.kv_heads) * p.head_dim;
     const int slices = p.gemm[kProjOut].slices > p.gemm[kProjDown].slices ? p.gemm[kProjOut].slices
                                                                           : p.gemm[kProjDown].slices;
     auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-    const size_t qkv = room(static_cast<size_t>(M) * pitch * 2), parts = room(static_cast<size_t>(slices) * M * H * 4),
+    const size_t parts = room(static_cast<size_t>(slices) * M * H * 4),
                  rotary = room(static_cast<size_t>(M) * (p.head_dim / 2) * 4), counters = room((p.steps + 2) * 4);
-    err = cudaMalloc(&st->scratch, qkv + parts + rotary + counters);
+    err = cudaMalloc(&st->scratch, parts + rotary + counters);
     if (err == cudaSuccess) {
-        p.qkv = reinterpret_cast<unsigned short*>(st->scratch);
-        p.parts = reinterpret_cast<float*>(st->scratch + qkv);
-        p.rotary = reinterpret_cast<unsigned int*>(st->scratch + qkv + parts);
-        p.counters = reinterpret_cast<unsigned int*>(st->scratch + qkv + parts + rotary);
+        p.parts = reinterpret_cast<float*>(st->scratch);
+        p.rotary = reinterpret_cast<unsigned int*>(st->scratch + parts);
+        p.counters = reinterpret_cast<unsigned int*>(st->scratch + parts + rotary);
         err = cudaMemset(p.counters, 0, counters);
     }
     // the form a launch takes, and the one it takes where it has fewer SMs
@@ -1404,6 +1394,7 @@ int prompt_bind(PromptState* st, const std::vector<unsigned long long>& slots, C
     p.table = rows_at(f[0].slot[MB_EM_S_TABLE]);
     p.hidden = rows_at(f[0].slot[MB_EM_S_OUT]);
     p.normed = rows_at(one[0].slot[MB_RN_S_OUT]);
+    p.q = rows_at(one[1].slot[MB_GV_S_OUT0]);
     p.attn = rows_at(one[3].slot[MB_AP_S_OUT]);
     p.glu = rows_at(one[6].slot[MB_GV_S_OUT0]);
     p.inv_freq = reinterpret_cast<const void*>(addr(one[2].slot[MB_RP_S_INVFREQ]));
@@ -1423,8 +1414,7 @@ int prompt_bind(PromptState* st, const std::vector<unsigned long long>& slots, C
         for (int s = 0; s < 3; ++s) layer.bias[s] = rows_at(P[1].slot[MB_GV_S_BIAS0 + s]);
         layer.bias[3] = rows_at(P[4].slot[MB_GV_S_BIAS0]);
         layer.bias[4] = rows_at(P[7].slot[MB_GV_S_BIAS0]);
-        layer.cache[0] = p.capacity > 0 ? rows_at(P[1].slot[MB_GV_S_OUT0 + 1]) : nullptr;
-        layer.cache[1] = p.capacity > 0 ? rows_at(P[1].slot[MB_GV_S_OUT0 + 2]) : nullptr;
+        for (int s = 0; s < 2; ++s) layer.kv[s] = rows_at(P[1].slot[MB_GV_S_OUT0 + 1 + s]);
         layer.length = reinterpret_cast<int*>(addr(P[2].slot[MB_RP_S_LEN]));
         for (int w = 0; w < 3; ++w)
             if (!make_head_map(&layer.w[w], addr(P[1].slot[MB_GV_S_W0 + w]), w == 0 ? p.heads : p.kv_heads, p.head_dim,

@@ -68,3 +68,27 @@ def test_fewer_sms_give_the_same_bits(name, batch, tokens, sms):
     assert torch.equal(got, expect)
     assert torch.equal(bound(*args), expect)
     bound.check()
+
+
+@pytest.mark.parametrize("name,batch,tokens", [("tiny-qwen2", 3, 31), ("tiny-gemma256", 1, 150)])
+def test_queries_keys_and_values_are_left_behind(monkeypatch, name, batch, tokens):
+    """The tensors that the records name are written, as by the launches of their own: bf16 results of sums in another
+    order, a few of them one step (2^-8) apart, and in the last layer of two what that step grew to."""
+    spec = models.get_spec(name)
+    args = _arguments(spec, tokens, batch)
+    layout = plan_prefill(models.direct_prefill_program(spec, batch, tokens))
+    names = {"q": spec.heads, "k": spec.kv_heads, "v": spec.kv_heads, "attention": spec.heads}
+    left = []
+    for switch in ("1", "0"):
+        monkeypatch.setenv(SWITCH, switch)
+        bound = BoundDecoder(layout, args)
+        bound.workspace.fill_(0)
+        bound(*args)
+        bound.check()
+        at = {s.name: s.offset for s in layout.slots if s.kind == "workspace"}
+        left.append({n: bound.workspace[at[n]:at[n] + 2 * batch * tokens * heads * spec.head_dim]
+                     .view(torch.bfloat16).float() for n, heads in names.items()})
+    assert bound.plan.launches > 1
+    for n in names:
+        one, chain = left[0][n], left[1][n]
+        assert chain.any() and float((one - chain).norm() / chain.norm()) < 0.018, n
