@@ -1222,6 +1222,8 @@ bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
         const int D = attn.i[MB_AP_I_HEAD_DIM], heads = attn.i[MB_AP_I_HEADS], kv = attn.i[MB_AP_I_KV_HEADS];
         const int T = attn.i[MB_AP_I_TOKENS];
         if (attn.i[MB_AP_I_BATCH] * T != M || attn.i[MB_AP_I_CAUSAL] != 1 || attn.slot[MB_AP_S_MASK] >= 0) return false;
+        // without scratch for transposed values the phase has another arithmetic (expf, exact division), which it keeps
+        if (attn.slot[MB_AP_S_VT] < 0) return false;
         if (qkv.i[MB_GV_I_K] != H || qkv.i[MB_GV_I_EPILOGUE] != MB_EPI_NONE || qkv.i[MB_GV_I_N0] != heads * D ||
             qkv.i[MB_GV_I_N0 + 1] != kv * D || qkv.i[MB_GV_I_N0 + 2] != kv * D)
             return false;

@@ -92,3 +92,21 @@ def test_queries_keys_and_values_are_left_behind(monkeypatch, name, batch, token
     for n in names:
         one, chain = left[0][n], left[1][n]
         assert chain.any() and float((one - chain).norm() / chain.norm()) < 0.018, n
+
+
+def test_without_room_for_transposed_values_the_launches_stay(monkeypatch):
+    """That record's attention computes with expf and exact division; it is not for the one launch to change that."""
+    spec = models.get_spec("tiny-llama")
+    args = _arguments(spec, 40)
+    layout = plan_prefill(models.direct_prefill_program(spec, 1, 40))
+    for phase in layout.phases:
+        if phase.body == rt.BODY_ATTN_PREFILL:
+            phase.slot[rt.AP_S_VT] = -1
+    results = []
+    for switch in ("1", "0"):
+        monkeypatch.setenv(SWITCH, switch)
+        bound = BoundDecoder(layout, args)
+        assert bound.plan.launches >= len(layout.phases)
+        results.append(bound(*args))
+        bound.check()
+    assert torch.equal(*results)
