@@ -360,6 +360,21 @@ int mb_plan_reset(mb_plan* plan);
  * one launch stamps its steps instead (CTA 0: 2 step done, 3 step before complete, 4 first operands
  * there, 5 products issued, 6 accumulators complete). */
 int mb_plan_set_trace(mb_plan* plan, uint64_t device_address, size_t bytes);
+
+/* Diagnostics, host only: how the phases of a prefill plan would run on a device of `sm_count` SMs.
+ * `form`: 0, a launch for each phase; 1 or 2, one launch, in the form for at most one block of keys and
+ * one row of tokens a CTA or in the general one, and then `out` is filled for q|k|v, o, gate|up, down
+ * and the logits. */
+typedef struct mb_prefill_cut {
+    int32_t features;         /* per work unit, of each matrix of a pair                  */
+    int32_t tokens;           /* per work unit                                            */
+    int32_t slices;           /* of the reduction                                         */
+    int32_t units;            /* shared out over the CTAs                                 */
+    int32_t accumulators;     /* 2: a pair, or more than 128 features                     */
+    int32_t first_cta;        /* of unit 0                                                */
+} mb_prefill_cut;
+int mb_prefill_cuts(const mb_phase* phases, uint32_t n_phases, uint32_t n_dynamic, int32_t sm_count,
+                    int32_t* form, mb_prefill_cut out[5]);
 void mb_plan_destroy(mb_plan* plan);
 
 /* ---- decode attention that allocates nothing ---------------------------------------------

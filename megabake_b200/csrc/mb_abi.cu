@@ -711,6 +711,16 @@ int mb_plan_reset(mb_plan* plan) {
     return MB_OK;
 }
 
+int mb_prefill_cuts(const mb_phase* phases, uint32_t n_phases, uint32_t n_dynamic, int32_t sm_count,
+                    int32_t* form, mb_prefill_cut out[5]) {
+    if (phases == nullptr || form == nullptr || out == nullptr || n_phases == 0 || sm_count < 1) return MB_ERR_INVALID;
+    for (unsigned int i = 0; i < n_phases; ++i) {
+        const int rc = mb::prefill_validate(phases[i], UINT_MAX, n_dynamic);
+        if (rc != MB_OK) return rc;
+    }
+    return mb::prompt_cuts(std::vector<mb_phase>(phases, phases + n_phases), n_dynamic, sm_count, form, out);
+}
+
 void mb_plan_destroy(mb_plan* plan) {
     if (plan == nullptr) return;
     {

@@ -52,6 +52,8 @@ struct PromptState;
 cudaError_t prompt_create(const std::vector<mb_phase>& phases, unsigned int n_dynamic, int sm_count,
                           unsigned int wait_limit_us, PromptState** out);
 void prompt_destroy(PromptState* state);
+int prompt_cuts(const std::vector<mb_phase>& phases, unsigned int n_dynamic, int sm_count, int* form,
+                mb_prefill_cut* out);
 cudaError_t prompt_reset(PromptState* state);
 int prompt_bind(PromptState* state, const std::vector<unsigned long long>& slots, Control* ctl);
 cudaError_t prompt_launch(const PromptState* state, const std::vector<unsigned long long>& slots,

@@ -27,6 +27,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -46,14 +47,42 @@ constexpr int kThreads = 128 + kWorkers;
 constexpr int kMaxLayers = 30;     // what fits the parameters of one launch
 // Tokens over all rows of the batch up to which one launch is the faster form, by the weights of a layer.  What it
 // saves is launches; what it costs grows with the tokens and the weights (tiles of 128 tokens take more operand
-// bytes than mb_prefill.cu's, attention does without tcgen05).  Launches of their own / one launch, us: 135M shape
-// (3.5 M weights a layer) 1,239 / 947 for 19 tokens, 1,847 / 1,360 for 256, 1,998 / 1,718 for 512, 2,120 / 2,106 for
-// 640; 0.5B (15 M) 1,427 / 1,018 for 64, 1,849 / 1,604 for 256, 2,124 / 2,031 for 400, 2,136 / 2,193 for 512; 1B (61 M)
-// 1,194 / 973 for 19, 1,489 / 1,339 for 128, 1,648 / 1,579 for 160, 1,655 / 1,674 for 176; 2B (110 M) 1,731 / 1,472 for
-// 19, 2,175 / 1,831 for 128, 2,442 / 2,459 for 130, 2,647 / 2,810 for 256.
+// bytes than mb_prefill.cu's, attention does without tcgen05).  Between the points the limit is interpolated over the
+// logarithm of the weights.  Time of the launches of their own over that of the one, each called directly /
+// replayed from a graph, one prompt (four and sixteen prompts of as many tokens together do better):
+//   0.6 M weights a layer  1.14 / 1.06 at 512 tokens, 1.02 / 0.97 at 640
+//   3.5 M (135M shape)     1.18 / 1.12 at 512, 1.07 / 1.02 at 576, 0.98 / 0.96 at 608
+//   5.9 M and 7.5 M        1.12 / 1.05 at 512, 1.04 / 1.00 at 576, 1.00 / 0.97 at 608
+//   9.4 M                  1.09 / 1.02 at 512, 0.96 / 0.92 at 544
+//   12.1 M                 1.05 / 0.99 at 448, 1.03 / 0.96 at 480
+//   14.9 M (0.5B shape)    1.17 / 1.11 at 256, 1.03 / 0.98 at 384
+//   19.9 M                 1.11 / 1.05 at 256, 1.01 / 0.96 at 288
+//   23.3 M                 1.05 / 1.00 at 192, 0.97 / 0.92 at 256
+//   29 M, 39 M, 47 M       1.17 / 1.10 at 160, 1.04 to 1.10 / 0.99 to 1.04 at 208
+//   60.8 M (1B shape)      1.12 / 1.07 at 128, 1.06 / 1.00 at 160, 1.01 / 0.96 at 176
+//   70 M to 212 M          1.13 to 1.22 / 1.09 to 1.15 at 128, 0.94 to 1.01 / 0.90 to 0.96 at 144
+struct Limit {
+    double weights;
+    int rows;
+};
+constexpr Limit kLimits[] = {{1.0e6, 640}, {4.2e6, 592}, {8.0e6, 576}, {12.0e6, 432}, {16.0e6, 384},
+                             {20.0e6, 272}, {24.0e6, 160}, {64.0e6, 160}, {66.0e6, 128}};
 inline int most_rows(long long layer_weights) {
-    return layer_weights <= 4ll << 20 ? 640 : layer_weights <= 16ll << 20 ? 400 : layer_weights <= 64ll << 20 ? 160 : 128;
+    const double w = static_cast<double>(layer_weights);
+    const Limit* below = kLimits;
+    for (const Limit& at : kLimits) {
+        if (w <= at.weights)
+            return &at == kLimits ? at.rows
+                                  : below->rows + static_cast<int>((at.rows - below->rows) * std::log(w / below->weights) /
+                                                                   std::log(at.weights / below->weights));
+        below = &at;
+    }
+    return below->rows;
 }
+// Blocks of keys that the attention units of one CTA may go over where a prompt has more than one (tcgen05 takes less
+// for them): 16 heads of 64 on a hidden size of 256, two waves of units and five blocks 1.01 / 0.96, three
+// waves 0.89 / 0.85.  Prompts of one block do better the more there are (128 of one token, 32 heads, 28 waves: 2.26 / 2.23).
+constexpr int kAttnSweeps = 10;
 constexpr int kAttnRows = 32;      // query rows of an attention unit
 constexpr int kSmemBytes = 232448 - 1024;  // 1 KB for what the kernel declares itself
 // A 128-row MMA reads 16 KB of weights from wherever a tile starts, also where the tile has fewer rows
@@ -1182,7 +1211,7 @@ Cut best_cut(const int* n, int segments, bool pair, bool sliced, int half, int K
 constexpr int kPhasesPerLayer = 8;  // norm, q|k|v, rotary, attention, o, norm, gate|up, down
 
 // The records of a decoder prefill in the planner's order, every layer of one shape.
-bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
+bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic, int sm_count) {
     const int count = static_cast<int>(f.size());
     if (count < 1 + kPhasesPerLayer + 2 || (count - 3) % kPhasesPerLayer != 0) return false;
     const int layers = (count - 3) / kPhasesPerLayer;
@@ -1221,6 +1250,8 @@ bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
                 return false;
         const int D = attn.i[MB_AP_I_HEAD_DIM], heads = attn.i[MB_AP_I_HEADS], kv = attn.i[MB_AP_I_KV_HEADS];
         const int T = attn.i[MB_AP_I_TOKENS];
+        const long long units = static_cast<long long>(attn.i[MB_AP_I_BATCH]) * heads * ((T + kAttnRows - 1) / kAttnRows);
+        if (T > kOneBlock && (units + sm_count - 1) / sm_count * ((T + kOneBlock - 1) / kOneBlock) > kAttnSweeps) return false;
         if (attn.i[MB_AP_I_BATCH] * T != M || attn.i[MB_AP_I_CAUSAL] != 1 || attn.slot[MB_AP_S_MASK] >= 0) return false;
         // without scratch for transposed values the phase has another arithmetic (expf, exact division), which it keeps
         if (attn.slot[MB_AP_S_VT] < 0) return false;
@@ -1272,6 +1303,50 @@ bool describes_prompt(const std::vector<mb_phase>& f, unsigned int n_dynamic) {
     return true;
 }
 
+// Sizes and options of such a list, and how its projections are cut.
+void plan_steps(const std::vector<mb_phase>& f, int grid, unsigned int wait_limit_us, Params* params) {
+    Params& p = *params;
+    std::memset(&p, 0, sizeof(p));
+    const mb_phase* one = &f[1];
+    const mb_phase &attn = one[3], &rope = one[2], &head = f.back();
+    p.limit_ns = wait_limit_us * 1000ull;
+    p.layers = (static_cast<int>(f.size()) - 3) / kPhasesPerLayer;
+    p.steps = 2 + p.layers * kStepsPerLayer;
+    p.rows = f[0].i[MB_EM_I_ROWS];
+    p.hidden_size = f[0].i[MB_EM_I_K];
+    p.vocab_in = f[0].i[MB_EM_I_VOCAB];
+    p.embed_scale = f[0].f[MB_EM_F_SCALE];
+    p.batch = attn.i[MB_AP_I_BATCH];
+    p.tokens = attn.i[MB_AP_I_TOKENS];
+    p.heads = attn.i[MB_AP_I_HEADS];
+    p.kv_heads = attn.i[MB_AP_I_KV_HEADS];
+    p.head_dim = attn.i[MB_AP_I_HEAD_DIM];
+    p.kv_rows = attn.i[MB_AP_I_KV_CAPACITY] > 0 ? attn.i[MB_AP_I_KV_CAPACITY] : p.tokens;
+    p.softmax_scale = attn.f[MB_AP_F_SCALE];
+    p.intermediate = one[6].i[MB_GV_I_N0];
+    p.activation = one[6].i[MB_GV_I_EPILOGUE];
+    p.norm_kind = one[0].i[MB_RN_I_KIND];
+    p.eps = one[0].f[MB_RN_F_EPS];
+    p.invfreq_bf16 = rope.i[MB_RP_I_INVFREQ_BF16];
+    p.rope_scale = rope.f[MB_RP_F_ROPE_SCALE];
+    p.q_scale = rope.f[MB_RP_F_Q_SCALE];
+    p.length_value = rope.i[MB_RP_I_LEN_VALUE];
+    p.length_count = rope.i[MB_RP_I_LEN_COUNT] > 1 ? rope.i[MB_RP_I_LEN_COUNT] : 1;
+    p.attn_blocks = (p.tokens + kAttnRows - 1) / kAttnRows;
+    p.attn_units = p.batch * p.heads * p.attn_blocks;
+    p.small = p.rows <= grid && p.tokens <= kOneBlock ? 1 : 0;
+
+    const int M = p.rows, H = p.hidden_size;
+    const int half = p.head_dim / 2, pairs[3] = {p.heads * half, p.kv_heads * half, p.kv_heads * half};
+    p.gemm[kProjQkv] = best_cut(pairs, 3, true, false, half, H, M, H, grid).gemm;
+    p.gemm[kProjOut] = best_cut(&one[4].i[MB_GV_I_N0], 1, false, true, 0, one[4].i[MB_GV_I_K], M, H, grid).gemm;
+    p.gemm[kProjGated] = best_cut(&one[6].i[MB_GV_I_N0], 1, true, false, 0, H, M, H, grid).gemm;
+    p.gemm[kProjDown] = best_cut(&one[7].i[MB_GV_I_N0], 1, false, true, 0, one[7].i[MB_GV_I_K], M, H, grid).gemm;
+    p.gemm[kProjHead] = best_cut(&head.i[MB_GV_I_N0], 1, false, false, 0, H, M, H, grid).gemm;
+    // CTAs with attention units cannot have their weights of the next projection ahead: others come first
+    p.gemm[kProjOut].first = p.attn_units % grid;
+}
+
 }  // namespace prompt
 
 struct PromptState {
@@ -1305,7 +1380,7 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
                              "MEGABAKE_B200_GEMM_BN", "MEGABAKE_B200_GEMM_STAGES", "MEGABAKE_B200_GEMM_SPLIT",
                              "MEGABAKE_B200_PREFILL_CHAIN"})
         if (std::getenv(name) != nullptr) return cudaSuccess;
-    if (!describes_prompt(f, n_dynamic)) return cudaSuccess;
+    if (!describes_prompt(f, n_dynamic, sm_count)) return cudaSuccess;
     int device = 0, cooperative = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
@@ -1316,45 +1391,8 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     st->grid = sm_count;
     st->n_dynamic = n_dynamic;
     Params& p = st->params;
-    std::memset(&p, 0, sizeof(p));
-    const mb_phase* one = &f[1];
-    const mb_phase &attn = one[3], &rope = one[2], &head = f.back();
-    p.limit_ns = wait_limit_us * 1000ull;
-    p.layers = (static_cast<int>(f.size()) - 3) / kPhasesPerLayer;
-    p.steps = 2 + p.layers * kStepsPerLayer;
-    p.rows = f[0].i[MB_EM_I_ROWS];
-    p.hidden_size = f[0].i[MB_EM_I_K];
-    p.vocab_in = f[0].i[MB_EM_I_VOCAB];
-    p.embed_scale = f[0].f[MB_EM_F_SCALE];
-    p.batch = attn.i[MB_AP_I_BATCH];
-    p.tokens = attn.i[MB_AP_I_TOKENS];
-    p.heads = attn.i[MB_AP_I_HEADS];
-    p.kv_heads = attn.i[MB_AP_I_KV_HEADS];
-    p.head_dim = attn.i[MB_AP_I_HEAD_DIM];
-    p.kv_rows = attn.i[MB_AP_I_KV_CAPACITY] > 0 ? attn.i[MB_AP_I_KV_CAPACITY] : p.tokens;
-    p.softmax_scale = attn.f[MB_AP_F_SCALE];
-    p.intermediate = one[6].i[MB_GV_I_N0];
-    p.activation = one[6].i[MB_GV_I_EPILOGUE];
-    p.norm_kind = one[0].i[MB_RN_I_KIND];
-    p.eps = one[0].f[MB_RN_F_EPS];
-    p.invfreq_bf16 = rope.i[MB_RP_I_INVFREQ_BF16];
-    p.rope_scale = rope.f[MB_RP_F_ROPE_SCALE];
-    p.q_scale = rope.f[MB_RP_F_Q_SCALE];
-    p.length_value = rope.i[MB_RP_I_LEN_VALUE];
-    p.length_count = rope.i[MB_RP_I_LEN_COUNT] > 1 ? rope.i[MB_RP_I_LEN_COUNT] : 1;
-    p.attn_blocks = (p.tokens + kAttnRows - 1) / kAttnRows;
-    p.attn_units = p.batch * p.heads * p.attn_blocks;
-    p.small = p.rows <= sm_count && p.tokens <= kOneBlock ? 1 : 0;
-
-    const int M = p.rows, H = p.hidden_size, grid = st->grid;
-    const int half = p.head_dim / 2, pairs[3] = {p.heads * half, p.kv_heads * half, p.kv_heads * half};
-    p.gemm[kProjQkv] = best_cut(pairs, 3, true, false, half, H, M, H, grid).gemm;
-    p.gemm[kProjOut] = best_cut(&one[4].i[MB_GV_I_N0], 1, false, true, 0, one[4].i[MB_GV_I_K], M, H, grid).gemm;
-    p.gemm[kProjGated] = best_cut(&one[6].i[MB_GV_I_N0], 1, true, false, 0, H, M, H, grid).gemm;
-    p.gemm[kProjDown] = best_cut(&one[7].i[MB_GV_I_N0], 1, false, true, 0, one[7].i[MB_GV_I_K], M, H, grid).gemm;
-    p.gemm[kProjHead] = best_cut(&head.i[MB_GV_I_N0], 1, false, false, 0, H, M, H, grid).gemm;
-    // CTAs with attention units cannot have their weights of the next projection ahead: others come first
-    p.gemm[kProjOut].first = p.attn_units % grid;
+    plan_steps(f, sm_count, wait_limit_us, &p);
+    const int M = p.rows, H = p.hidden_size;
     const int slices = p.gemm[kProjOut].slices > p.gemm[kProjDown].slices ? p.gemm[kProjOut].slices
                                                                           : p.gemm[kProjDown].slices;
     auto room = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
@@ -1383,6 +1421,22 @@ cudaError_t prompt_create(const std::vector<mb_phase>& f, unsigned int n_dynamic
     }
     *out = st;
     return cudaSuccess;
+}
+
+int prompt_cuts(const std::vector<mb_phase>& f, unsigned int n_dynamic, int sm_count, int* form, mb_prefill_cut* out) {
+    using namespace prompt;
+    *form = 0;
+    if (!describes_prompt(f, n_dynamic, sm_count)) return MB_OK;
+    Params* p = new (std::nothrow) Params;
+    if (p == nullptr) return MB_ERR_RESOURCE;
+    plan_steps(f, sm_count, 0, p);
+    for (int j = 0; j < 5; ++j) {
+        const Gemm& g = p->gemm[j];
+        out[j] = {g.rows, g.tokens, g.slices, g.units, g.accs, g.first};
+    }
+    *form = p->small ? 1 : 2;
+    delete p;
+    return MB_OK;
 }
 
 int prompt_bind(PromptState* st, const std::vector<unsigned long long>& slots, Control* ctl) {

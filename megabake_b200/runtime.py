@@ -156,6 +156,11 @@ class Status(ctypes.Structure):
     ]
 
 
+class PrefillCut(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_int32) for name in
+                ("features", "tokens", "slices", "units", "accumulators", "first_cta")]
+
+
 # The in-tree build, unless MEGABAKE_B200_LIBRARY names another build of the same ABI (a debug
 # build, or two builds compared in one session).
 LIBRARY_PATH = Path(os.environ.get("MEGABAKE_B200_LIBRARY") or
@@ -164,7 +169,7 @@ LIBRARY_PATH = Path(os.environ.get("MEGABAKE_B200_LIBRARY") or
 # Every symbol include/megabake_b200.h declares; the loader checks all of them.
 EXPORTS = (
     "mb_plan_create", "mb_plan_query", "mb_plan_bind", "mb_plan_launch", "mb_plan_status",
-    "mb_plan_reset", "mb_plan_set_trace", "mb_plan_destroy", "mb_strerror", "mb_status_string", "mb_last_cuda_error",
+    "mb_plan_reset", "mb_plan_set_trace", "mb_prefill_cuts", "mb_plan_destroy", "mb_strerror", "mb_status_string", "mb_last_cuda_error",
     "mb_abi_version", "mb_fixed_smem_bytes", "mb_stage_bytes", "mb_max_smem_bytes",
     "mb_attention_decode_static", "mb_greedy_advance",
 )
@@ -212,6 +217,9 @@ def load_library(path: Path | None = None) -> ctypes.CDLL:
                      "mb_plan_status", "mb_plan_reset", "mb_plan_set_trace", "mb_abi_version",
                      "mb_max_smem_bytes"):
             getattr(lib, name).restype = ctypes.c_int
+        lib.mb_prefill_cuts.argtypes = [ctypes.POINTER(Phase), ctypes.c_uint32, ctypes.c_uint32, ctypes.c_int32,
+                                        ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(PrefillCut)]
+        lib.mb_prefill_cuts.restype = ctypes.c_int
         for name in ("mb_fixed_smem_bytes", "mb_stage_bytes"):
             getattr(lib, name).argtypes = [ctypes.c_int]
             getattr(lib, name).restype = ctypes.c_int
@@ -284,6 +292,16 @@ def greedy_advance(logits, input_ids, position_ids=None, out_tokens=None, cursor
     with torch.cuda.device(logits.device):
         _check(lib, lib.mb_greedy_advance(ctypes.byref(args), ctypes.c_void_p(stream)),
                "runtime", "mb_greedy_advance")
+
+
+def prefill_cuts(phases: list[Phase], n_dynamic: int, sm_count: int) -> tuple[int, list[PrefillCut]]:
+    """How the phases of a prefill plan would run (``mb_prefill_cuts``): 0, a launch for each phase, or 1 or 2, the
+    form of the one launch, and then how q|k|v, o, gate|up, down and the logits are cut into units."""
+    lib = load_library()
+    form, cuts = ctypes.c_int32(), (PrefillCut * 5)()
+    _check(lib, lib.mb_prefill_cuts((Phase * len(phases))(*phases), len(phases), n_dynamic, sm_count,
+                                    ctypes.byref(form), cuts), "planner", "mb_prefill_cuts")
+    return form.value, list(cuts) if form.value else []
 
 
 class Plan:

@@ -113,3 +113,15 @@ def ulp_histogram(logits: torch.Tensor, reference: torch.Tensor) -> dict:
         ">4": float((steps > 4).sum()) / total,
         "max": float(steps.max()),
     }
+
+
+# Prompts that run as one launch and take a way through it that small models do not:
+# (overrides of tiny-llama, batch, tokens, what they reach).
+ONE_LAUNCH_SHAPES = {
+    "units-one-block": (dict(hidden=576, heads=9, kv_heads=3, layers=1), 20, 7, dict(form=1, attention=True)),
+    "units-two-sweeps": (dict(hidden=576, heads=9, kv_heads=3, layers=1), 1, 590, dict(form=2, attention=True)),
+    "units-256-wide": (dict(name="tiny-gemma256"), 1, 608, dict(form=2, attention=True)),
+    "logits-1": (dict(vocab=50000, layers=1), 1, 1, dict(form=1, logits=True)),
+    "logits-19": (dict(vocab=50002, layers=1), 1, 19, dict(form=1, logits=True)),
+    "logits-390": (dict(vocab=50000, layers=1), 1, 390, dict(form=2, logits=True)),
+}
