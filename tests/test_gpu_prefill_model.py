@@ -1,5 +1,6 @@
-"""Whole-model prefill parity: the prefill plan (tcgen05 GEMMs, prefill attention, row kernels;
-through the C ABI) against the CPU oracle and against the fixtures the reference produced.
+"""Whole-model prefill parity, through the C ABI, against the CPU oracle and against the fixtures the
+reference produced: as one launch, which is what prompts of this length get, and as one launch per phase
+(tcgen05 GEMMs, prefill attention, row kernels), which is what longer ones get.
 
 Bar: logits max-abs <= 3e-2 (two bf16 steps for large logits) and cosine >= 0.9999 per
 position; the arg-max of every position equal to the oracle's unless its two best logits tie
@@ -30,7 +31,13 @@ def from_bits(array) -> torch.Tensor:
     return torch.from_numpy(array.copy()).view(torch.bfloat16)
 
 
-def _prefill_on_gpu(name, seed, tokens):
+@pytest.fixture(params=["one launch", "a launch per phase"])
+def one_launch(request, monkeypatch):
+    monkeypatch.setenv("MEGABAKE_B200_PREFILL_ONE_LAUNCH", "1" if request.param == "one launch" else "0")
+    return request.param == "one launch"
+
+
+def _prefill_on_gpu(name, seed, tokens, one_launch=None):
     spec = models.get_spec(name)
     weights = models.init_weights(spec, seed)
     inv_freq = models.inv_freq_buffer(spec)
@@ -40,6 +47,8 @@ def _prefill_on_gpu(name, seed, tokens):
     args = models.direct_prefill_arguments(spec, {k: v.cuda() for k, v in weights.items()},
                                            inv_freq.cuda(), ids)
     bound = BoundDecoder(layout, args)
+    if one_launch is not None:
+        assert bound.plan.launches == 1 if one_launch else bound.plan.launches >= len(layout.phases)
     logits = bound(*args)
     bound.check()
     again = bound(*args)          # a second launch of the same plan gives the same bits
@@ -62,22 +71,22 @@ def _assert_close(logits, reference):
     ("tiny-llama", 1, 16), ("tiny-llama", 2, 70), ("tiny-llama3", 1, 33), ("tiny-qwen2", 2, 10),
     ("tiny-mha", 1, 130), ("tiny-gemma", 2, 12), ("tiny-gemma256", 1, 200),
 ])
-def test_tiny_prefill_matches_oracle(name, batch, length):
+def test_tiny_prefill_matches_oracle(one_launch, name, batch, length):
     spec = models.get_spec(name)
     tokens = torch.randint(0, spec.vocab, (batch, length),
                            generator=torch.Generator().manual_seed(length))
-    spec, weights, inv_freq, logits = _prefill_on_gpu(name, 3, tokens)
+    spec, weights, inv_freq, logits = _prefill_on_gpu(name, 3, tokens, one_launch)
     reference = oracle.prefill(oracle_config(spec), oracle_weights(weights, inv_freq), tokens)
     _assert_close(logits, reference)
 
 
 @pytest.mark.parametrize("key", sorted(k for k in INDEX if k.startswith("prefill_")))
-def test_prefill_matches_reference_fixture(key):
+def test_prefill_matches_reference_fixture(one_launch, key):
     """Logits the reference's declared attention op + Hugging Face eager produced."""
     meta = INDEX[key]
     data = np.load(GOLDEN / f"{key}.npz")
     tokens = torch.from_numpy(data["tokens"])
-    _, _, _, logits = _prefill_on_gpu(meta["model"], meta["seed"], tokens)
+    _, _, _, logits = _prefill_on_gpu(meta["model"], meta["seed"], tokens, one_launch)
     _assert_close(logits, from_bits(data["logits"]))
 
 
@@ -109,7 +118,7 @@ def test_plan_reports_its_kernel_launches(monkeypatch):
     assert BoundDecoder(layout, args).plan.launches == len(layout.phases) + spec.layers
 
 
-def test_prefill_reports_bad_token():
+def test_prefill_reports_bad_token(one_launch):
     from megabake_b200.diagnostics import CompilerError
 
     spec = models.get_spec("tiny-llama")
@@ -119,6 +128,7 @@ def test_prefill_reports_bad_token():
     args = models.direct_prefill_arguments(spec, {k: v.cuda() for k, v in weights.items()},
                                            models.inv_freq_buffer(spec).cuda(), ids)
     bound = BoundDecoder(layout, args)
+    assert (bound.plan.launches == 1) == one_launch
     bound(*args)
     with pytest.raises(CompilerError):
         bound.check()
