@@ -452,7 +452,8 @@ __device__ __forceinline__ void gate_pairs(unsigned int (&out)[4], const float (
 // tokens, an odd lane those of the odd ones (4 bytes a store instead of 2).  Tokens from `left` on, and
 // every `period` further, are `jump` elements further away.
 __device__ __forceinline__ void store_pairs(unsigned short* dst, int pitch, const unsigned int (&v)[4], int lane,
-                                            bool mine, int count, int left, int period, size_t jump) {
+                                            bool mine, int count, int left = 0x7fffffff, int period = 1,
+                                            size_t jump = 0) {
     const int odd = lane & 1;
     unsigned short* at = dst - odd;
 #pragma unroll
@@ -517,7 +518,8 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
                 pitch = p.hidden_size;
                 sum = p.parts + (static_cast<size_t>(x.slice) * p.rows + t0) * pitch + feature;
             }
-            const bool kv = proj == kProjQkv && x.seg > 0 && p.kv_rows != p.tokens;
+            // caches of keys and values have kv_rows rows for each prompt of the batch
+            const bool gaps = proj == kProjQkv && x.seg > 0 && p.kv_rows != p.tokens;
             float b1 = 0.f, b2 = 0.f;
             if (mine && bias != nullptr) {
                 b1 = bf16_bits_to_float(__ldg(bias + (proj == kProjQkv ? 2 * head * g.half + i0 : feature)));
@@ -571,13 +573,17 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
                     }
                     ask_angles(col + 16);
                 }
-                // caches of keys and values have kv_rows rows for each prompt of the batch
-                const int r = t0 + col, b = kv ? r / p.tokens : 0;
-                const int left = kv ? (b + 1) * p.tokens - r : 0x7fffffff;
-                const size_t gap = kv ? static_cast<size_t>(p.kv_rows - p.tokens) * pitch : 0;
-                unsigned short* dst = out + static_cast<size_t>(r) * pitch + b * gap;
-                store_pairs(dst, pitch, v2, lane, mine, count, left, p.tokens, gap);
-                if (proj == kProjQkv) store_pairs(dst + g.half, pitch, w2, lane, mine, count, left, p.tokens, gap);
+                if (!gaps) {
+                    unsigned short* dst = out + static_cast<size_t>(t0 + col) * pitch;
+                    store_pairs(dst, pitch, v2, lane, mine, count);
+                    if (proj == kProjQkv) store_pairs(dst + g.half, pitch, w2, lane, mine, count);
+                } else {
+                    const int r = t0 + col, b = r / p.tokens, left = (b + 1) * p.tokens - r;
+                    const size_t gap = static_cast<size_t>(p.kv_rows - p.tokens) * pitch;
+                    unsigned short* dst = out + static_cast<size_t>(r) * pitch + b * gap;
+                    store_pairs(dst, pitch, v2, lane, mine, count, left, p.tokens, gap);
+                    store_pairs(dst + g.half, pitch, w2, lane, mine, count, left, p.tokens, gap);
+                }
             }
         }
         tc_fence_before();
