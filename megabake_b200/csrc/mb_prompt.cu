@@ -143,7 +143,7 @@ struct Params {
     float eps, embed_scale, rope_scale, q_scale, softmax_scale;
     int attn_units, attn_blocks;  // units of the attention step; query blocks of a (row, head)
     int steps, small;
-    unsigned long long limit_ns;  // of a hand-off between steps; twice as much for the pipeline within a CTA
+    unsigned int limit_us;  // of a hand-over between steps; twice as much for the pipeline within a CTA
 };
 
 enum Step { kQkv = 0, kAttention, kOut, kRowsMid, kGated, kDown, kRowsEnd, kStepsPerLayer };
@@ -153,7 +153,7 @@ struct Shared {
     unsigned char* ring;
     unsigned long long *full, *empty, *acc_full, *acc_empty, *attn_done;
     unsigned int* tmem_slot;
-    volatile int* abort_flag;
+    volatile int* abort_flag;  // the word after it: the limit of a hand-over between steps, microseconds
 };
 
 // ---------------------------------------------------------------------------------------
@@ -163,8 +163,11 @@ struct Shared {
 // twice in a row.  So a body has one place in the code, waits that do not succeed at once continue
 // out of line, and loops stay rolled.
 // ---------------------------------------------------------------------------------------
-__device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, volatile int* abort_flag,
-                                       unsigned long long limit_ns) {
+// (The limit comes from shared memory when it is looked at: as an argument it cost 0.8 % of the shortest prompt.)
+__device__ __forceinline__ unsigned long long limit_ns(const volatile int* abort_flag) {
+    return 1000ull * static_cast<unsigned int>(abort_flag[1]);
+}
+__device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, volatile int* abort_flag) {
     const unsigned long long start = global_timer_ns();
     for (unsigned int tries = 1;; ++tries) {
         unsigned int done;
@@ -176,14 +179,13 @@ __device__ __noinline__ bool wait_long(unsigned int bar, unsigned int parity, vo
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((tries & 127u) == 0u && (*abort_flag || global_timer_ns() - start > limit_ns)) return false;
+        if ((tries & 127u) == 0u && (*abort_flag || global_timer_ns() - start > 2 * limit_ns(abort_flag))) return false;
     }
 }
 // All lanes of a warp; the compiler knows the result to be the same in all of them.
-__device__ __forceinline__ bool wait_warp(const Params& p, const Shared& sh, unsigned long long* bar,
-                                          unsigned int parity) {
+__device__ __forceinline__ bool wait_warp(const Shared& sh, unsigned long long* bar, unsigned int parity) {
     bool done = mbar_try_wait(bar, parity);
-    if (!__all_sync(0xffffffffu, done)) done = wait_long(smem_u32(bar), parity, sh.abort_flag, 2 * p.limit_ns);
+    if (!__all_sync(0xffffffffu, done)) done = wait_long(smem_u32(bar), parity, sh.abort_flag);
     return __all_sync(0xffffffffu, done) != 0;
 }
 
@@ -204,8 +206,7 @@ __device__ __forceinline__ void give_up(const Params& p, const Shared& sh, int c
 
 // Waits until `units` units of `step` are complete; one thread.
 __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned int units, const unsigned int* mark,
-                                         volatile int* abort_flag, Control* ctl, int step,
-                                         unsigned long long limit_ns) {
+                                         volatile int* abort_flag, Control* ctl, int step) {
     unsigned long long start = 0;
     for (unsigned int tries = 1;; ++tries) {
         unsigned int seen;
@@ -218,7 +219,7 @@ __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned i
                 *abort_flag = 1;
                 return false;
             }
-            if (global_timer_ns() - start > limit_ns) {
+            if (global_timer_ns() - start > limit_ns(abort_flag)) {
                 record_fault(ctl, const_cast<unsigned int*>(mark), abort_flag, MB_ST_HANDOFF_TIMEOUT, step,
                              static_cast<int>(blockIdx.x));
                 return false;
@@ -227,7 +228,7 @@ __device__ __noinline__ bool await_count(const unsigned int* counter, unsigned i
     }
 }
 __device__ __forceinline__ bool await_step(const Params& p, const Shared& sh, int step, unsigned int units) {
-    return await_count(p.counters + step, units, fault_mark(p), sh.abort_flag, p.ctl, step, p.limit_ns);
+    return await_count(p.counters + step, units, fault_mark(p), sh.abort_flag, p.ctl, step);
 }
 
 // The workers of this CTA have finished `units` units of `step`.  False: some wait ran out.
@@ -298,7 +299,7 @@ __device__ __forceinline__ bool produce_weights(const Params& p, const Shared& s
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x) {
         const Unit x = unit_of(g, u);
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (at.round > 0 && !wait_warp(p, sh, &sh.empty[at.s], (at.round - 1) & 1)) {
+            if (at.round > 0 && !wait_warp(sh, &sh.empty[at.s], (at.round - 1) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 1);
                 return false;
             }
@@ -341,7 +342,7 @@ __device__ __forceinline__ bool produce_activations(const Params& p, const Share
             waited = true;
         }
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (at.round > 0 && !wait_warp(p, sh, &sh.empty[at.s], (at.round - 1) & 1)) {
+            if (at.round > 0 && !wait_warp(sh, &sh.empty[at.s], (at.round - 1) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 2);
                 return false;
             }
@@ -364,14 +365,14 @@ __device__ __forceinline__ bool issue_products(const Params& p, const Shared& sh
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x, ++turn) {
         const Unit x = unit_of(g, u);
         const int buf = turn & 1;
-        if (turn >= 2 && !wait_warp(p, sh, &sh.acc_empty[buf], ((turn >> 1) - 1) & 1)) {
+        if (turn >= 2 && !wait_warp(sh, &sh.acc_empty[buf], ((turn >> 1) - 1) & 1)) {
             give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 3);
             return false;
         }
         tc_fence_after();
         const unsigned int acc = tmem + buf * 256;
         for (int kb = x.kb0; kb < x.kb1; kb += g.deep) {
-            if (!wait_warp(p, sh, &sh.full[at.s], at.round & 1)) {
+            if (!wait_warp(sh, &sh.full[at.s], at.round & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 4);
                 return false;
             }
@@ -479,7 +480,7 @@ __device__ __forceinline__ bool drain_units(const Params& p, const Shared& sh, c
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x, ++turn) {
         const Unit x = unit_of(g, u);
         const int buf = turn & 1;
-        if (!wait_warp(p, sh, &sh.acc_full[buf], (turn >> 1) & 1)) {
+        if (!wait_warp(sh, &sh.acc_full[buf], (turn >> 1) & 1)) {
             if (lane == 0) give_up(p, sh, MB_ST_PIPE_TIMEOUT, step, 5);
             return false;
         }
@@ -981,7 +982,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
             mbar_init(&sh.acc_empty[b], kWorkers / 32);
         }
         mbar_init(sh.attn_done, 1);
-        *sh.abort_flag = 0;
+        sh.abort_flag[0] = 0;
+        sh.abort_flag[1] = static_cast<int>(p.limit_us);
         mbar_init_fence();
     }
     if (warp == 1) tmem_alloc(sh.tmem_slot, 512);
@@ -997,7 +999,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt_kernel(const __grid_consta
         bool ok = true;
         for (int i = 0; ok && i < projections; ++i) {
             const Place x = place_of(p, i);
-            if (x.proj == kProjOut && attn_here > 0 && !wait_warp(p, sh, sh.attn_done, (i >> 2) & 1)) {
+            if (x.proj == kProjOut && attn_here > 0 && !wait_warp(sh, sh.attn_done, (i >> 2) & 1)) {
                 give_up(p, sh, MB_ST_PIPE_TIMEOUT, x.step, 6);
                 break;
             }
@@ -1315,7 +1317,7 @@ void plan_steps(const std::vector<mb_phase>& f, int grid, unsigned int wait_limi
     std::memset(&p, 0, sizeof(p));
     const mb_phase* one = &f[1];
     const mb_phase &attn = one[3], &rope = one[2], &head = f.back();
-    p.limit_ns = wait_limit_us * 1000ull;
+    p.limit_us = wait_limit_us;
     p.layers = (static_cast<int>(f.size()) - 3) / kPhasesPerLayer;
     p.steps = 2 + p.layers * kStepsPerLayer;
     p.rows = f[0].i[MB_EM_I_ROWS];
