@@ -329,15 +329,15 @@ __device__ __forceinline__ bool produce_activations(const Params& p, const Share
     for (int u = first_unit(g.first); u < g.units; u += gridDim.x) {
         const Unit x = unit_of(g, u);
         if (!waited) {
+            // The lane that waits is the one that issues the copies: elect.sync chooses the same lane of the same mask
+            // every time.  (A vote orders no memory between lanes; a warp barrier would, at 1.9 % of the shortest prompt.)
             bool ready = true;
-            if ((threadIdx.x & 31) == 0) {
+            if (elect_one()) {
                 ready = await_step(p, sh, step - 1, before);
                 stamp_at(p, step, 3);
             }
             if (!__all_sync(0xffffffffu, ready)) return false;
-            // What lane 0 acquired holds for whichever lane issues the copies: a vote says nothing about memory, this
-            // does.  Then the proxies: the step before wrote through the generic one, TMA reads through the async one.
-            __syncwarp();
+            // the step before wrote through the generic proxy, TMA reads through the async proxy
             asm volatile("fence.proxy.async;" ::: "memory");
             waited = true;
         }
