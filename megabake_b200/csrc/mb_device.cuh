@@ -264,7 +264,7 @@ __device__ __forceinline__ float ld_cg_f32(const void* p) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Shared-memory addresses, named barriers, mbarriers, bulk async copies.
+// Shared-memory addresses, named barriers, mbarriers.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned int smem_u32(const void* p) {
     return static_cast<unsigned int>(__cvta_generic_to_shared(p));
@@ -395,17 +395,6 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// 1-D bulk async copy global -> shared, completion counted in bytes on an mbarrier.
-// Source, destination and size must be multiples of 16 bytes.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst_smem, const void* src_gmem,
-                                              unsigned int bytes, unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(smem_u32(dst_smem)),
-        "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
 }
 
 // D(16x8, fp32) += A(16x16, bf16, row) * B(16x8, bf16, col)

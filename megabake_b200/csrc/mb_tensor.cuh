@@ -12,14 +12,14 @@ namespace prefill {
 
 constexpr int kTileK = 64;  // bf16 elements = one 128-byte swizzle row
 
-// Two floats to a bf16 pair in one instruction (same bits as two cvt.rn.bf16.f32, checked over
-// every finite float): the attention's softmax warps and the GEMM epilogue are bound by the
-// instructions they issue, and packing was four of them per pair.
 __device__ __forceinline__ float exp2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// Two floats to a bf16 pair in one instruction (same bits as two cvt.rn.bf16.f32, checked over
+// every finite float): the attention's softmax warps and the GEMM epilogue are bound by the
+// instructions they issue, and packing was four of them per pair.
 __device__ __forceinline__ unsigned int pack_bf16_pair(float lo, float hi) {
     unsigned int packed;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed) : "f"(hi), "f"(lo));
@@ -81,7 +81,7 @@ __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
                      smem_u32(bar))
                  : "memory");
 }
-// D[tmem] (+)= A[smem] . B[smem]^T, bf16 operands, fp32 accumulate, M = 128.
+// D[tmem] (+)= A[smem] . B[smem]^T, bf16 operands, fp32 accumulate, M = 64 or 128 (idesc).
 __device__ __forceinline__ void umma_bf16(unsigned int tmem_d, unsigned long long desc_a,
                                           unsigned long long desc_b, unsigned int idesc,
                                           unsigned int accumulate) {
